@@ -505,6 +505,9 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
             descs = ordered.data();
         }
         auto* ddev = static_cast<const aeonb_entropy_desc*>(ctx->upload(descs, sizeof(aeonb_entropy_desc) * n));
+        std::vector<int4> parts; // of the streams with restart markers
+        jpeg_restart_parts(descs, n, parts);
+        const int4* parts_dev = parts.empty() ? nullptr : static_cast<const int4*>(ctx->upload(parts.data(), sizeof(int4) * parts.size()));
         int64_t bytes = 0; // compressed scan in + the coefficient blocks of the region out
         if (ctx->profiling)
             for (int i = 0; i < n; ++i)
@@ -524,10 +527,11 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
         int       threads  = jpeg_entropy_threads();
         while (threads > 128 && segments <= threads / 2)
             threads /= 2;
-        cudaError_t  e = launch_jpeg_entropy(ddev, n, any_parallel, any_serial, jpeg_entropy_min_segment(), threads, ctx->stream);
+        cudaError_t  e = launch_jpeg_entropy(ddev, n, any_parallel, any_serial, jpeg_entropy_min_segment(), threads, parts_dev,
+                                             (int)parts.size(), ctx->stream);
         if (e != cudaSuccess)
             throw error(AEONB_ERR_CUDA, cuda_message("jpeg entropy kernel launch", e));
-        ctx->launches += (any_parallel ? 1 : 0) + (any_serial ? 1 : 0);
+        ctx->launches += (any_parallel ? 1 : 0) + (parts.empty() ? 0 : 2) + (any_serial ? 1 : 0);
         return AEONB_OK;
     });
 }

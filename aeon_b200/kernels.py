@@ -204,8 +204,8 @@ def jpeg_entropy_decode(data):
 
 
 def jpeg_entropy_decode_device(ctx, encoded, rois=None, parallel=True):
-    """Device entropy decode of JPEG byte strings: with `parallel` a thread block per stream (streams with
-    restart markers still take the one-warp serial kernel), without it the serial kernel for all.
+    """Device entropy decode of JPEG byte strings: with `parallel` a thread block per stream (several per
+    stream with restart markers), without it the one-warp serial kernel for all.
 
     Returns a list of (info, [coef planes as int16 tensors], quant uint16 numpy (3 x 64), status int) per
     record; with `rois` (MCU rectangles) the planes are the compact region planes."""

@@ -281,8 +281,9 @@ typedef struct aeonb_entropy_desc
     int32_t* status;         /* device: set to 0 on success, 1 when the stream is malformed (may be NULL) */
     void*    scratch;        /* device: work area of aeonb_jpeg_entropy_scratch_bytes() bytes, 16-byte aligned.  With it, a
                                 stream without restart markers is decoded by a whole thread block (speculative decoding
-                                of segments that synchronise on each other); without it (NULL), or with restart markers,
-                                by a single warp walking the stream serially */
+                                of segments that synchronise on each other), one with restart markers by several, each a
+                                run of the intervals between the markers; without it (NULL) a single warp walks the
+                                stream serially */
     uint64_t scratch_bytes;
 } aeonb_entropy_desc;
 

@@ -1,5 +1,5 @@
-"""Device entropy decoders (a thread block per JPEG stream decoding segments speculatively; one warp per stream for streams with
-restart markers) against the host decoder and against the oracle: identical coefficient planes."""
+"""Device entropy decoders (a thread block per JPEG stream decoding segments speculatively; a block per run of intervals for streams
+with restart markers; one warp per stream) against the host decoder and against the oracle: identical coefficient planes."""
 import ctypes as C
 import os
 
@@ -157,3 +157,64 @@ def test_streams_with_more_segments_than_the_smallest_segment_allows(ctx, golden
         big.append(jpeg_bytes(img, 92))
     assert min(len(b) for b in big) > 84000
     check(ctx, big)
+
+
+def restart_offsets(blob):
+    """Positions of the restart markers of a file (of their 0xFF)."""
+    start = blob.index(b"\xff\xda")
+    return [i for i in range(start, len(blob) - 1) if blob[i] == 0xFF and 0xD0 <= blob[i + 1] <= 0xD7]
+
+
+@pytest.mark.parametrize("interval", [1, 2, 7, 64, 65, 1000])
+def test_restart_intervals(ctx, interval):
+    """Interval decoding at the edges of its partition: intervals of one MCU (more of them than a part takes, fewer bytes than a
+    segment), of many MCUs (several segments each), more than the picture has; pictures with a ragged last interval; regions that
+    end inside an interval.  Identical planes to the host decoder."""
+    import cv2
+    from aeon_b200 import kernels as K
+    rng = np.random.default_rng(680 + interval)
+    blobs, rois = [], []
+    for (h, w), mode in [((8, 8), None), ((75, 333), None), ((210, 190), cv2.IMWRITE_JPEG_SAMPLING_FACTOR_422),
+                         ((130, 260), cv2.IMWRITE_JPEG_SAMPLING_FACTOR_444), ((520, 700), cv2.IMWRITE_JPEG_SAMPLING_FACTOR_420)]:
+        extra = [cv2.IMWRITE_JPEG_RST_INTERVAL, interval] + ([cv2.IMWRITE_JPEG_SAMPLING_FACTOR, mode] if mode else [])
+        for quality in (60, 95, 100):   # at 100 the noise brings stuffed bytes at every place of a vector
+            img = gradient_image(rng, h, w) if quality < 100 else rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
+            blob = jpeg_bytes(img, quality, extra)
+            info = K.jpeg_parse(blob)
+            mcux, mcuy = info.blocks_w[0] // info.hs[0], info.blocks_h[0] // info.vs[0]
+            x0, y0 = int(rng.integers(0, mcux)), int(rng.integers(0, mcuy))
+            blobs += [blob, blob]
+            rois += [(0, 0, mcux, mcuy), (x0, y0, int(rng.integers(x0 + 1, mcux + 1)), int(rng.integers(y0 + 1, mcuy + 1)))]
+    check(ctx, blobs, rois)
+    check(ctx, blobs[:1], rois[:1])
+
+
+def test_damaged_restart_streams_are_left_to_the_serial_decoder(ctx):
+    """Streams whose intervals are not all there, or do not end where they should: with and without a work area the same status,
+    and the same planes where the status is good."""
+    import cv2
+    from aeon_b200 import kernels as K
+    rng = np.random.default_rng(69)
+    good = jpeg_bytes(gradient_image(rng, 200, 330), 90, [cv2.IMWRITE_JPEG_RST_INTERVAL, 5])
+    at = restart_offsets(good)
+    assert len(at) > 30
+    a, b = at[10], at[11]
+    damaged = [good[:a] + good[a + 2:],                       # a marker lost
+               good[:a] + good[b:],                           # an interval lost
+               good[:a] + b"\xff" + good[a:],                 # a fill byte in front of a marker
+               good[:a] + b"\xff\xd3" + good[a:],             # an empty interval
+               good[:a] + bytes(40) + good[a:],               # bytes behind an interval's last block, few and many
+               good[:a] + bytes(90) + good[a:],
+               good[:a - 3] + good[a:],                       # an interval cut short
+               good[:b] + b"\xff\xd9",                        # the end of the stream lost
+               good[:a + 9] + b"\xff\xfe" + good[a + 9:],     # a foreign marker inside an interval
+               good[:a + 4] + bytes(rng.integers(0, 255, b - a - 8, dtype=np.uint8)) + good[b - 4:]]
+    blobs = [good] + damaged + [good]
+    serial = K.jpeg_entropy_decode_device(ctx, blobs, None, parallel=False)
+    got = K.jpeg_entropy_decode_device(ctx, blobs, None, parallel=True)
+    assert serial[0][3] == 0 and {s[3] for s in serial} == {0, 1}
+    for i, (g, s) in enumerate(zip(got, serial)):
+        assert g[3] == s[3], i
+        for c in range(3):
+            assert s[3] != 0 or np.array_equal(g[1][c].cpu().numpy(), s[1][c].cpu().numpy()), (i, c)
+    check(ctx, [good])
