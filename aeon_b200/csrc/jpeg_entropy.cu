@@ -472,8 +472,7 @@ namespace aeonb
         // average, 11 at most in that batch).  Tried and no faster: warming up on the tail of the left neighbour's
         // segment before the guess, a per-lane ring of stream words in shared memory topped up by asynchronous
         // copies, reading the two words under the bit position afresh for every symbol.
-        constexpr int PLOOK = 12; // bits of the lookup window: AC tables
-        constexpr int DLOOK = 9;  //                            DC tables (few, short codes)
+        constexpr int PLOOK = 12; // bits of the lookup window
         // One 16-bit lookup gives everything the symbol loop needs:
         //   bits 0-4  total bits the symbol takes (code + value bits)     bits 5-8  number of value bits (AC size / DC category)
         //   bits 9-15 advance of the zig-zag index: run + 1, 16 for ZRL, 64 for end of block, 1 for a DC category,
@@ -494,7 +493,6 @@ namespace aeonb
             int      valoff[17];
             uint8_t  vals[256];
             int      is_ac;
-            int      window; // bits of the lookup window in use
         };
 
         // One thread fills the canonical-code limits of a table from the DHT form (16 counts); the values are copied by the caller.
@@ -503,7 +501,6 @@ namespace aeonb
             int code = 0, k = 0;
             T.limit[0] = 0;
             T.is_ac    = is_ac;
-            T.window   = is_ac ? PLOOK : DLOOK;
             for (int len = 1; len <= 16; ++len)
             {
                 const int n   = dht[len - 1];
@@ -522,28 +519,27 @@ namespace aeonb
             int len = 1;
 #pragma unroll
             for (int l = 1; l < PLOOK; ++l)
-                len += l < T.window && i16 >= T.limit[l];
+                len += i16 >= T.limit[l];
             return len;
         }
         __device__ __forceinline__ uint32_t window_entry(const par_table& T, int i, int len)
         {
-            if ((i << (16 - T.window)) >= T.limit[len])
+            if ((i << (16 - PLOOK)) >= T.limit[len])
                 return 0;
-            return pack_symbol(len, T.vals[((i >> (T.window - len)) + T.valoff[len]) & 255], T.is_ac != 0);
+            return pack_symbol(len, T.vals[((i >> (PLOOK - len)) + T.valoff[len]) & 255], T.is_ac != 0);
         }
         // `nth` threads (index `tid`) fill the lookup windows of all four tables once limits and values are in place.  Eight
         // neighbouring entries go together: unless a code of the last three lengths starts among them they hold one symbol, so
         // the length is searched twice per eight entries and one 16-byte store does.
         __device__ void build_par_tables(par_table* tab, int tid, int nth)
         {
-            constexpr int dc8 = (1 << DLOOK) / 8, ac8 = (1 << PLOOK) / 8;
-            for (int j = tid; j < 2 * (dc8 + ac8); j += nth)
+            constexpr int groups = (1 << PLOOK) / 8;
+            for (int j = tid; j < 4 * groups; j += nth)
             {
-                const int  t = j < 2 * ac8 ? 2 + j / ac8 : (j - 2 * ac8) / dc8;
-                const int  i = (j < 2 * ac8 ? j % ac8 : (j - 2 * ac8) % dc8) * 8;
-                par_table& T = tab[t];
-                const int  sh = 16 - T.window, first = window_length(T, i << sh), last = window_length(T, (i + 7) << sh);
-                if (first == last && first <= T.window - 3)
+                const int  i = j % groups * 8;
+                par_table& T = tab[j / groups];
+                const int  first = window_length(T, i << (16 - PLOOK)), last = window_length(T, (i + 7) << (16 - PLOOK));
+                if (first == last && first <= PLOOK - 3)
                 {
                     const uint32_t e = window_entry(T, i, first) * 0x10001u;
                     *reinterpret_cast<uint4*>(&T.lookup[i]) = make_uint4(e, e, e, e);
@@ -552,7 +548,7 @@ namespace aeonb
                 {
 #pragma unroll 1
                     for (int k = 0; k < 8; ++k)
-                        T.lookup[i + k] = (uint16_t)window_entry(T, i + k, window_length(T, (i + k) << sh));
+                        T.lookup[i + k] = (uint16_t)window_entry(T, i + k, window_length(T, (i + k) << (16 - PLOOK)));
                 }
             }
         }
@@ -562,10 +558,10 @@ namespace aeonb
             const int c16 = (int)(h >> 16);
             if (c16 >= T.limit[16])
                 return k_invalid_symbol;
-            int len = T.window + 1;
+            int len = PLOOK + 1;
 #pragma unroll
-            for (int l = DLOOK + 1; l < 16; ++l)
-                len += l > T.window && c16 >= T.limit[l];
+            for (int l = PLOOK + 1; l < 16; ++l)
+                len += c16 >= T.limit[l];
             return pack_symbol(len, T.vals[((c16 >> (16 - len)) + T.valoff[len]) & 255], T.is_ac != 0);
         }
 
@@ -581,14 +577,12 @@ namespace aeonb
             uint32_t   warp_sums[3][32];
             uint8_t    zz[64];
             uint8_t    comp[16], bx[16], by[16]; // per block of an MCU: component and position inside the MCU,
-            const par_table* dct_of[16];         //                       its DC / AC table,
-            const par_table* act_of[16];
-            uint32_t   dc_look[16], ac_look[16]; //                       the shared-memory addresses of their lookup windows,
             int16_t*   blk_base[16];             //                       where its coefficients go: blk_base + (mcu row - first row) * blk_dy
             int64_t    blk_dy[16];               //                                                           + (mcu column - first column) * blk_dx
             int        blk_dx[16];
             aeonb_entropy_desc d;
             int        bpm;                      // blocks per MCU
+            uint32_t   dc_slots, ac_slots;       // bit b: the table slot of block b of an MCU
             int        bad;
             uint32_t   marker_at;                // first marker byte in the raw scan (or its size)
         };
@@ -598,6 +592,12 @@ namespace aeonb
             uint16_t v;
             asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
             return v;
+        }
+
+        // value = *p where `yes` is not 0
+        __device__ __forceinline__ void ldg_if(uint32_t& value, const uint32_t* p, uint32_t yes)
+        {
+            asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.u32 %0, [%1];\n\t}" : "+r"(value) : "l"(p), "r"(yes));
         }
 
         // Where block `b` of MCU (mx, my) lives in the compact coefficient planes, or NULL outside the region.
@@ -632,12 +632,12 @@ namespace aeonb
                                                           bool compare, uint32_t old_blocks)
         {
             seg_result R;
-            R.merged         = false;
-            uint32_t  blocks = 0;
-            int       bad    = 0;
-            const int bpm    = S.bpm;
-            int       mx = 0, my = 0;
-            int16_t*  out = nullptr;
+            R.merged            = false;
+            uint32_t       blocks = 0;
+            int            bad    = 0;
+            const int      bpm    = S.bpm;
+            int            mx = 0, my = 0;
+            int16_t*       out = nullptr;
             if (WRITE)
             {
                 const uint32_t mcu = g / (uint32_t)bpm;
@@ -648,7 +648,13 @@ namespace aeonb
                 else
                     out = block_home(S, mx, my, b);
             }
-            uint32_t dc_look = S.dc_look[b], ac_look = S.ac_look[b];
+            // The lookup window of the next symbol: the AC one of this block, or after the block's last symbol the DC one of the
+            // next.  Both are at hand before the symbol is known, so that only a select hangs on it.
+            const uint32_t windows = (uint32_t)__cvta_generic_to_shared(S.tab[0].lookup), dc_slots = S.dc_slots, ac_slots = S.ac_slots;
+            auto           dc_of   = [&](int blk) { return windows + (dc_slots >> blk & 1) * (uint32_t)sizeof(par_table); };
+            auto           ac_of   = [&](int blk) { return windows + (2 + (ac_slots >> blk & 1)) * (uint32_t)sizeof(par_table); };
+            int            bn      = b + 1 == bpm ? 0 : b + 1;
+            uint32_t       ac_look = ac_of(b), next_dc = dc_of(bn), look = k == 0 ? dc_of(b) : ac_look;
             // checkpoints: `slot` walks down this thread's column (state; the blocks so far NCHECK rows further on); `old_key` is
             // the state an earlier run noted at the next checkpoint (no state has all bits set)
             const uint32_t rows    = NCHECK * check_stride;
@@ -656,59 +662,48 @@ namespace aeonb
             uint32_t       old_key = !WRITE && compare ? chk[0] : 0xffffffffu;
             // A checkpoint at or past the segment's end is never taken: a run can step over it with its last symbol or stop short
             // of it, so what is noted there could be left from an older run than the one whose block count goes with it.
-            if (WRITE || check_at >= pend)
-                check_at = 0xffffffffu;
-            // The bits under p: `n` of them (33 to 64) at the top of `acc`; `next` is word `wp` of the copy, loaded a pass ahead.
-            uint32_t wp   = (p >> 5) + 2;
-            uint64_t acc  = ((uint64_t)words[wp - 2] << 32 | words[wp - 1]) << (p & 31);
-            int      n    = 64 - (int)(p & 31);
-            uint32_t next = words[wp];
-            while (p < pend)
+            uint32_t stop = WRITE || check_at >= pend ? pend : check_at;
+            // The 32 bits under p lie in w0 and w1; w2 is the word behind them, fetched when the one before it comes into use.
+            const uint32_t* ahead = words + (p >> 5) + 3;
+            uint32_t        w0 = ahead[-3], w1 = ahead[-2], w2 = ahead[-1];
+            for (;;)
             {
-                const uint32_t h = (uint32_t)(acc >> 32); // 32 valid bits; a symbol takes at most 31
-                const bool     dc = k == 0;
-                uint32_t       e  = lds_u16((dc ? dc_look : ac_look) + ((h >> (dc ? 32 - DLOOK : 32 - PLOOK)) << 1));
-                if (!e)
-                    e = long_symbol(dc ? *S.dct_of[b] : *S.act_of[b], h);
-                const int tot = e & 31, kinc = e >> 9;
-                if (WRITE)
+                while (p < stop)
                 {
-                    const int sz  = (e >> 5) & 15;
-                    const int raw = sz ? (int)((h << (tot - sz)) >> (32 - sz)) : 0;
-                    const int v   = raw - (sz && raw < ((1 << sz) >> 1) ? (1 << sz) - 1 : 0);
-                    if (kinc == 127)
-                        bad = 1; // invalid code, or a DC symbol that is no category
-                    if (dc)
-                        dcdiff[g] = (int16_t)v;
-                    else if (sz)
+                    const uint32_t h = __funnelshift_l(w1, w0, p); // 32 valid bits; a symbol takes at most 31
+                    uint32_t       e = lds_u16(look + ((h >> (32 - PLOOK)) << 1));
+                    if (!e)
+                        e = long_symbol(S.tab[k == 0 ? dc_slots >> b & 1 : 2 + (ac_slots >> b & 1)], h);
+                    const int tot = e & 31, kinc = e >> 9;
+                    if (WRITE)
                     {
-                        const int kk = k + kinc - 1; // position of this coefficient
-                        if (kk > 63)
-                            bad = 1; // the run leaves the block
-                        else if (out)
+                        const int      sz = (e >> 5) & 15, kk = k + kinc - 1; // value bits and position of this coefficient
+                        const uint32_t x  = h << (tot - sz);                  // the value bits at the top
+                        const int      v  = (int)__funnelshift_l(x, 0u, sz) + ((int)x >= 0 ? 1 - (1 << sz) : 0);
+                        // an invalid code, a DC symbol that is no category, or a run that leaves the block
+                        bad |= kinc == 127 || (sz && kk > 63);
+                        if (k == 0)
+                            dcdiff[g] = (int16_t)v;
+                        else if (sz && kk <= 63 && out)
                             out[S.zz[kk]] = (int16_t)v;
                     }
-                }
-                p += tot;
-                k += kinc;
-                acc <<= tot;
-                n -= tot;
-                if (n <= 32)
-                {
-                    // only lanes that took the word ask for the next one: few trips through the L1 pipeline per pass, and a
-                    // pass is longer than a hit takes, so `next` has arrived when a lane wants it
-                    acc |= (uint64_t)next << (32 - n);
-                    n += 32;
-                    next = words[++wp];
-                }
-                if (k >= 64)
-                {
-                    k = 0;
-                    ++blocks;
-                    b       = b + 1 == bpm ? 0 : b + 1;
-                    dc_look = S.dc_look[b];
-                    ac_look = S.ac_look[b];
-                    if (WRITE)
+                    const uint32_t q     = p + tot;
+                    const uint32_t cross = (p ^ q) & 32; // the read position has left w0
+                    p                    = q;
+                    w0                   = cross ? w1 : w0;
+                    w1                   = cross ? w2 : w1;
+                    ldg_if(w2, ahead, cross); // only lanes that used a word ask for one: few trips through the L1 pipeline
+                    ahead += cross >> 5;
+                    k += kinc;
+                    const bool end = k >= 64;
+                    look           = end ? next_dc : ac_look;
+                    k              = end ? 0 : k;
+                    b              = end ? bn : b;
+                    blocks += end;
+                    bn      = b + 1 == bpm ? 0 : b + 1;
+                    ac_look = ac_of(b);
+                    next_dc = dc_of(bn);
+                    if (WRITE && end)
                     {
                         if (++g >= gend)
                             break;
@@ -720,26 +715,26 @@ namespace aeonb
                         out = block_home(S, mx, my, b);
                     }
                 }
-                if (!WRITE && p >= check_at)
+                if (WRITE || stop == pend)
+                    break;
+                // a checkpoint
+                const uint32_t key = (p - stop) << 10 | (uint32_t)b << 6 | (uint32_t)k; // p - stop <= 30
+                if (key == old_key)
                 {
-                    const uint32_t key = (p - check_at) << 10 | (uint32_t)b << 6 | (uint32_t)k; // p - check_at <= 30
-                    if (key == old_key)
-                    {
-                        // in step with the earlier run: its blocks from here on are this run's too
-                        const uint32_t was = slot[rows];
-                        for (uint32_t* later = slot; later < chk + rows; later += check_stride)
-                            later[rows] += blocks - was;
-                        blocks += old_blocks - was;
-                        R.merged = true;
-                        break;
-                    }
-                    slot[0]    = key;
-                    slot[rows] = blocks;
-                    slot += check_stride;
-                    const bool more = slot < chk + rows && check_at + check_step < pend;
-                    check_at        = more ? check_at + check_step : 0xffffffffu;     // past the last checkpoint: none left
-                    old_key         = more && compare ? slot[0] : 0xffffffffu;        // fetched now, wanted at the next checkpoint
+                    // in step with the earlier run: its blocks from here on are this run's too
+                    const uint32_t was = slot[rows];
+                    for (uint32_t* later = slot; later < chk + rows; later += check_stride)
+                        later[rows] += blocks - was;
+                    blocks += old_blocks - was;
+                    R.merged = true;
+                    break;
                 }
+                slot[0]    = key;
+                slot[rows] = blocks;
+                slot += check_stride;
+                const bool more = slot < chk + rows && stop + check_step < pend;
+                old_key         = more && compare ? slot[0] : 0xffffffffu; // fetched now, wanted at the next checkpoint
+                stop            = more ? stop + check_step : pend;
             }
             R.p      = p;
             R.b      = b;
@@ -778,13 +773,58 @@ namespace aeonb
             return before + incl - v;
         }
 
+        // Appends bytes of all threads to the copy of a stream, which holds big-endian 32-bit words (byte i of the copy is byte
+        // i ^ 3 of memory).  A thread's bytes start anywhere, so they are laid out in a tile in shared memory first and leave it
+        // as whole words; stored byte by byte to global memory they were 11% of the kernel's time.
+        struct clean_writer
+        {
+            uint32_t* tile; // 16 bytes for each thread and 4 more
+            uint32_t* out;
+            uint32_t  size; // bytes appended so far (the same in every thread)
+            uint32_t  rest; // the last, incomplete word (thread 0)
+
+            // Appends the bytes of w whose bits are set in `keep`; returns the position of this thread's first one in the copy.
+            __device__ __forceinline__ uint32_t append(const uint32_t (&w)[4], uint32_t keep, uint32_t* sums)
+            {
+                uint8_t* const bytes = reinterpret_cast<uint8_t*>(tile);
+                const uint32_t carry = size & 3;
+                uint32_t       total;
+                const uint32_t at = cta_exclusive_scan((uint32_t)__popc(keep), sums, total); // and the last tile has been read
+                uint32_t       o  = carry + at;
+                if (threadIdx.x == 0)
+                    for (uint32_t c = 0; c < carry; ++c)
+                        bytes[c ^ 3] = (uint8_t)(rest >> (24 - 8 * c));
+#pragma unroll
+                for (int b = 0; b < 16; ++b)
+                    if (keep >> b & 1)
+                        bytes[o++ ^ 3] = (uint8_t)(w[b >> 2] >> (8 * (b & 3)));
+                __syncthreads();
+                const uint32_t whole = (carry + total) >> 2, first = size >> 2;
+                for (uint32_t i = threadIdx.x; i < whole; i += blockDim.x)
+                    out[first + i] = tile[i];
+                if (threadIdx.x == 0)
+                    rest = tile[whole];
+                const uint32_t mine = size + at;
+                size += total;
+                return mine;
+            }
+            // Ends the copy with 32 zero bytes that the readers may run into.
+            __device__ __forceinline__ void finish()
+            {
+                const uint32_t first = size >> 2, n = ((size + 31) >> 2) - first + 1, kept = 8 * (size & 3);
+                if (threadIdx.x < n)
+                    out[first + threadIdx.x] = threadIdx.x == 0 && kept ? rest & ~(0xffffffffu >> kept) : 0;
+            }
+        };
+
         // What the blocks of a stream need before its bits are looked at: where every block of an MCU goes, and the lookup tables.
         __device__ __forceinline__ void set_up_stream(par_state& S, int tid, int nth)
         {
             const aeonb_entropy_desc& d = S.d;
             if (tid == 0)
             {
-                int b = 0;
+                int      b        = 0;
+                uint32_t dc_slots = 0, ac_slots = 0;
                 for (int c = 0; c < d.ncomp; ++c)
                 {
                     const int64_t row_blocks = (int64_t)(d.roi[2] - d.roi[0]) * d.hs[c]; // blocks in a row of the compact plane
@@ -794,16 +834,16 @@ namespace aeonb
                             S.comp[b]     = (uint8_t)c;
                             S.bx[b]       = (uint8_t)x;
                             S.by[b]       = (uint8_t)y;
-                            S.dct_of[b]   = &S.tab[d.dc_table[c] & 1];
-                            S.act_of[b]   = &S.tab[2 + (d.ac_table[c] & 1)];
-                            S.dc_look[b]  = (uint32_t)__cvta_generic_to_shared(S.dct_of[b]->lookup);
-                            S.ac_look[b]  = (uint32_t)__cvta_generic_to_shared(S.act_of[b]->lookup);
+                            dc_slots |= (uint32_t)(d.dc_table[c] & 1) << b;
+                            ac_slots |= (uint32_t)(d.ac_table[c] & 1) << b;
                             S.blk_base[b] = d.coef[c] + (y * row_blocks + x) * 64;
                             S.blk_dy[b]   = d.vs[c] * row_blocks * 64;
                             S.blk_dx[b]   = d.hs[c] * 64;
                         }
                 }
                 S.bpm       = b;
+                S.dc_slots  = dc_slots;
+                S.ac_slots  = ac_slots;
                 S.marker_at = d.scan_size;
             }
             // The tables in DHT form are brought in whole: the head of a table is a chain over its 16 code counts, which one
@@ -910,8 +950,8 @@ namespace aeonb
                     atomicMin(&S.marker_at, first_marker);
             }
             __syncthreads();
-            const uint32_t raw_end    = S.marker_at;
-            uint32_t       clean_size = 0; // bytes written so far (the same in every thread)
+            const uint32_t raw_end = S.marker_at;
+            clean_writer   copy{chk_all, reinterpret_cast<uint32_t*>(clean), 0, 0}; // the checkpoints' room is not in use yet
             for (uint32_t tile = 0; tile < nv; tile += T)
             {
                 const uint32_t i = tile + tid;
@@ -922,18 +962,10 @@ namespace aeonb
                     classify(i, raw_end, w, valid, stuffed, marker);
                     keep = valid & ~stuffed;
                 }
-                uint32_t       tile_total;
-                uint32_t       o = clean_size + cta_exclusive_scan((uint32_t)__popc(keep), S.warp_sums[0], tile_total);
-#pragma unroll
-                for (int b = 0; b < 16; ++b)
-                    if (keep >> b & 1)
-                        clean[o++ ^ 3] = (uint8_t)(w[b >> 2] >> (8 * (b & 3)));
-                clean_size += tile_total;
+                copy.append(w, keep, S.warp_sums[0]);
             }
-            {
-                if (tid < 32)
-                    clean[(clean_size + tid) ^ 3] = 0; // padding the readers may run into
-            }
+            copy.finish();
+            const uint32_t clean_size = copy.size;
             __syncthreads();
             const uint32_t* words = reinterpret_cast<const uint32_t*>(clean);
 
@@ -1286,7 +1318,7 @@ namespace aeonb
             const uint32_t     lead  = (uint32_t)(reinterpret_cast<uintptr_t>(d.scan) & 15);
             const uint4* const vec   = reinterpret_cast<const uint4*>(d.scan - lead);
             const uint32_t     i0 = (lead + r0) >> 4, i1 = (lead + r1 + 15) >> 4;
-            uint32_t           clean_size = 0; // bytes written so far (the same in every thread)
+            clean_writer       copy{chk_all, reinterpret_cast<uint32_t*>(clean), 0, 0}; // the checkpoints' room is not in use yet
             if (tid == 0)
                 R.clean[0] = 0;
             for (uint32_t tile = i0; tile < i1; tile += T)
@@ -1320,8 +1352,7 @@ namespace aeonb
                         }
                     }
                 }
-                uint32_t tile_total;
-                uint32_t o = clean_size + cta_exclusive_scan((uint32_t)__popc(keep), S.warp_sums[0], tile_total);
+                const uint32_t o = copy.append(words, keep, S.warp_sums[0]);
                 for (uint32_t m = starts; m; m &= m - 1)
                 {
                     const uint32_t b = (uint32_t)__ffs(m) - 1, pos = 16 * i + b - lead + 1; // offset of the interval behind the marker
@@ -1336,14 +1367,9 @@ namespace aeonb
                     }
                     R.clean[lo] = o + (uint32_t)__popc(keep & ((1u << b) - 1));
                 }
-#pragma unroll
-                for (int b = 0; b < 16; ++b)
-                    if (keep >> b & 1)
-                        clean[o++ ^ 3] = (uint8_t)(words[b >> 2] >> (8 * (b & 3)));
-                clean_size += tile_total;
             }
-            if (tid < 32)
-                clean[(clean_size + tid) ^ 3] = 0; // padding the readers may run into
+            copy.finish();
+            const uint32_t clean_size = copy.size;
             if (tid == 0)
                 R.clean[I] = clean_size;
 
