@@ -19,6 +19,11 @@ namespace aeonb
                                         const float* window_dev, const float2* twiddle_dev, const int* filt_start_dev,
                                         const int* filt_bin_dev, const float* filt_weight_dev, const float* dct_dev, int dct_n,
                                         int n_out, cudaStream_t stream);
+    cudaError_t launch_specgram_split(const aeonb_specgram_desc* descs_dev, int n, const aeonb_specgram_config& cfg, const float* window_dev,
+                                      const float2* twiddle_dev, const float2* c1_dev, const float2* c2_dev, int n1, int n2, int frames,
+                                      const int* filt_start_dev, const int* filt_bin_dev, const float* filt_weight_dev, const float* dct_dev,
+                                      int dct_n, int n_out, cudaStream_t stream);
+    bool        specgram_split(int frame_length, int& n1, int& n2, int& frames);
     size_t      specgram_generic_smem(int frame_length);
     bool specgram_frame_length_supported(int frame_length);
 
@@ -107,7 +112,7 @@ namespace aeonb
         }
         else
         {
-            tw.resize(L); // the direct-sum kernel: exp(-2*pi*i*k/L), k = 0..L-1
+            tw.resize(L); // the split and the direct-sum kernel: exp(-2*pi*i*k/L), k = 0..L-1
             for (int k = 0; k < L; ++k)
             {
                 const double a = -2.0 * 3.14159265358979323846 * k / L;
@@ -115,6 +120,22 @@ namespace aeonb
             }
         }
         twiddle = to_device(tw);
+        split   = !fast && specgram_split(L, n1, n2, frames);
+        if (split)
+        {
+            auto table = [](int N) {
+                std::vector<float2> t;
+                for (int k = 0; k <= N / 2; ++k)
+                    for (int n = 1; n <= (N - 1) / 2; ++n)
+                    {
+                        const double a = 2.0 * 3.14159265358979323846 * ((k * n) % N) / N;
+                        t.push_back(make_float2((float)std::cos(a), (float)std::sin(a)));
+                    }
+                return t;
+            };
+            c1 = to_device(table(n1));
+            c2 = to_device(table(n2));
+        }
         n_out   = cfg.num_filters > 0 ? cfg.num_filters : H + 1;
         if (cfg.num_filters > 0)
         {
@@ -123,15 +144,20 @@ namespace aeonb
             std::vector<float>       weight;
             for (int j = 0; j < cfg.num_filters; ++j)
             {
-                start[j] = (int)bin.size();
+                // a filter is a triangle: its bins with a weight follow one another
+                start[j]  = (int)weight.size();
+                int first = 0, last = -1;
                 for (int i = 0; i <= H; ++i)
                     if (fb[(size_t)i * cfg.num_filters + j] != 0.f)
                     {
-                        bin.push_back(i);
-                        weight.push_back(fb[(size_t)i * cfg.num_filters + j]);
+                        first = last < 0 ? i : first;
+                        last  = i;
                     }
+                bin.push_back(first);
+                for (int i = first; i <= last; ++i)
+                    weight.push_back(fb[(size_t)i * cfg.num_filters + j]);
             }
-            start[cfg.num_filters] = (int)bin.size();
+            start[cfg.num_filters] = (int)weight.size();
             filt_start             = to_device(start);
             filt_bin               = to_device(bin);
             filt_weight            = to_device(weight);
@@ -157,6 +183,8 @@ namespace aeonb
     {
         cudaFree(window);
         cudaFree(twiddle);
+        cudaFree(c1);
+        cudaFree(c2);
         cudaFree(filt_start);
         cudaFree(filt_bin);
         cudaFree(filt_weight);
@@ -167,6 +195,9 @@ namespace aeonb
                                         cudaStream_t stream) const
     {
         return fast ? launch_specgram(descs_dev, n, cfg, window, twiddle, filt_start, filt_bin, filt_weight, dct, dct_n, n_out, stream)
+               : split
+                    ? launch_specgram_split(descs_dev, n, cfg, window, twiddle, c1, c2, n1, n2, frames, filt_start, filt_bin, filt_weight, dct, dct_n,
+                                            n_out, stream)
                     : launch_specgram_generic(descs_dev, n, cfg, window, twiddle, filt_start, filt_bin, filt_weight, dct, dct_n, n_out, stream);
     }
 

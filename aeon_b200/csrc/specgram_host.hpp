@@ -22,7 +22,10 @@ namespace aeonb
         float*  dct         = nullptr; // MFCC: num_cepstra x dct_n
         int     dct_n       = 0;
         int     n_out       = 0;
-        bool    fast        = true; // frame length 64*R: the shuffle-FFT kernel; otherwise the direct-sum kernel
+        bool    fast        = true;  // frame length 64*R: the shuffle-FFT kernel
+        bool    split       = false; // frame length n1*n2: the two-step kernel, `frames` frames a block; otherwise the direct-sum kernel
+        int     n1 = 0, n2 = 0, frames = 0;
+        float2 *c1 = nullptr, *c2 = nullptr;
         explicit specgram_tables(const aeonb_specgram_config& cfg);
         ~specgram_tables();
         specgram_tables(const specgram_tables&) = delete;

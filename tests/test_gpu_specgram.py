@@ -101,8 +101,21 @@ def test_mfcc(ctx):
     assert ctx.lib.aeonb_specgram_batch(ctx.handle, d, 1, C.byref(cfg)) == L.ERR_INVALID
 
 
+@pytest.mark.parametrize("length", [2, 3, 15, 49, 127, 131, 254, 441, 1936, 3600])
+def test_two_step_transform_at_the_edges_of_its_range(ctx, length):
+    """Frame lengths n1 * n2: one factor 1 (a prime up to 127), the next prime (131: direct sum), odd and even factors, fewer frames
+    per block than warps (3600), a last block that is not full.  Tolerance: a transform of L terms in float32 with exact tables
+    errs by less than a few times 2^-24 * sqrt(log2 L) of the largest bin; 2e-5 as for the other kernels."""
+    rng = np.random.default_rng(37)
+    clip = rng.integers(-32768, 32768, 13 * (length // 2 + 1) + length, dtype=np.int16)
+    got = run(ctx, [clip, clip[:length], clip[:length - 1]], frame_length=length, frame_stride=length // 2 + 1, max_time_steps=15, num_filters=0)
+    for g, c in zip(got, (clip, clip[:length], clip[:length - 1])):
+        want = ospec.log_mel(c, length, length // 2 + 1, 15, 0, 16000, "hann")
+        assert np.abs(g - want).max() <= 2e-5 * max(np.abs(want).max(), 1e-30), length
+
+
 def test_frame_lengths_without_a_factor_of_64(ctx):
-    """400 samples (25 ms at 16 kHz), odd and long frames take the direct-sum kernel: same tolerances as the FFT kernel."""
+    """400 samples (25 ms at 16 kHz), odd and long frames: same tolerances as the FFT kernel."""
     rng = np.random.default_rng(36)
     clip = synth_clip(rng, 0.9)
     for L_, win, name in [(400, 1, "hann"), (200, 0, "none"), (321, 2, "hamming"), (1000, 3, "blackman"), (7, 4, "bartlett"), (1024, 1, "hann")]:
