@@ -519,16 +519,23 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
             }
         launch_timer timer(ctx, AEONB_KERNEL_ENTROPY, bytes);
         // A launch of short streams (video frames) takes smaller blocks: its streams have few segments, and more blocks fit an SM.
-        uint32_t longest = 0;
+        uint32_t longest     = 0;
+        uint64_t most_blocks = 0;
         for (int i = 0; i < n; ++i)
             if (descs[i].scratch && descs[i].restart_interval == 0)
-                longest = std::max(longest, descs[i].scan_size);
+            {
+                uint64_t bpm = 0;
+                for (int c = 0; c < descs[i].ncomp; ++c)
+                    bpm += (uint64_t)descs[i].hs[c] * descs[i].vs[c];
+                longest     = std::max(longest, descs[i].scan_size);
+                most_blocks = std::max(most_blocks, bpm * descs[i].mcux * descs[i].roi[3]);
+            }
         const int segments = (int)((longest + (uint32_t)jpeg_entropy_min_segment() - 1) / (uint32_t)jpeg_entropy_min_segment());
         int       threads  = jpeg_entropy_threads();
         while (threads > 128 && segments <= threads / 2)
             threads /= 2;
-        cudaError_t  e = launch_jpeg_entropy(ddev, n, any_parallel, any_serial, jpeg_entropy_min_segment(), threads, parts_dev,
-                                             (int)parts.size(), ctx->stream);
+        cudaError_t  e = launch_jpeg_entropy(ddev, n, any_parallel, any_serial, jpeg_entropy_min_segment(), threads, longest, most_blocks,
+                                             parts_dev, (int)parts.size(), ctx->stream);
         if (e != cudaSuccess)
             throw error(AEONB_ERR_CUDA, cuda_message("jpeg entropy kernel launch", e));
         ctx->launches += (any_parallel ? 1 : 0) + (parts.empty() ? 0 : 2) + (any_serial ? 1 : 0);

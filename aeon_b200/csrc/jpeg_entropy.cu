@@ -458,20 +458,20 @@ namespace aeonb
         //
         // The threads of a warp sit in different segments, so the symbol loop is flat -- every pass of it
         // decodes one symbol in every lane, whatever kind (DC category, AC run/size, end of block, zero run),
-        // with the block-end bookkeeping predicated.  With every warp of an SM decoding, the loop is bound by
-        // trips through the L1 pipeline (a load by 32 lanes in 32 places of the stream takes one per cache
-        // line), so the bits under the read position live in a 64-bit register and a lane loads one word when
-        // it has used one up; the checkpoints live in shared memory, lane-major, for the same reason.
+        // with the block-end bookkeeping done by selects.  A launch lasts as long as the chain of symbols of its
+        // slowest stream, so what counts is how soon the next symbol's lookup can start.  The scan is fetched to
+        // shared memory while the tables are being built, cleaned of stuffed bytes in place and decoded from
+        // there: in global memory nearly every pass had some lane of the warp waiting for L2.
         //
-        // Measured on a B200 with 256 streams of 25-85 KB (4:2:0, quality 90, crop regions stored): 0.61 ms per batch
-        // with 512 threads per block and segments of at least 160 bytes (128-192 bytes within 3 %), against 20.9 ms
-        // for the one-warp kernel and about 10 ms for 14 host threads.  A wrong guess falls into step with the true
-        // decoder after about 10 blocks on average (the block's position inside the MCU has to match too), and not
-        // at all inside flat regions, where every block looks the same: there a chain of segments is settled one
-        // round per segment, which is what the slowest streams of a batch spend their time on (6.4 rounds on
-        // average, 11 at most in that batch).  Tried and no faster: warming up on the tail of the left neighbour's
-        // segment before the guess, a per-lane ring of stream words in shared memory topped up by asynchronous
-        // copies, reading the two words under the bit position afresh for every symbol.
+        // Measured on a B200: one 43 KB stream 0.32 ms at first, 0.27 ms with the selects, 0.23 ms with the stream
+        // in shared memory (435 k cycles: set-up 20 k, copy 25 k, first pass 78 k, four rounds 180 k, storing pass
+        // 115 k, DC 16 k); 256 streams of 25-85 KB (4:2:0, quality 90, crop regions stored), entropy, back end and
+        // image kernel together: 721 -> 639 -> 596 us.
+        // A wrong guess falls into step with the true decoder after about 10 blocks on average (the block's
+        // position inside the MCU has to match too), and not at all inside flat regions, where every block looks
+        // the same: there a chain of segments is settled one round per segment, which is what the slowest streams
+        // of a batch spend their time on (5 rounds on average, 11 at most).  Tried and no faster: warming up on the
+        // tail of the left neighbour's segment before the guess.
         constexpr int PLOOK = 12; // bits of the lookup window
         // One 16-bit lookup gives everything the symbol loop needs:
         //   bits 0-4  total bits the symbol takes (code + value bits)     bits 5-8  number of value bits (AC size / DC category)
@@ -568,24 +568,44 @@ namespace aeonb
         constexpr int PAR_THREADS = 512;  // most threads (= segments) a stream can have; the launch picks the actual number
         constexpr int NCHECK      = 3;    // checkpoints inside a segment (7 measured the same; 3 leaves room for a third kernel's CTA on the SM)
 
+        // Where the blocks of one place in an MCU go: base + (mcu row - first row) * dy + (mcu column - first column) * dx
+        struct alignas(16) block_place
+        {
+            int16_t* base;
+            int64_t  dy;
+            int32_t  dx;
+        };
+
         struct par_state
         {
             par_table  tab[4]; // DC slot 0, DC slot 1, AC slot 0, AC slot 1
             uint8_t    dht[4 * 272]; // the tables as they came
-            uint32_t   ent_p[PAR_THREADS], ext_p[PAR_THREADS], cnt[PAR_THREADS];
-            uint16_t   ent_bk[PAR_THREADS], ext_bk[PAR_THREADS];
             uint32_t   warp_sums[3][32];
             uint8_t    zz[64];
-            uint8_t    comp[16], bx[16], by[16]; // per block of an MCU: component and position inside the MCU,
-            int16_t*   blk_base[16];             //                       where its coefficients go: blk_base + (mcu row - first row) * blk_dy
-            int64_t    blk_dy[16];               //                                                           + (mcu column - first column) * blk_dx
-            int        blk_dx[16];
+            block_place place[16];               // per block of an MCU: its place, its component
+            uint8_t    comp[16];
             aeonb_entropy_desc d;
             int        bpm;                      // blocks per MCU
             uint32_t   dc_slots, ac_slots;       // bit b: the table slot of block b of an MCU
             int        bad;
             uint32_t   marker_at;                // first marker byte in the raw scan (or its size)
+            uint32_t   tile_end[2];              // last byte of an even / odd tile of the raw scan
         };
+
+        // Per thread (= segment): the state it was entered in and left in, its blocks, and the checkpoints.
+        struct seg_arrays
+        {
+            uint32_t *ent_p, *ext_p, *cnt, *chk; // chk: 2 x NCHECK rows of T words
+            uint16_t *ent_bk, *ext_bk;
+        };
+        constexpr uint32_t SEG_BYTES = 4 * (3 + 2 * NCHECK) + 2 * 2; // of shared memory for each thread
+
+        __device__ __forceinline__ seg_arrays seg_arrays_at(unsigned char* p, uint32_t T)
+        {
+            uint32_t* const w = reinterpret_cast<uint32_t*>(p);
+            uint16_t* const h = reinterpret_cast<uint16_t*>(w + (3 + 2 * NCHECK) * T);
+            return seg_arrays{w, w + T, w + 2 * T, w + 3 * T, h, h + T};
+        }
 
         __device__ __forceinline__ uint32_t lds_u16(uint32_t addr)
         {
@@ -594,11 +614,42 @@ namespace aeonb
             return v;
         }
 
-        // value = *p where `yes` is not 0
-        __device__ __forceinline__ void ldg_if(uint32_t& value, const uint32_t* p, uint32_t yes)
+        // Words of the copy of a stream, from shared or from global memory.  `next_if` replaces `value` by the next word where
+        // `yes` is not 0: only lanes that used a word ask for one.
+        struct shared_words
         {
-            asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.u32 %0, [%1];\n\t}" : "+r"(value) : "l"(p), "r"(yes));
-        }
+            uint32_t at;
+            __device__ __forceinline__ shared_words(const uint32_t* words, uint32_t i)
+                : at((uint32_t)__cvta_generic_to_shared(words) + 4 * i)
+            {
+            }
+            __device__ __forceinline__ uint32_t next()
+            {
+                uint32_t v;
+                asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at));
+                at += 4;
+                return v;
+            }
+            __device__ __forceinline__ void next_if(uint32_t& value, uint32_t yes)
+            {
+                asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.shared.u32 %0, [%1];\n\t}" : "+r"(value) : "r"(at), "r"(yes));
+                at += yes ? 4 : 0;
+            }
+        };
+        struct global_words
+        {
+            const uint32_t* at;
+            __device__ __forceinline__ global_words(const uint32_t* words, uint32_t i)
+                : at(words + i)
+            {
+            }
+            __device__ __forceinline__ uint32_t next() { return *at++; }
+            __device__ __forceinline__ void     next_if(uint32_t& value, uint32_t yes)
+            {
+                asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.u32 %0, [%1];\n\t}" : "+r"(value) : "l"(at), "r"(yes));
+                at += yes ? 1 : 0;
+            }
+        };
 
         // Where block `b` of MCU (mx, my) lives in the compact coefficient planes, or NULL outside the region.
         __device__ __forceinline__ int16_t* block_home(const par_state& S, int mx, int my, int b)
@@ -606,7 +657,8 @@ namespace aeonb
             const aeonb_entropy_desc& d = S.d;
             if (my < d.roi[1] || my >= d.roi[3] || mx < d.roi[0] || mx >= d.roi[2])
                 return nullptr;
-            return S.blk_base[b] + (my - d.roi[1]) * S.blk_dy[b] + (mx - d.roi[0]) * S.blk_dx[b];
+            const block_place& at = S.place[b];
+            return at.base + (my - d.roi[1]) * at.dy + (mx - d.roi[0]) * at.dx;
         }
 
         struct seg_result
@@ -625,8 +677,8 @@ namespace aeonb
         // chk[check_stride], ... and the blocks completed by then NCHECK rows further on; with `compare`, the run stops at the
         // first checkpoint that an earlier run over this segment (old_blocks blocks in all) passed in the same state, and the
         // block counts from there on are renumbered for this run.
-        template <bool WRITE>
-        __device__ __forceinline__ seg_result run_segment(const par_state& S, const uint32_t* __restrict__ words, uint32_t p, int b, int k,
+        template <bool WRITE, typename Words>
+        __device__ __forceinline__ seg_result run_segment(const par_state& S, const uint32_t* words, uint32_t p, int b, int k,
                                                           uint32_t pend, uint32_t g, uint32_t gend, int16_t* __restrict__ dcdiff,
                                                           uint32_t* chk, uint32_t check_stride, uint32_t check_at, uint32_t check_step,
                                                           bool compare, uint32_t old_blocks)
@@ -636,17 +688,29 @@ namespace aeonb
             uint32_t       blocks = 0;
             int            bad    = 0;
             const int      bpm    = S.bpm;
-            int            mx = 0, my = 0;
-            int16_t*       out = nullptr;
+            // WRITE: the MCU, counted from the region's first column and row (negative in front of it), and the region's size
+            int      mx = 0, my = 0;
+            int      mx_end = 0, mx_first = 0;
+            uint32_t roi_w = 0, roi_h = 0;
+            int16_t* out  = nullptr;
+            auto     home = [&]() -> int16_t* {
+                const block_place& at = S.place[b];
+                return (uint32_t)mx < roi_w && (uint32_t)my < roi_h ? at.base + my * at.dy + mx * at.dx : nullptr;
+            };
             if (WRITE)
             {
                 const uint32_t mcu = g / (uint32_t)bpm;
+                mx_first           = -S.d.roi[0];
+                mx_end             = S.d.mcux - S.d.roi[0];
+                roi_w              = (uint32_t)(S.d.roi[2] - S.d.roi[0]);
+                roi_h              = (uint32_t)(S.d.roi[3] - S.d.roi[1]);
                 my                 = (int)(mcu / (uint32_t)S.d.mcux);
-                mx                 = (int)(mcu - (uint32_t)my * S.d.mcux);
+                mx                 = (int)(mcu - (uint32_t)my * S.d.mcux) - S.d.roi[0];
+                my -= S.d.roi[1];
                 if (g >= gend)
                     pend = 0; // nothing of this segment is wanted
                 else
-                    out = block_home(S, mx, my, b);
+                    out = home();
             }
             // The lookup window of the next symbol: the AC one of this block, or after the block's last symbol the DC one of the
             // next.  Both are at hand before the symbol is known, so that only a select hangs on it.
@@ -664,8 +728,8 @@ namespace aeonb
             // of it, so what is noted there could be left from an older run than the one whose block count goes with it.
             uint32_t stop = WRITE || check_at >= pend ? pend : check_at;
             // The 32 bits under p lie in w0 and w1; w2 is the word behind them, fetched when the one before it comes into use.
-            const uint32_t* ahead = words + (p >> 5) + 3;
-            uint32_t        w0 = ahead[-3], w1 = ahead[-2], w2 = ahead[-1];
+            Words    ahead(words, p >> 5);
+            uint32_t w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
             for (;;)
             {
                 while (p < stop)
@@ -692,8 +756,7 @@ namespace aeonb
                     p                    = q;
                     w0                   = cross ? w1 : w0;
                     w1                   = cross ? w2 : w1;
-                    ldg_if(w2, ahead, cross); // only lanes that used a word ask for one: few trips through the L1 pipeline
-                    ahead += cross >> 5;
+                    ahead.next_if(w2, cross);
                     k += kinc;
                     const bool end = k >= 64;
                     look           = end ? next_dc : ac_look;
@@ -707,12 +770,12 @@ namespace aeonb
                     {
                         if (++g >= gend)
                             break;
-                        if (b == 0 && ++mx == S.d.mcux)
+                        if (b == 0 && ++mx == mx_end)
                         {
-                            mx = 0;
+                            mx = mx_first;
                             ++my;
                         }
-                        out = block_home(S, mx, my, b);
+                        out = home();
                     }
                 }
                 if (WRITE || stop == pend)
@@ -773,49 +836,68 @@ namespace aeonb
             return before + incl - v;
         }
 
-        // Appends bytes of all threads to the copy of a stream, which holds big-endian 32-bit words (byte i of the copy is byte
-        // i ^ 3 of memory).  A thread's bytes start anywhere, so they are laid out in a tile in shared memory first and leave it
-        // as whole words; stored byte by byte to global memory they were 11% of the kernel's time.
+        // The copy of a stream without stuffed bytes holds big-endian 32-bit words (byte i of the copy is byte i ^ 3 of memory).
+        // Resident: the raw scan lies in shared memory, from 16-byte vector 0 on, and the copy takes its place -- a tile's bytes are
+        // in registers before any of them is written, and never move up.  Otherwise the copy goes to global memory: a thread's
+        // bytes start anywhere, so they are laid out in a tile in shared memory first and leave it as whole words (stored byte by
+        // byte to global memory they were 11% of the kernel's time).
+        template <bool RESIDENT>
         struct clean_writer
         {
-            uint32_t* tile; // 16 bytes for each thread and 4 more
+            uint32_t* room; // resident: the scan.  Otherwise the tile: 16 bytes for each thread and 4 more
             uint32_t* out;
             uint32_t  size; // bytes appended so far (the same in every thread)
             uint32_t  rest; // the last, incomplete word (thread 0)
 
-            // Appends the bytes of w whose bits are set in `keep`; returns the position of this thread's first one in the copy.
-            __device__ __forceinline__ uint32_t append(const uint32_t (&w)[4], uint32_t keep, uint32_t* sums)
+            // Appends the bytes of w whose bits are set in `keep`, `at` being their place among the tile's `total` bytes; every
+            // thread has passed a barrier since it read its part of the tile.
+            __device__ __forceinline__ void append(const uint32_t (&w)[4], uint32_t keep, uint32_t at, uint32_t total)
             {
-                uint8_t* const bytes = reinterpret_cast<uint8_t*>(tile);
-                const uint32_t carry = size & 3;
-                uint32_t       total;
-                const uint32_t at = cta_exclusive_scan((uint32_t)__popc(keep), sums, total); // and the last tile has been read
-                uint32_t       o  = carry + at;
-                if (threadIdx.x == 0)
+                uint8_t* const bytes = reinterpret_cast<uint8_t*>(room);
+                const uint32_t carry = RESIDENT ? size : size & 3;
+                uint32_t       o     = carry + at;
+                if (!RESIDENT && threadIdx.x == 0)
                     for (uint32_t c = 0; c < carry; ++c)
                         bytes[c ^ 3] = (uint8_t)(rest >> (24 - 8 * c));
 #pragma unroll
                 for (int b = 0; b < 16; ++b)
                     if (keep >> b & 1)
                         bytes[o++ ^ 3] = (uint8_t)(w[b >> 2] >> (8 * (b & 3)));
-                __syncthreads();
-                const uint32_t whole = (carry + total) >> 2, first = size >> 2;
-                for (uint32_t i = threadIdx.x; i < whole; i += blockDim.x)
-                    out[first + i] = tile[i];
-                if (threadIdx.x == 0)
-                    rest = tile[whole];
-                const uint32_t mine = size + at;
+                if (!RESIDENT)
+                {
+                    __syncthreads();
+                    const uint32_t whole = (carry + total) >> 2, first = size >> 2;
+                    for (uint32_t i = threadIdx.x; i < whole; i += blockDim.x)
+                        out[first + i] = room[i];
+                    if (threadIdx.x == 0)
+                        rest = room[whole];
+                }
                 size += total;
-                return mine;
             }
             // Ends the copy with 32 zero bytes that the readers may run into.
             __device__ __forceinline__ void finish()
             {
+                if (RESIDENT)
+                {
+                    __syncthreads(); // the last tile has been read
+                    if (threadIdx.x < 32)
+                        reinterpret_cast<uint8_t*>(room)[(size + threadIdx.x) ^ 3] = 0;
+                    return;
+                }
                 const uint32_t first = size >> 2, n = ((size + 31) >> 2) - first + 1, kept = 8 * (size & 3);
                 if (threadIdx.x < n)
                     out[first + threadIdx.x] = threadIdx.x == 0 && kept ? rest & ~(0xffffffffu >> kept) : 0;
             }
         };
+
+        // Starts the transfer of 16-byte vectors [i0, i1) of the raw scan to shared memory.
+        __device__ __forceinline__ void fetch_raw(uint32_t* room, const uint4* vec, uint32_t i0, uint32_t i1)
+        {
+            const uint32_t at = (uint32_t)__cvta_generic_to_shared(room);
+            for (uint32_t i = i0 + threadIdx.x; i < i1; i += blockDim.x)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(at + 16 * (i - i0)), "l"(vec + i) : "memory");
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
 
         // What the blocks of a stream need before its bits are looked at: where every block of an MCU goes, and the lookup tables.
         __device__ __forceinline__ void set_up_stream(par_state& S, int tid, int nth)
@@ -831,20 +913,17 @@ namespace aeonb
                     for (int y = 0; y < d.vs[c]; ++y)
                         for (int x = 0; x < d.hs[c]; ++x, ++b)
                         {
-                            S.comp[b]     = (uint8_t)c;
-                            S.bx[b]       = (uint8_t)x;
-                            S.by[b]       = (uint8_t)y;
+                            S.comp[b] = (uint8_t)c;
                             dc_slots |= (uint32_t)(d.dc_table[c] & 1) << b;
                             ac_slots |= (uint32_t)(d.ac_table[c] & 1) << b;
-                            S.blk_base[b] = d.coef[c] + (y * row_blocks + x) * 64;
-                            S.blk_dy[b]   = d.vs[c] * row_blocks * 64;
-                            S.blk_dx[b]   = d.hs[c] * 64;
+                            S.place[b].base = d.coef[c] + (y * row_blocks + x) * 64;
+                            S.place[b].dy   = d.vs[c] * row_blocks * 64;
+                            S.place[b].dx   = d.hs[c] * 64;
                         }
                 }
                 S.bpm       = b;
                 S.dc_slots  = dc_slots;
                 S.ac_slots  = ac_slots;
-                S.marker_at = d.scan_size;
             }
             // The tables in DHT form are brought in whole: the head of a table is a chain over its 16 code counts, which one
             // thread walks from shared memory rather than from L2.
@@ -861,13 +940,241 @@ namespace aeonb
             __syncthreads();
         }
 
-        __global__ void __launch_bounds__(PAR_THREADS) jpeg_entropy_parallel_kernel(const aeonb_entropy_desc* __restrict__ descs, int min_segment)
+        // Sums the DC differences of MCUs [m0, m1) up from the predictors in front of them and stores the values.
+        __device__ __forceinline__ void store_dc(const par_state& S, const int16_t* dcdiff, uint32_t m0, uint32_t m1, int bpm, int (&pred)[3])
+        {
+            int my = (int)(m0 / (uint32_t)S.d.mcux), mx = (int)(m0 - (uint32_t)my * S.d.mcux);
+            for (uint32_t m = m0; m < m1; ++m)
+            {
+                for (int b = 0; b < bpm; ++b)
+                {
+                    const int v = dcdiff[(size_t)m * bpm + b];
+                    const int c = S.comp[b];
+                    int       now;
+                    if (c == 0)
+                        now = pred[0] += v;
+                    else if (c == 1)
+                        now = pred[1] += v;
+                    else
+                        now = pred[2] += v;
+                    int16_t* out = block_home(S, mx, my, b);
+                    if (out)
+                        out[0] = (int16_t)now;
+                }
+                if (++mx == S.d.mcux)
+                {
+                    mx = 0;
+                    ++my;
+                }
+            }
+        }
+
+        // Decodes every segment from a guessed state (`known`: the true one) and then, in rounds, from its left neighbour's exit state
+        // until nothing changes.  Returns the blocks this thread's segment completes; entry states and checkpoints stay in A.
+        template <typename Words>
+        __device__ __forceinline__ uint32_t settle_segments(const par_state& S, const seg_arrays& A, const uint32_t* words, uint32_t nseg,
+                                                            bool known, uint32_t pbeg, uint32_t pend, uint32_t step)
+        {
+            const uint32_t  tid = threadIdx.x, T = blockDim.x;
+            const bool      mine       = tid < nseg;
+            uint32_t* const chk        = A.chk + tid;
+            uint32_t        run_blocks = 0; // blocks of this thread's latest run
+            if (mine)
+            {
+                const seg_result r = run_segment<false, Words>(S, words, pbeg, 0, 0, pend, 0, 0, nullptr, chk, T, pbeg + step, step, false, 0);
+                A.ent_p[tid]  = pbeg;
+                A.ent_bk[tid] = 0;
+                A.ext_p[tid]  = r.p;
+                A.ext_bk[tid] = (uint16_t)((r.b << 8) | r.k);
+                run_blocks    = r.blocks;
+            }
+            __syncthreads();
+            for (uint32_t round = 1; round < nseg; ++round)
+            {
+                uint32_t cand_p  = 0;
+                uint16_t cand_bk = 0;
+                bool     redo    = false;
+                if (mine && !known)
+                {
+                    cand_p  = A.ext_p[tid - 1];
+                    cand_bk = A.ext_bk[tid - 1];
+                    redo    = cand_p != A.ent_p[tid] || cand_bk != A.ent_bk[tid];
+                }
+                __syncthreads(); // every candidate has been read before any exit state changes
+                if (redo)
+                {
+                    const seg_result r = run_segment<false, Words>(S, words, cand_p, cand_bk >> 8, cand_bk & 255, pend, 0, 0, nullptr, chk, T,
+                                                                   pbeg + step, step, true, run_blocks);
+                    A.ent_p[tid]  = cand_p;
+                    A.ent_bk[tid] = cand_bk;
+                    run_blocks    = r.blocks;
+                    if (!r.merged)
+                    {
+                        A.ext_p[tid]  = r.p;
+                        A.ext_bk[tid] = (uint16_t)((r.b << 8) | r.k);
+                    }
+                }
+                if (!__syncthreads_or(redo))
+                    break;
+            }
+            return run_blocks;
+        }
+
+        // The entry state of piece `piece` of segment t, which starts at bit `at`: position, block and zig-zag index, blocks so far.
+        __device__ __forceinline__ void piece_entry(const seg_arrays& A, uint32_t T, uint32_t t, uint32_t piece, uint32_t at, uint32_t& p,
+                                                    uint32_t& bk, uint32_t& before)
+        {
+            p = A.ent_p[t], bk = A.ent_bk[t], before = 0;
+            if (piece > 0)
+            {
+                const uint32_t key = A.chk[(piece - 1) * T + t];
+                p                  = at + (key >> 10);
+                bk                 = (key >> 6 & 15) << 8 | (key & 63);
+                before             = A.chk[(NCHECK + piece - 1) * T + t];
+            }
+        }
+
+        // Copies the scan without stuffed bytes, up to the first marker; returns the bytes of the copy.  RESIDENT: in place in `room`,
+        // where the scan's vectors have been brought; otherwise from `vec` to `out` through the tile `room`.
+        template <bool RESIDENT>
+        __device__ __forceinline__ uint32_t copy_scan(par_state& S, uint32_t* room, uint32_t* out, const uint4* vec, uint32_t nv, uint32_t lead)
+        {
+            const uint32_t         tid = threadIdx.x, T = blockDim.x, N = S.d.scan_size;
+            uint32_t               raw_end = S.marker_at;
+            clean_writer<RESIDENT> copy{room, out, 0, 0};
+            for (uint32_t tile = 0, odd = 0; tile < nv; tile += T, odd ^= 1)
+            {
+                // bit b of `keep` = byte b is part of the data, of `marker` = byte b is non-zero and follows 0xFF; the byte before
+                // the stream is not 0xFF
+                const uint32_t i = tile + tid;
+                uint32_t       w[4] = {0, 0, 0, 0}, keep = 0, marker = 0;
+                if (i < nv)
+                {
+                    const uint4 x = RESIDENT ? reinterpret_cast<const uint4*>(room)[i] : __ldg(vec + i);
+                    w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
+                    uint32_t prev = 0;
+                    if (i > 0)
+                        prev = !RESIDENT  ? (uint32_t)__ldg(reinterpret_cast<const uint8_t*>(vec) + 16 * i - 1)
+                               : tid == 0 ? S.tile_end[odd ^ 1] // its place may have been taken
+                                          : (uint32_t) reinterpret_cast<const uint8_t*>(room)[16 * i - 1];
+                    // Nearly every vector lies inside the stream and has no 0xFF in front of any of its bytes: all 16 are kept.
+                    const bool inside = 16 * i > lead && 16 * i + 16 - lead <= raw_end;
+                    const bool no_ff  = prev != 0xFF && !__vcmpeq4(w[0], 0xFFFFFFFFu) && !__vcmpeq4(w[1], 0xFFFFFFFFu) &&
+                                       !__vcmpeq4(w[2], 0xFFFFFFFFu) && !(__vcmpeq4(w[3], 0xFFFFFFFFu) & 0x00FFFFFFu);
+                    if (inside && no_ff)
+                        keep = 0xFFFF;
+                    else
+                    {
+#pragma unroll
+                        for (int b = 0; b < 16; ++b)
+                        {
+                            const uint32_t v   = (w[b >> 2] >> (8 * (b & 3))) & 255;
+                            const uint32_t pos = 16 * i + b; // offset from the aligned address
+                            if (pos == lead)
+                                prev = 0;
+                            const bool in = pos >= lead && pos - lead < N;
+                            keep |= (uint32_t)(in && pos - lead < raw_end && !(prev == 0xFF && v == 0)) << b;
+                            marker |= (uint32_t)(in && prev == 0xFF && v != 0) << b;
+                            prev = v;
+                        }
+                    }
+                }
+                if (RESIDENT && tid == T - 1)
+                    S.tile_end[odd] = w[3] >> 24;
+                uint32_t total, at = cta_exclusive_scan((uint32_t)__popc(keep) | (marker ? 1u << 20 : 0), S.warp_sums[0], total);
+                at &= (1u << 20) - 1;
+                if (total >> 20)
+                {
+                    // a marker (0xFF followed by anything but 0x00) ends the entropy-coded data
+                    if (marker)
+                        atomicMin(&S.marker_at, 16 * i + (uint32_t)__ffs(marker) - 1 - lead - 1); // the 0xFF before it
+                    __syncthreads();
+                    raw_end             = S.marker_at;
+                    const uint32_t left = lead + raw_end > 16 * i ? min(lead + raw_end - 16 * i, 16u) : 0;
+                    keep &= (1u << left) - 1;
+                    at = cta_exclusive_scan((uint32_t)__popc(keep), S.warp_sums[0], total);
+                }
+                copy.append(w, keep, at, total);
+                if (lead + raw_end <= 16 * (tile + T))
+                    break;
+            }
+            copy.finish();
+            return copy.size;
+        }
+
+        // Everything between the copy and the DC sums: segments, their true entry states, and the storing pass.
+        template <typename Words>
+        __device__ __forceinline__ void decode_scan(par_state& S, const seg_arrays& A, const uint32_t* words, uint32_t clean_size, int min_segment,
+                                                    uint32_t needed_blocks, int16_t* dcdiff)
+        {
+            const uint32_t            tid = threadIdx.x, T = blockDim.x;
+            const aeonb_entropy_desc& d = S.d;
+            // ---- segments: one per thread, a multiple of 4 bytes, at least min_segment bytes
+            uint32_t seg = (clean_size + T - 1) / T;
+            seg          = max((seg + 3u) & ~3u, (uint32_t)max(min_segment, 64) & ~3u);
+            const uint32_t nseg      = (clean_size + seg - 1) / seg; // <= T
+            const uint32_t total_bit = clean_size * 8;
+            const uint32_t pbeg = tid * seg * 8, pend = min(total_bit, pbeg + seg * 8);
+            // checkpoints of a segment, evenly spaced (at least 64 bits apart; a symbol is shorter, so it passes at most one)
+            const uint32_t step = seg * 8 / (NCHECK + 1); // bits between checkpoints (seg is a multiple of 4 bytes)
+
+            // ---- clear the coefficient planes now: the stores drain while the segments are being decoded, and the barriers
+            // between here and the storing pass order them before that pass's stores.  Warps without a segment do it, if there
+            // are four of them, while the others start decoding.
+            const uint32_t busy = (nseg + 31) & ~31u, from = T >= busy + 128 ? busy : 0;
+            if (tid >= from)
+                for (int c = 0; c < d.ncomp; ++c)
+                {
+                    const size_t n16 = (size_t)(d.roi[2] - d.roi[0]) * d.hs[c] * (d.roi[3] - d.roi[1]) * d.vs[c] * 8; // 16-byte units
+                    uint4*       p   = reinterpret_cast<uint4*>(d.coef[c]);
+                    for (size_t i = tid - from; i < n16; i += T - from)
+                        p[i] = make_uint4(0, 0, 0, 0);
+                }
+
+            const uint32_t run_blocks = settle_segments<Words>(S, A, words, nseg, tid == 0, pbeg, pend, step);
+
+            // ---- first block number of every segment
+            uint32_t       counted;
+            const uint32_t g0 = cta_exclusive_scan(run_blocks, S.warp_sums[0], counted);
+            if (tid == 0 && counted < needed_blocks)
+                S.bad = 1;
+
+            // ---- decode once more from the true entry states, storing (the planes were cleared above).  The checkpoints now
+            // describe every segment's final run, so each segment falls into NCHECK + 1 pieces with known entry states and block
+            // numbers, and the pieces -- not the segments -- are dealt out to the threads: streams with fewer segments than
+            // threads keep every warp busy, and neighbouring lanes work on neighbouring pieces.
+            A.cnt[tid] = g0;
+            __syncthreads();
+            for (uint32_t q = tid; q < nseg * (NCHECK + 1); q += T)
+            {
+                const uint32_t t = q / (NCHECK + 1), piece = q % (NCHECK + 1);
+                const uint32_t seg_beg = t * seg * 8, seg_end = min(total_bit, seg_beg + seg * 8);
+                const uint32_t at = seg_beg + piece * step; // the checkpoint this piece starts from
+                if (at >= seg_end)
+                    continue;
+                uint32_t p0, bk, before;
+                piece_entry(A, T, t, piece, at, p0, bk, before);
+                const seg_result r = run_segment<true, Words>(S, words, p0, bk >> 8, bk & 255, min(seg_end, at + step), A.cnt[t] + before,
+                                                              needed_blocks, dcdiff, nullptr, 0, 0, 0, false, 0);
+                if (r.bad)
+                    S.bad = 1;
+            }
+            __syncthreads();
+        }
+
+        // Shared memory of a block: par_state, SEG_BYTES per thread, and what is left of `smem_bytes` for the scan and behind it
+        // the DC differences, where they fit; otherwise they live in the record's work area.
+        __global__ void __launch_bounds__(PAR_THREADS) jpeg_entropy_parallel_kernel(const aeonb_entropy_desc* __restrict__ descs, int min_segment,
+                                                                                    uint32_t smem_bytes)
         {
             const uint32_t T = blockDim.x; // threads = most segments of this launch
             extern __shared__ __align__(16) unsigned char smem_raw[];
-            par_state&      S       = *reinterpret_cast<par_state*>(smem_raw);
-            uint32_t* const chk_all = reinterpret_cast<uint32_t*>(smem_raw + sizeof(par_state)); // 2 x NCHECK rows of T words
-            const int       tid     = threadIdx.x;
+            par_state&       S          = *reinterpret_cast<par_state*>(smem_raw);
+            const seg_arrays A          = seg_arrays_at(smem_raw + sizeof(par_state), T);
+            const uint32_t   room_at    = ((uint32_t)sizeof(par_state) + SEG_BYTES * T + 15) & ~15u;
+            uint32_t* const  room       = reinterpret_cast<uint32_t*>(smem_raw + room_at);
+            const uint32_t   room_bytes = smem_bytes - room_at;
+            const int        tid        = threadIdx.x;
             for (int i = tid; i < (int)(sizeof(aeonb_entropy_desc) / 4); i += T)
                 reinterpret_cast<uint32_t*>(&S.d)[i] = reinterpret_cast<const uint32_t*>(descs + blockIdx.x)[i];
             if (tid < 64)
@@ -877,7 +1184,7 @@ namespace aeonb
             __syncthreads();
             const aeonb_entropy_desc& d = S.d;
             if (!d.scratch || d.restart_interval != 0)
-                return; // the serial kernel's stream
+                return; // the other kernels' stream
             int bpm = 0;
             for (int c = 0; c < 3; ++c)
                 if (c < d.ncomp)
@@ -894,180 +1201,41 @@ namespace aeonb
                     *d.status = 1;
                 return;
             }
-            set_up_stream(S, tid, (int)T);
-
-            // ---- copy without stuffed bytes, as big-endian 32-bit words (byte i of the stream is byte i ^ 3 of the copy)
-            uint8_t* const  clean  = static_cast<uint8_t*>(d.scratch);
-            int16_t* const  dcdiff = reinterpret_cast<int16_t*>(clean + clean_room);
-            const uint32_t  N      = d.scan_size;
             // The raw scan is read as 16-byte vectors from the aligned address below it; `lead` bytes precede it there.
+            const uint32_t     N    = d.scan_size;
             const uint32_t     lead = (uint32_t)(reinterpret_cast<uintptr_t>(d.scan) & 15);
             const uint4* const vec  = reinterpret_cast<const uint4*>(d.scan - lead);
             const uint32_t     nv   = (lead + N + 15) >> 4;
-            // For vector i: bit b of `stuffed` = byte b is a zero that follows 0xFF, of `marker` = byte b is non-zero and
-            // follows 0xFF; only bytes at stream offsets [0, limit) count, and the byte before the stream is not 0xFF.
-            auto classify = [&](uint32_t i, uint32_t limit, uint32_t (&w)[4], uint32_t& valid, uint32_t& stuffed, uint32_t& marker) {
-                const uint4 x = __ldg(vec + i);
-                w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
-                uint32_t prev = i > 0 ? (uint32_t)__ldg(reinterpret_cast<const uint8_t*>(vec) + 16 * i - 1) : 0;
-                valid = stuffed = marker = 0;
-                // Nearly every vector lies inside the stream and has no 0xFF in front of any of its bytes: all 16 are kept.
-                const bool inside = 16 * i >= lead && 16 * i + 16 - lead <= limit && 16 * i != lead;
-                const bool no_ff  = prev != 0xFF && !__vcmpeq4(w[0], 0xFFFFFFFFu) && !__vcmpeq4(w[1], 0xFFFFFFFFu) &&
-                                   !__vcmpeq4(w[2], 0xFFFFFFFFu) && !(__vcmpeq4(w[3], 0xFFFFFFFFu) & 0x00FFFFFFu);
-                if (inside && no_ff)
-                {
-                    valid = 0xFFFF;
-                    return;
-                }
-#pragma unroll
-                for (int b = 0; b < 16; ++b)
-                {
-                    const uint32_t v   = (w[b >> 2] >> (8 * (b & 3))) & 255;
-                    const uint32_t pos = 16 * i + b; // offset from the aligned address
-                    if (pos == lead)
-                        prev = 0;
-                    const bool in = pos >= lead && pos - lead < limit;
-                    valid |= (uint32_t)in << b;
-                    stuffed |= (uint32_t)(in && prev == 0xFF && v == 0) << b;
-                    marker |= (uint32_t)(in && prev == 0xFF && v != 0) << b;
-                    prev = v;
-                }
-            };
-            {
-                // a marker (0xFF followed by anything but 0x00, or 0xFF as the last byte) ends the entropy-coded data
-                uint32_t first_marker = N;
-                for (uint32_t i = tid; i < nv; i += T)
-                {
-                    uint32_t w[4], valid, stuffed, marker;
-                    classify(i, N, w, valid, stuffed, marker);
-                    if (marker)
-                        first_marker = min(first_marker, 16 * i + (uint32_t)__ffs(marker) - 1 - lead - 1); // the 0xFF before it
-                }
-                if (tid == 0 && N > 0 && __ldg(d.scan + N - 1) == 0xFF)
-                    first_marker = min(first_marker, N - 1);
-                if (first_marker < N)
-                    atomicMin(&S.marker_at, first_marker);
-            }
+            const uint32_t     scan_room = 16 * nv + 48; // the zero bytes behind the copy, too
+            const bool         resident  = scan_room <= room_bytes;
+            if (resident)
+                fetch_raw(room, vec, 0, nv); // arrives while the tables are being built
+            if (tid == 0)
+                S.marker_at = N > 0 && __ldg(d.scan + N - 1) == 0xFF ? N - 1 : N;
+            set_up_stream(S, tid, (int)T);
+            asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
-            const uint32_t raw_end = S.marker_at;
-            clean_writer   copy{chk_all, reinterpret_cast<uint32_t*>(clean), 0, 0}; // the checkpoints' room is not in use yet
-            for (uint32_t tile = 0; tile < nv; tile += T)
-            {
-                const uint32_t i = tile + tid;
-                uint32_t       w[4] = {0, 0, 0, 0}, keep = 0;
-                if (i < nv)
-                {
-                    uint32_t valid, stuffed, marker;
-                    classify(i, raw_end, w, valid, stuffed, marker);
-                    keep = valid & ~stuffed;
-                }
-                copy.append(w, keep, S.warp_sums[0]);
-            }
-            copy.finish();
-            const uint32_t clean_size = copy.size;
-            __syncthreads();
-            const uint32_t* words = reinterpret_cast<const uint32_t*>(clean);
 
-            // ---- clear the coefficient planes now: the stores drain while the segments are being decoded, and the
-            // barriers between here and the storing pass order them before that pass's stores
-            for (int c = 0; c < d.ncomp; ++c)
-            {
-                const size_t n16 = (size_t)(d.roi[2] - d.roi[0]) * d.hs[c] * (d.roi[3] - d.roi[1]) * d.vs[c] * 8; // 16-byte units
-                uint4*       p   = reinterpret_cast<uint4*>(d.coef[c]);
-                for (size_t i = tid; i < n16; i += T)
-                    p[i] = make_uint4(0, 0, 0, 0);
-            }
-            // ---- segments: one per thread, a multiple of 4 bytes, at least min_segment bytes
-            uint32_t seg = (clean_size + T - 1) / T;
-            seg          = max((seg + 3u) & ~3u, (uint32_t)max(min_segment, 64) & ~3u);
-            const uint32_t nseg      = (clean_size + seg - 1) / seg; // <= T
-            const uint32_t total_bit = clean_size * 8;
-            const bool     mine      = (uint32_t)tid < nseg;
-            const uint32_t pbeg = (uint32_t)tid * seg * 8, pend = min(total_bit, pbeg + seg * 8);
-            // checkpoints of this thread's segment, evenly spaced (at least 64 bits apart; a symbol is shorter, so it passes at most one)
-            const uint32_t  step       = seg * 8 / (NCHECK + 1); // bits between checkpoints (seg is a multiple of 4 bytes)
-            uint32_t* const chk        = chk_all + tid;
-            uint32_t        run_blocks = 0; // blocks of this thread's latest run
-            // first decoding pass: guessed entry states (segment 0: the true one)
-            if (mine)
-            {
-                const seg_result r = run_segment<false>(S, words, pbeg, 0, 0, pend, 0, 0, nullptr, chk, T, pbeg + step, step, false, 0);
-                S.ent_p[tid]  = pbeg;
-                S.ent_bk[tid] = 0;
-                S.ext_p[tid]  = r.p;
-                S.ext_bk[tid] = (uint16_t)((r.b << 8) | r.k);
-                S.cnt[tid]    = r.blocks;
-                run_blocks    = r.blocks;
-            }
-            else
-                S.cnt[tid] = 0;
-            __syncthreads();
-            for (uint32_t round = 1; round < nseg; ++round)
-            {
-                uint32_t cand_p  = 0;
-                uint16_t cand_bk = 0;
-                bool     redo    = false;
-                if (mine && tid > 0)
-                {
-                    cand_p  = S.ext_p[tid - 1];
-                    cand_bk = S.ext_bk[tid - 1];
-                    redo    = cand_p != S.ent_p[tid] || cand_bk != S.ent_bk[tid];
-                }
-                __syncthreads(); // every candidate has been read before any exit state changes
-                if (redo)
-                {
-                    const seg_result r =
-                        run_segment<false>(S, words, cand_p, cand_bk >> 8, cand_bk & 255, pend, 0, 0, nullptr, chk, T, pbeg + step, step, true, run_blocks);
-                    S.ent_p[tid]  = cand_p;
-                    S.ent_bk[tid] = cand_bk;
-                    S.cnt[tid]    = r.blocks;
-                    run_blocks    = r.blocks;
-                    if (!r.merged)
-                    {
-                        S.ext_p[tid]  = r.p;
-                        S.ext_bk[tid] = (uint16_t)((r.b << 8) | r.k);
-                    }
-                }
-                if (!__syncthreads_or(redo))
-                    break;
-            }
-
-            // ---- first block number of every segment
-            uint32_t       counted;
-            const uint32_t g0            = cta_exclusive_scan(S.cnt[tid], S.warp_sums[0], counted);
             const uint32_t needed_mcus   = (uint32_t)min(d.roi[3], d.mcuy) * d.mcux;
             const uint32_t needed_blocks = needed_mcus * bpm;
-            if (tid == 0 && counted < needed_blocks)
-                S.bad = 1;
-
-            // ---- decode once more from the true entry states, storing (the planes were cleared above).  The checkpoints now
-            // describe every segment's final run, so each segment falls into NCHECK + 1 pieces with known entry states and block
-            // numbers, and the pieces -- not the segments -- are dealt out to the threads: streams with fewer segments than
-            // threads keep every warp busy, and neighbouring lanes work on neighbouring pieces.
-            S.ext_p[tid] = g0; // the exit states have served
-            __syncthreads();
-            for (uint32_t q = tid; q < nseg * (NCHECK + 1); q += T)
+            uint8_t* const clean         = static_cast<uint8_t*>(d.scratch);
+            int16_t*       dcdiff        = reinterpret_cast<int16_t*>(clean + clean_room);
+            if (resident)
             {
-                const uint32_t t = q / (NCHECK + 1), piece = q % (NCHECK + 1);
-                const uint32_t seg_beg = t * seg * 8, seg_end = min(total_bit, seg_beg + seg * 8);
-                const uint32_t at = seg_beg + piece * step; // the checkpoint this piece starts from
-                if (at >= seg_end)
-                    continue;
-                uint32_t p0 = S.ent_p[t], bk = S.ent_bk[t], before = 0;
-                if (piece > 0)
-                {
-                    const uint32_t key = chk_all[(piece - 1) * T + t];
-                    p0                 = at + (key >> 10);
-                    bk                 = (key >> 6 & 15) << 8 | (key & 63);
-                    before             = chk_all[(NCHECK + piece - 1) * T + t];
-                }
-                const seg_result r = run_segment<true>(S, words, p0, bk >> 8, bk & 255, min(seg_end, at + step), S.ext_p[t] + before, needed_blocks,
-                                                       dcdiff, nullptr, 0, 0, 0, false, 0);
-                if (r.bad)
-                    S.bad = 1;
+                if (2ull * needed_blocks <= room_bytes - scan_room)
+                    dcdiff = reinterpret_cast<int16_t*>(reinterpret_cast<uint8_t*>(room) + scan_room);
+                const uint32_t clean_size = copy_scan<true>(S, room, nullptr, vec, nv, lead);
+                __syncthreads();
+                decode_scan<shared_words>(S, A, room, clean_size, min_segment, needed_blocks, dcdiff);
             }
-            __syncthreads();
+            else
+            {
+                uint32_t* const words = reinterpret_cast<uint32_t*>(clean);
+                // the checkpoints' room and what follows is not in use yet
+                const uint32_t clean_size = copy_scan<false>(S, A.chk, words, vec, nv, lead);
+                __syncthreads();
+                decode_scan<global_words>(S, A, words, clean_size, min_segment, needed_blocks, dcdiff);
+            }
 
             // ---- DC: sum the differences per component in scan order.  Thread t owns MCUs [m0, m1).
             const uint32_t mchunk = (needed_mcus + T - 1) / T;
@@ -1089,33 +1257,7 @@ namespace aeonb
                 uint32_t total;
                 pred[c] = (int)cta_exclusive_scan((uint32_t)sum[c], S.warp_sums[c], total);
             }
-            if (m0 < m1)
-            {
-                int my = (int)(m0 / (uint32_t)d.mcux), mx = (int)(m0 - (uint32_t)my * d.mcux);
-                for (uint32_t m = m0; m < m1; ++m)
-                {
-                    for (int b = 0; b < bpm; ++b)
-                    {
-                        const int v = dcdiff[(size_t)m * bpm + b];
-                        const int c = S.comp[b];
-                        int       now;
-                        if (c == 0)
-                            now = pred[0] += v;
-                        else if (c == 1)
-                            now = pred[1] += v;
-                        else
-                            now = pred[2] += v;
-                        int16_t* out = block_home(S, mx, my, b);
-                        if (out)
-                            out[0] = (int16_t)now;
-                    }
-                    if (++mx == d.mcux)
-                    {
-                        mx = 0;
-                        ++my;
-                    }
-                }
-            }
+            store_dc(S, dcdiff, m0, m1, bpm, pred);
             __syncthreads();
             if (tid == 0 && d.status)
                 *d.status = S.bad ? 1 : 0;
@@ -1139,6 +1281,7 @@ namespace aeonb
         // with these.  A part of 4 to 16 KB per block fills the chip (about 20 parts per picture) and keeps segments at 160 bytes.
         constexpr int RST_THREADS       = 128;
         constexpr int RST_INDEX_THREADS = 1024;
+        constexpr int RST_ROOM          = 12 * 1024 + 512; // shared memory for a part's bytes (see jpeg_restart_parts): 4 blocks fit an SM
 
         struct rst_state
         {
@@ -1268,17 +1411,165 @@ namespace aeonb
             }
         }
 
-        // Part blockIdx.x = {record, first interval, intervals, number of the part within its stream}.
+        // Copies intervals R.raw[0..I) without stuffed bytes and markers and notes in R.clean where each starts; returns the bytes of
+        // the copy.  RESIDENT as in copy_scan, vector i0 being the first in `room`.
+        template <bool RESIDENT>
+        __device__ __forceinline__ uint32_t copy_intervals(rst_state& R, uint32_t I, uint32_t* room, uint32_t* out, const uint4* vec, uint32_t lead)
+        {
+            constexpr uint32_t     T   = RST_THREADS;
+            const uint32_t         tid = threadIdx.x;
+            const uint32_t         r0 = R.raw[0], r1 = R.raw[I] - 2;
+            const uint32_t         i0 = (lead + r0) >> 4, i1 = (lead + r1 + 15) >> 4;
+            const uint8_t* const   base = reinterpret_cast<const uint8_t*>(vec);
+            clean_writer<RESIDENT> copy{room, out, 0, 0};
+            for (uint32_t tile = i0, odd = 0; tile < i1; tile += T, odd ^= 1)
+            {
+                const uint32_t i = tile + tid;
+                uint32_t       words[4] = {0, 0, 0, 0}, keep = 0, starts = 0;
+                if (i < i1)
+                {
+                    const uint4 x = RESIDENT ? reinterpret_cast<const uint4*>(room)[i - i0] : __ldg(vec + i);
+                    words[0] = x.x, words[1] = x.y, words[2] = x.z, words[3] = x.w;
+                    uint32_t prev = 0;
+                    if (i > i0)
+                        prev = !RESIDENT  ? (uint32_t)__ldg(base + 16 * i - 1)
+                               : tid == 0 ? R.S.tile_end[odd ^ 1] // its place may have been taken
+                                          : (uint32_t) reinterpret_cast<const uint8_t*>(room)[16 * (i - i0) - 1];
+                    if (16 * i >= lead + r0 && 16 * i + 16 <= lead + r1 && !has_ff(x, prev))
+                        keep = 0xFFFF;
+                    else
+                    {
+                        const uint32_t last = 16 * i + 16 < lead + r1 ? (uint32_t)__ldg(base + 16 * i + 16) : 0;
+#pragma unroll
+                        for (int b = 0; b < 16; ++b)
+                        {
+                            const uint32_t v    = (words[b >> 2] >> (8 * (b & 3))) & 255;
+                            const uint32_t pos  = 16 * i + b;
+                            const uint32_t next = b < 15 ? (words[(b + 1) >> 2] >> (8 * ((b + 1) & 3))) & 255 : last;
+                            if (pos == lead + r0)
+                                prev = 0; // the second byte of the marker in front of the part
+                            const bool in     = pos >= lead + r0 && pos < lead + r1;
+                            const bool follow = prev == 0xFF; // a stuffed zero, or a marker's second byte
+                            const bool head   = v == 0xFF && next != 0 && pos + 1 < lead + r1;
+                            keep |= (uint32_t)(in && !follow && !head) << b;
+                            starts |= (uint32_t)(in && follow && v != 0) << b;
+                            prev = v;
+                        }
+                    }
+                }
+                if (RESIDENT && tid == T - 1)
+                    R.S.tile_end[odd] = words[3] >> 24;
+                uint32_t       total;
+                const uint32_t at = cta_exclusive_scan((uint32_t)__popc(keep), R.S.warp_sums[0], total);
+                for (uint32_t m = starts; m; m &= m - 1)
+                {
+                    const uint32_t b = (uint32_t)__ffs(m) - 1, pos = 16 * i + b - lead + 1; // offset of the interval behind the marker
+                    uint32_t       lo = 0, hi = I; // the last interval that starts at or before it
+                    while (hi - lo > 1)
+                    {
+                        const uint32_t mid = (lo + hi) >> 1;
+                        if (R.raw[mid] <= pos)
+                            lo = mid;
+                        else
+                            hi = mid;
+                    }
+                    R.clean[lo] = copy.size + at + (uint32_t)__popc(keep & ((1u << b) - 1));
+                }
+                copy.append(words, keep, at, total);
+            }
+            copy.finish();
+            if (tid == 0)
+                R.clean[0] = 0, R.clean[I] = copy.size;
+            return copy.size;
+        }
+
+        // Segments of a part's intervals, their true entry states, and the storing pass.
+        template <typename Words>
+        __device__ __forceinline__ void decode_intervals(rst_state& R, const seg_arrays& A, const uint32_t* words, uint32_t first, uint32_t I,
+                                                         uint32_t clean_size, int min_segment, int bpm, uint32_t needed_mcus, int16_t* dcdiff)
+        {
+            constexpr uint32_t T   = RST_THREADS;
+            par_state&         S   = R.S;
+            const uint32_t     tid = threadIdx.x, ri = (uint32_t)S.d.restart_interval;
+            auto first_block = [&](uint32_t i) { return (uint32_t)min((uint64_t)needed_mcus, (uint64_t)(first + i) * ri) * (uint32_t)bpm; };
+            // an interval has ceil(its bytes / seg) segments; I < T of them are shorter than seg, so this many fit
+            uint32_t seg = (clean_size + (T - I) - 1) / (T - I);
+            seg          = max((seg + 3u) & ~3u, (uint32_t)max(min_segment, 64) & ~3u);
+            uint32_t       nseg; // <= T
+            const uint32_t mine_of = tid < I ? (R.clean[tid + 1] - R.clean[tid] + seg - 1) / seg : 0;
+            const uint32_t seg0    = cta_exclusive_scan(mine_of, S.warp_sums[0], nseg);
+            if (tid < I)
+                R.seg[tid] = seg0;
+            if (tid == 0)
+                R.seg[I] = nseg;
+            __syncthreads();
+            const bool mine = tid < nseg;
+            uint32_t   iv   = 0; // this thread's interval: the last one whose first segment is not behind it
+            for (uint32_t hi = I; hi - iv > 1;)
+            {
+                const uint32_t mid = (iv + hi) >> 1;
+                if (R.seg[mid] <= tid)
+                    iv = mid;
+                else
+                    hi = mid;
+            }
+            const uint32_t pbeg = (R.clean[iv] + (tid - R.seg[iv]) * seg) * 8, pend = min(R.clean[iv + 1] * 8, pbeg + seg * 8);
+            const uint32_t step       = seg * 8 / (NCHECK + 1);
+            const uint32_t run_blocks = settle_segments<Words>(S, A, words, nseg, R.seg[iv] == tid, pbeg, pend, step);
+
+            // ---- first block number of every segment, counted from its interval's first block
+            uint32_t counted;
+            A.cnt[tid] = cta_exclusive_scan(run_blocks, S.warp_sums[0], counted);
+            if (mine)
+                A.ext_bk[tid] = (uint16_t)iv; // the exit states have served
+            __syncthreads();
+            if (mine)
+                A.ext_p[tid] = first_block(iv) + A.cnt[tid] - A.cnt[R.seg[iv]];
+            if (tid < I)
+            {
+                const uint32_t a = R.seg[tid], b = R.seg[tid + 1];
+                const uint32_t has = a == b ? 0 : (b < nseg ? A.cnt[b] : counted) - A.cnt[a];
+                if (has < first_block(tid + 1) - first_block(tid))
+                    S.bad = 1;
+            }
+            __syncthreads();
+
+            // ---- decode once more, storing; the pieces between checkpoints are dealt out to the threads
+            for (uint32_t q = tid; q < nseg * (NCHECK + 1); q += T)
+            {
+                const uint32_t t = q / (NCHECK + 1), piece = q % (NCHECK + 1), i = A.ext_bk[t];
+                const uint32_t all_end = R.clean[i + 1] * 8;
+                const uint32_t seg_beg = (R.clean[i] + (t - R.seg[i]) * seg) * 8, seg_end = min(all_end, seg_beg + seg * 8);
+                const uint32_t at = seg_beg + piece * step; // the checkpoint this piece starts from
+                if (at >= seg_end)
+                    continue;
+                uint32_t p0, bk, before;
+                piece_entry(A, T, t, piece, at, p0, bk, before);
+                const uint32_t   g = A.ext_p[t] + before, gend = first_block(i + 1);
+                const seg_result r = run_segment<true, Words>(S, words, p0, bk >> 8, bk & 255, min(seg_end, at + step), g, gend, dcdiff, nullptr, 0,
+                                                              0, 0, false, 0);
+                // the interval's last block leaves less than a byte
+                if (r.bad || (r.blocks > 0 && g + r.blocks == gend && (r.p > all_end || all_end - r.p > 7)))
+                    S.bad = 1;
+            }
+            __syncthreads();
+        }
+
+        // Part blockIdx.x = {record, first interval, intervals, number of the part within its stream}.  Shared memory: rst_state,
+        // SEG_BYTES per thread, and what is left of `smem_bytes` for the part's bytes, where they fit.
         __global__ void __launch_bounds__(RST_THREADS) jpeg_entropy_restart_kernel(const aeonb_entropy_desc* __restrict__ descs,
-                                                                                   const int4* __restrict__ parts, int min_segment)
+                                                                                   const int4* __restrict__ parts, int min_segment,
+                                                                                   uint32_t smem_bytes)
         {
             constexpr uint32_t T = RST_THREADS;
             extern __shared__ __align__(16) unsigned char smem_raw[];
-            rst_state&      R       = *reinterpret_cast<rst_state*>(smem_raw);
-            par_state&      S       = R.S;
-            uint32_t* const chk_all = reinterpret_cast<uint32_t*>(smem_raw + sizeof(rst_state)); // 2 x NCHECK rows of T words
-            const uint32_t  tid     = threadIdx.x;
-            const int4      part    = __ldg(parts + blockIdx.x);
+            rst_state&       R       = *reinterpret_cast<rst_state*>(smem_raw);
+            par_state&       S       = R.S;
+            const seg_arrays A       = seg_arrays_at(smem_raw + sizeof(rst_state), T);
+            const uint32_t   room_at = ((uint32_t)sizeof(rst_state) + SEG_BYTES * T + 15) & ~15u;
+            uint32_t* const  room    = reinterpret_cast<uint32_t*>(smem_raw + room_at);
+            const uint32_t   tid     = threadIdx.x;
+            const int4       part    = __ldg(parts + blockIdx.x);
             for (uint32_t i = tid; i < sizeof(aeonb_entropy_desc) / 4; i += T)
                 reinterpret_cast<uint32_t*>(&S.d)[i] = reinterpret_cast<const uint32_t*>(descs + part.x)[i];
             if (tid < 64)
@@ -1309,74 +1600,19 @@ namespace aeonb
                     w.header->doubtful = 1;
                 return;
             }
+            const uint32_t     lead = (uint32_t)(reinterpret_cast<uintptr_t>(d.scan) & 15);
+            const uint4* const vec  = reinterpret_cast<const uint4*>(d.scan - lead);
+            const uint32_t     r0 = R.raw[0], i0 = (lead + r0) >> 4, i1 = (lead + R.raw[I] - 2 + 15) >> 4;
+            const bool         resident = 16 * (i1 - i0) + 48 <= smem_bytes - room_at;
+            if (resident)
+                fetch_raw(room, vec, i0, i1); // arrives while the tables are being built
             set_up_stream(S, (int)tid, (int)T);
-
-            // ---- copy without stuffed bytes and markers, as big-endian 32-bit words (byte i of the copy is byte i ^ 3 of memory).
-            // The parts' copies follow one another with 64 bytes between them.
-            const uint32_t     r0 = R.raw[0], r1 = R.raw[I] - 2;
-            uint8_t* const     clean = w.clean + (r0 & ~15u) + 64u * (uint32_t)part.w;
-            const uint32_t     lead  = (uint32_t)(reinterpret_cast<uintptr_t>(d.scan) & 15);
-            const uint4* const vec   = reinterpret_cast<const uint4*>(d.scan - lead);
-            const uint32_t     i0 = (lead + r0) >> 4, i1 = (lead + r1 + 15) >> 4;
-            clean_writer       copy{chk_all, reinterpret_cast<uint32_t*>(clean), 0, 0}; // the checkpoints' room is not in use yet
-            if (tid == 0)
-                R.clean[0] = 0;
-            for (uint32_t tile = i0; tile < i1; tile += T)
-            {
-                const uint32_t i = tile + tid;
-                uint32_t       words[4] = {0, 0, 0, 0}, keep = 0, starts = 0;
-                if (i < i1)
-                {
-                    const uint4 x    = __ldg(vec + i);
-                    uint32_t    prev = i > i0 ? (uint32_t)__ldg(reinterpret_cast<const uint8_t*>(vec) + 16 * i - 1) : 0;
-                    words[0] = x.x, words[1] = x.y, words[2] = x.z, words[3] = x.w;
-                    if (16 * i >= lead + r0 && 16 * i + 16 <= lead + r1 && !has_ff(x, prev))
-                        keep = 0xFFFF;
-                    else
-                    {
-                        const uint32_t last = 16 * i + 16 < lead + r1 ? (uint32_t)__ldg(reinterpret_cast<const uint8_t*>(vec) + 16 * i + 16) : 0;
-#pragma unroll
-                        for (int b = 0; b < 16; ++b)
-                        {
-                            const uint32_t v    = (words[b >> 2] >> (8 * (b & 3))) & 255;
-                            const uint32_t pos  = 16 * i + b;
-                            const uint32_t next = b < 15 ? (words[(b + 1) >> 2] >> (8 * ((b + 1) & 3))) & 255 : last;
-                            if (pos == lead + r0)
-                                prev = 0; // the second byte of the marker in front of the part
-                            const bool in     = pos >= lead + r0 && pos < lead + r1;
-                            const bool follow = prev == 0xFF; // a stuffed zero, or a marker's second byte
-                            const bool head   = v == 0xFF && next != 0 && pos + 1 < lead + r1;
-                            keep |= (uint32_t)(in && !follow && !head) << b;
-                            starts |= (uint32_t)(in && follow && v != 0) << b;
-                            prev = v;
-                        }
-                    }
-                }
-                const uint32_t o = copy.append(words, keep, S.warp_sums[0]);
-                for (uint32_t m = starts; m; m &= m - 1)
-                {
-                    const uint32_t b = (uint32_t)__ffs(m) - 1, pos = 16 * i + b - lead + 1; // offset of the interval behind the marker
-                    uint32_t       lo = 0, hi = I; // the last interval that starts at or before it
-                    while (hi - lo > 1)
-                    {
-                        const uint32_t mid = (lo + hi) >> 1;
-                        if (R.raw[mid] <= pos)
-                            lo = mid;
-                        else
-                            hi = mid;
-                    }
-                    R.clean[lo] = o + (uint32_t)__popc(keep & ((1u << b) - 1));
-                }
-            }
-            copy.finish();
-            const uint32_t clean_size = copy.size;
-            if (tid == 0)
-                R.clean[I] = clean_size;
 
             // ---- clear the coefficients of this part's MCUs (a warp per MCU, a lane per 16 bytes)
             const uint32_t needed_mcus = (uint32_t)min(d.roi[3], d.mcuy) * d.mcux;
             const uint32_t ri          = (uint32_t)d.restart_interval;
-            const uint32_t mcu0 = min(needed_mcus, first * ri), mcu1 = (uint32_t)min((uint64_t)needed_mcus, (uint64_t)(first + I) * ri);
+            const uint32_t mcu0 = (uint32_t)min((uint64_t)needed_mcus, (uint64_t)first * ri);
+            const uint32_t mcu1 = (uint32_t)min((uint64_t)needed_mcus, (uint64_t)(first + I) * ri);
             const uint32_t lane = tid & 31, warp = tid >> 5;
             for (uint32_t m = mcu0 + warp; m < mcu1; m += T / 32)
             {
@@ -1386,119 +1622,23 @@ namespace aeonb
                 for (uint32_t u = lane; u < (uint32_t)bpm * 8; u += 32)
                     reinterpret_cast<uint4*>(block_home(S, mx, my, (int)(u >> 3)))[u & 7] = make_uint4(0, 0, 0, 0);
             }
+            asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
-            const uint32_t* words = reinterpret_cast<const uint32_t*>(clean);
-
-            // ---- segments: an interval has ceil(its bytes / seg) of them; I < T of them are shorter than seg, so this many fit
-            uint32_t seg = (clean_size + (T - I) - 1) / (T - I);
-            seg          = max((seg + 3u) & ~3u, (uint32_t)max(min_segment, 64) & ~3u);
-            uint32_t       nseg; // <= T
-            const uint32_t mine_of = tid < I ? (R.clean[tid + 1] - R.clean[tid] + seg - 1) / seg : 0;
-            const uint32_t seg0    = cta_exclusive_scan(mine_of, S.warp_sums[0], nseg);
-            if (tid < I)
-                R.seg[tid] = seg0;
-            if (tid == 0)
-                R.seg[I] = nseg;
-            __syncthreads();
-            const bool mine = tid < nseg;
-            uint32_t   iv   = 0; // this thread's interval: the last one whose first segment is not behind it
-            for (uint32_t lo = 0, hi = I; hi - lo > 1;)
-            {
-                const uint32_t mid = (lo + hi) >> 1;
-                if (R.seg[mid] <= tid)
-                    lo = mid;
-                else
-                    hi = mid;
-                iv = lo;
-            }
-            const bool      heads = mine && R.seg[iv] == tid; // its entry state is known
-            const uint32_t  pbeg = (R.clean[iv] + (tid - R.seg[iv]) * seg) * 8, pend = min(R.clean[iv + 1] * 8, pbeg + seg * 8);
-            const uint32_t  step = seg * 8 / (NCHECK + 1);
-            uint32_t* const chk  = chk_all + tid;
-            uint32_t        run_blocks = 0;
-            if (mine)
-            {
-                const seg_result r = run_segment<false>(S, words, pbeg, 0, 0, pend, 0, 0, nullptr, chk, T, pbeg + step, step, false, 0);
-                S.ent_p[tid]  = pbeg;
-                S.ent_bk[tid] = 0;
-                S.ext_p[tid]  = r.p;
-                S.ext_bk[tid] = (uint16_t)((r.b << 8) | r.k);
-                run_blocks    = r.blocks;
-            }
-            __syncthreads();
-            for (uint32_t round = 1; round < nseg; ++round)
-            {
-                uint32_t cand_p  = 0;
-                uint16_t cand_bk = 0;
-                bool     redo    = false;
-                if (mine && !heads)
-                {
-                    cand_p  = S.ext_p[tid - 1];
-                    cand_bk = S.ext_bk[tid - 1];
-                    redo    = cand_p != S.ent_p[tid] || cand_bk != S.ent_bk[tid];
-                }
-                __syncthreads(); // every candidate has been read before any exit state changes
-                if (redo)
-                {
-                    const seg_result r =
-                        run_segment<false>(S, words, cand_p, cand_bk >> 8, cand_bk & 255, pend, 0, 0, nullptr, chk, T, pbeg + step, step, true, run_blocks);
-                    S.ent_p[tid]  = cand_p;
-                    S.ent_bk[tid] = cand_bk;
-                    run_blocks    = r.blocks;
-                    if (!r.merged)
-                    {
-                        S.ext_p[tid]  = r.p;
-                        S.ext_bk[tid] = (uint16_t)((r.b << 8) | r.k);
-                    }
-                }
-                if (!__syncthreads_or(redo))
-                    break;
-            }
-
-            // ---- first block number of every segment, counted from its interval's first block
-            uint32_t counted;
-            S.cnt[tid] = cta_exclusive_scan(run_blocks, S.warp_sums[0], counted);
-            if (mine)
-                S.ext_bk[tid] = (uint16_t)iv; // the exit states have served
-            __syncthreads();
-            auto first_block = [&](uint32_t i) { return (uint32_t)min((uint64_t)needed_mcus, (uint64_t)(first + i) * ri) * (uint32_t)bpm; };
-            if (mine)
-                S.ext_p[tid] = first_block(iv) + S.cnt[tid] - S.cnt[R.seg[iv]];
-            if (tid < I)
-            {
-                const uint32_t a = R.seg[tid], b = R.seg[tid + 1];
-                const uint32_t has = a == b ? 0 : (b < nseg ? S.cnt[b] : counted) - S.cnt[a];
-                if (has < first_block(tid + 1) - first_block(tid))
-                    S.bad = 1;
-            }
-            __syncthreads();
-
-            // ---- decode once more, storing; the pieces between checkpoints are dealt out to the threads
             int16_t* const dcdiff = w.dcdiff;
-            for (uint32_t q = tid; q < nseg * (NCHECK + 1); q += T)
+            if (resident)
             {
-                const uint32_t t = q / (NCHECK + 1), piece = q % (NCHECK + 1), i = S.ext_bk[t];
-                const uint32_t all_end = R.clean[i + 1] * 8;
-                const uint32_t seg_beg = (R.clean[i] + (t - R.seg[i]) * seg) * 8, seg_end = min(all_end, seg_beg + seg * 8);
-                const uint32_t at = seg_beg + piece * step; // the checkpoint this piece starts from
-                if (at >= seg_end)
-                    continue;
-                uint32_t p0 = S.ent_p[t], bk = S.ent_bk[t], before = 0;
-                if (piece > 0)
-                {
-                    const uint32_t key = chk_all[(piece - 1) * T + t];
-                    p0                 = at + (key >> 10);
-                    bk                 = (key >> 6 & 15) << 8 | (key & 63);
-                    before             = chk_all[(NCHECK + piece - 1) * T + t];
-                }
-                const uint32_t   g = S.ext_p[t] + before, gend = first_block(i + 1);
-                const seg_result r = run_segment<true>(S, words, p0, bk >> 8, bk & 255, min(seg_end, at + step), g, gend, dcdiff, nullptr, 0, 0, 0,
-                                                       false, 0);
-                // the interval's last block leaves less than a byte
-                if (r.bad || (r.blocks > 0 && g + r.blocks == gend && (r.p > all_end || all_end - r.p > 7)))
-                    S.bad = 1;
+                const uint32_t clean_size = copy_intervals<true>(R, I, room, nullptr, vec, lead);
+                __syncthreads();
+                decode_intervals<shared_words>(R, A, room, first, I, clean_size, min_segment, bpm, needed_mcus, dcdiff);
             }
-            __syncthreads();
+            else
+            {
+                // the parts' copies follow one another with 64 bytes between them; the checkpoints' room is not in use yet
+                uint32_t* const clean      = reinterpret_cast<uint32_t*>(w.clean + (r0 & ~15u) + 64u * (uint32_t)part.w);
+                const uint32_t  clean_size = copy_intervals<false>(R, I, A.chk, clean, vec, lead);
+                __syncthreads();
+                decode_intervals<global_words>(R, A, clean, first, I, clean_size, min_segment, bpm, needed_mcus, dcdiff);
+            }
             if (S.bad)
             {
                 if (tid == 0)
@@ -1509,7 +1649,8 @@ namespace aeonb
             // ---- DC: a warp per interval sums the differences in scan order, lane l the l-th run of MCUs
             for (uint32_t i = warp; i < I; i += T / 32)
             {
-                const uint32_t b0 = first_block(i) / (uint32_t)bpm, b1 = first_block(i + 1) / (uint32_t)bpm, chunk = (b1 - b0 + 31) / 32;
+                const uint32_t b0 = (uint32_t)min((uint64_t)needed_mcus, (uint64_t)(first + i) * ri);
+                const uint32_t b1 = (uint32_t)min((uint64_t)needed_mcus, (uint64_t)(first + i + 1) * ri), chunk = (b1 - b0 + 31) / 32;
                 const uint32_t m0 = min(b1, b0 + lane * chunk), m1 = min(b1, m0 + chunk);
                 int            sum[3] = {0, 0, 0};
                 for (uint32_t m = m0; m < m1; ++m)
@@ -1535,30 +1676,7 @@ namespace aeonb
                     }
                     pred[c] = incl - sum[c];
                 }
-                int my = (int)(m0 / (uint32_t)d.mcux), mx = (int)(m0 - (uint32_t)my * d.mcux);
-                for (uint32_t m = m0; m < m1; ++m)
-                {
-                    for (int b = 0; b < bpm; ++b)
-                    {
-                        const int v = dcdiff[(size_t)m * bpm + b];
-                        const int c = S.comp[b];
-                        int       now;
-                        if (c == 0)
-                            now = pred[0] += v;
-                        else if (c == 1)
-                            now = pred[1] += v;
-                        else
-                            now = pred[2] += v;
-                        int16_t* out = block_home(S, mx, my, b);
-                        if (out)
-                            out[0] = (int16_t)now;
-                    }
-                    if (++mx == d.mcux)
-                    {
-                        mx = 0;
-                        ++my;
-                    }
-                }
+                store_dc(S, dcdiff, m0, m1, bpm, pred);
             }
         }
     }
@@ -1605,8 +1723,9 @@ namespace aeonb
                 total += descs[i].scan_size;
         if (total == 0)
             return;
-        // Five blocks of a part fit an SM; parts of less than 4 KB are mostly set-up, parts of more than 16 KB mean longer segments.
-        const uint64_t target = std::min<uint64_t>(std::max<uint64_t>(total / (148 * 5), 4096), 16384);
+        // Four blocks of a part fit an SM; parts of less than 4 KB are mostly set-up, parts of more than 12 KB do not fit its
+        // shared memory.
+        const uint64_t target = std::min<uint64_t>(std::max<uint64_t>(total / (148 * 4), 4096), 10240);
         for (int i = 0; i < n; ++i)
         {
             const aeonb_entropy_desc& d = descs[i];
@@ -1623,26 +1742,39 @@ namespace aeonb
         }
     }
 
+    // Shared memory of a block of the block-parallel kernel: room for the launch's longest stream and its DC differences.  More
+    // streams than SMs: as much as lets as many blocks share an SM as there are streams for it (four at most), the longest
+    // streams falling back on global memory.
+    static size_t jpeg_entropy_smem(int n, int threads, uint32_t longest, uint64_t most_blocks)
+    {
+        const size_t fixed = sizeof(par_state) + (size_t)SEG_BYTES * threads + 16;
+        const size_t want  = fixed + (size_t)longest + 16 + 64 + (size_t)most_blocks * 2;
+        const int    share = std::min({(n + 147) / 148, 4, std::max(1, 1280 / threads)}); // the kernel's registers allow 1280 threads
+        const size_t most  = (size_t)(228 * 1024) / share - 1024;
+        return std::max(fixed, std::min(want, std::min<size_t>(most, 227 * 1024)));
+    }
+
     cudaError_t launch_jpeg_entropy(const aeonb_entropy_desc* descs_dev, int n, bool any_parallel, bool any_serial, int min_segment,
-                                    int threads, const int4* parts_dev, int n_parts, cudaStream_t stream)
+                                    int threads, uint32_t longest, uint64_t most_blocks, const int4* parts_dev, int n_parts,
+                                    cudaStream_t stream)
     {
         if (n <= 0)
             return cudaSuccess;
         if (any_parallel)
         {
             threads           = std::min(std::max(threads, 64), jpeg_entropy_threads()) & ~31;
-            const size_t smem = sizeof(par_state) + (size_t)2 * NCHECK * threads * sizeof(uint32_t);
+            const size_t smem = jpeg_entropy_smem(n, threads, longest, most_blocks);
             cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_parallel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (err != cudaSuccess)
                 return err;
-            jpeg_entropy_parallel_kernel<<<n, threads, smem, stream>>>(descs_dev, min_segment);
+            jpeg_entropy_parallel_kernel<<<n, threads, smem, stream>>>(descs_dev, min_segment, (uint32_t)smem);
             err = cudaGetLastError();
             if (err != cudaSuccess)
                 return err;
         }
         if (n_parts > 0)
         {
-            const size_t smem = sizeof(rst_state) + (size_t)2 * NCHECK * RST_THREADS * sizeof(uint32_t);
+            const size_t smem = sizeof(rst_state) + 16 + (size_t)SEG_BYTES * RST_THREADS + RST_ROOM;
             cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_restart_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (err != cudaSuccess)
                 return err;
@@ -1650,7 +1782,7 @@ namespace aeonb
             err = cudaGetLastError();
             if (err != cudaSuccess)
                 return err;
-            jpeg_entropy_restart_kernel<<<n_parts, RST_THREADS, smem, stream>>>(descs_dev, parts_dev, min_segment);
+            jpeg_entropy_restart_kernel<<<n_parts, RST_THREADS, smem, stream>>>(descs_dev, parts_dev, min_segment, (uint32_t)smem);
             err = cudaGetLastError();
             if (err != cudaSuccess)
                 return err;
