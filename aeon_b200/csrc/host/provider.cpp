@@ -261,7 +261,10 @@ aeonb_provider::aeonb_provider(aeonb_ctx* c, const json& cfg) : ctx(c)
             const char* names[10] = {"bbtargets", "bbtargets_mask", "labels_flat", "labels_mask", "image_shape", "gt_boxes",
                                      "gt_box_count", "gt_class_count", "image_scale", "difficult_flag"};
             for (int i = 0; i < 10; ++i)
+            {
                 add(prefixed(st.rcnn.name, names[i]), st.rcnn.shapes[i], true);
+                outputs.back().anchor_plane = i < RCNN_PLANES;
+            }
         }
         else if (t == "audio")
         {

@@ -67,6 +67,7 @@ namespace aeonb
         shape_type  shape;
         std::string axes;          // comma separated axis names
         bool        host_produced; // small outputs computed on the CPU (labels, boxes)
+        bool        anchor_plane = false; // localization_rcnn: filled on the GPU where the output lies in device memory
     };
 
     // One JPEG stream to decode: where its bytes are and where its pieces live in the arenas.
@@ -153,6 +154,7 @@ namespace aeonb
         size_t stage_bytes = 0, pixel_bytes = 0, coef_bytes = 0, oriented_bytes = 0, rotated_bytes = 0;
         size_t status_room   = 0; // bytes reserved for the entropy decoder's status words at the start of the coefficient arena
         int    n_device_jobs = 0; // streams Huffman-decoded on the GPU
+        bool   anchor_planes_on_device = false; // localization_rcnn: the planes with a value or four per anchor are written by kernels
         std::vector<char*> produced; // where each device-produced output is written
     };
 }
@@ -202,6 +204,7 @@ struct aeonb_provider
     std::vector<aeonb::device_buffer>    rcnn_anchor_dev, rcnn_result_dev;
     std::vector<aeonb::pinned_buffer>    rcnn_result_host;
     aeonb::random_engine_t               rcnn_engine;
+    cudaEvent_t                          m_labelled = nullptr; // the labels of the batch in hand are on the host
     // Device-side outputs of batches delivered to host memory: the copy of batch t to the host (on the copy stream)
     // overlaps the kernels of the next batches, which write the other sets.
     std::vector<aeonb::device_buffer>    out_dev[k_sets];   // per output, batch_size records
@@ -268,6 +271,6 @@ private:
     void plan_records(aeonb::batch_plan& plan, const void* const* elems, const size_t* sizes, int n);
     void reserve_arenas(aeonb::batch_plan& plan, void* const* outs, bool on_device, int par);
     void stage_inputs(aeonb::batch_plan& plan, int par);
-    void launch_kernels(aeonb::batch_plan& plan, int n, int par);
+    void launch_kernels(aeonb::batch_plan& plan, void* const* outs, int n, int par);
     void deliver(aeonb::batch_plan& plan, void* const* outs, int n, bool on_device, int par, int64_t ticket);
 };

@@ -169,6 +169,8 @@ aeonb_provider::~aeonb_provider()
     for (cudaEvent_t e : m_kernels)
         if (e)
             cudaEventDestroy(e);
+    if (m_labelled)
+        cudaEventDestroy(m_labelled);
     for (auto& slot : m_trace)
         for (cudaEvent_t e : slot)
             if (e)
@@ -294,6 +296,11 @@ void aeonb_provider::run(const void* const* elems, const size_t* sizes, int n, v
         throw std::invalid_argument("aeonb_provider_run: record count must be in [1, batch_size]");
     const auto t0 = std::chrono::steady_clock::now();
     auto job = std::make_unique<batch_job>((int)stages.size());
+    // the big planes of localization_rcnn never exist on the host when they are delivered to device memory as they are
+    job->plan.anchor_planes_on_device = on_device && batch_major;
+    for (size_t o = 0; o < outputs.size(); ++o)
+        if (outputs[o].anchor_plane && ((uintptr_t)outs[o] & 3))
+            job->plan.anchor_planes_on_device = false;
     plan_records(job->plan, elems, sizes, n); // sequential planning pass (record order == RNG order), on the calling thread
     job->outs.assign(outs, outs + outputs.size());
     job->n         = n;
@@ -410,7 +417,7 @@ void aeonb_provider::process(batch_job& job)
     mark(2);
     stage_inputs(B, par); // host work on the pool, uploads
     mark(3);
-    launch_kernels(B, n, par);
+    launch_kernels(B, job.outs.data(), n, par);
     mark(4);
     deliver(B, job.outs.data(), n, on_device, par, T);
     launches = (int32_t)(ctx->launches - launches_before);
@@ -429,7 +436,7 @@ void aeonb_provider::plan_records(batch_plan& B, const void* const* elems, const
     const int nin = (int)stages.size();
     B.out_host.resize(outputs.size());
     for (size_t o = 0; o < outputs.size(); ++o)
-        if (outputs[o].host_produced)
+        if (outputs[o].host_produced && !(outputs[o].anchor_plane && B.anchor_planes_on_device))
             B.out_host[o].assign((size_t)batch_size * outputs[o].shape.byte_size(), 0);
 
     // Parses the headers of one JPEG stream and registers it as a decode job (sizes only; no layout yet).
@@ -1077,12 +1084,75 @@ void aeonb_provider::stage_inputs(batch_plan& B, int par)
 }
 
 // Phase 4: one launch per kernel for the whole batch.
-void aeonb_provider::launch_kernels(batch_plan& B, int n, int par)
+void aeonb_provider::launch_kernels(batch_plan& B, void* const* outs, int n, int par)
 {
     cudaStream_t st     = ctx->stream;
     const int    nin    = (int)stages.size();
     const int    njobs  = (int)B.jobs.size();
     char* const  dstage = static_cast<char*>(staging_dev[par].p);
+    // localization_rcnn first: its kernels need the boxes only, so they run, and the labels are back on the host, while the
+    // pictures are still being decoded on the entropy stream.
+    bool any_labels = false;
+    for (int s = 0; s < nin; ++s)
+    {
+        const stage& sg = stages[s];
+        if (sg.kind == stage_kind::rcnn)
+        {
+            // one launch labels every anchor of every record; labels and best boxes come back for the host's sampling
+            const size_t A = sg.anchors.size();
+            const int    m = (int)B.rcnn[s].size();
+            if (!rcnn_anchor_dev[s].p)
+            {
+                rcnn_anchor_dev[s].reserve(A * sizeof(box4));
+                AEONB_CUDA(cudaMemcpyAsync(rcnn_anchor_dev[s].p, sg.anchors.data(), A * sizeof(box4), cudaMemcpyHostToDevice, st));
+                AEONB_CUDA(cudaStreamSynchronize(st)); // the source is pageable memory owned by the stage
+                h2d_bytes += (int64_t)(A * sizeof(box4));
+            }
+            const size_t per = align_up(A, 16) + align_up(A * sizeof(int16_t), 16); // labels, then best boxes
+            rcnn_result_dev[s].reserve(per * m + 16);
+            rcnn_result_host[s].reserve(per * m + 16);
+            vector<box4>   gt;
+            vector<size_t> first(m);
+            for (int r = 0; r < m; ++r)
+            {
+                first[r] = gt.size();
+                for (const bbox& b : B.rcnn[s][r].gt_boxes)
+                    gt.push_back(box4{b.xmin, b.ymin, b.xmax, b.ymax});
+            }
+            gt.push_back(box4{0, 0, 0, 0}); // never empty
+            const box4* gt_dev = static_cast<const box4*>(ctx->upload(gt.data(), gt.size() * sizeof(box4)));
+            h2d_bytes += (int64_t)(gt.size() * sizeof(box4));
+            vector<aeonb_rcnn_desc> rd(m);
+            for (int r = 0; r < m; ++r)
+            {
+                const rcnn_record& rec = B.rcnn[s][r];
+                char*              out = static_cast<char*>(rcnn_result_dev[s].p) + per * r;
+                rd[r].gt_boxes  = reinterpret_cast<const float*>(gt_dev + first[r]);
+                rd[r].n_gt      = (int32_t)rec.gt_boxes.size();
+                rd[r].im_width  = rec.im_width;
+                rd[r].im_height = rec.im_height;
+                rd[r].labels    = reinterpret_cast<int8_t*>(out);
+                rd[r].best_box  = reinterpret_cast<int16_t*>(out + align_up(A, 16));
+            }
+            check_status(aeonb_rcnn_label_batch(ctx, static_cast<const float*>(rcnn_anchor_dev[s].p), (int32_t)A, rd.data(), m,
+                                                sg.rcnn.negative_overlap, sg.rcnn.positive_overlap));
+            h2d_bytes += (int64_t)(sizeof(aeonb_rcnn_desc) * m);
+            AEONB_CUDA(cudaMemcpyAsync(rcnn_result_host[s].p, rcnn_result_dev[s].p, per * m, cudaMemcpyDeviceToHost, st));
+            d2h_bytes += (int64_t)(per * m);
+        }
+        if (sg.kind == stage_kind::rcnn && B.anchor_planes_on_device)
+        {
+            AEONB_CUDA(launch_rcnn_clear(outs + sg.first_output, sg.anchors.size(), (int)B.rcnn[s].size(), st));
+            ctx->launches++;
+        }
+        any_labels |= sg.kind == stage_kind::rcnn;
+    }
+    if (any_labels)
+    {
+        if (!m_labelled)
+            AEONB_CUDA(cudaEventCreateWithFlags(&m_labelled, cudaEventDisableTiming));
+        AEONB_CUDA(cudaEventRecord(m_labelled, st));
+    }
     // ---- 4. kernels
     B.n_device_jobs = 0;
     if (njobs > 0)
@@ -1393,50 +1463,6 @@ void aeonb_provider::launch_kernels(batch_plan& B, int n, int par)
             check_status(aeonb_image_batch(ctx, B.descs[s].data(), (int)B.descs[s].size(), &L));
             h2d_bytes += (int64_t)(sizeof(aeonb_image_desc) * B.descs[s].size());
         }
-        else if (sg.kind == stage_kind::rcnn)
-        {
-            // one launch labels every anchor of every record; labels and best boxes come back for the host's sampling
-            const size_t A = sg.anchors.size();
-            const int    m = (int)B.rcnn[s].size();
-            if (!rcnn_anchor_dev[s].p)
-            {
-                rcnn_anchor_dev[s].reserve(A * sizeof(box4));
-                AEONB_CUDA(cudaMemcpyAsync(rcnn_anchor_dev[s].p, sg.anchors.data(), A * sizeof(box4), cudaMemcpyHostToDevice, st));
-                AEONB_CUDA(cudaStreamSynchronize(st)); // the source is pageable memory owned by the stage
-                h2d_bytes += (int64_t)(A * sizeof(box4));
-            }
-            const size_t per = align_up(A, 16) + align_up(A * sizeof(int16_t), 16); // labels, then best boxes
-            rcnn_result_dev[s].reserve(per * m + 16);
-            rcnn_result_host[s].reserve(per * m + 16);
-            vector<box4>   gt;
-            vector<size_t> first(m);
-            for (int r = 0; r < m; ++r)
-            {
-                first[r] = gt.size();
-                for (const bbox& b : B.rcnn[s][r].gt_boxes)
-                    gt.push_back(box4{b.xmin, b.ymin, b.xmax, b.ymax});
-            }
-            gt.push_back(box4{0, 0, 0, 0}); // never empty
-            const box4* gt_dev = static_cast<const box4*>(ctx->upload(gt.data(), gt.size() * sizeof(box4)));
-            h2d_bytes += (int64_t)(gt.size() * sizeof(box4));
-            vector<aeonb_rcnn_desc> rd(m);
-            for (int r = 0; r < m; ++r)
-            {
-                const rcnn_record& rec = B.rcnn[s][r];
-                char*              out = static_cast<char*>(rcnn_result_dev[s].p) + per * r;
-                rd[r].gt_boxes  = reinterpret_cast<const float*>(gt_dev + first[r]);
-                rd[r].n_gt      = (int32_t)rec.gt_boxes.size();
-                rd[r].im_width  = rec.im_width;
-                rd[r].im_height = rec.im_height;
-                rd[r].labels    = reinterpret_cast<int8_t*>(out);
-                rd[r].best_box  = reinterpret_cast<int16_t*>(out + align_up(A, 16));
-            }
-            check_status(aeonb_rcnn_label_batch(ctx, static_cast<const float*>(rcnn_anchor_dev[s].p), (int32_t)A, rd.data(), m,
-                                                sg.rcnn.negative_overlap, sg.rcnn.positive_overlap));
-            h2d_bytes += (int64_t)(sizeof(aeonb_rcnn_desc) * m);
-            AEONB_CUDA(cudaMemcpyAsync(rcnn_result_host[s].p, rcnn_result_dev[s].p, per * m, cudaMemcpyDeviceToHost, st));
-            d2h_bytes += (int64_t)(per * m);
-        }
         else if (sg.kind == stage_kind::audio)
         {
             const int             o = sg.first_output;
@@ -1464,15 +1490,16 @@ void aeonb_provider::deliver(batch_plan& B, void* const* outs, int n, bool on_de
     cudaStream_t st = ctx->stream;
     // ---- 5. deliver
     // localization_rcnn: the labels of the GPU pass are needed on the host now -- sampling draws from them and the ten
-    // buffers are filled from the sample -- so a batch with such a stage waits for its kernels here.
+    // buffers are filled from the sample -- so a batch with such a stage waits for its labels here.
     for (size_t s = 0; s < stages.size(); ++s)
     {
         const stage& sg = stages[s];
         if (sg.kind != stage_kind::rcnn)
             continue;
-        AEONB_CUDA(cudaStreamSynchronize(st));
-        const size_t A   = sg.anchors.size();
-        const size_t per = align_up(A, 16) + align_up(A * sizeof(int16_t), 16);
+        AEONB_CUDA(cudaEventSynchronize(m_labelled));
+        const size_t        A   = sg.anchors.size();
+        const size_t        per = align_up(A, 16) + align_up(A * sizeof(int16_t), 16);
+        vector<rcnn_target> targets;
         for (size_t r = 0; r < B.rcnn[s].size(); ++r)
         {
             const char*    res    = static_cast<const char*>(rcnn_result_host[s].p) + per * r;
@@ -1481,9 +1508,20 @@ void aeonb_provider::deliver(batch_plan& B, void* const* outs, int n, bool on_de
             const vector<int> sampled = rcnn_sample_anchors(labels, (int)A, sg.rcnn.rois_per_image, sg.rcnn.foreground_fraction,
                                                             sg.rcnn.deterministic_sampling ? nullptr : &rcnn_engine);
             void* bufs[10];
-            for (int k = 0; k < 10; ++k)
+            for (int k = B.anchor_planes_on_device ? RCNN_PLANES : 0; k < 10; ++k)
                 bufs[k] = B.out_host[sg.first_output + k].data() + r * (size_t)outputs[sg.first_output + k].shape.byte_size();
-            rcnn_load(sg.rcnn, sg.anchors, B.rcnn[s][r], labels, best, sampled, bufs);
+            const size_t first = targets.size();
+            rcnn_targets((int)r, sg.anchors, B.rcnn[s][r], labels, best, sampled, targets);
+            if (!B.anchor_planes_on_device)
+                rcnn_load_planes(A, targets.data() + first, targets.size() - first, bufs);
+            rcnn_load_boxes(sg.rcnn, B.rcnn[s][r], bufs);
+        }
+        if (B.anchor_planes_on_device && !targets.empty())
+        {
+            const auto* dev = static_cast<const rcnn_target*>(ctx->upload(targets.data(), targets.size() * sizeof(rcnn_target)));
+            AEONB_CUDA(launch_rcnn_scatter(outs + sg.first_output, A, dev, targets.size(), st));
+            ctx->launches++;
+            h2d_bytes += (int64_t)(targets.size() * sizeof(rcnn_target));
         }
     }
     size_t small_total = 0;
@@ -1499,7 +1537,7 @@ void aeonb_provider::deliver(batch_plan& B, void* const* outs, int n, bool on_de
         const size_t  rec   = (size_t)outputs[o].shape.byte_size();
         const int     esz   = (int)outputs[o].shape.otype.size;
         const int64_t elems_per_rec = outputs[o].shape.element_count();
-        if (outputs[o].host_produced)
+        if (outputs[o].host_produced && !(outputs[o].anchor_plane && B.anchor_planes_on_device))
         {
             vector<char>  tmp;
             const char*   src = B.out_host[o].data();

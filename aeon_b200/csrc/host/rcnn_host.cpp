@@ -86,11 +86,13 @@ namespace aeonb
     {
         const int        num_fg = (int)(foreground_fraction * (float)rois_per_image);
         std::vector<int> fg, bg;
-        for (int i = 0; i < n_anchors; ++i)
+        // in index order no more than this of either kind are ever taken; a shuffle draws from all of them
+        const size_t most = engine ? (size_t)n_anchors : (size_t)std::max({rois_per_image, num_fg, 0}) + 1;
+        for (int i = 0; i < n_anchors && (fg.size() < most || bg.size() < most); ++i)
         {
             if (labels[i] >= 1)
                 fg.push_back(i);
-            else if (labels[i] == 0)
+            else if (labels[i] == 0 && bg.size() < most)
                 bg.push_back(i);
         }
         if (engine)
@@ -107,28 +109,37 @@ namespace aeonb
         return fg;
     }
 
-    void rcnn_load(const rcnn_config& cfg, const std::vector<box4>& anchors, const rcnn_record& rec, const int8_t* labels,
-                   const int16_t* best_box, const std::vector<int>& sampled, void* const bufs[10])
+    void rcnn_targets(int record, const std::vector<box4>& anchors, const rcnn_record& rec, const int8_t* labels, const int16_t* best_box,
+                      const std::vector<int>& sampled, std::vector<rcnn_target>& out)
     {
-        const size_t A = anchors.size();
+        for (int index : sampled)
+        {
+            // compute_targets (:265-300) against the box this anchor overlaps most
+            const bbox& gt = rec.gt_boxes[best_box[index]];
+            const box4& rp = anchors[index];
+            const float rw = extent(rp.xmin, rp.xmax), rh = extent(rp.ymin, rp.ymax);
+            out.push_back(rcnn_target{record, index, labels[index] == 1, 0,
+                                      {(centre(gt.xmin, gt.xmax) - centre(rp.xmin, rp.xmax)) / rw,
+                                       (centre(gt.ymin, gt.ymax) - centre(rp.ymin, rp.ymax)) / rh, std::log(extent(gt.xmin, gt.xmax) / rw),
+                                       std::log(extent(gt.ymin, gt.ymax) / rh)}});
+        }
+    }
+
+    void rcnn_load_planes(size_t A, const rcnn_target* targets, size_t n, void* const bufs[RCNN_PLANES])
+    {
         float*   bbtargets      = static_cast<float*>(bufs[0]);
         float*   bbtargets_mask = static_cast<float*>(bufs[1]);
         int32_t* labels_flat    = static_cast<int32_t*>(bufs[2]);
         int32_t* labels_mask    = static_cast<int32_t*>(bufs[3]);
-        int32_t* im_shape       = static_cast<int32_t*>(bufs[4]);
-        float*   gt_boxes       = static_cast<float*>(bufs[5]);
-        int32_t* num_gt_boxes   = static_cast<int32_t*>(bufs[6]);
-        int32_t* gt_classes     = static_cast<int32_t*>(bufs[7]);
-        float*   im_scale       = static_cast<float*>(bufs[8]);
-        int32_t* gt_difficult   = static_cast<int32_t*>(bufs[9]);
         std::memset(bbtargets, 0, 4 * A * sizeof(float));
         std::memset(bbtargets_mask, 0, 4 * A * sizeof(float));
         std::fill(labels_flat, labels_flat + A, 1);
         std::fill(labels_flat + A, labels_flat + 2 * A, 0);
         std::memset(labels_mask, 0, 2 * A * sizeof(int32_t));
-        for (int index : sampled)
+        for (const rcnn_target* t = targets; t < targets + n; ++t)
         {
-            if (labels[index] == 1)
+            const size_t index = (size_t)t->anchor;
+            if (t->positive)
             {
                 labels_flat[index]     = 0;
                 labels_flat[index + A] = 1;
@@ -137,15 +148,19 @@ namespace aeonb
             }
             labels_mask[index]     = 1;
             labels_mask[index + A] = 1;
-            // compute_targets (:265-300) against the box this anchor overlaps most
-            const bbox& gt = rec.gt_boxes[best_box[index]];
-            const box4& rp = anchors[index];
-            const float rw = extent(rp.xmin, rp.xmax), rh = extent(rp.ymin, rp.ymax);
-            bbtargets[index + A * 0] = (centre(gt.xmin, gt.xmax) - centre(rp.xmin, rp.xmax)) / rw;
-            bbtargets[index + A * 1] = (centre(gt.ymin, gt.ymax) - centre(rp.ymin, rp.ymax)) / rh;
-            bbtargets[index + A * 2] = std::log(extent(gt.xmin, gt.xmax) / rw);
-            bbtargets[index + A * 3] = std::log(extent(gt.ymin, gt.ymax) / rh);
+            for (int k = 0; k < 4; ++k)
+                bbtargets[index + A * k] = t->target[k];
         }
+    }
+
+    void rcnn_load_boxes(const rcnn_config& cfg, const rcnn_record& rec, void* const bufs[10])
+    {
+        int32_t* im_shape     = static_cast<int32_t*>(bufs[4]);
+        float*   gt_boxes     = static_cast<float*>(bufs[5]);
+        int32_t* num_gt_boxes = static_cast<int32_t*>(bufs[6]);
+        int32_t* gt_classes   = static_cast<int32_t*>(bufs[7]);
+        float*   im_scale     = static_cast<float*>(bufs[8]);
+        int32_t* gt_difficult = static_cast<int32_t*>(bufs[9]);
         im_shape[0]   = rec.im_width;
         im_shape[1]   = rec.im_height;
         *num_gt_boxes = std::min<int>(cfg.max_gt_boxes, (int)rec.gt_boxes.size());

@@ -2,6 +2,8 @@
 // the GPU labelling pass -- anchor sampling, the regression targets of the sampled anchors and the ten output buffers.
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 #include <random>
 #include <string>
@@ -58,8 +60,22 @@ namespace aeonb
     std::vector<int> rcnn_sample_anchors(const int8_t* labels, int n_anchors, int rois_per_image, float foreground_fraction,
                                          random_engine_t* engine);
 
-    // loader::load (:340-432) into the ten buffers of one record; the regression targets (compute_targets, :265-300) are
-    // formed here for the sampled anchors only, each against the box the GPU pass found best for it.
-    void rcnn_load(const rcnn_config& cfg, const std::vector<box4>& anchors, const rcnn_record& rec, const int8_t* labels,
-                   const int16_t* best_box, const std::vector<int>& sampled, void* const bufs[10]);
+    // A sampled anchor: its regression targets (compute_targets, :265-300) against the box the GPU pass found best for it.
+    struct alignas(16) rcnn_target
+    {
+        int32_t record, anchor, positive, reserved;
+        float   target[4];
+    };
+    void rcnn_targets(int record, const std::vector<box4>& anchors, const rcnn_record& rec, const int8_t* labels, const int16_t* best_box,
+                      const std::vector<int>& sampled, std::vector<rcnn_target>& out);
+
+    // loader::load (:340-432): the first four buffers of a record (targets, their mask, labels, their mask: a value or four per
+    // anchor, of which only the sampled anchors' differ from the fill), and the other six.
+    constexpr int RCNN_PLANES = 4;
+    void rcnn_load_planes(size_t n_anchors, const rcnn_target* targets, size_t n, void* const bufs[RCNN_PLANES]);
+    void rcnn_load_boxes(const rcnn_config& cfg, const rcnn_record& rec, void* const bufs[10]);
+
+    // The same planes of a whole batch in device memory, record after record: the fill, then the sampled anchors.
+    cudaError_t launch_rcnn_clear(void* const planes[RCNN_PLANES], size_t n_anchors, int records, cudaStream_t stream);
+    cudaError_t launch_rcnn_scatter(void* const planes[RCNN_PLANES], size_t n_anchors, const rcnn_target* targets_dev, size_t n, cudaStream_t stream);
 }
