@@ -472,35 +472,35 @@ namespace aeonb
         // the same: there a chain of segments is settled one round per segment, which is what the slowest streams
         // of a batch spend their time on (5 rounds on average, 11 at most).  Tried and no faster: warming up on the
         // tail of the left neighbour's segment before the guess.
-        constexpr int PLOOK = 12; // bits of the lookup window
-        // One 16-bit lookup gives everything the symbol loop needs:
-        //   bits 0-4  total bits the symbol takes (code + value bits)     bits 5-8  number of value bits (AC size / DC category)
-        //   bits 9-15 advance of the zig-zag index: run + 1, 16 for ZRL, 64 for end of block, 1 for a DC category,
-        //             127 for an invalid code (which still takes bits and ends the block, so that a decoder in a wrong state moves on)
-        // 0 = the code is longer than the window.
+        constexpr int AC_BITS = 11; // bits of the lookup window: AC tables (12: 28 us slower for 256 streams, fewer of which then fit shared memory)
+        constexpr int DC_BITS = 9;  //                            DC tables (few, short codes)
+        // One 32-bit lookup gives everything the symbol loop needs:
+        //   bits 0-4   total bits the symbol takes (code + value bits)     bits 5-8  number of value bits (AC size / DC category)
+        //   bits 24-31 advance of the zig-zag index: run + 1, 16 for ZRL, 64 for end of block, 1 for a DC category,
+        //              127 for an invalid code (which still takes bits and ends the block, so that a decoder in a wrong state moves on)
+        // 0 = the code is longer than the window.  Without the value bits the entry is what the decoder's state -- bit position in
+        // bits 0-23, zig-zag index in bits 24-31 -- advances by, in one addition.
+        constexpr uint32_t k_advance = 0xff00001fu, k_position = 0x00ffffffu, k_block_end = 64u << 24;
         __device__ __forceinline__ uint32_t pack_symbol(int len, int sym, bool is_ac)
         {
             const int s = sym & 15, r = sym >> 4;
             const int kinc = is_ac ? (s ? r + 1 : (r == 15 ? 16 : 64)) : (r == 0 ? 1 : 127);
-            return (uint32_t)(len + s) | (uint32_t)s << 5 | (uint32_t)kinc << 9;
+            return (uint32_t)(len + s) | (uint32_t)s << 5 | (uint32_t)kinc << 24;
         }
-        constexpr uint32_t k_invalid_symbol = 16u | 127u << 9;
+        constexpr uint32_t k_invalid_symbol = 16u | 127u << 24;
 
-        struct par_table
+        struct code_table
         {
-            alignas(16) uint16_t lookup[1 << PLOOK];
-            int      limit[17]; // limit[len]: exclusive upper bound of the codes of length <= len, left-justified to 16 bits
-            int      valoff[17];
-            uint8_t  vals[256];
-            int      is_ac;
+            int     limit[17]; // limit[len]: exclusive upper bound of the codes of length <= len, left-justified to 16 bits
+            int     valoff[17];
+            uint8_t vals[256];
         };
 
         // One thread fills the canonical-code limits of a table from the DHT form (16 counts); the values are copied by the caller.
-        __device__ void build_par_table_head(par_table& T, const uint8_t* __restrict__ dht, bool is_ac, int* bad)
+        __device__ void build_code_table(code_table& T, const uint8_t* __restrict__ dht, int* bad)
         {
             int code = 0, k = 0;
             T.limit[0] = 0;
-            T.is_ac    = is_ac;
             for (int len = 1; len <= 16; ++len)
             {
                 const int n   = dht[len - 1];
@@ -513,80 +513,90 @@ namespace aeonb
                 code <<= 1;
             }
         }
-        // One entry of the lookup window: the symbol whose code heads the window's bits `i`.
-        __device__ __forceinline__ int window_length(const par_table& T, int i16)
+        // Length of the code at the head of the 16 bits c16, if it is no longer than `bits`.
+        __device__ __forceinline__ int code_length(const code_table& T, int c16, int bits)
         {
             int len = 1;
 #pragma unroll
-            for (int l = 1; l < PLOOK; ++l)
-                len += i16 >= T.limit[l];
+            for (int l = 1; l < AC_BITS; ++l)
+                len += l < bits && c16 >= T.limit[l];
             return len;
         }
-        __device__ __forceinline__ uint32_t window_entry(const par_table& T, int i, int len)
+        __device__ __forceinline__ uint32_t window_entry(const code_table& T, int i, int len, int bits, bool is_ac)
         {
-            if ((i << (16 - PLOOK)) >= T.limit[len])
+            if ((i << (16 - bits)) >= T.limit[len])
                 return 0;
-            return pack_symbol(len, T.vals[((i >> (PLOOK - len)) + T.valoff[len]) & 255], T.is_ac != 0);
+            return pack_symbol(len, T.vals[((i >> (bits - len)) + T.valoff[len]) & 255], is_ac);
         }
-        // `nth` threads (index `tid`) fill the lookup windows of all four tables once limits and values are in place.  Eight
-        // neighbouring entries go together: unless a code of the last three lengths starts among them they hold one symbol, so
-        // the length is searched twice per eight entries and one 16-byte store does.
-        __device__ void build_par_tables(par_table* tab, int tid, int nth)
+        // `nth` threads (index `tid`) fill the four lookup windows once limits and values are in place.  Eight neighbouring entries
+        // go together: unless a code of the last three lengths starts among them they hold one symbol, so the length is searched
+        // twice per eight entries.
+        __device__ void build_windows(uint32_t* ac, uint32_t* dc, const code_table* codes, int tid, int nth)
         {
-            constexpr int groups = (1 << PLOOK) / 8;
-            for (int j = tid; j < 4 * groups; j += nth)
+            constexpr int ac8 = (1 << AC_BITS) / 8, dc8 = (1 << DC_BITS) / 8;
+            for (int j = tid; j < 2 * (ac8 + dc8); j += nth)
             {
-                const int  i = j % groups * 8;
-                par_table& T = tab[j / groups];
-                const int  first = window_length(T, i << (16 - PLOOK)), last = window_length(T, (i + 7) << (16 - PLOOK));
-                if (first == last && first <= PLOOK - 3)
+                const bool        is_ac = j < 2 * ac8;
+                const int         slot = is_ac ? j / ac8 : (j - 2 * ac8) / dc8, i = (is_ac ? j % ac8 : (j - 2 * ac8) % dc8) * 8;
+                const int         bits = is_ac ? AC_BITS : DC_BITS;
+                const code_table& T    = codes[is_ac ? 2 + slot : slot];
+                uint32_t* const   out  = (is_ac ? ac + (slot << AC_BITS) : dc + (slot << DC_BITS)) + i;
+                const int first = code_length(T, i << (16 - bits), bits), last = code_length(T, (i + 7) << (16 - bits), bits);
+                if (first == last && first <= bits - 3)
                 {
-                    const uint32_t e = window_entry(T, i, first) * 0x10001u;
-                    *reinterpret_cast<uint4*>(&T.lookup[i]) = make_uint4(e, e, e, e);
+                    const uint32_t e = window_entry(T, i, first, bits, is_ac);
+                    reinterpret_cast<uint4*>(out)[0] = make_uint4(e, e, e, e);
+                    reinterpret_cast<uint4*>(out)[1] = make_uint4(e, e, e, e);
                 }
                 else
                 {
 #pragma unroll 1
                     for (int k = 0; k < 8; ++k)
-                        T.lookup[i + k] = (uint16_t)window_entry(T, i + k, window_length(T, (i + k) << (16 - PLOOK)));
+                        out[k] = window_entry(T, i + k, code_length(T, (i + k) << (16 - bits), bits), bits, is_ac);
                 }
             }
         }
         // A code longer than the window, or an invalid one.
-        __device__ __noinline__ uint32_t long_symbol(const par_table& T, uint32_t h)
+        __device__ __noinline__ uint32_t long_symbol(const code_table& T, uint32_t h, bool is_ac)
         {
             const int c16 = (int)(h >> 16);
             if (c16 >= T.limit[16])
                 return k_invalid_symbol;
-            int len = PLOOK + 1;
+            int len = 1;
 #pragma unroll
-            for (int l = PLOOK + 1; l < 16; ++l)
+            for (int l = 1; l < 16; ++l)
                 len += c16 >= T.limit[l];
-            return pack_symbol(len, T.vals[((c16 >> (16 - len)) + T.valoff[len]) & 255], T.is_ac != 0);
+            return pack_symbol(len, T.vals[((c16 >> (16 - len)) + T.valoff[len]) & 255], is_ac);
         }
 
         constexpr int PAR_THREADS = 512;  // most threads (= segments) a stream can have; the launch picks the actual number
         constexpr int NCHECK      = 3;    // checkpoints inside a segment (7 measured the same; 3 leaves room for a third kernel's CTA on the SM)
 
-        // Where the blocks of one place in an MCU go: base + (mcu row - first row) * dy + (mcu column - first column) * dx
+        // Where the blocks of one place in an MCU go: base + 64 * ((mcu row - first row) * dy + (mcu column - first column) * dx)
         struct alignas(16) block_place
         {
             int16_t* base;
-            int64_t  dy;
-            int32_t  dx;
+            int32_t  dy, dx;
+        };
+        // What the symbol loop wants to know of a block of an MCU, in one 16-byte load: the shared-memory addresses of its AC window,
+        // of the next block's DC window and of the next block's link.
+        struct alignas(16) block_link
+        {
+            uint32_t ac, next_dc, next, block;
         };
 
         struct par_state
         {
-            par_table  tab[4]; // DC slot 0, DC slot 1, AC slot 0, AC slot 1
-            uint8_t    dht[4 * 272]; // the tables as they came
-            uint32_t   warp_sums[3][32];
-            uint8_t    zz[64];
-            block_place place[16];               // per block of an MCU: its place, its component
-            uint8_t    comp[16];
+            uint32_t    ac_window[2][1 << AC_BITS], dc_window[2][1 << DC_BITS];
+            code_table  codes[4]; // DC slot 0, DC slot 1, AC slot 0, AC slot 1
+            uint8_t     dht[4 * 272]; // the tables as they came
+            uint32_t    warp_sums[3][32];
+            uint8_t     zz[64];
+            block_place place[16];               // per block of an MCU
+            block_link  link[16];
+            uint8_t     comp[16];
             aeonb_entropy_desc d;
             int        bpm;                      // blocks per MCU
-            uint32_t   dc_slots, ac_slots;       // bit b: the table slot of block b of an MCU
             int        bad;
             uint32_t   marker_at;                // first marker byte in the raw scan (or its size)
             uint32_t   tile_end[2];              // last byte of an even / odd tile of the raw scan
@@ -607,11 +617,19 @@ namespace aeonb
             return seg_arrays{w, w + T, w + 2 * T, w + 3 * T, h, h + T};
         }
 
-        __device__ __forceinline__ uint32_t lds_u16(uint32_t addr)
+        __device__ __forceinline__ uint32_t shared_address(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+        __device__ __forceinline__ uint32_t lds_u32(uint32_t addr)
         {
-            uint16_t v;
-            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+            uint32_t v;
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
             return v;
+        }
+        // link = the link at its `next` where `yes`
+        __device__ __forceinline__ void follow_if(block_link& link, bool yes)
+        {
+            asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %4, 0;\n\t@q ld.shared.v4.u32 {%0, %1, %2, %3}, [%2];\n\t}"
+                         : "+r"(link.ac), "+r"(link.next_dc), "+r"(link.next), "+r"(link.block)
+                         : "r"((uint32_t)yes));
         }
 
         // Words of the copy of a stream, from shared or from global memory.  `next_if` replaces `value` by the next word where
@@ -658,7 +676,7 @@ namespace aeonb
             if (my < d.roi[1] || my >= d.roi[3] || mx < d.roi[0] || mx >= d.roi[2])
                 return nullptr;
             const block_place& at = S.place[b];
-            return at.base + (my - d.roi[1]) * at.dy + (mx - d.roi[0]) * at.dx;
+            return at.base + (int64_t)((my - d.roi[1]) * at.dy + (mx - d.roi[0]) * at.dx) * 64;
         }
 
         struct seg_result
@@ -695,7 +713,7 @@ namespace aeonb
             int16_t* out  = nullptr;
             auto     home = [&]() -> int16_t* {
                 const block_place& at = S.place[b];
-                return (uint32_t)mx < roi_w && (uint32_t)my < roi_h ? at.base + my * at.dy + mx * at.dx : nullptr;
+                return (uint32_t)mx < roi_w && (uint32_t)my < roi_h ? at.base + (int64_t)(my * at.dy + mx * at.dx) * 64 : nullptr;
             };
             if (WRITE)
             {
@@ -714,11 +732,12 @@ namespace aeonb
             }
             // The lookup window of the next symbol: the AC one of this block, or after the block's last symbol the DC one of the
             // next.  Both are at hand before the symbol is known, so that only a select hangs on it.
-            const uint32_t windows = (uint32_t)__cvta_generic_to_shared(S.tab[0].lookup), dc_slots = S.dc_slots, ac_slots = S.ac_slots;
-            auto           dc_of   = [&](int blk) { return windows + (dc_slots >> blk & 1) * (uint32_t)sizeof(par_table); };
-            auto           ac_of   = [&](int blk) { return windows + (2 + (ac_slots >> blk & 1)) * (uint32_t)sizeof(par_table); };
-            int            bn      = b + 1 == bpm ? 0 : b + 1;
-            uint32_t       ac_look = ac_of(b), next_dc = dc_of(bn), look = k == 0 ? dc_of(b) : ac_look;
+            block_link link = S.link[b];
+            uint32_t   look = k == 0 ? S.link[b ? b - 1 : bpm - 1].next_dc : link.ac, shift = k == 0 ? 32 - DC_BITS : 32 - AC_BITS;
+            // Bit positions count from the word that the run starts in; `at` is the state (see k_advance).
+            const uint32_t base = p & ~31u;
+            uint32_t       at   = (p - base) | (uint32_t)k << 24;
+            pend                = pend > base ? pend - base : 0;
             // checkpoints: `slot` walks down this thread's column (state; the blocks so far NCHECK rows further on); `old_key` is
             // the state an earlier run noted at the next checkpoint (no state has all bits set)
             const uint32_t rows    = NCHECK * check_stride;
@@ -726,50 +745,51 @@ namespace aeonb
             uint32_t       old_key = !WRITE && compare ? chk[0] : 0xffffffffu;
             // A checkpoint at or past the segment's end is never taken: a run can step over it with its last symbol or stop short
             // of it, so what is noted there could be left from an older run than the one whose block count goes with it.
+            check_at -= base;
             uint32_t stop = WRITE || check_at >= pend ? pend : check_at;
-            // The 32 bits under p lie in w0 and w1; w2 is the word behind them, fetched when the one before it comes into use.
+            // The 32 bits under the position lie in w0 and w1; w2 is the word behind them, fetched when the one before it comes into use.
             Words    ahead(words, p >> 5);
             uint32_t w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
             for (;;)
             {
-                while (p < stop)
+                while ((at & k_position) < stop)
                 {
-                    const uint32_t h = __funnelshift_l(w1, w0, p); // 32 valid bits; a symbol takes at most 31
-                    uint32_t       e = lds_u16(look + ((h >> (32 - PLOOK)) << 1));
+                    const uint32_t h = __funnelshift_l(w1, w0, at); // 32 valid bits; a symbol takes at most 31
+                    uint32_t       e = lds_u32(look + ((h >> shift) << 2));
                     if (!e)
-                        e = long_symbol(S.tab[k == 0 ? dc_slots >> b & 1 : 2 + (ac_slots >> b & 1)], h);
-                    const int tot = e & 31, kinc = e >> 9;
+                    {
+                        const bool is_ac = at > k_position;
+                        e = long_symbol(is_ac ? S.codes[look == shared_address(S.ac_window[0]) ? 2 : 3] : S.codes[look == shared_address(S.dc_window[0]) ? 0 : 1],
+                                        h, is_ac);
+                    }
+                    const uint32_t to    = at + (e & k_advance);
+                    const uint32_t cross = (at ^ to) & 32; // the read position has left w0
                     if (WRITE)
                     {
-                        const int      sz = (e >> 5) & 15, kk = k + kinc - 1; // value bits and position of this coefficient
-                        const uint32_t x  = h << (tot - sz);                  // the value bits at the top
-                        const int      v  = (int)__funnelshift_l(x, 0u, sz) + ((int)x >= 0 ? 1 - (1 << sz) : 0);
+                        const int      tot = e & 31, sz = (e >> 5) & 15, kk = (int)((at >> 24) + (e >> 24)) - 1; // kk: the coefficient's place
+                        const uint32_t x   = h << (tot - sz);                                                   // the value bits at the top
+                        const int      v   = (int)__funnelshift_l(x, 0u, sz) + ((int)x >= 0 ? 1 - (1 << sz) : 0);
                         // an invalid code, a DC symbol that is no category, or a run that leaves the block
-                        bad |= kinc == 127 || (sz && kk > 63);
-                        if (k == 0)
+                        bad |= e >= 127u << 24 || (sz && kk > 63);
+                        if (at <= k_position)
                             dcdiff[g] = (int16_t)v;
                         else if (sz && kk <= 63 && out)
                             out[S.zz[kk]] = (int16_t)v;
                     }
-                    const uint32_t q     = p + tot;
-                    const uint32_t cross = (p ^ q) & 32; // the read position has left w0
-                    p                    = q;
-                    w0                   = cross ? w1 : w0;
-                    w1                   = cross ? w2 : w1;
+                    w0 = cross ? w1 : w0;
+                    w1 = cross ? w2 : w1;
                     ahead.next_if(w2, cross);
-                    k += kinc;
-                    const bool end = k >= 64;
-                    look           = end ? next_dc : ac_look;
-                    k              = end ? 0 : k;
-                    b              = end ? bn : b;
+                    const bool end = to >= k_block_end;
+                    look           = end ? link.next_dc : link.ac;
+                    shift          = end ? 32 - DC_BITS : 32 - AC_BITS;
+                    at             = end ? to & k_position : to;
                     blocks += end;
-                    bn      = b + 1 == bpm ? 0 : b + 1;
-                    ac_look = ac_of(b);
-                    next_dc = dc_of(bn);
+                    follow_if(link, end);
                     if (WRITE && end)
                     {
                         if (++g >= gend)
                             break;
+                        b = (int)link.block;
                         if (b == 0 && ++mx == mx_end)
                         {
                             mx = mx_first;
@@ -781,7 +801,7 @@ namespace aeonb
                 if (WRITE || stop == pend)
                     break;
                 // a checkpoint
-                const uint32_t key = (p - stop) << 10 | (uint32_t)b << 6 | (uint32_t)k; // p - stop <= 30
+                const uint32_t key = ((at & k_position) - stop) << 10 | link.block << 6 | at >> 24; // position - stop <= 30
                 if (key == old_key)
                 {
                     // in step with the earlier run: its blocks from here on are this run's too
@@ -799,9 +819,9 @@ namespace aeonb
                 old_key         = more && compare ? slot[0] : 0xffffffffu; // fetched now, wanted at the next checkpoint
                 stop            = more ? stop + check_step : pend;
             }
-            R.p      = p;
-            R.b      = b;
-            R.k      = k;
+            R.p      = base + (at & k_position);
+            R.b      = (int)link.block;
+            R.k      = (int)(at >> 24);
             R.blocks = blocks;
             R.bad    = bad;
             return R;
@@ -905,38 +925,41 @@ namespace aeonb
             const aeonb_entropy_desc& d = S.d;
             if (tid == 0)
             {
-                int      b        = 0;
-                uint32_t dc_slots = 0, ac_slots = 0;
+                int b = 0;
                 for (int c = 0; c < d.ncomp; ++c)
                 {
                     const int64_t row_blocks = (int64_t)(d.roi[2] - d.roi[0]) * d.hs[c]; // blocks in a row of the compact plane
                     for (int y = 0; y < d.vs[c]; ++y)
                         for (int x = 0; x < d.hs[c]; ++x, ++b)
                         {
-                            S.comp[b] = (uint8_t)c;
-                            dc_slots |= (uint32_t)(d.dc_table[c] & 1) << b;
-                            ac_slots |= (uint32_t)(d.ac_table[c] & 1) << b;
+                            S.comp[b]       = (uint8_t)c;
+                            S.link[b].ac    = shared_address(S.ac_window[d.ac_table[c] & 1]);
+                            S.link[b].block = (uint32_t)b;
                             S.place[b].base = d.coef[c] + (y * row_blocks + x) * 64;
-                            S.place[b].dy   = d.vs[c] * row_blocks * 64;
-                            S.place[b].dx   = d.hs[c] * 64;
+                            S.place[b].dy   = (int32_t)(d.vs[c] * row_blocks);
+                            S.place[b].dx   = d.hs[c];
                         }
                 }
-                S.bpm       = b;
-                S.dc_slots  = dc_slots;
-                S.ac_slots  = ac_slots;
+                S.bpm = b;
             }
             // The tables in DHT form are brought in whole: the head of a table is a chain over its 16 code counts, which one
             // thread walks from shared memory rather than from L2.
             for (int i = tid; i < 4 * 272; i += nth)
                 S.dht[i] = __ldg(d.tables + i);
             __syncthreads();
+            if (tid < S.bpm)
+            {
+                const int next       = tid + 1 < S.bpm ? tid + 1 : 0;
+                S.link[tid].next_dc = shared_address(S.dc_window[d.dc_table[S.comp[next]] & 1]);
+                S.link[tid].next    = shared_address(&S.link[next]);
+            }
             if ((tid & 31) == 0)
                 for (int t = tid >> 5; t < 4; t += nth >> 5)
-                    build_par_table_head(S.tab[t], S.dht + t * 272, t >= 2, &S.bad);
+                    build_code_table(S.codes[t], S.dht + t * 272, &S.bad);
             for (int i = tid; i < 4 * 256; i += nth)
-                S.tab[i >> 8].vals[i & 255] = S.dht[(i >> 8) * 272 + 16 + (i & 255)];
+                S.codes[i >> 8].vals[i & 255] = S.dht[(i >> 8) * 272 + 16 + (i & 255)];
             __syncthreads();
-            build_par_tables(S.tab, tid, nth);
+            build_windows(S.ac_window[0], S.dc_window[0], S.codes, tid, nth);
             __syncthreads();
         }
 
@@ -1281,7 +1304,7 @@ namespace aeonb
         // with these.  A part of 4 to 16 KB per block fills the chip (about 20 parts per picture) and keeps segments at 160 bytes.
         constexpr int RST_THREADS       = 128;
         constexpr int RST_INDEX_THREADS = 1024;
-        constexpr int RST_ROOM          = 12 * 1024 + 512; // shared memory for a part's bytes (see jpeg_restart_parts): 4 blocks fit an SM
+        constexpr int RST_ROOM          = 12 * 1024 + 512; // shared memory for a part's bytes (see jpeg_restart_parts): 5 blocks fit an SM
 
         struct rst_state
         {
@@ -1304,7 +1327,7 @@ namespace aeonb
             for (int c = 0; c < 3; ++c)
                 if (c < d.ncomp)
                     bpm += d.hs[c] * d.vs[c];
-            return d.ncomp >= 1 && d.ncomp <= 3 && d.mcux > 0 && d.mcuy > 0 && d.scan && d.tables && bpm <= 16 && d.scan_size < (1u << 27) &&
+            return d.ncomp >= 1 && d.ncomp <= 3 && d.mcux > 0 && d.mcuy > 0 && d.scan && d.tables && bpm <= 16 && d.scan_size < (1u << 26) &&
                    (uint64_t)d.mcux * d.mcuy * bpm < (1ull << 30) && d.scratch_bytes >= w.bytes && (reinterpret_cast<uintptr_t>(d.scratch) & 15) == 0;
         }
 
@@ -1698,7 +1721,7 @@ namespace aeonb
             int v = 512;
             if (const char* e = std::getenv("AEONB_ENTROPY_THREADS"))
                 v = std::atoi(e);
-            v = v < 64 ? 64 : v > PAR_THREADS ? PAR_THREADS : v;
+            v = v < 128 ? 128 : v > PAR_THREADS ? PAR_THREADS : v;
             return v & ~31;
         }();
         return value;
@@ -1723,9 +1746,9 @@ namespace aeonb
                 total += descs[i].scan_size;
         if (total == 0)
             return;
-        // Four blocks of a part fit an SM; parts of less than 4 KB are mostly set-up, parts of more than 12 KB do not fit its
+        // Five blocks of a part fit an SM; parts of less than 4 KB are mostly set-up, parts of more than 12 KB do not fit its
         // shared memory.
-        const uint64_t target = std::min<uint64_t>(std::max<uint64_t>(total / (148 * 4), 4096), 10240);
+        const uint64_t target = std::min<uint64_t>(std::max<uint64_t>(total / (148 * 5), 4096), 10240);
         for (int i = 0; i < n; ++i)
         {
             const aeonb_entropy_desc& d = descs[i];
@@ -1762,7 +1785,7 @@ namespace aeonb
             return cudaSuccess;
         if (any_parallel)
         {
-            threads           = std::min(std::max(threads, 64), jpeg_entropy_threads()) & ~31;
+            threads           = std::min(std::max(threads, 128), jpeg_entropy_threads()) & ~31;
             const size_t smem = jpeg_entropy_smem(n, threads, longest, most_blocks);
             cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_parallel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (err != cudaSuccess)
