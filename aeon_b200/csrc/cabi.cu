@@ -518,7 +518,6 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
                     bytes += (int64_t)(r.roi[2] - r.roi[0]) * r.hs[c] * (r.roi[3] - r.roi[1]) * r.vs[c] * 128;
             }
         launch_timer timer(ctx, AEONB_KERNEL_ENTROPY, bytes);
-        // A launch of short streams (video frames) takes smaller blocks: its streams have few segments, and more blocks fit an SM.
         uint32_t longest     = 0;
         uint64_t most_blocks = 0;
         for (int i = 0; i < n; ++i)
@@ -530,11 +529,7 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
                 longest     = std::max(longest, descs[i].scan_size);
                 most_blocks = std::max(most_blocks, bpm * descs[i].mcux * descs[i].roi[3]);
             }
-        const int segments = (int)((longest + (uint32_t)jpeg_entropy_min_segment() - 1) / (uint32_t)jpeg_entropy_min_segment());
-        int       threads  = jpeg_entropy_threads();
-        while (threads > 128 && segments <= threads / 2)
-            threads /= 2;
-        cudaError_t  e = launch_jpeg_entropy(ddev, n, any_parallel, any_serial, jpeg_entropy_min_segment(), threads, longest, most_blocks,
+        cudaError_t  e = launch_jpeg_entropy(ddev, n, any_parallel, any_serial, jpeg_entropy_min_segment(), longest, most_blocks,
                                              parts_dev, (int)parts.size(), ctx->stream);
         if (e != cudaSuccess)
             throw error(AEONB_ERR_CUDA, cuda_message("jpeg entropy kernel launch", e));

@@ -474,20 +474,32 @@ namespace aeonb
         // tail of the left neighbour's segment before the guess.
         constexpr int AC_BITS = 11; // bits of the lookup window: AC tables (12: 28 us slower for 256 streams, fewer of which then fit shared memory)
         constexpr int DC_BITS = 9;  //                            DC tables (few, short codes)
-        // One 32-bit lookup gives everything the symbol loop needs:
-        //   bits 0-4   total bits the symbol takes (code + value bits)     bits 5-8  number of value bits (AC size / DC category)
-        //   bits 24-31 advance of the zig-zag index: run + 1, 16 for ZRL, 64 for end of block, 1 for a DC category,
+        // One 32-bit lookup gives everything the symbol loops need.  Of the symbol at the head of the window:
+        //   bits 5-8   number of value bits (AC size / DC category)       bits 9-13  total bits it takes (code + value bits)
+        //   bits 14-20 advance of the zig-zag index: run + 1, 16 for ZRL, 64 for end of block, 1 for a DC category,
         //              127 for an invalid code (which still takes bits and ends the block, so that a decoder in a wrong state moves on)
-        // 0 = the code is longer than the window.  Without the value bits the entry is what the decoder's state -- bit position in
-        // bits 0-23, zig-zag index in bits 24-31 -- advances by, in one addition.
+        // and of the pair it makes with the symbol behind it, where it fits the window whole and does not end the block, and the
+        // second one's code lies in the window too (otherwise of the one symbol again):
+        //   bits 0-4   total bits                                          bits 24-31 advance of the zig-zag index
+        // 0 = the code is longer than the window.  The pair's part is what the decoder's state -- bit position in bits 0-23, zig-zag
+        // index in bits 24-31 -- advances by, in one addition.
         constexpr uint32_t k_advance = 0xff00001fu, k_position = 0x00ffffffu, k_block_end = 64u << 24;
+        constexpr uint32_t k_pair_first = AC_BITS - 1;  // most bits of the first symbol of a pair
+        constexpr uint32_t k_pair_limit = 48u << 24;    // from this zig-zag index on (63 - 15) the first symbol can end the block
+        __device__ __forceinline__ uint32_t entry_total(uint32_t e) { return e >> 9 & 31; }
+        __device__ __forceinline__ uint32_t entry_size(uint32_t e) { return e >> 5 & 15; }
+        __device__ __forceinline__ uint32_t entry_advance(uint32_t e) { return e >> 14 & 127; }
+        __device__ __forceinline__ uint32_t single_step(uint32_t e) { return entry_total(e) | (e << 10 & 0x7f000000u); }
+        __device__ __forceinline__ uint32_t make_entry(uint32_t size, uint32_t total, uint32_t advance)
+        {
+            return total | size << 5 | total << 9 | advance << 14 | advance << 24;
+        }
         __device__ __forceinline__ uint32_t pack_symbol(int len, int sym, bool is_ac)
         {
             const int s = sym & 15, r = sym >> 4;
             const int kinc = is_ac ? (s ? r + 1 : (r == 15 ? 16 : 64)) : (r == 0 ? 1 : 127);
-            return (uint32_t)(len + s) | (uint32_t)s << 5 | (uint32_t)kinc << 24;
+            return make_entry((uint32_t)s, (uint32_t)(len + s), (uint32_t)kinc);
         }
-        constexpr uint32_t k_invalid_symbol = 16u | 127u << 24;
 
         struct code_table
         {
@@ -556,12 +568,26 @@ namespace aeonb
                 }
             }
         }
+        // Pairs the entries of the AC windows (see above).  Only the parts of an entry that stay as they are are read of others.
+        __device__ void pair_windows(uint32_t* ac, int tid, int nth)
+        {
+            for (int j = tid; j < 2 << AC_BITS; j += nth)
+            {
+                uint32_t* const T = ac + (j >> AC_BITS << AC_BITS);
+                const uint32_t  i = (uint32_t)j & ((1 << AC_BITS) - 1), e = T[i], total = entry_total(e), advance = entry_advance(e);
+                if (e == 0 || advance >= 64 || total > k_pair_first)
+                    continue;
+                const uint32_t f = reinterpret_cast<volatile uint32_t*>(T)[i << total & ((1 << AC_BITS) - 1)]; // the bits behind, zeros after them
+                if (f != 0 && entry_total(f) - entry_size(f) <= AC_BITS - total)
+                    T[i] = (e & 0x001fffe0u) | (total + entry_total(f)) | (advance + entry_advance(f)) << 24;
+            }
+        }
         // A code longer than the window, or an invalid one.
         __device__ __noinline__ uint32_t long_symbol(const code_table& T, uint32_t h, bool is_ac)
         {
             const int c16 = (int)(h >> 16);
             if (c16 >= T.limit[16])
-                return k_invalid_symbol;
+                return make_entry(0, 16, 127);
             int len = 1;
 #pragma unroll
             for (int l = 1; l < 16; ++l)
@@ -569,7 +595,7 @@ namespace aeonb
             return pack_symbol(len, T.vals[((c16 >> (16 - len)) + T.valoff[len]) & 255], is_ac);
         }
 
-        constexpr int PAR_THREADS = 512;  // most threads (= segments) a stream can have; the launch picks the actual number
+        constexpr int PAR_THREADS = 1024; // most threads (= segments) a stream can have; the launch picks the actual number
         constexpr int NCHECK      = 3;    // checkpoints inside a segment (7 measured the same; 3 leaves room for a third kernel's CTA on the SM)
 
         // Where the blocks of one place in an MCU go: base + 64 * ((mcu row - first row) * dy + (mcu column - first column) * dx)
@@ -750,41 +776,63 @@ namespace aeonb
             // The 32 bits under the position lie in w0 and w1; w2 is the word behind them, fetched when the one before it comes into use.
             Words    ahead(words, p >> 5);
             uint32_t w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
+            // The entry of the symbol under the position, and the state after an advance.
+            uint32_t h;
+            auto     lookup = [&]() -> uint32_t {
+                h          = __funnelshift_l(w1, w0, at); // 32 valid bits; a symbol or a pair takes at most 31
+                uint32_t e = lds_u32(look + ((h >> shift) << 2));
+                if (!e)
+                {
+                    const bool is_ac = at > k_position;
+                    e = long_symbol(is_ac ? S.codes[look == shared_address(S.ac_window[0]) ? 2 : 3] : S.codes[look == shared_address(S.dc_window[0]) ? 0 : 1], h,
+                                    is_ac);
+                }
+                return e;
+            };
+            auto step = [&](uint32_t by) -> bool {
+                const uint32_t to    = at + by;
+                const uint32_t cross = (at ^ to) & 32; // the read position has left w0
+                w0                   = cross ? w1 : w0;
+                w1                   = cross ? w2 : w1;
+                ahead.next_if(w2, cross);
+                const bool end = to >= k_block_end;
+                look           = end ? link.next_dc : link.ac;
+                shift          = end ? 32 - DC_BITS : 32 - AC_BITS;
+                at             = end ? to & k_position : to;
+                blocks += end;
+                follow_if(link, end);
+                return end;
+            };
             for (;;)
             {
+                // Two symbols at a time as long as the first one cannot reach `stop`: a run stops at the first symbol at or past it,
+                // however it came there.
+                if (!WRITE)
+                    while ((at & k_position) + k_pair_first < stop)
+                    {
+                        const uint32_t e  = lookup();
+                        uint32_t       by = e & k_advance;
+                        if (at >= k_pair_limit)
+                            by = single_step(e);
+                        step(by);
+                    }
                 while ((at & k_position) < stop)
                 {
-                    const uint32_t h = __funnelshift_l(w1, w0, at); // 32 valid bits; a symbol takes at most 31
-                    uint32_t       e = lds_u32(look + ((h >> shift) << 2));
-                    if (!e)
-                    {
-                        const bool is_ac = at > k_position;
-                        e = long_symbol(is_ac ? S.codes[look == shared_address(S.ac_window[0]) ? 2 : 3] : S.codes[look == shared_address(S.dc_window[0]) ? 0 : 1],
-                                        h, is_ac);
-                    }
-                    const uint32_t to    = at + (e & k_advance);
-                    const uint32_t cross = (at ^ to) & 32; // the read position has left w0
+                    const uint32_t e = lookup();
                     if (WRITE)
                     {
-                        const int      tot = e & 31, sz = (e >> 5) & 15, kk = (int)((at >> 24) + (e >> 24)) - 1; // kk: the coefficient's place
-                        const uint32_t x   = h << (tot - sz);                                                   // the value bits at the top
-                        const int      v   = (int)__funnelshift_l(x, 0u, sz) + ((int)x >= 0 ? 1 - (1 << sz) : 0);
+                        const int      tot = (int)entry_total(e), sz = (int)entry_size(e), kinc = (int)entry_advance(e);
+                        const int      kk = (int)(at >> 24) + kinc - 1; // the coefficient's place
+                        const uint32_t x  = h << (tot - sz);            // the value bits at the top
+                        const int      v  = (int)__funnelshift_l(x, 0u, sz) + ((int)x >= 0 ? 1 - (1 << sz) : 0);
                         // an invalid code, a DC symbol that is no category, or a run that leaves the block
-                        bad |= e >= 127u << 24 || (sz && kk > 63);
+                        bad |= kinc == 127 || (sz && kk > 63);
                         if (at <= k_position)
                             dcdiff[g] = (int16_t)v;
                         else if (sz && kk <= 63 && out)
                             out[S.zz[kk]] = (int16_t)v;
                     }
-                    w0 = cross ? w1 : w0;
-                    w1 = cross ? w2 : w1;
-                    ahead.next_if(w2, cross);
-                    const bool end = to >= k_block_end;
-                    look           = end ? link.next_dc : link.ac;
-                    shift          = end ? 32 - DC_BITS : 32 - AC_BITS;
-                    at             = end ? to & k_position : to;
-                    blocks += end;
-                    follow_if(link, end);
+                    const bool end = step(single_step(e));
                     if (WRITE && end)
                     {
                         if (++g >= gend)
@@ -960,6 +1008,8 @@ namespace aeonb
                 S.codes[i >> 8].vals[i & 255] = S.dht[(i >> 8) * 272 + 16 + (i & 255)];
             __syncthreads();
             build_windows(S.ac_window[0], S.dc_window[0], S.codes, tid, nth);
+            __syncthreads();
+            pair_windows(S.ac_window[0], tid, nth);
             __syncthreads();
         }
 
@@ -1715,16 +1765,27 @@ namespace aeonb
         return value;
     }
 
-    int jpeg_entropy_threads()
+    int jpeg_entropy_threads(int n)
     {
         static const int value = [] {
-            int v = 512;
+            int v = 0;
             if (const char* e = std::getenv("AEONB_ENTROPY_THREADS"))
-                v = std::atoi(e);
-            v = v < 128 ? 128 : v > PAR_THREADS ? PAR_THREADS : v;
-            return v & ~31;
+                v = std::max(128, std::min(std::atoi(e), PAR_THREADS)) & ~31;
+            return v;
         }();
-        return value;
+        return value ? value : n <= 148 ? PAR_THREADS : 512;
+    }
+
+    int jpeg_entropy_block(int n, uint32_t longest)
+    {
+        // A stream that has an SM to itself gets a thread for each piece of the storing pass; of more streams than SMs two share one,
+        // and a thread per segment has to do.
+        const int segments = (int)((longest + (uint32_t)jpeg_entropy_min_segment() - 1) / (uint32_t)jpeg_entropy_min_segment());
+        const int wanted   = n <= 148 ? segments * (NCHECK + 1) : segments;
+        int       threads  = jpeg_entropy_threads(n);
+        while (threads > 128 && wanted <= threads / 2)
+            threads /= 2;
+        return threads & ~31;
     }
 
     int64_t jpeg_entropy_scratch_bytes(const aeonb_entropy_desc& d)
@@ -1778,14 +1839,14 @@ namespace aeonb
     }
 
     cudaError_t launch_jpeg_entropy(const aeonb_entropy_desc* descs_dev, int n, bool any_parallel, bool any_serial, int min_segment,
-                                    int threads, uint32_t longest, uint64_t most_blocks, const int4* parts_dev, int n_parts,
+                                    uint32_t longest, uint64_t most_blocks, const int4* parts_dev, int n_parts,
                                     cudaStream_t stream)
     {
         if (n <= 0)
             return cudaSuccess;
         if (any_parallel)
         {
-            threads           = std::min(std::max(threads, 128), jpeg_entropy_threads()) & ~31;
+            const int    threads = jpeg_entropy_block(n, longest);
             const size_t smem = jpeg_entropy_smem(n, threads, longest, most_blocks);
             cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_parallel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (err != cudaSuccess)

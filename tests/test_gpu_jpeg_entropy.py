@@ -218,3 +218,18 @@ def test_damaged_restart_streams_are_left_to_the_serial_decoder(ctx):
         for c in range(3):
             assert s[3] != 0 or np.array_equal(g[1][c].cpu().numpy(), s[1][c].cpu().numpy()), (i, c)
     check(ctx, [good])
+
+
+@pytest.mark.parametrize("copies", [1, 148, 149])
+def test_block_sizes_on_either_side_of_a_stream_per_sm(ctx, golden_dir, copies):
+    """Up to one stream per SM a stream gets a thread per piece of the storing pass, above that a thread per segment and less shared
+    memory.  A stream of 507 segments, noise at quality 100 (long codes, blocks that end at coefficient 63 without an end-of-block code)
+    and a stream too long for the shared memory of a block that shares its SM."""
+    rng = np.random.default_rng(78)
+    blobs = [open(os.path.join(golden_dir, "entropy_stream_507_segments.jpg"), "rb").read(),
+             jpeg_bytes(rng.integers(0, 256, (168, 200, 3), dtype=np.uint8), 100),
+             jpeg_bytes(rng.integers(0, 256, (300, 400, 3), dtype=np.uint8), 97),
+             jpeg_bytes(gradient_image(rng, 24, 40), 75)]
+    assert len(blobs[2]) > 115_000
+    for blob in blobs if copies == 1 else [None]:
+        check(ctx, [blob] if blob else [blobs[i % len(blobs)] for i in range(copies)])
