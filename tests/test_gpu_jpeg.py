@@ -155,3 +155,40 @@ def test_440_and_411_sampling(ctx):
     got = decode_gpu(ctx, cases)
     for i, b in enumerate(cases):
         assert np.array_equal(got[i], cv2.imdecode(np.frombuffer(b, np.uint8), cv2.IMREAD_COLOR)), "case %d" % i
+
+
+@pytest.mark.parametrize("pitch_step", [4, 8])
+def test_422_and_420_rows_at_the_edges_of_the_eight_pixel_groups(ctx, pitch_step):
+    """Widths around multiples of eight and sixteen (the last group of a row takes the generic path), strips of one and two MCU rows, and
+    destinations whose rows are 4-byte but not 8-byte aligned."""
+    import ctypes as C
+    import cv2
+    import torch
+    from aeon_b200 import _lib as L, kernels as K
+    rng = np.random.default_rng(24)
+    dev = torch.device("cuda", ctx.device)
+    blobs = [jpeg_bytes(rng.integers(0, 256, (h, w, 3), dtype=np.uint8), 95, [cv2.IMWRITE_JPEG_SAMPLING_FACTOR, mode])
+             for mode in (cv2.IMWRITE_JPEG_SAMPLING_FACTOR_422, cv2.IMWRITE_JPEG_SAMPLING_FACTOR_420)
+             for h, w in [(1, 7), (8, 8), (9, 9), (16, 15), (17, 16), (33, 17), (40, 23), (7, 24), (24, 25), (31, 31), (64, 32), (5, 33), (48, 257)]]
+    descs, keep, outs = (L.JpegDesc * len(blobs))(), [], []
+    for d, blob in zip(descs, blobs):
+        info, coefs, quants = K.jpeg_entropy_decode(blob)
+        pitch = (info.width * 3 + 3) // 4 * 4
+        pitch += 4 if pitch % 8 != pitch_step % 8 else 0
+        out = torch.full((info.height + 1, pitch), 77, dtype=torch.uint8, device=dev)
+        d.width, d.height, d.ncomp = info.width, info.height, info.ncomp
+        for c in range(info.ncomp):
+            d.hs[c], d.vs[c], d.blocks_w[c], d.blocks_h[c] = info.hs[c], info.vs[c], info.blocks_w[c], info.blocks_h[c]
+            t, q = torch.from_numpy(coefs[c]).to(dev), torch.from_numpy(quants[c].view(np.int16)).to(dev)
+            keep += [t, q]
+            d.coef[c], d.quant[c] = t.data_ptr(), q.data_ptr()
+        d.dst, d.dst_pitch, d.dst_pixel_stride = out.data_ptr(), pitch, 3
+        outs.append(out)
+    torch.cuda.synchronize(dev)
+    L.check(ctx.lib.aeonb_jpeg_backend_batch(ctx.handle, descs, len(blobs)))
+    ctx.synchronize()
+    for d, blob, out in zip(descs, blobs, outs):
+        want = cv2.imdecode(np.frombuffer(blob, np.uint8), cv2.IMREAD_COLOR)
+        got = out.cpu().numpy()
+        assert np.array_equal(got[:-1, :d.width * 3].reshape(want.shape), want), (want.shape, d.dst_pitch)
+        assert (got[-1] == 77).all()
