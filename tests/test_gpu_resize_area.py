@@ -102,3 +102,20 @@ def test_lanczos4_matches_the_oracle(ctx):
     got = resize_gpu(ctx, jobs, interp=L.INTERP_LANCZOS4)
     for (img, _, _, (dw, dh)), g in zip(jobs, got):
         assert np.array_equal(g, ops.resize_lanczos4_u8(img, dw, dh)), (img.shape, dw, dh)
+
+
+@pytest.mark.parametrize("records", [1, 40])
+def test_shrinking_cells_over_blocks_of_rows_and_columns(ctx, records):
+    """More columns than a block holds cells for (512), rows that do not fill a block's group (one row a block for one record, eight for
+    many), cells of one to nine pixels, cells that hang over the picture's edge on an expanded canvas, 4-byte source pixels."""
+    rng = np.random.default_rng(85)
+    jobs = []
+    for i in range(records):
+        ow, oh = [(513, 3), (512, 9), (1030, 2), (64, 230), (31, 17)][i % 5] if records > 1 else (1030, 230)
+        sw, sh = int(ow * rng.uniform(1.01, 1.9)) + 1, int(oh * rng.uniform(1.01, 8.0)) + 1
+        img = rng.integers(0, 256, (sh, sw, 3), dtype=np.uint8)
+        cx, cy = (0, 0) if i % 2 else (5, 3)
+        jobs.append((img, (cx, cy), (0, 0, sw + cx, sh + cy), (ow, oh)))
+    for stride in (3, 4):
+        for (img, cxy, crop, (ow, oh)), g in zip(jobs, resize_gpu(ctx, jobs, stride)):
+            assert np.array_equal(g, ops.resize_area_u8(window(img, cxy, crop), ow, oh)), (img.shape, ow, oh, stride)
