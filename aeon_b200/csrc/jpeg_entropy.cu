@@ -481,8 +481,11 @@ namespace aeonb
         // and of the pair it makes with the symbol behind it, where it fits the window whole and does not end the block, and the
         // second one's code lies in the window too (otherwise of the one symbol again):
         //   bits 0-4   total bits                                          bits 24-31 advance of the zig-zag index
-        // 0 = the code is longer than the window.  The pair's part is what the decoder's state -- bit position in bits 0-23, zig-zag
+        // A code longer than an AC window: bits 0-4 are 0, bits 8-24 hold the 16 bits at which such codes begin; the entry is found
+        // behind the window, at the distance of the 16 bits at hand from there.  0 = look the code up the long way (long_symbol).
+        // The pair's part is what the decoder's state -- bit position in bits 0-23, zig-zag
         // index in bits 24-31 -- advances by, in one addition.
+        constexpr int      AC_LONG = 256, AC_ENTRIES = (1 << AC_BITS) + AC_LONG; // entries behind an AC window, and all of them
         constexpr uint32_t k_advance = 0xff00001fu, k_position = 0x00ffffffu, k_block_end = 64u << 24;
         constexpr uint32_t k_pair_first = AC_BITS - 1;  // most bits of the first symbol of a pair
         constexpr uint32_t k_pair_limit = 48u << 24;    // from this zig-zag index on (63 - 15) the first symbol can end the block
@@ -537,7 +540,7 @@ namespace aeonb
         __device__ __forceinline__ uint32_t window_entry(const code_table& T, int i, int len, int bits, bool is_ac)
         {
             if ((i << (16 - bits)) >= T.limit[len])
-                return 0;
+                return is_ac && (i << (16 - bits) | ((1 << (16 - bits)) - 1)) - T.limit[AC_BITS] < AC_LONG ? (uint32_t)T.limit[AC_BITS] << 8 : 0;
             return pack_symbol(len, T.vals[((i >> (bits - len)) + T.valoff[len]) & 255], is_ac);
         }
         // `nth` threads (index `tid`) fill the four lookup windows once limits and values are in place.  Eight neighbouring entries
@@ -552,7 +555,7 @@ namespace aeonb
                 const int         slot = is_ac ? j / ac8 : (j - 2 * ac8) / dc8, i = (is_ac ? j % ac8 : (j - 2 * ac8) % dc8) * 8;
                 const int         bits = is_ac ? AC_BITS : DC_BITS;
                 const code_table& T    = codes[is_ac ? 2 + slot : slot];
-                uint32_t* const   out  = (is_ac ? ac + (slot << AC_BITS) : dc + (slot << DC_BITS)) + i;
+                uint32_t* const   out  = (is_ac ? ac + slot * AC_ENTRIES : dc + (slot << DC_BITS)) + i;
                 const int first = code_length(T, i << (16 - bits), bits), last = code_length(T, (i + 7) << (16 - bits), bits);
                 if (first == last && first <= bits - 3)
                 {
@@ -568,24 +571,9 @@ namespace aeonb
                 }
             }
         }
-        // Pairs the entries of the AC windows (see above).  Only the parts of an entry that stay as they are are read of others.
-        __device__ void pair_windows(uint32_t* ac, int tid, int nth)
-        {
-            for (int j = tid; j < 2 << AC_BITS; j += nth)
-            {
-                uint32_t* const T = ac + (j >> AC_BITS << AC_BITS);
-                const uint32_t  i = (uint32_t)j & ((1 << AC_BITS) - 1), e = T[i], total = entry_total(e), advance = entry_advance(e);
-                if (e == 0 || advance >= 64 || total > k_pair_first)
-                    continue;
-                const uint32_t f = reinterpret_cast<volatile uint32_t*>(T)[i << total & ((1 << AC_BITS) - 1)]; // the bits behind, zeros after them
-                if (f != 0 && entry_total(f) - entry_size(f) <= AC_BITS - total)
-                    T[i] = (e & 0x001fffe0u) | (total + entry_total(f)) | (advance + entry_advance(f)) << 24;
-            }
-        }
         // A code longer than the window, or an invalid one.
-        __device__ __noinline__ uint32_t long_symbol(const code_table& T, uint32_t h, bool is_ac)
+        __device__ __noinline__ uint32_t long_symbol(const code_table& T, int c16, bool is_ac)
         {
-            const int c16 = (int)(h >> 16);
             if (c16 >= T.limit[16])
                 return make_entry(0, 16, 127);
             int len = 1;
@@ -593,6 +581,35 @@ namespace aeonb
             for (int l = 1; l < 16; ++l)
                 len += c16 >= T.limit[l];
             return pack_symbol(len, T.vals[((c16 >> (16 - len)) + T.valoff[len]) & 255], is_ac);
+        }
+        // Pairs the entries of the AC windows (see above), four neighbours per thread and pass so that their second lookups overlap, and
+        // fills what lies behind the windows.  Only the parts of an entry that stay as they are are read of others.
+        __device__ void pair_windows(uint32_t* ac, const code_table* codes, int tid, int nth)
+        {
+            constexpr uint32_t mask = (1 << AC_BITS) - 1;
+            for (int j = tid; j < 2 << (AC_BITS - 2); j += nth)
+            {
+                uint32_t* const T = ac + (j >> (AC_BITS - 2)) * AC_ENTRIES;
+                const uint32_t  i = 4 * ((uint32_t)j & (mask >> 2));
+                const uint4     four = *reinterpret_cast<uint4*>(T + i);
+                uint32_t        e[4] = {four.x, four.y, four.z, four.w}, f[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                    f[k] = reinterpret_cast<volatile uint32_t*>(T)[(i + k) << entry_total(e[k]) & mask]; // the bits behind, zeros after them
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                {
+                    const uint32_t total = entry_total(e[k]), advance = entry_advance(e[k]);
+                    if ((e[k] & 31) && advance < 64 && total <= k_pair_first && (f[k] & 31) && entry_total(f[k]) - entry_size(f[k]) <= AC_BITS - total)
+                        e[k] = (e[k] & 0x001fffe0u) | (total + entry_total(f[k])) | (advance + entry_advance(f[k])) << 24;
+                }
+                *reinterpret_cast<uint4*>(T + i) = make_uint4(e[0], e[1], e[2], e[3]);
+            }
+            for (int j = tid; j < 2 * AC_LONG; j += nth)
+            {
+                const code_table& T = codes[2 + j / AC_LONG];
+                ac[j / AC_LONG * AC_ENTRIES + (1 << AC_BITS) + j % AC_LONG] = long_symbol(T, min(T.limit[AC_BITS] + j % AC_LONG, 0xffff), true);
+            }
         }
 
         constexpr int PAR_THREADS = 1024; // most threads (= segments) a stream can have; the launch picks the actual number
@@ -613,7 +630,7 @@ namespace aeonb
 
         struct par_state
         {
-            uint32_t    ac_window[2][1 << AC_BITS], dc_window[2][1 << DC_BITS];
+            uint32_t    ac_window[2][AC_ENTRIES], dc_window[2][1 << DC_BITS];
             code_table  codes[4]; // DC slot 0, DC slot 1, AC slot 0, AC slot 1
             uint8_t     dht[4 * 272]; // the tables as they came
             uint32_t    warp_sums[3][32];
@@ -649,6 +666,11 @@ namespace aeonb
             uint32_t v;
             asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
             return v;
+        }
+        // value = the word at addr where `yes`
+        __device__ __forceinline__ void lds_if(uint32_t& value, uint32_t addr, bool yes)
+        {
+            asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.shared.u32 %0, [%1];\n\t}" : "+r"(value) : "r"(addr), "r"((uint32_t)yes));
         }
         // link = the link at its `next` where `yes`
         __device__ __forceinline__ void follow_if(block_link& link, bool yes)
@@ -781,11 +803,12 @@ namespace aeonb
             auto     lookup = [&]() -> uint32_t {
                 h          = __funnelshift_l(w1, w0, at); // 32 valid bits; a symbol or a pair takes at most 31
                 uint32_t e = lds_u32(look + ((h >> shift) << 2));
+                lds_if(e, look + (((h >> 16) - (e >> 8) + (1 << AC_BITS)) << 2), (e & 31) == 0 && e != 0);
                 if (!e)
                 {
                     const bool is_ac = at > k_position;
-                    e = long_symbol(is_ac ? S.codes[look == shared_address(S.ac_window[0]) ? 2 : 3] : S.codes[look == shared_address(S.dc_window[0]) ? 0 : 1], h,
-                                    is_ac);
+                    e = long_symbol(is_ac ? S.codes[look == shared_address(S.ac_window[0]) ? 2 : 3] : S.codes[look == shared_address(S.dc_window[0]) ? 0 : 1],
+                                    (int)(h >> 16), is_ac);
                 }
                 return e;
             };
@@ -805,20 +828,14 @@ namespace aeonb
             };
             for (;;)
             {
-                // Two symbols at a time as long as the first one cannot reach `stop`: a run stops at the first symbol at or past it,
-                // however it came there.
-                if (!WRITE)
-                    while ((at & k_position) + k_pair_first < stop)
-                    {
-                        const uint32_t e  = lookup();
-                        uint32_t       by = e & k_advance;
-                        if (at >= k_pair_limit)
-                            by = single_step(e);
-                        step(by);
-                    }
                 while ((at & k_position) < stop)
                 {
-                    const uint32_t e = lookup();
+                    const uint32_t e  = lookup();
+                    uint32_t       by = single_step(e);
+                    // Two symbols at a time as long as the first one cannot reach `stop`: a run stops at the first symbol at or past
+                    // it, however it came there.
+                    if (!WRITE)
+                        by = at < k_pair_limit && (at & k_position) + k_pair_first < stop ? e & k_advance : by;
                     if (WRITE)
                     {
                         const int      tot = (int)entry_total(e), sz = (int)entry_size(e), kinc = (int)entry_advance(e);
@@ -832,7 +849,7 @@ namespace aeonb
                         else if (sz && kk <= 63 && out)
                             out[S.zz[kk]] = (int16_t)v;
                     }
-                    const bool end = step(single_step(e));
+                    const bool end = step(by);
                     if (WRITE && end)
                     {
                         if (++g >= gend)
@@ -1009,7 +1026,7 @@ namespace aeonb
             __syncthreads();
             build_windows(S.ac_window[0], S.dc_window[0], S.codes, tid, nth);
             __syncthreads();
-            pair_windows(S.ac_window[0], tid, nth);
+            pair_windows(S.ac_window[0], S.codes, tid, nth);
             __syncthreads();
         }
 
