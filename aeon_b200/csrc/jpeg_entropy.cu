@@ -528,14 +528,12 @@ namespace aeonb
                 code <<= 1;
             }
         }
-        // Length of the code at the head of the 16 bits c16, if it is no longer than `bits`.
-        __device__ __forceinline__ int code_length(const code_table& T, int c16, int bits)
+        // Length of the code at the head of the 16 bits c16, known to be at least `from`, if it is no longer than `to`.
+        __device__ __forceinline__ int code_length(const code_table& T, int c16, int from, int to)
         {
-            int len = 1;
-#pragma unroll
-            for (int l = 1; l < AC_BITS; ++l)
-                len += l < bits && c16 >= T.limit[l];
-            return len;
+            while (from < to && c16 >= T.limit[from])
+                ++from;
+            return from;
         }
         __device__ __forceinline__ uint32_t window_entry(const code_table& T, int i, int len, int bits, bool is_ac)
         {
@@ -556,7 +554,7 @@ namespace aeonb
                 const int         bits = is_ac ? AC_BITS : DC_BITS;
                 const code_table& T    = codes[is_ac ? 2 + slot : slot];
                 uint32_t* const   out  = (is_ac ? ac + slot * AC_ENTRIES : dc + (slot << DC_BITS)) + i;
-                const int first = code_length(T, i << (16 - bits), bits), last = code_length(T, (i + 7) << (16 - bits), bits);
+                const int first = code_length(T, i << (16 - bits), 1, bits), last = code_length(T, (i + 7) << (16 - bits), first, bits);
                 if (first == last && first <= bits - 3)
                 {
                     const uint32_t e = window_entry(T, i, first, bits, is_ac);
@@ -567,19 +565,16 @@ namespace aeonb
                 {
 #pragma unroll 1
                     for (int k = 0; k < 8; ++k)
-                        out[k] = window_entry(T, i + k, code_length(T, (i + k) << (16 - bits), bits), bits, is_ac);
+                        out[k] = window_entry(T, i + k, code_length(T, (i + k) << (16 - bits), first, last), bits, is_ac);
                 }
             }
         }
         // A code longer than the window, or an invalid one.
-        __device__ __noinline__ uint32_t long_symbol(const code_table& T, int c16, bool is_ac)
+        __device__ __noinline__ uint32_t long_symbol(const code_table& T, int c16, bool is_ac, int from)
         {
             if (c16 >= T.limit[16])
                 return make_entry(0, 16, 127);
-            int len = 1;
-#pragma unroll
-            for (int l = 1; l < 16; ++l)
-                len += c16 >= T.limit[l];
+            const int len = code_length(T, c16, from, 16);
             return pack_symbol(len, T.vals[((c16 >> (16 - len)) + T.valoff[len]) & 255], is_ac);
         }
         // Pairs the entries of the AC windows (see above), four neighbours per thread and pass so that their second lookups overlap, and
@@ -608,7 +603,7 @@ namespace aeonb
             for (int j = tid; j < 2 * AC_LONG; j += nth)
             {
                 const code_table& T = codes[2 + j / AC_LONG];
-                ac[j / AC_LONG * AC_ENTRIES + (1 << AC_BITS) + j % AC_LONG] = long_symbol(T, min(T.limit[AC_BITS] + j % AC_LONG, 0xffff), true);
+                ac[j / AC_LONG * AC_ENTRIES + (1 << AC_BITS) + j % AC_LONG] = long_symbol(T, min(T.limit[AC_BITS] + j % AC_LONG, 0xffff), true, AC_BITS + 1);
             }
         }
 
@@ -632,7 +627,7 @@ namespace aeonb
         {
             uint32_t    ac_window[2][AC_ENTRIES], dc_window[2][1 << DC_BITS];
             code_table  codes[4]; // DC slot 0, DC slot 1, AC slot 0, AC slot 1
-            uint8_t     dht[4 * 272]; // the tables as they came
+            alignas(16) uint8_t dht[4 * 272]; // the tables as they came
             uint32_t    warp_sums[3][32];
             uint8_t     zz[64];
             block_place place[16];               // per block of an MCU
@@ -808,7 +803,7 @@ namespace aeonb
                 {
                     const bool is_ac = at > k_position;
                     e = long_symbol(is_ac ? S.codes[look == shared_address(S.ac_window[0]) ? 2 : 3] : S.codes[look == shared_address(S.dc_window[0]) ? 0 : 1],
-                                    (int)(h >> 16), is_ac);
+                                    (int)(h >> 16), is_ac, 1);
                 }
                 return e;
             };
@@ -908,17 +903,17 @@ namespace aeonb
             if (lane == 31)
                 sums[warp] = incl;
             __syncthreads();
-            uint32_t  before = 0, all = 0;
-            const int nwarps = (int)(blockDim.x >> 5);
-            for (int w = 0; w < nwarps; ++w)
+            uint32_t to = lane < (int)(blockDim.x >> 5) ? sums[lane] : 0; // the sums up to warp `lane`
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
             {
-                const uint32_t s = sums[w];
-                if (w < warp)
-                    before += s;
-                all += s;
+                const uint32_t up = __shfl_up_sync(0xffffffffu, to, o);
+                if (lane >= o)
+                    to += up;
             }
-            total = all;
-            return before + incl - v;
+            const uint32_t before = __shfl_sync(0xffffffffu, to, max(warp - 1, 0));
+            total                 = __shfl_sync(0xffffffffu, to, 31);
+            return (warp ? before : 0) + incl - v;
         }
 
         // The copy of a stream without stuffed bytes holds big-endian 32-bit words (byte i of the copy is byte i ^ 3 of memory).
@@ -1009,8 +1004,14 @@ namespace aeonb
             }
             // The tables in DHT form are brought in whole: the head of a table is a chain over its 16 code counts, which one
             // thread walks from shared memory rather than from L2.
-            for (int i = tid; i < 4 * 272; i += nth)
-                S.dht[i] = __ldg(d.tables + i);
+            if ((reinterpret_cast<uintptr_t>(d.tables) & 15) == 0)
+            {
+                for (int i = tid; i < 4 * 272 / 16; i += nth)
+                    reinterpret_cast<uint4*>(S.dht)[i] = __ldg(reinterpret_cast<const uint4*>(d.tables) + i);
+            }
+            else
+                for (int i = tid; i < 4 * 272; i += nth)
+                    S.dht[i] = __ldg(d.tables + i);
             __syncthreads();
             if (tid < S.bpm)
             {
@@ -1202,6 +1203,10 @@ namespace aeonb
             // ---- segments: one per thread, a multiple of 4 bytes, at least min_segment bytes
             uint32_t seg = (clean_size + T - 1) / T;
             seg          = max((seg + 3u) & ~3u, (uint32_t)max(min_segment, 64) & ~3u);
+            // The storing pass deals its pieces out in rounds of T.  Up to a quarter more than a whole number of rounds is avoided by
+            // longer segments: the last round would take as long as the others.
+            const uint32_t rounds = max(((NCHECK + 1) * ((clean_size + seg - 1) / seg) * 4 + 3 * T) / (4 * T), 1u);
+            seg                   = max(seg, ((NCHECK + 1) * clean_size / (rounds * T) + 4u) & ~3u);
             const uint32_t nseg      = (clean_size + seg - 1) / seg; // <= T
             const uint32_t total_bit = clean_size * 8;
             const uint32_t pbeg = tid * seg * 8, pend = min(total_bit, pbeg + seg * 8);
