@@ -151,6 +151,7 @@ namespace aeonb
         std::vector<std::vector<rcnn_record>>      rcnn; // per stage: what transformer::transform leaves for the loader
         std::vector<std::vector<aeonb_specgram_desc>> sdescs;
         std::vector<std::vector<size_t>>           sdesc_off;
+        std::vector<int> slice_end; // clips uploaded in slices that the kernels wait for one by one: the end of each; else empty
         size_t stage_bytes = 0, pixel_bytes = 0, coef_bytes = 0, oriented_bytes = 0, rotated_bytes = 0;
         size_t status_room   = 0; // bytes reserved for the entropy decoder's status words at the start of the coefficient arena
         int    n_device_jobs = 0; // streams Huffman-decoded on the GPU
@@ -212,6 +213,8 @@ struct aeonb_provider
     aeonb::pinned_buffer                 small_pinned[k_sets]; // host-produced outputs on their way to device memory
 
     static constexpr int k_events = 8;
+    static constexpr int k_slices = 8;  // of the staging upload of a batch
+    cudaEvent_t m_slice[k_slices]   = {}; // a slice of the batch in hand has arrived
     cudaEvent_t m_done[k_events]    = {}; // batch t complete: m_done[t % k_events]
     cudaEvent_t m_kernels[k_events] = {}; // the kernels of batch t have finished
     cudaStream_t m_copy             = nullptr; // device -> host copies of finished batches

@@ -171,6 +171,9 @@ aeonb_provider::~aeonb_provider()
             cudaEventDestroy(e);
     if (m_labelled)
         cudaEventDestroy(m_labelled);
+    for (cudaEvent_t e : m_slice)
+        if (e)
+            cudaEventDestroy(e);
     for (auto& slot : m_trace)
         for (cudaEvent_t e : slot)
             if (e)
@@ -991,7 +994,13 @@ void aeonb_provider::stage_inputs(batch_plan& B, int par)
     const int   nwork  = njobs + (int)B.copies.size();
     if (nwork > 0)
     {
-        const int                     groups = std::max(1, std::min(8, nwork));
+        const int                     groups = std::max(1, std::min(k_slices, nwork));
+        // A batch of nothing but clips: the spectrogram kernel of a slice runs while the next slices are on their way.  Under
+        // 2 MB the copy takes about as long as the launches that this adds.
+        int clip_stages = 0;
+        for (const auto& d : B.sdescs)
+            clip_stages += !d.empty();
+        const bool in_slices = njobs == 0 && clip_stages == 1 && B.stage_bytes >= (size_t)2 << 20;
         vector<std::atomic<int>>      remaining(groups);
         vector<int>                   first(groups + 1);
         for (int g = 0; g <= groups; ++g)
@@ -1066,6 +1075,14 @@ void aeonb_provider::stage_inputs(batch_plan& B, int par)
                 copy_error = cudaMemcpyAsync(dstage + begin, hstage + begin, end - begin, cudaMemcpyHostToDevice, m_upload);
                 h2d_bytes += (int64_t)(end - begin);
             }
+            if (in_slices && copy_error == cudaSuccess && !failure)
+            {
+                if (!m_slice[g])
+                    copy_error = cudaEventCreateWithFlags(&m_slice[g], cudaEventDisableTiming);
+                if (copy_error == cudaSuccess)
+                    copy_error = cudaEventRecord(m_slice[g], m_upload);
+                B.slice_end.push_back(first[g + 1]);
+            }
         }
         pool->wait();
         if (failure)
@@ -1079,7 +1096,8 @@ void aeonb_provider::stage_inputs(batch_plan& B, int par)
     }
     AEONB_CUDA(cudaEventRecord(m_staged[par], m_upload));
     m_staged_valid[par] = true;
-    AEONB_CUDA(cudaStreamWaitEvent(st, m_staged[par], 0)); // the kernels of this batch start once its inputs have arrived
+    if (B.slice_end.empty())
+        AEONB_CUDA(cudaStreamWaitEvent(st, m_staged[par], 0)); // the kernels of this batch start once its inputs have arrived
 
 }
 
@@ -1475,7 +1493,14 @@ void aeonb_provider::launch_kernels(batch_plan& B, void* const* outs, int n, int
                 B.sdescs[s][i].samples = reinterpret_cast<const int16_t*>(dstage + B.sdesc_off[s][i]);
                 B.sdescs[s][i].dst     = reinterpret_cast<float*>(B.produced[o] + (int64_t)i * outputs[o].shape.byte_size());
             }
-            check_status(aeonb_specgram_batch(ctx, B.sdescs[s].data(), (int)B.sdescs[s].size(), &cfg));
+            if (B.slice_end.empty())
+                check_status(aeonb_specgram_batch(ctx, B.sdescs[s].data(), (int)B.sdescs[s].size(), &cfg));
+            int begin = 0;
+            for (size_t g = 0; g < B.slice_end.size(); begin = B.slice_end[g++])
+            {
+                AEONB_CUDA(cudaStreamWaitEvent(st, m_slice[g], 0));
+                check_status(aeonb_specgram_batch(ctx, B.sdescs[s].data() + begin, B.slice_end[g] - begin, &cfg));
+            }
             h2d_bytes += (int64_t)(sizeof(aeonb_specgram_desc) * B.sdescs[s].size());
         }
     }

@@ -669,3 +669,22 @@ def test_errors_of_pipelined_batches(ctx):
     prov.wait(t2)
     assert np.array_equal(bufs[0]["image"], want) and np.array_equal(bufs[2]["image"], want)
     assert np.array_equal(prov.run_host([(good,), (good,)])["image"], want)
+
+
+def test_audio_batches_uploaded_in_slices(ctx):
+    """Batches of more than 2 MB of samples go through the spectrogram kernel slice by slice as they arrive: eleven clips (slices of one
+    and two), one of them empty of frames, several batches in a row; the same rows as the oracle."""
+    from oracle import specgram as ospec
+    rng = np.random.default_rng(91)
+    steps = (240000 - 400) // 160 + 1
+    cfg = {"batch_size": 11, "etl": [{"type": "audio", "frame_length": 400, "frame_stride": 160, "max_samples": 240000, "num_filters": 40,
+                                      "sample_rate": 16000, "window_type": "hann", "feature_type": "mfsc"}]}
+    prov = make_provider(ctx, cfg)
+    for _ in range(4):
+        clips = [(rng.normal(0, 2000, int(n))).astype(np.int16) for n in [240000, 399, 400] + list(rng.integers(120000, 240000, 8))]
+        got = prov.run_host([(c.tobytes(),) for c in clips])["audio"].reshape(11, steps, 40)
+        for g, c in zip(got, clips):
+            want = ospec.log_mel(c, 400, 160, steps, 40)
+            fin = np.isfinite(want)
+            assert np.array_equal(np.isfinite(g), fin)
+            assert np.all(np.abs(g[fin] - want[fin]) <= 1e-4 * np.abs(want[fin]) + 2e-4)

@@ -208,3 +208,34 @@ def test_provider_with_random_crops_thresholds_and_small_samples(ctx):
         want = PipelineOracle(oracle_cfg).batch(recs)
         assert np.array_equal(got["image"], want["image"])
         compare_rcnn(got, want)
+
+
+@pytest.mark.parametrize("rc", [{}, {"scaling_factor": 0.125, "base_size": 8, "ratios": [0.5, 1, 2], "scales": [4]}])
+def test_planes_written_on_the_device_equal_the_host_planes(ctx, rc):
+    """Delivered to device memory the per-anchor planes come from kernels: the same values as in host delivery, buffers that hold
+    something else before are fully overwritten, records past a short batch are left alone, an odd number of anchors."""
+    import cv2
+    import torch
+    from aeon_b200 import kernels as K
+    from aeon_b200.provider import Provider
+    rng = np.random.default_rng(84)
+    recs = []
+    for i in range(3):
+        h, w = int(rng.integers(150, 240)), int(rng.integers(200, 319))
+        png = cv2.imencode(".png", rng.integers(0, 256, (h, w, 3), dtype=np.uint8))[1].tobytes()
+        objs = [{"bndbox": {"xmin": 10 * k, "ymin": 12 * k, "xmax": 10 * k + 70, "ymax": 12 * k + 55}, "name": "a", "difficult": False} for k in range(i + 1)]
+        recs.append((png, json.dumps({"object": objs, "size": {"width": w, "height": h, "depth": 3}}).encode()))
+    cfg = {"batch_size": 4, "random_seed": 3,
+           "etl": [{"type": "image", "height": 248, "width": 328},
+                   dict({"type": "localization_rcnn", "height": 248, "width": 328, "class_names": ["a"], "debug_deterministic": True}, **rc)],
+           "augmentation": [{"type": "image", "fixed_aspect_ratio": True, "fixed_scaling_factor": 1.0, "crop_enable": False}]}
+    want = Provider(ctx, cfg).run_host(recs)
+    prov = Provider(ctx, cfg)
+    outs = {name: torch.full((4,) + dims, 7, dtype=K._TORCH_DTYPE[dt], device="cuda") for name, dims, dt, _ in prov.outputs}
+    torch.cuda.synchronize()
+    for _ in range(4):      # more batches than the provider has buffer sets, into the same outputs
+        prov.run_device(recs, outs)
+        for name, t in outs.items():
+            got = t.cpu().numpy()
+            assert np.array_equal(got[:3], np.asarray(want[name])[:3].reshape(got[:3].shape)), name
+            assert (got[3] == 7).all(), name
