@@ -1057,33 +1057,50 @@ void aeonb_provider::stage_inputs(batch_plan& B, int par)
             }
             remaining[group_of(i)].fetch_sub(1, std::memory_order_release);
         }, !heavy);
-        // the calling thread copies too (it is awake already), then ships the slices as their last job finishes
-        pool->help();
+        // The calling thread copies too (it is awake already) and ships every slice as its last job finishes, so that the copy
+        // engine works while the rest is being staged.
         static const bool trace = std::getenv("AEONB_TRACE") != nullptr;
         if (trace && m_trace[m_trace_slot][3])
             AEONB_CUDA(cudaEventRecord(m_trace[m_trace_slot][3], m_upload));
         cudaError_t copy_error = cudaSuccess;
-        for (int g = 0; g < groups; ++g)
-        {
-            for (int spin = 0; remaining[g].load(std::memory_order_acquire) > 0; ++spin)
-                if (spin > 2000)
-                    std::this_thread::sleep_for(std::chrono::microseconds(20));
-            const size_t begin = offset_of(first[g]);
-            const size_t end   = first[g + 1] < nwork ? offset_of(first[g + 1]) : B.stage_bytes;
-            if (end > begin && copy_error == cudaSuccess && !failure)
+        auto        failed     = [&] {
+            std::lock_guard<std::mutex> lk(failure_mutex);
+            return failure != nullptr;
+        };
+        int  shipped = 0;
+        auto ship    = [&](bool wait) {
+            for (; shipped < groups; ++shipped)
             {
-                copy_error = cudaMemcpyAsync(dstage + begin, hstage + begin, end - begin, cudaMemcpyHostToDevice, m_upload);
-                h2d_bytes += (int64_t)(end - begin);
+                const int g = shipped;
+                for (int spin = 0; remaining[g].load(std::memory_order_acquire) > 0; ++spin)
+                {
+                    if (!wait)
+                        return;
+                    if (spin > 2000)
+                        std::this_thread::sleep_for(std::chrono::microseconds(20));
+                }
+                const size_t begin = offset_of(first[g]);
+                const size_t end   = first[g + 1] < nwork ? offset_of(first[g + 1]) : B.stage_bytes;
+                if (copy_error != cudaSuccess || failed())
+                    continue;
+                if (end > begin)
+                {
+                    copy_error = cudaMemcpyAsync(dstage + begin, hstage + begin, end - begin, cudaMemcpyHostToDevice, m_upload);
+                    h2d_bytes += (int64_t)(end - begin);
+                }
+                if (in_slices && copy_error == cudaSuccess)
+                {
+                    if (!m_slice[g])
+                        copy_error = cudaEventCreateWithFlags(&m_slice[g], cudaEventDisableTiming);
+                    if (copy_error == cudaSuccess)
+                        copy_error = cudaEventRecord(m_slice[g], m_upload);
+                    B.slice_end.push_back(first[g + 1]);
+                }
             }
-            if (in_slices && copy_error == cudaSuccess && !failure)
-            {
-                if (!m_slice[g])
-                    copy_error = cudaEventCreateWithFlags(&m_slice[g], cudaEventDisableTiming);
-                if (copy_error == cudaSuccess)
-                    copy_error = cudaEventRecord(m_slice[g], m_upload);
-                B.slice_end.push_back(first[g + 1]);
-            }
-        }
+        };
+        while (pool->help(1) > 0)
+            ship(false);
+        ship(true);
         pool->wait();
         if (failure)
             std::rethrow_exception(failure);

@@ -63,10 +63,10 @@ namespace aeonb
             m_wake_rest.notify_all();
     }
 
-    int worker_pool::help()
+    int worker_pool::help(int most)
     {
         int ran = 0;
-        for (;;)
+        while (ran < most)
         {
             const int i = m_next.fetch_add(1);
             if (i >= m_count)
@@ -83,6 +83,7 @@ namespace aeonb
             }
             ++ran;
         }
+        return ran;
     }
 
     void worker_pool::wait()

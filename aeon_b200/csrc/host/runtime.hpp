@@ -32,8 +32,9 @@ namespace aeonb
         void start(int count, std::function<void(int)> fn, bool light = false);
         void wait();
         // The calling thread takes part in the job started last: runs fn(i) for indices it draws from the same counter until
-        // none is left.  Returns how many it ran.  (The workers' wake-up takes tens of microseconds; the caller is already awake.)
-        int help();
+        // none is left or it has run `most`.  Returns how many it ran.  (The workers' wake-up takes tens of microseconds; the caller
+        // is already awake.)
+        int help(int most = 1 << 30);
         void run(int count, std::function<void(int)> fn)
         {
             start(count, std::move(fn));
