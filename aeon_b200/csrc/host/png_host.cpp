@@ -1,5 +1,8 @@
 #include "png_host.hpp"
 
+#if defined(__x86_64__)
+#include <tmmintrin.h>
+#endif
 #include <algorithm>
 #include <cstring>
 #include <string>
@@ -82,6 +85,17 @@ namespace aeonb
             int            over = 0; // bytes made up past the end of the data
             inline void refill()
             {
+                if (end - p >= 8)
+                {
+                    // eight bytes at once; the bits of the last, partial one are or-ed in again by the next refill
+                    uint64_t next;
+                    std::memcpy(&next, p, 8);
+                    acc |= next << n;
+                    const int bytes = (63 - n) >> 3;
+                    p += bytes;
+                    n += 8 * bytes;
+                    return;
+                }
                 while (n <= 56)
                 {
                     uint64_t b = 0;
@@ -245,8 +259,16 @@ namespace aeonb
                         const size_t d = k_dist_base[ds] + in.bits(k_dist_extra[ds]);
                         if (d > o || o + len > want)
                             bad("distance too far back or too much data");
-                        for (size_t i = 0; i < len; ++i, ++o) // the ranges may overlap: byte by byte
-                            out[o] = out[o - d];
+                        // the ranges may overlap: the last d bytes are repeated, each copy doubling what there is of them
+                        uint8_t* const to   = out + o;
+                        size_t         done = std::min(d, len);
+                        if (d == 1)
+                            std::memset(to, to[-1], done = len);
+                        else
+                            std::memcpy(to, to - d, done);
+                        for (size_t more; done < len; done += more)
+                            std::memcpy(to + done, to, more = std::min(done, len - done));
+                        o += len;
                     }
                 }
             }
@@ -361,6 +383,36 @@ namespace aeonb
         // integers, the blue weight being what is left of 32768.  8-bit samples are truncated, 16-bit samples rounded.
         constexpr int k_grey_r = 9797, k_grey_g = 19234, k_grey_b = 3737;
 
+        // Every sample three times.  Sixteen samples become three vectors, each picked from them by one byte shuffle.
+#if defined(__x86_64__)
+        __attribute__((target("ssse3"))) int grey_to_bgr_ssse3(const uint8_t* s, int count, uint8_t* o)
+        {
+            const __m128i a = _mm_setr_epi8(0, 0, 0, 1, 1, 1, 2, 2, 2, 3, 3, 3, 4, 4, 4, 5), b = _mm_setr_epi8(5, 5, 6, 6, 6, 7, 7, 7, 8, 8, 8, 9, 9, 9, 10, 10),
+                          c = _mm_setr_epi8(10, 11, 11, 11, 12, 12, 12, 13, 13, 13, 14, 14, 14, 15, 15, 15);
+            int i = 0;
+            for (; i + 16 <= count; i += 16)
+            {
+                const __m128i v = _mm_loadu_si128(reinterpret_cast<const __m128i*>(s + i));
+                __m128i*      t = reinterpret_cast<__m128i*>(o + 3 * static_cast<size_t>(i));
+                _mm_storeu_si128(t, _mm_shuffle_epi8(v, a));
+                _mm_storeu_si128(t + 1, _mm_shuffle_epi8(v, b));
+                _mm_storeu_si128(t + 2, _mm_shuffle_epi8(v, c));
+            }
+            return i;
+        }
+#endif
+        void grey_to_bgr(const uint8_t* s, int count, uint8_t* o)
+        {
+            int i = 0;
+#if defined(__x86_64__)
+            static const bool ssse3 = __builtin_cpu_supports("ssse3");
+            if (ssse3)
+                i = grey_to_bgr_ssse3(s, count, o);
+#endif
+            for (; i < count; ++i)
+                o[3 * static_cast<size_t>(i)] = o[3 * static_cast<size_t>(i) + 1] = o[3 * static_cast<size_t>(i) + 2] = s[i];
+        }
+
         // Writes `count` pixels of one unfiltered row to out[3 * (x0 + i * xstep)].
         void emit_row(const uint8_t* cur, int count, int x0, int xstep, const png_info& info, const chunks& c, int channels,
                       bool grey, uint8_t* out)
@@ -396,6 +448,8 @@ namespace aeonb
                         put(i, s[2 * step], s[step], s[0]);
                 }
             }
+            else if (info.color_type == 0 && info.bit_depth == 8 && xstep == 1) // masks, as a rule
+                grey_to_bgr(cur, count, out + 3 * static_cast<size_t>(x0));
             else if (info.bit_depth >= 8) // grey, grey + alpha, or an 8-bit palette index
             {
                 for (int i = 0; i < count; ++i)

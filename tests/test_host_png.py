@@ -172,3 +172,16 @@ def test_colour_files_read_as_one_channel():
         assert np.array_equal(got, reference(blob, grey=True)), i
         if i not in (2, 3):   # 8-bit files: the pixelmask extractor's IMREAD_ANYDEPTH read gives the same picture
             assert np.array_equal(got, cv2.imdecode(np.frombuffer(blob, np.uint8), cv2.IMREAD_ANYDEPTH)), i
+
+
+@pytest.mark.parametrize("width", [1, 15, 16, 17, 31, 48, 300])
+def test_grey_rows_around_the_vector_width_and_repeats(width):
+    """Rows of 8-bit grey samples are widened sixteen at a time; matches that overlap what they copy (distances 1 to 9 and a
+    whole row) and data that ends within eight bytes of the last code."""
+    import cv2
+    rng = np.random.default_rng(width)
+    for period in (1, 2, 3, 7, 8, 9):
+        img = np.tile(rng.integers(0, 256, period, dtype=np.uint8), width * 6 // period + 1)[:width * 6].reshape(6, width)
+        for level in (0, 1, 9):
+            ok, enc = cv2.imencode(".png", img, [cv2.IMWRITE_PNG_COMPRESSION, level])
+            assert ok and np.array_equal(decode(enc.tobytes()), cv2.imdecode(enc, cv2.IMREAD_COLOR))
