@@ -477,7 +477,22 @@ namespace aeonb
         }
     }
 
-    void png_decode_bgr(const void* data, size_t size, const png_info& info, uint8_t* dst, size_t pitch, bool grey)
+    namespace
+    {
+        // One row to memory that the copy engine reads next and no CPU again: past the caches, from which the engine would have to
+        // fetch it (9 MB of masks took 1.5 ms to upload).  dst is 16-byte aligned; n is rounded up to 16 bytes.
+        void stream_row(uint8_t* dst, const uint8_t* src, size_t n)
+        {
+#if defined(__x86_64__)
+            for (size_t i = 0; i < n; i += 16)
+                _mm_stream_si128(reinterpret_cast<__m128i*>(dst + i), _mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i)));
+#else
+            std::memcpy(dst, src, n);
+#endif
+        }
+    }
+
+    void png_decode_bgr(const void* data, size_t size, const png_info& info, uint8_t* dst, size_t pitch, bool grey, bool for_upload)
     {
         const uint8_t* d = static_cast<const uint8_t*>(data);
         chunks         c;
@@ -517,6 +532,20 @@ namespace aeonb
                 continue;
             const size_t row = (static_cast<size_t>(pw) * bits_pp + 7) / 8;
             unfilter(at, row, ph, bpp);
+            const size_t wide = (static_cast<size_t>(info.width) * 3 + 15) & ~static_cast<size_t>(15);
+            if (for_upload && npass == 1 && ((reinterpret_cast<uintptr_t>(dst) | pitch) & 15) == 0 && pitch >= wide)
+            {
+                std::vector<uint8_t> line(wide);
+                for (int y = 0; y < ph; ++y)
+                {
+                    emit_row(at + static_cast<size_t>(y) * (row + 1) + 1, pw, 0, 1, info, c, channels, grey, line.data());
+                    stream_row(dst + static_cast<size_t>(y) * pitch, line.data(), wide);
+                }
+#if defined(__x86_64__)
+                _mm_sfence();
+#endif
+                return;
+            }
             for (int y = 0; y < ph; ++y)
                 emit_row(at + static_cast<size_t>(y) * (row + 1) + 1, pw, passes[p].x0, passes[p].dx, info, c, channels, grey,
                          dst + static_cast<size_t>(passes[p].y0 + y * passes[p].dy) * pitch);

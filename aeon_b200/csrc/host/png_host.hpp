@@ -29,5 +29,7 @@ namespace aeonb
     // With `grey` the three bytes of a pixel all carry the grey value cv::imdecode(IMREAD_GRAYSCALE / IMREAD_ANYDEPTH)
     // returns: libpng's integer colour -> grey conversion (15-bit weights 9797, 19234, 3737 for R, G, B; truncated for 8-bit
     // samples; for 16-bit samples computed on the 16-bit values with rounding, then cut to the high byte).
-    void png_decode_bgr(const void* data, size_t size, const png_info& info, uint8_t* dst, size_t pitch, bool grey = false);
+    // `for_upload`: dst is staging memory that is read by the copy engine next (rows may be written up to the next 16 bytes).
+    void png_decode_bgr(const void* data, size_t size, const png_info& info, uint8_t* dst, size_t pitch, bool grey = false,
+                        bool for_upload = false);
 }

@@ -1026,7 +1026,7 @@ void aeonb_provider::stage_inputs(batch_plan& B, int par)
                     if (job.png)
                     {
                         png_decode_bgr(job.data, job.size, job.pinfo, reinterpret_cast<uint8_t*>(hstage + job.stage_off), job.pitch,
-                                       job.grey);
+                                       job.grey, true);
                         remaining[group_of(i)].fetch_sub(1, std::memory_order_release);
                         return;
                     }
