@@ -463,10 +463,11 @@ namespace aeonb
         // shared memory while the tables are being built, cleaned of stuffed bytes in place and decoded from
         // there: in global memory nearly every pass had some lane of the warp waiting for L2.
         //
-        // Measured on a B200: one 43 KB stream 0.32 ms at first, 0.27 ms with the selects, 0.23 ms with the stream
-        // in shared memory (435 k cycles: set-up 20 k, copy 25 k, first pass 78 k, four rounds 180 k, storing pass
-        // 115 k, DC 16 k); 256 streams of 25-85 KB (4:2:0, quality 90, crop regions stored), entropy, back end and
-        // image kernel together: 721 -> 639 -> 596 us.
+        // Measured on a B200 (kernel times): one stream of about 40 KB 0.33 ms with branches and the copy in global memory, 0.18 ms
+        // now; 256 streams of up to 55 KB (4:2:0, quality 90, crop regions stored) 0.456 ms, now 0.263 ms.  Phases of a 43 KB
+        // stream, thousand cycles before and after: first pass 83 / 62, rounds 201 / 125 (four of them), storing pass 112 / 107,
+        // copy and marker scan 44 / 26, DC 42 / 19, set-up 30 / 17 (the two last are shorter still since).  Without its stores
+        // the storing pass takes 81, without finding out where blocks go 70: it is bound by the issue of its instructions.
         // A wrong guess falls into step with the true decoder after about 10 blocks on average (the block's
         // position inside the MCU has to match too), and not at all inside flat regions, where every block looks
         // the same: there a chain of segments is settled one round per segment, which is what the slowest streams
@@ -1372,8 +1373,8 @@ namespace aeonb
         // marked doubtful and the serial kernel, launched behind, decodes it anew.
         //
         // Measured on a B200, 32 pictures of 900-1400 pixels a side (4:2:2, quality 92, a marker after every MCU row, 0.3 MB
-        // each): 92.1 ms for a provider batch of them with the serial kernel (91 ms of it in that kernel, one warp per stream), 1.45 ms
-        // with these.  A part of 4 to 16 KB per block fills the chip (about 20 parts per picture) and keeps segments at 160 bytes.
+        // each): 88 ms with the serial kernel (one warp per stream), 0.38 ms with these two; 92.1 and 1.1 ms for a provider batch of them.
+        // A part of 4 to 10 KB per block fills the chip (about 30 parts per picture) and keeps segments at 160 bytes.
         constexpr int RST_THREADS       = 128;
         constexpr int RST_INDEX_THREADS = 1024;
         constexpr int RST_ROOM          = 12 * 1024 + 512; // shared memory for a part's bytes (see jpeg_restart_parts): 5 blocks fit an SM
