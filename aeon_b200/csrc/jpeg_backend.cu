@@ -587,7 +587,8 @@ namespace aeonb
     {
         if (n_work <= 0)
             return cudaSuccess;
-        cudaError_t err = cudaFuncSetAttribute(jpeg_backend_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the most the callers let through, so that threads with smaller pictures do not lower it between this call and the launch
+        cudaError_t err = cudaFuncSetAttribute(jpeg_backend_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (err != cudaSuccess)
             return err;
         jpeg_launch L{descs_dev, work_dev};

@@ -1871,7 +1871,9 @@ namespace aeonb
         {
             const int    threads = jpeg_entropy_block(n, longest);
             const size_t smem = jpeg_entropy_smem(n, threads, longest, most_blocks);
-            cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_parallel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            // always the most a block can have: the setting is the kernel's, and another thread may launch it with another size between
+            // this call and the launch
+            cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_parallel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (err != cudaSuccess)
                 return err;
             jpeg_entropy_parallel_kernel<<<n, threads, smem, stream>>>(descs_dev, min_segment, (uint32_t)smem);

@@ -464,7 +464,8 @@ namespace aeonb
         spec_launch      P{descs_dev, cfg, window_dev, twiddle_dev, filt_start_dev, filt_bin_dev, filt_weight_dev, dct_dev, dct_n, n_out};
         const split_plan S{n1, n2, frames, c1_dev, c2_dev};
         const size_t     smem = split_smem(n1, n2, frames);
-        cudaError_t      err  = cudaFuncSetAttribute(specgram_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the most any frame length takes, so that threads with other lengths do not lower it between this call and the launch
+        cudaError_t      err  = cudaFuncSetAttribute(specgram_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 216 * 1024);
         if (err != cudaSuccess)
             return err;
         dim3 grid((cfg.max_time_steps + frames - 1) / frames, n, 1);
