@@ -1824,12 +1824,11 @@ namespace aeonb
 
     void jpeg_restart_parts(const aeonb_entropy_desc* descs, int n, std::vector<int4>& parts)
     {
+        // A stream of no bytes gets its parts too: the serial kernel reads the header that the index kernel writes.
         uint64_t total = 0;
         for (int i = 0; i < n; ++i)
             if (descs[i].scratch && descs[i].restart_interval > 0)
                 total += descs[i].scan_size;
-        if (total == 0)
-            return;
         // Five blocks of a part fit an SM; parts of less than 4 KB are mostly set-up, parts of more than 12 KB do not fit its
         // shared memory.
         const uint64_t target = std::min<uint64_t>(std::max<uint64_t>(total / (148 * 5), 4096), 10240);

@@ -233,3 +233,55 @@ def test_block_sizes_on_either_side_of_a_stream_per_sm(ctx, golden_dir, copies):
     assert len(blobs[2]) > 115_000
     for blob in blobs if copies == 1 else [None]:
         check(ctx, [blob] if blob else [blobs[i % len(blobs)] for i in range(copies)])
+
+
+def decode_descs(ctx, blobs, rois=None, lead=0, scratch=True, scan_bytes=None):
+    """Entropy decode with the descriptors in hand: (status, [planes], work area, descriptor) of every record.  `lead`: offset of a scan from a
+    16-byte boundary; `scan_bytes`: cuts the scans off; work areas are zeroed before."""
+    import torch
+    from aeon_b200 import _lib as L
+    lib, dev = ctx.lib, torch.device("cuda", ctx.device)
+    descs = (L.EntropyDesc * len(blobs))()
+    status = torch.full((len(blobs),), -1, dtype=torch.int32, device=dev)
+    keep, out = [], []
+    for i, (d, blob) in enumerate(zip(descs, blobs)):
+        info, quant, tables, off = L.JpegInfo(), np.zeros(192, np.uint16), np.zeros(1088, np.uint8), C.c_size_t()
+        buf = (C.c_char * len(blob)).from_buffer_copy(blob)
+        L.check(lib.aeonb_jpeg_entropy_prepare(buf, len(blob), C.byref(info), quant.ctypes.data_as(C.POINTER(C.c_uint16)),
+                                               tables.ctypes.data_as(C.POINTER(C.c_uint8)), C.byref(d), C.byref(off)))
+        d.scan_size = d.scan_size if scan_bytes is None else min(d.scan_size, scan_bytes)
+        scan = np.full(d.scan_size + 64, 0xFF, np.uint8)
+        scan[lead:lead + d.scan_size] = np.frombuffer(blob, np.uint8)[off.value:off.value + d.scan_size]
+        scan, tables = torch.from_numpy(scan).to(dev), torch.from_numpy(tables).to(dev)
+        for k in range(4 if rois else 0):
+            d.roi[k] = rois[i][k]
+        planes = [torch.full(((d.roi[2] - d.roi[0]) * d.hs[c] * (d.roi[3] - d.roi[1]) * d.vs[c] * 64,), 0x5555, dtype=torch.int16, device=dev)
+                  for c in range(info.ncomp)]
+        for c, p in enumerate(planes):
+            d.coef[c] = p.data_ptr()
+        d.scan, d.tables, d.status = scan.data_ptr() + lead, tables.data_ptr(), status.data_ptr() + 4 * i
+        d.scratch_bytes = int(lib.aeonb_jpeg_entropy_scratch_bytes(C.byref(d)))
+        work = torch.zeros(d.scratch_bytes, dtype=torch.uint8, device=dev)
+        d.scratch = work.data_ptr() if scratch else None
+        keep += [scan, tables]
+        out.append((planes, work))
+    torch.cuda.synchronize(dev)
+    L.check(lib.aeonb_jpeg_entropy_batch(ctx.handle, descs, len(blobs)))
+    ctx.synchronize()
+    return [(int(s), [p.cpu().numpy() for p in planes], work.cpu().numpy(), d)
+            for s, (planes, work), d in zip(status.cpu().numpy(), out, descs)]
+
+
+@pytest.mark.parametrize("interval", [1, 3, 1000])
+def test_restart_streams_without_a_byte_of_data(ctx, interval):
+    """A file with restart markers that ends behind its scan header, alone in a batch and beside a whole one: whatever the work area
+    holds, the status is the serial decoder's."""
+    import cv2
+    blob = jpeg_bytes(gradient_image(np.random.default_rng(70), 64, 96), 90, [cv2.IMWRITE_JPEG_RST_INTERVAL, interval])
+    want = decode_descs(ctx, [blob], scratch=False, scan_bytes=0)[0]
+    for lead in (0, 5):
+        for got in (decode_descs(ctx, [blob], lead=lead, scan_bytes=0), decode_descs(ctx, [blob] * 3, lead=lead, scan_bytes=0)):
+            for status, planes, _, _ in got:
+                assert status == want[0]
+                assert status != 0 or all(np.array_equal(a, b) for a, b in zip(planes, want[1]))
+    assert want[0] == (1 if interval < 1000 else 0)
