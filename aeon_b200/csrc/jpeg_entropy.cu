@@ -1136,8 +1136,8 @@ namespace aeonb
             clean_writer<RESIDENT> copy{room, out, 0, 0};
             for (uint32_t tile = 0, odd = 0; tile < nv; tile += T, odd ^= 1)
             {
-                // bit b of `keep` = byte b is part of the data, of `marker` = byte b is non-zero and follows 0xFF; the byte before
-                // the stream is not 0xFF
+                // bit b of `keep` = byte b is part of the data, of `marker` = byte b (16: of the next vector) is non-zero and follows
+                // 0xFF; the byte before the stream is not 0xFF
                 const uint32_t i = tile + tid;
                 uint32_t       w[4] = {0, 0, 0, 0}, keep = 0, marker = 0;
                 if (i < nv)
@@ -1170,6 +1170,10 @@ namespace aeonb
                             prev = v;
                         }
                     }
+                    // The second byte of a marker whose first is the tile's last lies in the next tile, which is too late.
+                    if (tid == T - 1 && i + 1 < nv && w[3] >> 24 == 0xFF)
+                        marker |= (uint32_t)((RESIDENT ? reinterpret_cast<const uint8_t*>(room)[16 * i + 16]
+                                                       : __ldg(reinterpret_cast<const uint8_t*>(vec) + 16 * i + 16)) != 0) << 16;
                 }
                 if (RESIDENT && tid == T - 1)
                     S.tile_end[odd] = w[3] >> 24;

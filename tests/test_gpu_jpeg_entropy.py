@@ -285,3 +285,68 @@ def test_restart_streams_without_a_byte_of_data(ctx, interval):
                 assert status == want[0]
                 assert status != 0 or all(np.array_equal(a, b) for a, b in zip(planes, want[1]))
     assert want[0] == (1 if interval < 1000 else 0)
+
+
+def coded_grey(rng, size, whole):
+    """A grey JPEG whose entropy-coded data takes `size` bytes: its table gives the end of a block nine bits, eight ones and a zero.  Without
+    the end of the last block (`whole` false) the data ends at a byte's end just in front of it."""
+    dc = [("00", 0), ("01", 1), ("10", 5)]
+    ac = [("0", 0x01), ("10", 0x02), ("110", 0x11), ("1110", 0x03), ("11110", 0x04), ("111110", 0x22), ("1111110", 0x05), ("11111110", 0x31)]
+    plain = [a for a in ac if a[1] < 16]
+    out, bits, blocks = bytearray(), "", 0
+
+    def put(code, value_bits=0):
+        nonlocal bits
+        bits += code + (format(int(rng.integers(1 << value_bits)), "b").zfill(value_bits) if value_bits else "")
+        while len(bits) >= 8:
+            out.append(int(bits[:8], 2))
+            if out[-1] == 0xFF:
+                out.append(0)
+            bits = bits[8:]
+
+    def symbol(table):
+        code, sym = table[rng.integers(len(table))]
+        put(code, sym & 15)
+
+    while len(out) < size - (20 if size < 10000 else 60):
+        symbol(dc)
+        for _ in range(rng.integers(0, 6) if size < 10000 else 55):      # a picture has at most 8191 blocks in a row
+            symbol(ac if size < 10000 else plain)
+        put("111111110")
+        blocks += 1
+    kept = bytes(out), bits
+    while True:      # the last block: symbols until the data ends where it should
+        out[:], bits = kept
+        symbol(dc)
+        for _ in range(60):
+            if len(out) == size and (not whole) and bits == "":
+                break
+            if whole and len(out) + 3 > size:
+                put("111111110")
+                if bits:
+                    put("1" * (8 - len(bits)))
+                break
+            symbol(plain)
+        if len(out) == size and bits == "":
+            break
+    blocks += 1
+    mark = lambda m, body: bytes([0xFF, m]) + (len(body) + 2).to_bytes(2, "big") + body  # noqa: E731
+    dht = lambda cls, lens, syms: mark(0xC4, bytes([cls]) + bytes(lens + [0] * (16 - len(lens))) + bytes(syms))  # noqa: E731
+    return (b"\xff\xd8" + mark(0xDB, bytes([0]) + bytes([1] * 64)) +
+            mark(0xC0, bytes([8, 0, 8]) + (8 * blocks).to_bytes(2, "big") + bytes([1, 1, 0x11, 0])) +
+            dht(0x00, [0, 3], [s for _, s in dc]) + dht(0x10, [1] * 9, [s for _, s in ac] + [0]) +
+            mark(0xDA, bytes([1, 1, 0, 0, 63, 0])) + bytes(out) + b"\xff\xd9" + bytes(20))
+
+
+@pytest.mark.parametrize("tile", [2048, 4096, 13 * 16384])
+def test_streams_that_end_at_the_edge_of_a_tile(ctx, tile):
+    """The end marker at every place around a multiple of the bytes a block copies at a time (128 threads for a short stream; 1024 and the
+    copy in the work area for the long one): a whole stream decodes, one cut short in front of its last code is reported, also where the
+    marker's first byte is the last of a tile."""
+    rng = np.random.default_rng(tile)
+    for size, lead in [(tile - 2, 0), (tile - 1, 0), (tile, 0), (tile - 1 - 6, 6), (tile - 1 - 15, 15)][:5 if tile < 10000 else 3]:
+        blob = coded_grey(rng, size, True)
+        (status, planes, _, _), = decode_descs(ctx, [blob], lead=lead)
+        assert status == 0 and np.array_equal(planes[0], host_planes(blob)[1][0][:planes[0].size]), (size, lead)
+        (status, _, _, _), = decode_descs(ctx, [coded_grey(rng, size, False)], lead=lead)
+        assert status == 1, (size, lead)
