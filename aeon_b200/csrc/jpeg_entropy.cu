@@ -1592,6 +1592,8 @@ namespace aeonb
             par_state&         S   = R.S;
             const uint32_t     tid = threadIdx.x, ri = (uint32_t)S.d.restart_interval;
             auto first_block = [&](uint32_t i) { return (uint32_t)min((uint64_t)needed_mcus, (uint64_t)(first + i) * ri) * (uint32_t)bpm; };
+            // interval i goes on below the region
+            auto cut = [&](uint32_t i) { return needed_mcus < min((uint64_t)S.d.mcux * S.d.mcuy, (uint64_t)(first + i + 1) * ri); };
             // an interval has ceil(its bytes / seg) segments; I < T of them are shorter than seg, so this many fit
             uint32_t seg = (clean_size + (T - I) - 1) / (T - I);
             seg          = max((seg + 3u) & ~3u, (uint32_t)max(min_segment, 64) & ~3u);
@@ -1648,8 +1650,8 @@ namespace aeonb
                 const uint32_t   g = A.ext_p[t] + before, gend = first_block(i + 1);
                 const seg_result r = run_segment<true, Words>(S, words, p0, bk >> 8, bk & 255, min(seg_end, at + step), g, gend, dcdiff, nullptr, 0,
                                                               0, 0, false, 0);
-                // the interval's last block leaves less than a byte
-                if (r.bad || (r.blocks > 0 && g + r.blocks == gend && (r.p > all_end || all_end - r.p > 7)))
+                // the interval's last block leaves less than a byte, unless the region ends in front of that block
+                if (r.bad || (r.blocks > 0 && g + r.blocks == gend && (r.p > all_end || (all_end - r.p > 7 && !cut(i)))))
                     S.bad = 1;
             }
             __syncthreads();

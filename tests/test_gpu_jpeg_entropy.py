@@ -350,3 +350,25 @@ def test_streams_that_end_at_the_edge_of_a_tile(ctx, tile):
         assert status == 0 and np.array_equal(planes[0], host_planes(blob)[1][0][:planes[0].size]), (size, lead)
         (status, _, _, _), = decode_descs(ctx, [coded_grey(rng, size, False)], lead=lead)
         assert status == 1, (size, lead)
+
+
+def left_to_the_serial_decoder(work, d):
+    """The first word of the work area's header: not 0 where the interval decoder has given a stream up."""
+    mcus, bpm = d.mcux * d.mcuy, sum(d.hs[c] * d.vs[c] for c in range(d.ncomp))
+    intervals = -(-mcus // d.restart_interval)
+    parts = intervals if intervals < 96 else intervals // 64 + 96
+    at = (d.scan_size + 64 * (parts + 2) + 15) // 16 * 16 + (mcus * bpm * 2 + 15) // 16 * 16
+    return int(work[at:at + 4].view(np.uint32)[0])
+
+
+@pytest.mark.parametrize("interval", [2, 7, 13, 40, 64, 1000])
+def test_regions_that_end_inside_a_restart_interval(ctx, interval):
+    """A region whose last row is not the end of an interval: the rest of that interval is not looked at, and the stream stays with the
+    interval decoder.  Every last row of a picture of 13 x 9 MCUs, and the same planes as the host decoder."""
+    import cv2
+    blob = jpeg_bytes(gradient_image(np.random.default_rng(71), 9 * 16 - 3, 13 * 16 - 5), 90, [cv2.IMWRITE_JPEG_RST_INTERVAL, interval])
+    rois = [(x0, y0, x1, y1) for y1 in range(1, 10) for x0, x1, y0 in ((0, 13, 0), (3, 9, y1 // 2))]
+    for roi, (status, planes, work, d) in zip(rois, decode_descs(ctx, [blob] * len(rois), rois)):
+        _, want, _ = host_planes(blob, roi)
+        assert status == 0 and all(np.array_equal(p, w[:p.size]) for p, w in zip(planes, want)), roi
+        assert left_to_the_serial_decoder(work, d) == 0, roi
