@@ -27,7 +27,6 @@
 // this file is compiled with -fmad=false and uses explicit fused operations only where
 // OpenCV's own code is fused.
 #include <algorithm>
-#include <atomic>
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
@@ -44,6 +43,7 @@ namespace aeonb
     {
         constexpr int AUG_MAX_THREADS = 224;
         constexpr int AUG_MAX_BAND    = 8;  // portable cluster size limit
+        constexpr int AUG_MAX_SMEM    = 200 * 1024; // most dynamic shared memory of a launch
         constexpr int AUG_MAX_GROUP   = 16; // source rows staged per group, at most
         constexpr int AUG_STAGE_PAD   = 16; // bytes kept free before and after a staged row
 
@@ -838,20 +838,10 @@ namespace aeonb
                                  cudaStream_t stream)
         {
             auto kern = pix == 4 ? aug_pack_kernel<T, 4> : aug_pack_kernel<T, 3>;
-            // the dynamic shared-memory limit of a kernel is a per-device setting: raised only when a launch needs more
-            static std::atomic<int> limit[2][64];
-            int                     device = 0;
-            cudaError_t             err    = cudaGetDevice(&device);
+            // the most launch_aug_pack lets through, so that threads with smaller tiles do not lower it between this call and the launch
+            cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AUG_MAX_SMEM);
             if (err != cudaSuccess)
                 return err;
-            std::atomic<int>& have = limit[pix == 4][device & 63];
-            if ((int)smem > have.load(std::memory_order_relaxed))
-            {
-                err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (err != cudaSuccess)
-                    return err;
-                have.store((int)smem, std::memory_order_relaxed);
-            }
             cudaLaunchConfig_t cfg = {};
             cfg.gridDim            = dim3(bands, clusters, 1);
             cfg.blockDim           = dim3(threads, 1, 1);
@@ -905,7 +895,7 @@ namespace aeonb
         // contrast step needs (the per-image mean travels through distributed shared memory).  Larger outputs (a
         // 1000 x 1000 detection input, say) take more, independent bands -- possible whenever no record of the batch
         // changes the contrast.
-        while (smem_for(bands) > 200 * 1024 && bands < 256 && layout.slot_h / (bands * 2) >= 1)
+        while (smem_for(bands) > AUG_MAX_SMEM && bands < 256 && layout.slot_h / (bands * 2) >= 1)
             bands *= 2;
         // Few records leave SMs idle with 8 bands each, so they get more, until there are about four CTAs for every SM or a band
         // has four rows (the row shared with the next band is read twice).  Kernel times: one picture 26.6 -> 14.4 us, 32 of 300 x 300
@@ -926,7 +916,7 @@ namespace aeonb
         L.vector_ok = slots_aligned && layout.stride_x == 1 && (layout.stride_y * elem) % 16 == 0 &&
                       (layout.stride_c * elem) % 16 == 0;
         const size_t smem = smem_for(bands);
-        if (smem > 200 * 1024)
+        if (smem > AUG_MAX_SMEM)
         {
             *why = "output image too large for the on-chip band tile (one row of width * 3 bytes must stay under 200 KB)";
             return cudaErrorInvalidValue;

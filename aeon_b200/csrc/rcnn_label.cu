@@ -260,7 +260,8 @@ extern "C" int aeonb_rcnn_label_batch(aeonb_ctx* ctx, const float* anchors_dev, 
         if (n_anchors <= 65535)
         {
             const size_t smem = ((size_t)n_anchors * sizeof(uint16_t) + 15) & ~(size_t)15;
-            e = cudaFuncSetAttribute(rcnn_label_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            // the most any anchor count takes, so that threads with fewer anchors do not lower it between this call and the launch
+            e = cudaFuncSetAttribute(rcnn_label_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
             if (e == cudaSuccess)
                 rcnn_label_kernel<true><<<n, RCNN_THREADS, smem, ctx->stream>>>(L);
         }

@@ -483,7 +483,8 @@ namespace aeonb
     {
         spec_launch  P{descs_dev, cfg, window_dev, twiddle_dev, filt_start_dev, filt_bin_dev, filt_weight_dev, dct_dev, dct_n, n_out};
         const size_t smem = specgram_generic_smem(cfg.frame_length);
-        cudaError_t  err  = cudaFuncSetAttribute(specgram_generic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // the most specgram_tables lets through, for the same reason as above
+        cudaError_t  err  = cudaFuncSetAttribute(specgram_generic_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (err != cudaSuccess)
             return err;
         dim3 grid((cfg.max_time_steps + SPEC_GENERIC_WARPS - 1) / SPEC_GENERIC_WARPS, n, 1);

@@ -2,6 +2,8 @@
 
 Bar: bit-exact for uint8 outputs (geometry and photometric alike, since the oracle restates
 OpenCV's integer / float32 arithmetic), 1e-6 absolute for standardised float outputs."""
+import os
+
 import numpy as np
 import pytest
 import torch
@@ -10,6 +12,7 @@ from oracle import image_ops as ops
 from tests.synth import gradient_image
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 def run_kernel(ctx, srcs, params, slot_w, slot_h, output_type="uint8_t", channel_major=True, bgr_to_rgb=False,
@@ -213,3 +216,54 @@ def test_invalid_descriptors_are_rejected(ctx):
     big = ops.ImageParams(cropbox=(0, 0, 32, 32), output_size=(40, 16))
     with pytest.raises(AeonError, match="does not fit"):
         run_kernel(ctx, [src], [big], 16, 16)
+
+
+
+SIZES_AT_ONCE = """
+import sys, threading
+import numpy as np, torch
+from aeon_b200 import kernels as K
+from oracle import image_ops as ops
+from tests.test_gpu_specgram import run as specgram
+barrier, failures = threading.Barrier(4), []
+rng = np.random.default_rng(0)
+src = torch.from_numpy(rng.integers(0, 256, (64, 64, 4), dtype=np.uint8)).cuda()
+clip = rng.integers(-999, 999, 12000, dtype=np.int16)
+box = np.array([[10, 10, 60, 60]], np.float32)
+
+def work(size, frame, anchors):
+    ctx = K.Context(0)
+    def attempt(what, fn):
+        torch.cuda.synchronize()
+        barrier.wait(60)
+        try:
+            fn()
+        except Exception as e:
+            failures.append((what, str(e)))
+    for dt in K._TORCH_DTYPE:
+        for stride in (3, 4):
+            out = torch.zeros((1, size, size, 3), dtype=K._TORCH_DTYPE[dt], device="cuda")
+            lay = K.make_layout(size, size, dt, False)
+            p = ops.ImageParams(cropbox=(0, 0, 64, 64), output_size=(size, size))
+            attempt(("image", size, dt, stride), lambda: (K.image_batch(ctx, [src[:, :, :stride].contiguous()], [p], out, lay), ctx.synchronize()))
+    for _ in range(20):
+        attempt(("specgram", frame), lambda: specgram(ctx, [clip], frame_length=frame, frame_stride=frame, max_time_steps=2, num_filters=0))
+        attempt(("rcnn", anchors), lambda: K.rcnn_label_batch(ctx, np.tile(box, (anchors, 1)), [box], [(100, 100)]))
+
+threads = [threading.Thread(target=work, args=a) for a in ((32, 131, 100), (400, 6007, 60000), (240, 1009, 30000), (64, 257, 25600))]
+[t.start() for t in threads]
+[t.join() for t in threads]
+print(len(failures), failures[:4])
+sys.exit(1 if failures else 0)
+"""
+
+
+def test_launches_of_several_sizes_at_once(ctx):
+    """Four threads with contexts of their own launch every variant of the image kernel for the first time in the process, and the
+    direct-sum spectrogram and the anchor kernel, each with another amount of shared memory: no thread's launch may find the limit that
+    another has set for a smaller one."""
+    import subprocess
+    import sys
+    for _ in range(3):
+        done = subprocess.run([sys.executable, "-c", SIZES_AT_ONCE], capture_output=True, text=True, timeout=180, cwd=ROOT)
+        assert done.returncode == 0, done.stdout[-2000:] + done.stderr[-2000:]
