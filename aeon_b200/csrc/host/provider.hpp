@@ -273,7 +273,7 @@ private:
     // the phases of run()
     void plan_records(aeonb::batch_plan& plan, const void* const* elems, const size_t* sizes, int n);
     void reserve_arenas(aeonb::batch_plan& plan, void* const* outs, bool on_device, int par);
-    void stage_inputs(aeonb::batch_plan& plan, int par);
+    void stage_inputs(aeonb::batch_plan& plan, int par, bool alone);
     void launch_kernels(aeonb::batch_plan& plan, void* const* outs, int n, int par);
     void deliver(aeonb::batch_plan& plan, void* const* outs, int n, bool on_device, int par, int64_t ticket);
 };

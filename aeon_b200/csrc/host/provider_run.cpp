@@ -418,7 +418,10 @@ void aeonb_provider::process(batch_job& job)
     }
     reserve_arenas(B, job.outs.data(), on_device, par);
     mark(2);
-    stage_inputs(B, par); // host work on the pool, uploads
+    const bool alone = T == 1 || cudaEventQuery(m_done[(T - 1) % k_events]) != cudaErrorNotReady; // no earlier batch is under way
+    if (!alone)
+        cudaGetLastError(); // not ready is no error
+    stage_inputs(B, par, alone); // host work on the pool, uploads
     mark(3);
     launch_kernels(B, job.outs.data(), n, par);
     mark(4);
@@ -981,7 +984,8 @@ void aeonb_provider::reserve_arenas(batch_plan& B, void* const* outs, bool on_de
 
 // Phase 3: the worker pool fills the pinned staging buffer (compressed scans and tables, or coefficient planes when
 // Huffman decoding runs on the host; audio samples), shipped to the device in slices while the pool is still working.
-void aeonb_provider::stage_inputs(batch_plan& B, int par)
+// `alone`: no earlier batch is under way.
+void aeonb_provider::stage_inputs(batch_plan& B, int par, bool alone)
 {
     cudaStream_t st = ctx->stream;
     // ---- 3. entropy decode on the pool, shipping finished slices while the rest decode
@@ -996,11 +1000,13 @@ void aeonb_provider::stage_inputs(batch_plan& B, int par)
     {
         const int                     groups = std::max(1, std::min(k_slices, nwork));
         // A batch of nothing but clips: the spectrogram kernel of a slice runs while the next slices are on their way.  Under
-        // 2 MB the copy takes about as long as the launches that this adds.
+        // 2 MB the copy takes about as long as the launches that this adds.  Behind a batch that is still under way it gains
+        // nothing, since that one's kernel runs beside the upload already, and the launches cost: with four batches in flight 32 clips
+        // (400-sample frames, 13 cepstra) take 266 us in slices and 190 us in one launch, 64 clips (320, 64 filters) 490 and 420 us.
         int clip_stages = 0;
         for (const auto& d : B.sdescs)
             clip_stages += !d.empty();
-        const bool in_slices = njobs == 0 && clip_stages == 1 && B.stage_bytes >= (size_t)2 << 20;
+        const bool in_slices = alone && njobs == 0 && clip_stages == 1 && B.stage_bytes >= (size_t)2 << 20;
         vector<std::atomic<int>>      remaining(groups);
         vector<int>                   first(groups + 1);
         for (int g = 0; g <= groups; ++g)

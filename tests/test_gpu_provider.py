@@ -688,3 +688,23 @@ def test_audio_batches_uploaded_in_slices(ctx):
             fin = np.isfinite(want)
             assert np.array_equal(np.isfinite(g), fin)
             assert np.all(np.abs(g[fin] - want[fin]) <= 1e-4 * np.abs(want[fin]) + 2e-4)
+
+
+def test_audio_slices_only_when_no_earlier_batch_is_under_way(ctx):
+    """One call at a time takes a launch per slice; behind a batch whose direct sums (331 is a prime) are still being computed one launch
+    does.  The same rows either way."""
+    rng = np.random.default_rng(92)
+    cfg = {"batch_size": 11, "etl": [{"type": "audio", "frame_length": 331, "frame_stride": 160, "max_samples": 240000, "num_filters": 40,
+                                      "sample_rate": 16000, "window_type": "hann", "feature_type": "mfsc"}]}
+    prov = make_provider(ctx, cfg)
+    batches = [[((rng.normal(0, 2000, int(n))).astype(np.int16).tobytes(),) for n in rng.integers(120000, 240000, 11)] for _ in range(3)]
+    want = []
+    for b in batches:
+        want.append(prov.run_host(b)["audio"])
+        assert prov.stats()["launches"] == 8
+    outs = [{"audio": np.zeros_like(want[0])} for _ in range(6)]
+    for t in [prov.submit_host(batches[i % 3], outs[i]) for i in range(6)]:
+        prov.wait(t)
+    assert prov.stats()["launches"] == 1
+    for i, o in enumerate(outs):
+        assert np.array_equal(o["audio"], want[i % 3])
