@@ -1237,13 +1237,14 @@ void aeonb_provider::launch_kernels(batch_plan& B, void* const* outs, int n, int
             static const bool trace = std::getenv("AEONB_TRACE") != nullptr;
             if (trace && m_trace[m_trace_slot][5])
                 AEONB_CUDA(cudaEventRecord(m_trace[m_trace_slot][5], ectx->stream));
+            const int64_t launched = ectx->launches;
             check_status(aeonb_jpeg_entropy_batch(ectx, ed.data(), B.n_device_jobs));
             h2d_bytes += (int64_t)(sizeof(aeonb_entropy_desc) * B.n_device_jobs);
             if (trace && m_trace[m_trace_slot][6])
                 AEONB_CUDA(cudaEventRecord(m_trace[m_trace_slot][6], ectx->stream));
             if (ectx != ctx)
             {
-                ctx->launches += 1;
+                ctx->launches += ectx->launches - launched;
                 AEONB_CUDA(cudaEventRecord(m_entropy_done[par], ectx->stream));
                 AEONB_CUDA(cudaStreamWaitEvent(st, m_entropy_done[par], 0));
             }

@@ -299,6 +299,18 @@ def test_device_and_host_entropy_decoding_give_identical_batches(ctx):
         assert a.stats()["launches"] == b.stats()["launches"] + 1
 
 
+def test_launch_count_of_streams_with_restart_markers(ctx):
+    """Index, interval and serial kernel, back end and image kernel; with plain streams in the batch the block-parallel kernel too."""
+    import cv2
+    rng = np.random.default_rng(54)
+    imgs = [gradient_image(rng, 90, 120) for _ in range(3)]
+    plain, marked = ([(jpeg_bytes(img, 90, extra),) for img in imgs] for extra in ([], [cv2.IMWRITE_JPEG_RST_INTERVAL, 4]))
+    prov = make_provider(ctx, {"batch_size": 3, "etl": [{"type": "image", "height": 48, "width": 64, "output_type": "uint8_t"}]})
+    for recs, launches in ((plain, 3), (marked, 5), (plain[:1] + marked[:2], 6)):
+        prov.run_host(recs)
+        assert prov.stats()["launches"] == launches
+
+
 def test_device_entropy_decoding_reports_malformed_streams(ctx):
     cfg = {"batch_size": 2, "random_seed": 34, "entropy_decode": "device",
            "etl": [{"type": "image", "height": 64, "width": 64, "output_type": "uint8_t"}], "augmentation": [{"type": "image"}]}
