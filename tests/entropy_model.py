@@ -1,7 +1,8 @@
 """Model of the bookkeeping of the block-parallel JPEG entropy kernel (aeon_b200/csrc/jpeg_entropy.cu): segments, guessed
 entry states, checkpoints, rounds of re-decoding with an early exit at a checkpoint passed in a noted state, block counts,
 and the storing pass dealt out in pieces between checkpoints.  Plain python over the bit string of a baseline JPEG; the
-kernel follows the same steps.  `simulate` returns what the kernel would count and every inconsistency it finds: a segment
+kernel follows the same steps (it takes AC symbols in pairs where the first cannot reach the place a run looks for, which comes to the
+same).  `simulate` returns what the kernel would count and every inconsistency it finds: a segment
 whose block count differs from the true one, a piece that would start at a wrong block number or meet an invalid symbol, a
 checkpoint the storing pass needs that no run has written.  Test infrastructure only."""
 import numpy as np
@@ -87,6 +88,8 @@ def simulate(blob, threads=512, checkpoint_past_end=False):
     block_ends = np.array(block_ends)
 
     seg = max((-(-len(clean) // threads) + 3) & ~3, MIN_SEGMENT)
+    deals = max(((NCHECK + 1) * -(-len(clean) // seg) * 4 + 3 * threads) // (4 * threads), 1)   # rounds of the storing pass
+    seg = max(seg, ((NCHECK + 1) * len(clean) // (deals * threads) + 4) & ~3)                   # no nearly empty last one
     nseg = -(-len(clean) // seg)
     step = seg * 8 // (NCHECK + 1)
 

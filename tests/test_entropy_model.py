@@ -36,3 +36,17 @@ def test_random_streams_in_every_sampling_mode_and_block_size(seed):
         assert ok
         r = simulate(enc.tobytes(), threads=int(rng.choice([512, 256, 128])))
         assert r["counted"] == r["total_blocks"] and not r["problems"], (seed, k, r)
+
+
+@pytest.mark.parametrize("quality", [75, 95])
+def test_a_thread_for_every_piece_of_the_storing_pass(golden_dir, quality):
+    """1024 threads, as for streams that have an SM to themselves: segments are lengthened so that the pieces fill whole rounds."""
+    rng = np.random.default_rng(quality)
+    blobs = [open(os.path.join(golden_dir, "entropy_stream_507_segments.jpg"), "rb").read()] if quality == 95 else []
+    for h, w in ((300, 420), (500, 375), (90, 60)):
+        blobs.append(cv2.imencode(".jpg", gradient_image(rng, h, w), [cv2.IMWRITE_JPEG_QUALITY, quality])[1].tobytes())
+    for blob in blobs:
+        r = simulate(blob, threads=1024)
+        assert r["counted"] == r["total_blocks"] and not r["problems"], r
+        pieces = 4 * r["segments"]
+        assert pieces <= 1024 or r["segment"] == 160 or pieces % 1024 == 0 or pieces % 1024 > 256, r
