@@ -192,3 +192,18 @@ def test_422_and_420_rows_at_the_edges_of_the_eight_pixel_groups(ctx, pitch_step
         got = out.cpu().numpy()
         assert np.array_equal(got[:-1, :d.width * 3].reshape(want.shape), want), (want.shape, d.dst_pitch)
         assert (got[-1] == 77).all()
+
+
+@pytest.mark.parametrize("mode,widest", [("420", 3440), ("422", 5376), ("444", 3584), (None, 10752)])
+def test_pictures_as_wide_as_two_mcu_rows_in_shared_memory_allow(ctx, mode, widest):
+    """The sample planes of two MCU rows and the warps' 32 KB of coefficients take 200 KB at most: 50 bytes a column in 4:2:0, 32 in 4:2:2,
+    48 in 4:4:4, 16 in grey.  The widest picture decodes, the next one is refused."""
+    import cv2
+    from aeon_b200._lib import AeonError
+    rng = np.random.default_rng(25)
+    extra = [cv2.IMWRITE_JPEG_SAMPLING_FACTOR, getattr(cv2, "IMWRITE_JPEG_SAMPLING_FACTOR_" + mode)] if mode else []
+    blobs = [jpeg_bytes(gradient_image(rng, 40, w) if mode else gradient_image(rng, 40, w)[..., 0], 90, extra) for w in (widest, widest - 5, widest + 1)]
+    for got, blob in zip(decode_gpu(ctx, blobs[:2]), blobs):
+        assert np.array_equal(got, cv2.imdecode(np.frombuffer(blob, np.uint8), cv2.IMREAD_COLOR))
+    with pytest.raises(AeonError, match="too wide"):
+        decode_gpu(ctx, blobs[2:])
