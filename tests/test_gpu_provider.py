@@ -703,8 +703,9 @@ def test_audio_batches_uploaded_in_slices(ctx):
 
 
 def test_audio_slices_only_when_no_earlier_batch_is_under_way(ctx):
-    """One call at a time takes a launch per slice; behind a batch whose direct sums (331 is a prime) are still being computed one launch
-    does.  The same rows either way."""
+    """One call at a time takes a launch per slice; behind a batch that cannot have finished (a tenth of a second of other work lies in
+    front of its kernels) one launch does.  The same rows either way."""
+    import torch
     rng = np.random.default_rng(92)
     cfg = {"batch_size": 11, "etl": [{"type": "audio", "frame_length": 331, "frame_stride": 160, "max_samples": 240000, "num_filters": 40,
                                       "sample_rate": 16000, "window_type": "hann", "feature_type": "mfsc"}]}
@@ -714,9 +715,17 @@ def test_audio_slices_only_when_no_earlier_batch_is_under_way(ctx):
     for b in batches:
         want.append(prov.run_host(b)["audio"])
         assert prov.stats()["launches"] == 8
-    outs = [{"audio": np.zeros_like(want[0])} for _ in range(6)]
-    for t in [prov.submit_host(batches[i % 3], outs[i]) for i in range(6)]:
+    outs = [{"audio": torch.zeros(want[0].shape, device="cuda")} for _ in range(3)]
+    big = torch.zeros(1 << 28, device="cuda")
+    torch.cuda.synchronize()
+    with torch.cuda.stream(ctx.torch_stream):
+        for _ in range(300):
+            big.add_(1.0)
+    tickets = [prov.submit_device(b, o) for b, o in zip(batches[:2], outs)]
+    for t in tickets:
         prov.wait(t)
     assert prov.stats()["launches"] == 1
-    for i, o in enumerate(outs):
-        assert np.array_equal(o["audio"], want[i % 3])
+    prov.wait(prov.submit_device(batches[2], outs[2]))
+    assert prov.stats()["launches"] == 8
+    for w, o in zip(want, outs):
+        assert np.array_equal(o["audio"].cpu().numpy(), w)
