@@ -1377,7 +1377,7 @@ namespace aeonb
         // marked doubtful and the serial kernel, launched behind, decodes it anew.
         //
         // Measured on a B200, 32 pictures of 900-1400 pixels a side (4:2:2, quality 92, a marker after every MCU row, 0.3 MB
-        // each): 88 ms with the serial kernel (one warp per stream), 0.38 ms with these two; 92.1 and 1.1 ms for a provider batch of them.
+        // each): 88 ms with the serial kernel (one warp per stream), 0.38 ms with these two; 92 and 1.06 ms for a provider batch of them.
         // A part of 4 to 10 KB per block fills the chip (about 30 parts per picture) and keeps segments at 160 bytes.
         constexpr int RST_THREADS       = 128;
         constexpr int RST_INDEX_THREADS = 1024;
