@@ -1065,8 +1065,8 @@ void aeonb_provider::stage_inputs(batch_plan& B, int par, bool alone)
         }, !heavy);
         // The calling thread copies too (it is awake already).  From 4 MB on it ships every slice as its last job finishes, so that
         // the copy engine works while the rest is being staged (64 clips of 17 MB 714 -> 642 us).  Of less the whole upload takes
-        // under 0.1 ms; nothing is gained, and planning of the next batch beside it is slower (32 video clips of 2.6 MB, four batches
-        // in flight: 593 us a batch with it, 566 without).  Clips behind a batch under way find the copy engine busy with that one's
+        // under 0.1 ms; little is gained, and planning of the next batch beside it is slower (32 video clips of 2.6 MB: one call at a
+        // time 1293 us with it and 1316 without, within the spread of the runs; four batches in flight 593 and 566).  Clips behind a batch under way find the copy engine busy with that one's
         // (64 clips, four batches in flight: 415 us a batch with it, 387 without; 256 photos in flight do gain, 532 -> 485 us).
         static const bool trace = std::getenv("AEONB_TRACE") != nullptr;
         if (trace && m_trace[m_trace_slot][3])
