@@ -53,7 +53,7 @@ namespace aeonb
             uint64_t        bytes; // of the whole area
             uint32_t        intervals;
         };
-        constexpr int RST_MAX_INTERVALS = 64; // of a part (= what one thread block decodes)
+        constexpr int RST_MAX_INTERVALS = 256; // of a part (= what one thread block decodes)
         __host__ __device__ inline uint32_t restart_most_parts(uint32_t intervals)
         {
             return intervals < 96 ? intervals : intervals / RST_MAX_INTERVALS + 96;
@@ -463,11 +463,15 @@ namespace aeonb
         // shared memory while the tables are being built, cleaned of stuffed bytes in place and decoded from
         // there: in global memory nearly every pass had some lane of the warp waiting for L2.
         //
-        // Measured on a B200 (kernel times): one stream of about 40 KB 0.33 ms with branches and the copy in global memory, 0.18 ms
-        // now; 256 streams of up to 55 KB (4:2:0, quality 90, crop regions stored) 0.456 ms, now 0.263 ms.  Phases of a 43 KB
-        // stream, thousand cycles before and after: first pass 83 / 62, rounds 201 / 125 (four of them), storing pass 112 / 107,
-        // copy and marker scan 44 / 26, DC 42 / 19, set-up 30 / 17 (the two last are shorter still since).  Without its stores
-        // the storing pass takes 81, without finding out where blocks go 70: it is bound by the issue of its instructions.
+        // A pass of the loop is one lookup, one byte permute and one addition from position to position, and every other
+        // decision (the next table, the window's refill, the end of a block, a code that the window does not hold) is a select or
+        // a predicated load beside that chain; with a second, dependent lookup for long codes and a branch for codes in no table a
+        // pass took half as long again.
+        //
+        // Measured on a B200 (kernel times): one stream of about 40 KB 0.183 ms before, 0.146 ms now; 256 streams of up to 55 KB (4:2:0,
+        // quality 90, crop regions stored) 0.263 / 0.207 ms; 512 streams of 6 KB 0.232 / 0.147 ms.  Phases of a 43 KB stream, thousand
+        // cycles: first pass 62 / 44 (16 of them beside the clearing of the planes), rounds 126 / 77 (five of them), storing pass
+        // 110 / 102 (one 2-byte store per coefficient, each to a line of its own), copy and marker scan 21, DC 14, set-up 18.
         // A wrong guess falls into step with the true decoder after about 10 blocks on average (the block's
         // position inside the MCU has to match too), and not at all inside flat regions, where every block looks
         // the same: there a chain of segments is settled one round per segment, which is what the slowest streams
@@ -475,34 +479,40 @@ namespace aeonb
         // tail of the left neighbour's segment before the guess.
         constexpr int AC_BITS = 11; // bits of the lookup window: AC tables (12: 28 us slower for 256 streams, fewer of which then fit shared memory)
         constexpr int DC_BITS = 9;  //                            DC tables (few, short codes)
-        // One 32-bit lookup gives everything the symbol loops need.  Of the symbol at the head of the window:
-        //   bits 5-8   number of value bits (AC size / DC category)       bits 9-13  total bits it takes (code + value bits)
-        //   bits 14-20 advance of the zig-zag index: run + 1, 16 for ZRL, 64 for end of block, 1 for a DC category,
-        //              127 for an invalid code (which still takes bits and ends the block, so that a decoder in a wrong state moves on)
-        // and of the pair it makes with the symbol behind it, where it fits the window whole and does not end the block, and the
-        // second one's code lies in the window too (otherwise of the one symbol again):
-        //   bits 0-4   total bits                                          bits 24-31 advance of the zig-zag index
-        // A code longer than an AC window: bits 0-4 are 0, bits 8-24 hold the 16 bits at which such codes begin; the entry is found
-        // behind the window, at the distance of the 16 bits at hand from there.  0 = look the code up the long way (long_symbol).
-        // The pair's part is what the decoder's state -- bit position in bits 0-23, zig-zag
-        // index in bits 24-31 -- advances by, in one addition.
-        constexpr int      AC_LONG = 256, AC_ENTRIES = (1 << AC_BITS) + AC_LONG; // entries behind an AC window, and all of them
-        constexpr uint32_t k_advance = 0xff00001fu, k_position = 0x00ffffffu, k_block_end = 64u << 24;
+        // Each of the four tables is a window, indexed by the bits at hand, behind LONG entries indexed by 16 bits from LONG_FROM on:
+        // the codes that are longer than the window are nearly always among the last ones, which start with eight ones.
+        //
+        // An entry of the passes that only look for states holds, a byte each, what the state -- bit position in bits 0-23, zig-zag
+        // index in bits 24-31 -- advances by: byte 0 bits of the pair that the symbol at the head of the window makes with the one
+        // behind it, where the pair fits the window (the second one's value bits may lie outside) and the first one does not end the
+        // block, otherwise of the symbol alone; byte 1 bits of the symbol alone; byte 2 its advance of the zig-zag index: run + 1, 16 for
+        // ZRL, 64 for end of block, 1 for a DC category, 127 for an invalid code (which still takes bits and ends the block, so that a
+        // decoder in a wrong state moves on); byte 3 the advance of the pair.  One byte permute turns an entry into the advance.
+        // An entry of the storing pass: bits 0-4 bits of the symbol, 5-8 number of value bits (AC size / DC category, 1 for an
+        // invalid code, which then looks like a run that leaves the block), 9-15 advance.
+        // 0: look the 16 bits up in front of the window.  k_slow: neither window nor LONG entries hold the code (long_symbol finds it).
+        constexpr int      LONG = 256, LONG_FROM = 0x10000 - LONG;
+        constexpr int      AC_ENTRIES = LONG + (1 << AC_BITS), DC_ENTRIES = LONG + (1 << DC_BITS), ENTRIES = 2 * (AC_ENTRIES + DC_ENTRIES);
+        constexpr uint32_t k_position = 0x00ffffffu, k_block_end = 64u << 24;
         constexpr uint32_t k_pair_first = AC_BITS - 1;  // most bits of the first symbol of a pair
         constexpr uint32_t k_pair_limit = 48u << 24;    // from this zig-zag index on (63 - 15) the first symbol can end the block
-        __device__ __forceinline__ uint32_t entry_total(uint32_t e) { return e >> 9 & 31; }
+        constexpr uint32_t k_take_pair = 0x3440, k_take_one = 0x2441; // byte selectors
+        constexpr uint32_t k_slow = 0xffff;
+        __device__ __forceinline__ uint32_t store_entry(uint32_t total, uint32_t size, uint32_t advance) { return total | size << 5 | advance << 9; }
+        constexpr uint32_t k_invalid = 16 | 1 << 5 | 127 << 9;
+        __device__ __forceinline__ uint32_t entry_total(uint32_t e) { return e & 31; }
         __device__ __forceinline__ uint32_t entry_size(uint32_t e) { return e >> 5 & 15; }
-        __device__ __forceinline__ uint32_t entry_advance(uint32_t e) { return e >> 14 & 127; }
-        __device__ __forceinline__ uint32_t single_step(uint32_t e) { return entry_total(e) | (e << 10 & 0x7f000000u); }
-        __device__ __forceinline__ uint32_t make_entry(uint32_t size, uint32_t total, uint32_t advance)
+        __device__ __forceinline__ uint32_t entry_advance(uint32_t e) { return e >> 9; }
+        __device__ __forceinline__ uint32_t scan_entry(uint32_t e) // of a storing pass entry, no pair
         {
-            return total | size << 5 | total << 9 | advance << 14 | advance << 24;
+            return e == k_slow ? k_slow : entry_total(e) * 0x101u + entry_advance(e) * 0x1010000u;
         }
         __device__ __forceinline__ uint32_t pack_symbol(int len, int sym, bool is_ac)
         {
             const int s = sym & 15, r = sym >> 4;
-            const int kinc = is_ac ? (s ? r + 1 : (r == 15 ? 16 : 64)) : (r == 0 ? 1 : 127);
-            return make_entry((uint32_t)s, (uint32_t)(len + s), (uint32_t)kinc);
+            if (!is_ac && r)
+                return k_invalid;
+            return store_entry((uint32_t)(len + s), (uint32_t)s, is_ac ? (s ? r + 1 : (r == 15 ? 16 : 64)) : 1);
         }
 
         struct code_table
@@ -536,124 +546,144 @@ namespace aeonb
                 ++from;
             return from;
         }
-        __device__ __forceinline__ uint32_t window_entry(const code_table& T, int i, int len, int bits, bool is_ac)
+        // A code known to be at least `from` bits long, or an invalid one, at the head of the 16 bits c16.
+        __device__ __noinline__ uint32_t long_symbol(const code_table& T, int c16, bool is_ac, int from)
         {
-            if ((i << (16 - bits)) >= T.limit[len])
-                return is_ac && (i << (16 - bits) | ((1 << (16 - bits)) - 1)) - T.limit[AC_BITS] < AC_LONG ? (uint32_t)T.limit[AC_BITS] << 8 : 0;
-            return pack_symbol(len, T.vals[((i >> (bits - len)) + T.valoff[len]) & 255], is_ac);
+            if (c16 >= T.limit[16])
+                return k_invalid;
+            const int len = code_length(T, c16, from, 16);
+            return pack_symbol(len, T.vals[((c16 >> (16 - len)) + T.valoff[len]) & 255], is_ac);
         }
-        // `nth` threads (index `tid`) fill the four lookup windows once limits and values are in place.  Eight neighbouring entries
-        // go together: unless a code of the last three lengths starts among them they hold one symbol, so the length is searched
-        // twice per eight entries.
-        __device__ void build_windows(uint32_t* ac, uint32_t* dc, const code_table* codes, int tid, int nth)
+        __device__ __forceinline__ uint32_t window_entry(const code_table& T, int i, int len, int bits, bool is_ac, int* slow)
+        {
+            const int c16 = i << (16 - bits);
+            if (c16 < T.limit[len])
+                return pack_symbol(len, T.vals[((i >> (bits - len)) + T.valoff[len]) & 255], is_ac);
+            if (c16 >= LONG_FROM)
+                return 0;
+            if (c16 >= T.limit[16])
+                return k_invalid;
+            *slow = 1;
+            return k_slow;
+        }
+        // Where a table starts among the ENTRIES: DC slot 0, DC slot 1, AC slot 0, AC slot 1.
+        __device__ __forceinline__ int table_at(int t) { return t < 2 ? t * DC_ENTRIES : 2 * DC_ENTRIES + (t - 2) * AC_ENTRIES; }
+        // `nth` threads (index `tid`) fill the storing pass's entries of the four tables once limits and values are in place.  Eight
+        // neighbouring entries go together: unless a code of the last three lengths starts among them they hold one symbol, so the
+        // length is searched twice per eight entries.
+        __device__ void build_tables(uint16_t* store, const code_table* codes, int tid, int nth, int* slow)
         {
             constexpr int ac8 = (1 << AC_BITS) / 8, dc8 = (1 << DC_BITS) / 8;
             for (int j = tid; j < 2 * (ac8 + dc8); j += nth)
             {
                 const bool        is_ac = j < 2 * ac8;
-                const int         slot = is_ac ? j / ac8 : (j - 2 * ac8) / dc8, i = (is_ac ? j % ac8 : (j - 2 * ac8) % dc8) * 8;
+                const int         t = is_ac ? 2 + j / ac8 : (j - 2 * ac8) / dc8, i = (is_ac ? j % ac8 : (j - 2 * ac8) % dc8) * 8;
                 const int         bits = is_ac ? AC_BITS : DC_BITS;
-                const code_table& T    = codes[is_ac ? 2 + slot : slot];
-                uint32_t* const   out  = (is_ac ? ac + slot * AC_ENTRIES : dc + (slot << DC_BITS)) + i;
+                const code_table& T    = codes[t];
+                uint16_t* const   out  = store + table_at(t) + LONG + i;
                 const int first = code_length(T, i << (16 - bits), 1, bits), last = code_length(T, (i + 7) << (16 - bits), first, bits);
                 if (first == last && first <= bits - 3)
                 {
-                    const uint32_t e = window_entry(T, i, first, bits, is_ac);
-                    reinterpret_cast<uint4*>(out)[0] = make_uint4(e, e, e, e);
-                    reinterpret_cast<uint4*>(out)[1] = make_uint4(e, e, e, e);
+                    const uint32_t e = window_entry(T, i, first, bits, is_ac, slow) * 0x10001u;
+                    *reinterpret_cast<uint4*>(out) = make_uint4(e, e, e, e);
                 }
                 else
                 {
 #pragma unroll 1
                     for (int k = 0; k < 8; ++k)
-                        out[k] = window_entry(T, i + k, code_length(T, (i + k) << (16 - bits), first, last), bits, is_ac);
+                        out[k] = (uint16_t)window_entry(T, i + k, code_length(T, (i + k) << (16 - bits), first, last), bits, is_ac, slow);
                 }
             }
+            for (int j = tid; j < 4 * LONG; j += nth)
+                store[table_at(j / LONG) + j % LONG] = (uint16_t)long_symbol(codes[j / LONG], LONG_FROM + j % LONG, j >= 2 * LONG, 1);
         }
-        // A code longer than the window, or an invalid one.
-        __device__ __noinline__ uint32_t long_symbol(const code_table& T, int c16, bool is_ac, int from)
-        {
-            if (c16 >= T.limit[16])
-                return make_entry(0, 16, 127);
-            const int len = code_length(T, c16, from, 16);
-            return pack_symbol(len, T.vals[((c16 >> (16 - len)) + T.valoff[len]) & 255], is_ac);
-        }
-        // Pairs the entries of the AC windows (see above), four neighbours per thread and pass so that their second lookups overlap, and
-        // fills what lies behind the windows.  Only the parts of an entry that stay as they are are read of others.
-        __device__ void pair_windows(uint32_t* ac, const code_table* codes, int tid, int nth)
+        // The entries of the other passes from those of the storing pass; eight neighbours per thread and pass so that the lookups of
+        // the second symbols overlap.
+        __device__ void pair_tables(uint32_t* scan, const uint16_t* store, int tid, int nth)
         {
             constexpr uint32_t mask = (1 << AC_BITS) - 1;
-            for (int j = tid; j < 2 << (AC_BITS - 2); j += nth)
+            for (int j = tid; j < ENTRIES / 8; j += nth)
             {
-                uint32_t* const T = ac + (j >> (AC_BITS - 2)) * AC_ENTRIES;
-                const uint32_t  i = 4 * ((uint32_t)j & (mask >> 2));
-                const uint4     four = *reinterpret_cast<uint4*>(T + i);
-                uint32_t        e[4] = {four.x, four.y, four.z, four.w}, f[4];
+                const uint4    in    = reinterpret_cast<const uint4*>(store)[j];
+                const uint32_t raw[4] = {in.x, in.y, in.z, in.w};
+                uint32_t       e[8], f[8], out[8];
+                // the place in an AC window; the entries in front of it, and DC tables, have no pairs
+                int i = 8 * j - 2 * DC_ENTRIES - LONG;
+                const uint16_t* window = store + 2 * DC_ENTRIES + LONG;
+                if (i >= AC_ENTRIES)
+                    i -= AC_ENTRIES, window += AC_ENTRIES;
+                const bool is_ac = i >= 0 && i <= (int)mask;
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
-                    f[k] = reinterpret_cast<volatile uint32_t*>(T)[(i + k) << entry_total(e[k]) & mask]; // the bits behind, zeros after them
+                for (int k = 0; k < 8; ++k)
+                {
+                    e[k] = raw[k >> 1] >> (16 * (k & 1)) & 0xffff;
+                    f[k] = is_ac ? window[(uint32_t)(i + k) << entry_total(e[k]) & mask] : 0; // the bits behind, zeros after them
+                }
 #pragma unroll
-                for (int k = 0; k < 4; ++k)
+                for (int k = 0; k < 8; ++k)
                 {
                     const uint32_t total = entry_total(e[k]), advance = entry_advance(e[k]);
-                    if ((e[k] & 31) && advance < 64 && total <= k_pair_first && (f[k] & 31) && entry_total(f[k]) - entry_size(f[k]) <= AC_BITS - total)
-                        e[k] = (e[k] & 0x001fffe0u) | (total + entry_total(f[k])) | (advance + entry_advance(f[k])) << 24;
+                    out[k] = scan_entry(e[k]);
+                    if (e[k] && e[k] != k_slow && advance < 64 && total <= k_pair_first && f[k] && f[k] != k_slow &&
+                        entry_total(f[k]) - entry_size(f[k]) <= AC_BITS - total && entry_advance(f[k]) != 127)
+                        out[k] = (out[k] & 0x00ffff00u) | (total + entry_total(f[k])) | (advance + entry_advance(f[k])) << 24;
                 }
-                *reinterpret_cast<uint4*>(T + i) = make_uint4(e[0], e[1], e[2], e[3]);
-            }
-            for (int j = tid; j < 2 * AC_LONG; j += nth)
-            {
-                const code_table& T = codes[2 + j / AC_LONG];
-                ac[j / AC_LONG * AC_ENTRIES + (1 << AC_BITS) + j % AC_LONG] = long_symbol(T, min(T.limit[AC_BITS] + j % AC_LONG, 0xffff), true, AC_BITS + 1);
+                reinterpret_cast<uint4*>(scan)[2 * j]     = make_uint4(out[0], out[1], out[2], out[3]);
+                reinterpret_cast<uint4*>(scan)[2 * j + 1] = make_uint4(out[4], out[5], out[6], out[7]);
             }
         }
 
         constexpr int PAR_THREADS = 1024; // most threads (= segments) a stream can have; the launch picks the actual number
         constexpr int NCHECK      = 3;    // checkpoints inside a segment (7 measured the same; 3 leaves room for a third kernel's CTA on the SM)
 
-        // Where the blocks of one place in an MCU go: base + 64 * ((mcu row - first row) * dy + (mcu column - first column) * dx)
-        struct alignas(16) block_place
-        {
-            int16_t* base;
-            int32_t  dy, dx;
-        };
-        // What the symbol loop wants to know of a block of an MCU, in one 16-byte load: the shared-memory addresses of its AC window,
-        // of the next block's DC window and of the next block's link.
+        // What the symbol loops want to know of a block of an MCU, in 16-byte loads: the shared-memory addresses of its AC window, of the
+        // next block's DC window and of the next block's link.
         struct alignas(16) block_link
         {
             uint32_t ac, next_dc, next, block;
         };
+        // The storing pass also wants to know whether it is the MCU's last block, and where the blocks of this place go:
+        // base + 64 * ((mcu row - first row) * dy + (mcu column - first column) * dx)
+        struct alignas(16) block_place
+        {
+            uint32_t ac, next_dc, next, last;
+            int16_t* base;
+            int32_t  dy, dx;
+        };
 
         struct par_state
         {
-            uint32_t    ac_window[2][AC_ENTRIES], dc_window[2][1 << DC_BITS];
+            alignas(16) uint32_t scan[ENTRIES];
+            alignas(16) uint16_t store[ENTRIES];
             code_table  codes[4]; // DC slot 0, DC slot 1, AC slot 0, AC slot 1
             alignas(16) uint8_t dht[4 * 272]; // the tables as they came
             uint32_t    warp_sums[3][32];
-            uint8_t     zz[64];
+            uint8_t     zz[64 + 128];            // in front of a run that leaves the block, or of a look further on, anything is read
             block_place place[16];               // per block of an MCU
             block_link  link[16];
             uint8_t     comp[16];
             aeonb_entropy_desc d;
             int        bpm;                      // blocks per MCU
             int        bad;
+            int        slow;                     // some code is not in the tables (see k_slow)
             uint32_t   marker_at;                // first marker byte in the raw scan (or its size)
             uint32_t   tile_end[2];              // last byte of an even / odd tile of the raw scan
         };
 
-        // Per thread (= segment): the state it was entered in and left in, its blocks, and the checkpoints.
+        // Per segment (= thread): the state it was entered in and left in, its blocks, and the checkpoints.
         struct seg_arrays
         {
             uint32_t *ent_p, *ext_p, *cnt, *chk; // chk: 2 x NCHECK rows of T words
             uint16_t *ent_bk, *ext_bk;
+            uint32_t rows; // most segments
         };
-        constexpr uint32_t SEG_BYTES = 4 * (3 + 2 * NCHECK) + 2 * 2; // of shared memory for each thread
+        constexpr uint32_t SEG_BYTES = 4 * (3 + 2 * NCHECK) + 2 * 2; // of shared memory for each segment
 
-        __device__ __forceinline__ seg_arrays seg_arrays_at(unsigned char* p, uint32_t T)
+        __device__ __forceinline__ seg_arrays seg_arrays_at(unsigned char* p, uint32_t rows)
         {
             uint32_t* const w = reinterpret_cast<uint32_t*>(p);
-            uint16_t* const h = reinterpret_cast<uint16_t*>(w + (3 + 2 * NCHECK) * T);
-            return seg_arrays{w, w + T, w + 2 * T, w + 3 * T, h, h + T};
+            uint16_t* const h = reinterpret_cast<uint16_t*>(w + (3 + 2 * NCHECK) * rows);
+            return seg_arrays{w, w + rows, w + 2 * rows, w + 3 * rows, h, h + rows, rows};
         }
 
         __device__ __forceinline__ uint32_t shared_address(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -663,10 +693,11 @@ namespace aeonb
             asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
             return v;
         }
-        // value = the word at addr where `yes`
-        __device__ __forceinline__ void lds_if(uint32_t& value, uint32_t addr, bool yes)
+        __device__ __forceinline__ uint32_t lds_u16(uint32_t addr)
         {
-            asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.shared.u32 %0, [%1];\n\t}" : "+r"(value) : "r"(addr), "r"((uint32_t)yes));
+            uint16_t v;
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+            return v;
         }
         // link = the link at its `next` where `yes`
         __device__ __forceinline__ void follow_if(block_link& link, bool yes)
@@ -674,6 +705,15 @@ namespace aeonb
             asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %4, 0;\n\t@q ld.shared.v4.u32 {%0, %1, %2, %3}, [%2];\n\t}"
                          : "+r"(link.ac), "+r"(link.next_dc), "+r"(link.next), "+r"(link.block)
                          : "r"((uint32_t)yes));
+        }
+        __device__ __forceinline__ void follow_if(block_place& at, bool yes)
+        {
+            uint64_t base = reinterpret_cast<uint64_t>(at.base);
+            asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 a;\n\tsetp.ne.u32 q, %7, 0;\n\tmov.b32 a, %2;\n\t"
+                         "@q ld.shared.v4.u32 {%0, %1, %2, %3}, [a];\n\t@q ld.shared.u64 %4, [a + 16];\n\t@q ld.shared.v2.s32 {%5, %6}, [a + 24];\n\t}"
+                         : "+r"(at.ac), "+r"(at.next_dc), "+r"(at.next), "+r"(at.last), "+l"(base), "+r"(at.dy), "+r"(at.dx)
+                         : "r"((uint32_t)yes));
+            at.base = reinterpret_cast<int16_t*>(base);
         }
 
         // Words of the copy of a stream, from shared or from global memory.  `next_if` replaces `value` by the next word where
@@ -728,57 +768,28 @@ namespace aeonb
             uint32_t p;      // exit state: bit position of the first symbol past the segment,
             int      b, k;   //             block inside the MCU, zig-zag index
             uint32_t blocks; // blocks completed
-            int      bad;
             bool     merged; // the run fell into step with the remembered run: the exit state is that run's (p, b, k unset)
         };
 
         // Decodes symbols from bit position p in state (b, k) until the first symbol that starts at or past pend.  The copy of the
         // stream holds big-endian words, so the 32 bits under p are one funnel shift of two words.
-        // WRITE: stores coefficients and DC differences, `g` being the number of the block in progress, up to block `gend`.
-        // Otherwise the state at the checkpoints (first one at bit check_at, then every check_step bits) goes to chk[0],
+        // The state at the checkpoints (first one at bit check_at, then every check_step bits) goes to chk[0],
         // chk[check_stride], ... and the blocks completed by then NCHECK rows further on; with `compare`, the run stops at the
         // first checkpoint that an earlier run over this segment (old_blocks blocks in all) passed in the same state, and the
         // block counts from there on are renumbered for this run.
-        template <bool WRITE, typename Words>
-        __device__ __forceinline__ seg_result run_segment(const par_state& S, const uint32_t* words, uint32_t p, int b, int k,
-                                                          uint32_t pend, uint32_t g, uint32_t gend, int16_t* __restrict__ dcdiff,
-                                                          uint32_t* chk, uint32_t check_stride, uint32_t check_at, uint32_t check_step,
-                                                          bool compare, uint32_t old_blocks)
+        template <bool SLOW, typename Words>
+        __device__ __forceinline__ seg_result scan_segment(const par_state& S, const uint32_t* words, uint32_t p, int b, int k, uint32_t pend,
+                                                           uint32_t* chk, uint32_t check_stride, uint32_t check_at, uint32_t check_step,
+                                                           bool compare, uint32_t old_blocks)
         {
             seg_result R;
-            R.merged            = false;
-            uint32_t       blocks = 0;
-            int            bad    = 0;
-            const int      bpm    = S.bpm;
-            // WRITE: the MCU, counted from the region's first column and row (negative in front of it), and the region's size
-            int      mx = 0, my = 0;
-            int      mx_end = 0, mx_first = 0;
-            uint32_t roi_w = 0, roi_h = 0;
-            int16_t* out  = nullptr;
-            auto     home = [&]() -> int16_t* {
-                const block_place& at = S.place[b];
-                return (uint32_t)mx < roi_w && (uint32_t)my < roi_h ? at.base + (int64_t)(my * at.dy + mx * at.dx) * 64 : nullptr;
-            };
-            if (WRITE)
-            {
-                const uint32_t mcu = g / (uint32_t)bpm;
-                mx_first           = -S.d.roi[0];
-                mx_end             = S.d.mcux - S.d.roi[0];
-                roi_w              = (uint32_t)(S.d.roi[2] - S.d.roi[0]);
-                roi_h              = (uint32_t)(S.d.roi[3] - S.d.roi[1]);
-                my                 = (int)(mcu / (uint32_t)S.d.mcux);
-                mx                 = (int)(mcu - (uint32_t)my * S.d.mcux) - S.d.roi[0];
-                my -= S.d.roi[1];
-                if (g >= gend)
-                    pend = 0; // nothing of this segment is wanted
-                else
-                    out = home();
-            }
-            // The lookup window of the next symbol: the AC one of this block, or after the block's last symbol the DC one of the
+            R.merged        = false;
+            uint32_t blocks = 0;
+            // The table of the next symbol: the AC one of this block, or after the block's last symbol the DC one of the
             // next.  Both are at hand before the symbol is known, so that only a select hangs on it.
             block_link link = S.link[b];
-            uint32_t   look = k == 0 ? S.link[b ? b - 1 : bpm - 1].next_dc : link.ac, shift = k == 0 ? 32 - DC_BITS : 32 - AC_BITS;
-            // Bit positions count from the word that the run starts in; `at` is the state (see k_advance).
+            uint32_t   look = k == 0 ? S.link[b ? b - 1 : S.bpm - 1].next_dc : link.ac, shift = k == 0 ? 32 - DC_BITS : 32 - AC_BITS;
+            // Bit positions count from the word that the run starts in; `at` is the state: position, and zig-zag index in the top byte.
             const uint32_t base = p & ~31u;
             uint32_t       at   = (p - base) | (uint32_t)k << 24;
             pend                = pend > base ? pend - base : 0;
@@ -786,80 +797,44 @@ namespace aeonb
             // the state an earlier run noted at the next checkpoint (no state has all bits set)
             const uint32_t rows    = NCHECK * check_stride;
             uint32_t*      slot    = chk;
-            uint32_t       old_key = !WRITE && compare ? chk[0] : 0xffffffffu;
+            uint32_t       old_key = compare ? chk[0] : 0xffffffffu;
             // A checkpoint at or past the segment's end is never taken: a run can step over it with its last symbol or stop short
             // of it, so what is noted there could be left from an older run than the one whose block count goes with it.
             check_at -= base;
-            uint32_t stop = WRITE || check_at >= pend ? pend : check_at;
+            uint32_t stop = check_at >= pend ? pend : check_at;
             // The 32 bits under the position lie in w0 and w1; w2 is the word behind them, fetched when the one before it comes into use.
             Words    ahead(words, p >> 5);
             uint32_t w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
-            // The entry of the symbol under the position, and the state after an advance.
-            uint32_t h;
-            auto     lookup = [&]() -> uint32_t {
-                h          = __funnelshift_l(w1, w0, at); // 32 valid bits; a symbol or a pair takes at most 31
-                uint32_t e = lds_u32(look + ((h >> shift) << 2));
-                lds_if(e, look + (((h >> 16) - (e >> 8) + (1 << AC_BITS)) << 2), (e & 31) == 0 && e != 0);
-                if (!e)
-                {
-                    const bool is_ac = at > k_position;
-                    e = long_symbol(is_ac ? S.codes[look == shared_address(S.ac_window[0]) ? 2 : 3] : S.codes[look == shared_address(S.dc_window[0]) ? 0 : 1],
-                                    (int)(h >> 16), is_ac, 1);
-                }
-                return e;
-            };
-            auto step = [&](uint32_t by) -> bool {
-                const uint32_t to    = at + by;
-                const uint32_t cross = (at ^ to) & 32; // the read position has left w0
-                w0                   = cross ? w1 : w0;
-                w1                   = cross ? w2 : w1;
-                ahead.next_if(w2, cross);
-                const bool end = to >= k_block_end;
-                look           = end ? link.next_dc : link.ac;
-                shift          = end ? 32 - DC_BITS : 32 - AC_BITS;
-                at             = end ? to & k_position : to;
-                blocks += end;
-                follow_if(link, end);
-                return end;
-            };
             for (;;)
             {
-                while ((at & k_position) < stop)
+                for (uint32_t pos = at & k_position; pos < stop;)
                 {
-                    const uint32_t e  = lookup();
-                    uint32_t       by = single_step(e);
                     // Two symbols at a time as long as the first one cannot reach `stop`: a run stops at the first symbol at or past
                     // it, however it came there.
-                    if (!WRITE)
-                        by = at < k_pair_limit && (at & k_position) + k_pair_first < stop ? e & k_advance : by;
-                    if (WRITE)
+                    const uint32_t take = at < k_pair_limit && pos + k_pair_first < stop ? k_take_pair : k_take_one;
+                    const uint32_t h    = __funnelshift_l(w1, w0, at); // 32 valid bits; a symbol or a pair takes at most 31
+                    uint32_t       e    = lds_u32(look + ((h >> shift) << 2));
+                    if (SLOW && e == k_slow)
                     {
-                        const int      tot = (int)entry_total(e), sz = (int)entry_size(e), kinc = (int)entry_advance(e);
-                        const int      kk = (int)(at >> 24) + kinc - 1; // the coefficient's place
-                        const uint32_t x  = h << (tot - sz);            // the value bits at the top
-                        const int      v  = (int)__funnelshift_l(x, 0u, sz) + ((int)x >= 0 ? 1 - (1 << sz) : 0);
-                        // an invalid code, a DC symbol that is no category, or a run that leaves the block
-                        bad |= kinc == 127 || (sz && kk > 63);
-                        if (at <= k_position)
-                            dcdiff[g] = (int16_t)v;
-                        else if (sz && kk <= 63 && out)
-                            out[S.zz[kk]] = (int16_t)v;
+                        const bool is_ac = at > k_position;
+                        const int  slot1 = look == shared_address(S.scan + table_at(is_ac ? 3 : 1) + LONG);
+                        e = scan_entry(long_symbol(S.codes[(is_ac ? 2 : 0) + slot1], (int)(h >> 16), is_ac, 1));
                     }
-                    const bool end = step(by);
-                    if (WRITE && end)
-                    {
-                        if (++g >= gend)
-                            break;
-                        b = (int)link.block;
-                        if (b == 0 && ++mx == mx_end)
-                        {
-                            mx = mx_first;
-                            ++my;
-                        }
-                        out = home();
-                    }
+                    const uint32_t by    = __byte_perm(e, 0, take);
+                    const uint32_t to    = at + by;
+                    const bool     cross = (at ^ to) & 32; // the read position has left w0
+                    const bool     end = to >= k_block_end, again = by == 0;
+                    w0                   = cross ? w1 : w0;
+                    w1                   = cross ? w2 : w1;
+                    ahead.next_if(w2, cross);
+                    look  = again ? look - 4 * LONG - 4 * LONG_FROM : end ? link.next_dc : link.ac;
+                    shift = again ? 16 : end ? 32 - DC_BITS : 32 - AC_BITS;
+                    at    = end ? to & k_position : to;
+                    pos   = to & k_position;
+                    blocks += end;
+                    follow_if(link, end);
                 }
-                if (WRITE || stop == pend)
+                if (stop == pend)
                     break;
                 // a checkpoint
                 const uint32_t key = ((at & k_position) - stop) << 10 | link.block << 6 | at >> 24; // position - stop <= 30
@@ -884,7 +859,77 @@ namespace aeonb
             R.b      = (int)link.block;
             R.k      = (int)(at >> 24);
             R.blocks = blocks;
-            R.bad    = bad;
+            return R;
+        }
+
+        // Decodes symbols as above and stores coefficients and DC differences; `g` is the number of the block in progress, block `gend`
+        // the first that is not wanted.  There is nothing to branch around: where a block goes is worked out anew for
+        // every symbol (three multiply-adds), and what a symbol has no part in is a store that is not made.
+        struct store_result
+        {
+            uint32_t p, blocks; // where the first symbol past the segment starts; blocks completed
+            bool     bad;
+        };
+        template <bool SLOW, typename Words>
+        __device__ __forceinline__ store_result store_segment(const par_state& S, const uint32_t* words, uint32_t p, int b, int k, uint32_t pend,
+                                                              uint32_t g, uint32_t gend, int16_t* __restrict__ dcdiff)
+        {
+            store_result R{p, 0, false};
+            if (g >= gend)
+                return R; // nothing of this segment is wanted
+            const uint32_t first = g;
+            // the MCU, counted from the region's first column and row (negative in front of it), and the region's size
+            const int      mx_first = -S.d.roi[0], mx_end = S.d.mcux - S.d.roi[0];
+            const uint32_t roi_w = (uint32_t)(S.d.roi[2] - S.d.roi[0]), roi_h = (uint32_t)(S.d.roi[3] - S.d.roi[1]);
+            const uint32_t mcu = g / (uint32_t)S.bpm, row = mcu / (uint32_t)S.d.mcux;
+            int            my = (int)row - S.d.roi[1], mx = (int)(mcu - row * (uint32_t)S.d.mcux) - S.d.roi[0];
+            block_place    place = S.place[b];
+            uint32_t       look = k == 0 ? S.place[b ? b - 1 : S.bpm - 1].next_dc : place.ac, shift = k == 0 ? 32 - DC_BITS : 32 - AC_BITS;
+            const uint32_t base = p & ~31u;
+            uint32_t       at   = (p - base) | (uint32_t)k << 24, pos = p - base;
+            pend                = pend > base ? pend - base : 0;
+            const uint32_t zz   = shared_address(S.zz);
+            Words          ahead(words, p >> 5);
+            uint32_t       w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
+            while (pos < pend && g < gend)
+            {
+                const uint32_t h = __funnelshift_l(w1, w0, at);
+                uint32_t       e = lds_u16(look + ((h >> shift) << 1));
+                if (SLOW && e == k_slow)
+                {
+                    const bool is_ac = at > k_position;
+                    const int  slot1 = look == shared_address(S.store + table_at(is_ac ? 3 : 1) + LONG);
+                    e                = long_symbol(S.codes[(is_ac ? 2 : 0) + slot1], (int)(h >> 16), is_ac, 1);
+                }
+                const uint32_t total = entry_total(e), size = entry_size(e), advance = entry_advance(e);
+                const uint32_t kk = (at >> 24) + advance - 1; // the coefficient's place
+                const uint32_t x  = h << (total - size);      // the value bits at the top
+                const int      v  = (int)__funnelshift_l(x, 0u, size) + ((int)x >= 0 ? 1 - (1 << size) : 0);
+                const bool     inside = (uint32_t)mx < roi_w && (uint32_t)my < roi_h;
+                // an invalid code, or a run that leaves the block
+                R.bad |= size != 0 && (int)kk > 63;
+                if (at <= k_position)
+                    dcdiff[g] = (int16_t)v;
+                else if (size != 0 && kk <= 63 && inside)
+                    place.base[(int64_t)(my * place.dy + mx * place.dx) * 64 + S.zz[kk]] = (int16_t)v;
+                const uint32_t to    = at + (total | advance << 24);
+                const bool     cross = (at ^ to) & 32;
+                const bool     end = to >= k_block_end, again = e == 0;
+                w0                   = cross ? w1 : w0;
+                w1                   = cross ? w2 : w1;
+                ahead.next_if(w2, cross);
+                look  = again ? look - 2 * LONG - 2 * LONG_FROM : end ? place.next_dc : place.ac;
+                shift = again ? 16 : end ? 32 - DC_BITS : 32 - AC_BITS;
+                at    = end ? to & k_position : to;
+                pos   = to & k_position;
+                g += end;
+                mx += end ? place.last : 0;
+                my += mx == mx_end;
+                mx = mx == mx_end ? mx_first : mx;
+                follow_if(place, end);
+            }
+            R.p      = base + pos;
+            R.blocks = g - first;
             return R;
         }
 
@@ -994,7 +1039,8 @@ namespace aeonb
                         for (int x = 0; x < d.hs[c]; ++x, ++b)
                         {
                             S.comp[b]       = (uint8_t)c;
-                            S.link[b].ac    = shared_address(S.ac_window[d.ac_table[c] & 1]);
+                            S.link[b].ac    = shared_address(S.scan + table_at(2 + (d.ac_table[c] & 1)) + LONG);
+                            S.place[b].ac   = shared_address(S.store + table_at(2 + (d.ac_table[c] & 1)) + LONG);
                             S.link[b].block = (uint32_t)b;
                             S.place[b].base = d.coef[c] + (y * row_blocks + x) * 64;
                             S.place[b].dy   = (int32_t)(d.vs[c] * row_blocks);
@@ -1017,8 +1063,12 @@ namespace aeonb
             if (tid < S.bpm)
             {
                 const int next       = tid + 1 < S.bpm ? tid + 1 : 0;
-                S.link[tid].next_dc = shared_address(S.dc_window[d.dc_table[S.comp[next]] & 1]);
-                S.link[tid].next    = shared_address(&S.link[next]);
+                const int dc         = table_at(d.dc_table[S.comp[next]] & 1) + LONG;
+                S.link[tid].next_dc  = shared_address(S.scan + dc);
+                S.link[tid].next     = shared_address(&S.link[next]);
+                S.place[tid].next_dc = shared_address(S.store + dc);
+                S.place[tid].next    = shared_address(&S.place[next]);
+                S.place[tid].last    = next == 0;
             }
             if ((tid & 31) == 0)
                 for (int t = tid >> 5; t < 4; t += nth >> 5)
@@ -1026,9 +1076,9 @@ namespace aeonb
             for (int i = tid; i < 4 * 256; i += nth)
                 S.codes[i >> 8].vals[i & 255] = S.dht[(i >> 8) * 272 + 16 + (i & 255)];
             __syncthreads();
-            build_windows(S.ac_window[0], S.dc_window[0], S.codes, tid, nth);
+            build_tables(S.store, S.codes, tid, nth, &S.slow);
             __syncthreads();
-            pair_windows(S.ac_window[0], S.codes, tid, nth);
+            pair_tables(S.scan, S.store, tid, nth);
             __syncthreads();
         }
 
@@ -1063,17 +1113,17 @@ namespace aeonb
 
         // Decodes every segment from a guessed state (`known`: the true one) and then, in rounds, from its left neighbour's exit state
         // until nothing changes.  Returns the blocks this thread's segment completes; entry states and checkpoints stay in A.
-        template <typename Words>
+        template <bool SLOW, typename Words>
         __device__ __forceinline__ uint32_t settle_segments(const par_state& S, const seg_arrays& A, const uint32_t* words, uint32_t nseg,
                                                             bool known, uint32_t pbeg, uint32_t pend, uint32_t step)
         {
-            const uint32_t  tid = threadIdx.x, T = blockDim.x;
+            const uint32_t  tid = threadIdx.x, T = A.rows;
             const bool      mine       = tid < nseg;
             uint32_t* const chk        = A.chk + tid;
             uint32_t        run_blocks = 0; // blocks of this thread's latest run
             if (mine)
             {
-                const seg_result r = run_segment<false, Words>(S, words, pbeg, 0, 0, pend, 0, 0, nullptr, chk, T, pbeg + step, step, false, 0);
+                const seg_result r = scan_segment<SLOW, Words>(S, words, pbeg, 0, 0, pend, chk, T, pbeg + step, step, false, 0);
                 A.ent_p[tid]  = pbeg;
                 A.ent_bk[tid] = 0;
                 A.ext_p[tid]  = r.p;
@@ -1095,8 +1145,8 @@ namespace aeonb
                 __syncthreads(); // every candidate has been read before any exit state changes
                 if (redo)
                 {
-                    const seg_result r = run_segment<false, Words>(S, words, cand_p, cand_bk >> 8, cand_bk & 255, pend, 0, 0, nullptr, chk, T,
-                                                                   pbeg + step, step, true, run_blocks);
+                    const seg_result r = scan_segment<SLOW, Words>(S, words, cand_p, cand_bk >> 8, cand_bk & 255, pend, chk, T, pbeg + step, step,
+                                                                    true, run_blocks);
                     A.ent_p[tid]  = cand_p;
                     A.ent_bk[tid] = cand_bk;
                     run_blocks    = r.blocks;
@@ -1113,16 +1163,16 @@ namespace aeonb
         }
 
         // The entry state of piece `piece` of segment t, which starts at bit `at`: position, block and zig-zag index, blocks so far.
-        __device__ __forceinline__ void piece_entry(const seg_arrays& A, uint32_t T, uint32_t t, uint32_t piece, uint32_t at, uint32_t& p,
+        __device__ __forceinline__ void piece_entry(const seg_arrays& A, uint32_t t, uint32_t piece, uint32_t at, uint32_t& p,
                                                     uint32_t& bk, uint32_t& before)
         {
             p = A.ent_p[t], bk = A.ent_bk[t], before = 0;
             if (piece > 0)
             {
-                const uint32_t key = A.chk[(piece - 1) * T + t];
+                const uint32_t key = A.chk[(piece - 1) * A.rows + t];
                 p                  = at + (key >> 10);
                 bk                 = (key >> 6 & 15) << 8 | (key & 63);
-                before             = A.chk[(NCHECK + piece - 1) * T + t];
+                before             = A.chk[(NCHECK + piece - 1) * A.rows + t];
             }
         }
 
@@ -1199,20 +1249,20 @@ namespace aeonb
         }
 
         // Everything between the copy and the DC sums: segments, their true entry states, and the storing pass.
-        template <typename Words>
+        template <bool SLOW, typename Words>
         __device__ __forceinline__ void decode_scan(par_state& S, const seg_arrays& A, const uint32_t* words, uint32_t clean_size, int min_segment,
                                                     uint32_t needed_blocks, int16_t* dcdiff)
         {
             const uint32_t            tid = threadIdx.x, T = blockDim.x;
             const aeonb_entropy_desc& d = S.d;
-            // ---- segments: one per thread, a multiple of 4 bytes, at least min_segment bytes
-            uint32_t seg = (clean_size + T - 1) / T;
+            // ---- segments: at most one per thread, a multiple of 4 bytes, at least min_segment bytes
+            uint32_t seg = (clean_size + A.rows - 1) / A.rows;
             seg          = max((seg + 3u) & ~3u, (uint32_t)max(min_segment, 64) & ~3u);
             // The storing pass deals its pieces out in rounds of T.  Up to a quarter more than a whole number of rounds is avoided by
             // longer segments: the last round would take as long as the others.
             const uint32_t rounds = max(((NCHECK + 1) * ((clean_size + seg - 1) / seg) * 4 + 3 * T) / (4 * T), 1u);
             seg                   = max(seg, ((NCHECK + 1) * clean_size / (rounds * T) + 4u) & ~3u);
-            const uint32_t nseg      = (clean_size + seg - 1) / seg; // <= T
+            const uint32_t nseg      = (clean_size + seg - 1) / seg; // <= A.rows <= T
             const uint32_t total_bit = clean_size * 8;
             const uint32_t pbeg = tid * seg * 8, pend = min(total_bit, pbeg + seg * 8);
             // checkpoints of a segment, evenly spaced (at least 64 bits apart; a symbol is shorter, so it passes at most one)
@@ -1231,7 +1281,7 @@ namespace aeonb
                         p[i] = make_uint4(0, 0, 0, 0);
                 }
 
-            const uint32_t run_blocks = settle_segments<Words>(S, A, words, nseg, tid == 0, pbeg, pend, step);
+            const uint32_t run_blocks = settle_segments<SLOW, Words>(S, A, words, nseg, tid == 0, pbeg, pend, step);
 
             // ---- first block number of every segment
             uint32_t       counted;
@@ -1243,7 +1293,8 @@ namespace aeonb
             // describe every segment's final run, so each segment falls into NCHECK + 1 pieces with known entry states and block
             // numbers, and the pieces -- not the segments -- are dealt out to the threads: streams with fewer segments than
             // threads keep every warp busy, and neighbouring lanes work on neighbouring pieces.
-            A.cnt[tid] = g0;
+            if (tid < nseg)
+                A.cnt[tid] = g0;
             __syncthreads();
             for (uint32_t q = tid; q < nseg * (NCHECK + 1); q += T)
             {
@@ -1253,25 +1304,25 @@ namespace aeonb
                 if (at >= seg_end)
                     continue;
                 uint32_t p0, bk, before;
-                piece_entry(A, T, t, piece, at, p0, bk, before);
-                const seg_result r = run_segment<true, Words>(S, words, p0, bk >> 8, bk & 255, min(seg_end, at + step), A.cnt[t] + before,
-                                                              needed_blocks, dcdiff, nullptr, 0, 0, 0, false, 0);
+                piece_entry(A, t, piece, at, p0, bk, before);
+                const store_result r = store_segment<SLOW, Words>(S, words, p0, bk >> 8, bk & 255, min(seg_end, at + step), A.cnt[t] + before,
+                                                                needed_blocks, dcdiff);
                 if (r.bad)
                     S.bad = 1;
             }
             __syncthreads();
         }
 
-        // Shared memory of a block: par_state, SEG_BYTES per thread, and what is left of `smem_bytes` for the scan and behind it
-        // the DC differences, where they fit; otherwise they live in the record's work area.
+        // Shared memory of a block: par_state, SEG_BYTES for each of `rows` segments, and what is left of `smem_bytes` for the scan and
+        // behind it the DC differences, where they fit; otherwise they live in the record's work area.
         __global__ void __launch_bounds__(PAR_THREADS) jpeg_entropy_parallel_kernel(const aeonb_entropy_desc* __restrict__ descs, int min_segment,
-                                                                                    uint32_t smem_bytes)
+                                                                                    uint32_t rows, uint32_t smem_bytes)
         {
-            const uint32_t T = blockDim.x; // threads = most segments of this launch
+            const uint32_t T = blockDim.x;
             extern __shared__ __align__(16) unsigned char smem_raw[];
             par_state&       S          = *reinterpret_cast<par_state*>(smem_raw);
-            const seg_arrays A          = seg_arrays_at(smem_raw + sizeof(par_state), T);
-            const uint32_t   room_at    = ((uint32_t)sizeof(par_state) + SEG_BYTES * T + 15) & ~15u;
+            const seg_arrays A          = seg_arrays_at(smem_raw + sizeof(par_state), rows);
+            const uint32_t   room_at    = ((uint32_t)sizeof(par_state) + SEG_BYTES * rows + 15) & ~15u;
             uint32_t* const  room       = reinterpret_cast<uint32_t*>(smem_raw + room_at);
             const uint32_t   room_bytes = smem_bytes - room_at;
             const int        tid        = threadIdx.x;
@@ -1280,7 +1331,7 @@ namespace aeonb
             if (tid < 64)
                 S.zz[tid] = k_zz_colmajor[tid];
             if (tid == 0)
-                S.bad = 0;
+                S.bad = S.slow = 0;
             __syncthreads();
             const aeonb_entropy_desc& d = S.d;
             if (!d.scratch || d.restart_interval != 0)
@@ -1326,7 +1377,10 @@ namespace aeonb
                     dcdiff = reinterpret_cast<int16_t*>(reinterpret_cast<uint8_t*>(room) + scan_room);
                 const uint32_t clean_size = copy_scan<true>(S, room, nullptr, vec, nv, lead);
                 __syncthreads();
-                decode_scan<shared_words>(S, A, room, clean_size, min_segment, needed_blocks, dcdiff);
+                if (S.slow)
+                    decode_scan<true, shared_words>(S, A, room, clean_size, min_segment, needed_blocks, dcdiff);
+                else
+                    decode_scan<false, shared_words>(S, A, room, clean_size, min_segment, needed_blocks, dcdiff);
             }
             else
             {
@@ -1334,7 +1388,7 @@ namespace aeonb
                 // the checkpoints' room and what follows is not in use yet
                 const uint32_t clean_size = copy_scan<false>(S, A.chk, words, vec, nv, lead);
                 __syncthreads();
-                decode_scan<global_words>(S, A, words, clean_size, min_segment, needed_blocks, dcdiff);
+                decode_scan<true, global_words>(S, A, words, clean_size, min_segment, needed_blocks, dcdiff);
             }
 
             // ---- DC: sum the differences per component in scan order.  Thread t owns MCUs [m0, m1).
@@ -1377,11 +1431,11 @@ namespace aeonb
         // marked doubtful and the serial kernel, launched behind, decodes it anew.
         //
         // Measured on a B200, 32 pictures of 900-1400 pixels a side (4:2:2, quality 92, a marker after every MCU row, 0.3 MB
-        // each): 88 ms with the serial kernel (one warp per stream), 0.38 ms with these two; 92 and 1.06 ms for a provider batch of them.
-        // A part of 4 to 10 KB per block fills the chip (about 30 parts per picture) and keeps segments at 160 bytes.
-        constexpr int RST_THREADS       = 128;
+        // each): 88 ms with the serial kernel (one warp per stream), 0.30 ms with these two.  Two blocks of 512 threads fit an SM by
+        // their tables; five of 128 threads with parts of at most 10 KB took 0.38 ms, most of it spent on building tables.
+        constexpr int RST_THREADS       = 512;
         constexpr int RST_INDEX_THREADS = 1024;
-        constexpr int RST_ROOM          = 12 * 1024 + 512; // shared memory for a part's bytes (see jpeg_restart_parts): 5 blocks fit an SM
+        constexpr int RST_ROOM          = 46 * 1024; // shared memory for a part's bytes (see jpeg_restart_parts): 2 blocks fit an SM
 
         struct rst_state
         {
@@ -1584,7 +1638,7 @@ namespace aeonb
         }
 
         // Segments of a part's intervals, their true entry states, and the storing pass.
-        template <typename Words>
+        template <bool SLOW, typename Words>
         __device__ __forceinline__ void decode_intervals(rst_state& R, const seg_arrays& A, const uint32_t* words, uint32_t first, uint32_t I,
                                                          uint32_t clean_size, int min_segment, int bpm, uint32_t needed_mcus, int16_t* dcdiff)
         {
@@ -1617,7 +1671,7 @@ namespace aeonb
             }
             const uint32_t pbeg = (R.clean[iv] + (tid - R.seg[iv]) * seg) * 8, pend = min(R.clean[iv + 1] * 8, pbeg + seg * 8);
             const uint32_t step       = seg * 8 / (NCHECK + 1);
-            const uint32_t run_blocks = settle_segments<Words>(S, A, words, nseg, R.seg[iv] == tid, pbeg, pend, step);
+            const uint32_t run_blocks = settle_segments<SLOW, Words>(S, A, words, nseg, R.seg[iv] == tid, pbeg, pend, step);
 
             // ---- first block number of every segment, counted from its interval's first block
             uint32_t counted;
@@ -1646,10 +1700,9 @@ namespace aeonb
                 if (at >= seg_end)
                     continue;
                 uint32_t p0, bk, before;
-                piece_entry(A, T, t, piece, at, p0, bk, before);
-                const uint32_t   g = A.ext_p[t] + before, gend = first_block(i + 1);
-                const seg_result r = run_segment<true, Words>(S, words, p0, bk >> 8, bk & 255, min(seg_end, at + step), g, gend, dcdiff, nullptr, 0,
-                                                              0, 0, false, 0);
+                piece_entry(A, t, piece, at, p0, bk, before);
+                const uint32_t     g = A.ext_p[t] + before, gend = first_block(i + 1);
+                const store_result r = store_segment<SLOW, Words>(S, words, p0, bk >> 8, bk & 255, min(seg_end, at + step), g, gend, dcdiff);
                 // the interval's last block leaves less than a byte, unless the region ends in front of that block
                 if (r.bad || (r.blocks > 0 && g + r.blocks == gend && (r.p > all_end || (all_end - r.p > 7 && !cut(i)))))
                     S.bad = 1;
@@ -1659,7 +1712,7 @@ namespace aeonb
 
         // Part blockIdx.x = {record, first interval, intervals, number of the part within its stream}.  Shared memory: rst_state,
         // SEG_BYTES per thread, and what is left of `smem_bytes` for the part's bytes, where they fit.
-        __global__ void __launch_bounds__(RST_THREADS) jpeg_entropy_restart_kernel(const aeonb_entropy_desc* __restrict__ descs,
+        __global__ void __launch_bounds__(RST_THREADS, 2) jpeg_entropy_restart_kernel(const aeonb_entropy_desc* __restrict__ descs,
                                                                                    const int4* __restrict__ parts, int min_segment,
                                                                                    uint32_t smem_bytes)
         {
@@ -1677,7 +1730,7 @@ namespace aeonb
             if (tid < 64)
                 S.zz[tid] = k_zz_colmajor[tid];
             if (tid == 0)
-                S.bad = 0;
+                S.bad = S.slow = 0;
             __syncthreads();
             const aeonb_entropy_desc& d = S.d;
             const restart_layout      w = restart_work(d);
@@ -1731,7 +1784,10 @@ namespace aeonb
             {
                 const uint32_t clean_size = copy_intervals<true>(R, I, room, nullptr, vec, lead);
                 __syncthreads();
-                decode_intervals<shared_words>(R, A, room, first, I, clean_size, min_segment, bpm, needed_mcus, dcdiff);
+                if (S.slow)
+                    decode_intervals<true, shared_words>(R, A, room, first, I, clean_size, min_segment, bpm, needed_mcus, dcdiff);
+                else
+                    decode_intervals<false, shared_words>(R, A, room, first, I, clean_size, min_segment, bpm, needed_mcus, dcdiff);
             }
             else
             {
@@ -1739,7 +1795,7 @@ namespace aeonb
                 uint32_t* const clean      = reinterpret_cast<uint32_t*>(w.clean + (r0 & ~15u) + 64u * (uint32_t)part.w);
                 const uint32_t  clean_size = copy_intervals<false>(R, I, A.chk, clean, vec, lead);
                 __syncthreads();
-                decode_intervals<global_words>(R, A, clean, first, I, clean_size, min_segment, bpm, needed_mcus, dcdiff);
+                decode_intervals<true, global_words>(R, A, clean, first, I, clean_size, min_segment, bpm, needed_mcus, dcdiff);
             }
             if (S.bad)
             {
@@ -1812,7 +1868,7 @@ namespace aeonb
         const int segments = (int)((longest + (uint32_t)jpeg_entropy_min_segment() - 1) / (uint32_t)jpeg_entropy_min_segment());
         const int wanted   = n <= 148 ? segments * (NCHECK + 1) : segments;
         int       threads  = jpeg_entropy_threads(n);
-        while (threads > 128 && wanted <= threads / 2)
+        while (threads > 256 && wanted <= threads / 2)
             threads /= 2;
         return threads & ~31;
     }
@@ -1835,9 +1891,9 @@ namespace aeonb
         for (int i = 0; i < n; ++i)
             if (descs[i].scratch && descs[i].restart_interval > 0)
                 total += descs[i].scan_size;
-        // Five blocks of a part fit an SM; parts of less than 4 KB are mostly set-up, parts of more than 12 KB do not fit its
-        // shared memory.
-        const uint64_t target = std::min<uint64_t>(std::max<uint64_t>(total / (148 * 5), 4096), 10240);
+        // Two blocks of a part fit an SM, and all parts should run at once; parts of less than 4 KB are mostly set-up, parts of more than
+        // 46 KB do not fit a block's shared memory.
+        const uint64_t target = std::min<uint64_t>(std::max<uint64_t>(total / (148 * 2), 4096), 36 * 1024);
         for (int i = 0; i < n; ++i)
         {
             const aeonb_entropy_desc& d = descs[i];
@@ -1846,7 +1902,8 @@ namespace aeonb
             const uint32_t all    = restart_work(d).intervals;
             const uint64_t mcus   = (uint64_t)std::min(d.roi[3], d.mcuy) * d.mcux;
             const uint32_t needed = (uint32_t)((mcus + d.restart_interval - 1) / d.restart_interval);
-            uint64_t       per    = std::max<uint64_t>(1, target * all / std::max<uint32_t>(d.scan_size, 1));
+            const uint64_t split  = std::max<uint64_t>(1, (d.scan_size + target / 2) / target);
+            uint64_t       per    = std::max<uint64_t>(1, (all + split - 1) / split);
             per = std::max<uint64_t>(per, (needed + restart_most_parts(all) - 1) / restart_most_parts(all));
             per = std::min<uint64_t>(per, RST_MAX_INTERVALS);
             for (uint32_t first = 0, k = 0; first < needed; first += (uint32_t)per, ++k)
@@ -1857,9 +1914,10 @@ namespace aeonb
     // Shared memory of a block of the block-parallel kernel: room for the launch's longest stream and its DC differences.  More
     // streams than SMs: as much as lets as many blocks share an SM as there are streams for it (four at most), the longest
     // streams falling back on global memory.
-    static size_t jpeg_entropy_smem(int n, int threads, uint32_t longest, uint64_t most_blocks)
+    static size_t jpeg_entropy_smem(int n, int threads, int rows, uint32_t longest, uint64_t most_blocks)
     {
-        const size_t fixed = sizeof(par_state) + (size_t)SEG_BYTES * threads + 16;
+        // (a copy in global memory leaves through a tile of 16 bytes per thread, laid over the checkpoints and what follows)
+        const size_t fixed = sizeof(par_state) + std::max((size_t)SEG_BYTES * rows + 16, (size_t)12 * rows + 16 * (size_t)threads + 32);
         const size_t want  = fixed + (size_t)longest + 16 + 64 + (size_t)most_blocks * 2;
         const int    share = std::min({(n + 147) / 148, 4, std::max(1, 1280 / threads)}); // the kernel's registers allow 1280 threads
         const size_t most  = (size_t)(228 * 1024) / share - 1024;
@@ -1875,13 +1933,14 @@ namespace aeonb
         if (any_parallel)
         {
             const int    threads = jpeg_entropy_block(n, longest);
-            const size_t smem = jpeg_entropy_smem(n, threads, longest, most_blocks);
+            const int    rows = std::min(threads, (int)(longest / (uint32_t)min_segment) + 1);
+            const size_t smem = jpeg_entropy_smem(n, threads, rows, longest, most_blocks);
             // always the most a block can have: the setting is the kernel's, and another thread may launch it with another size between
             // this call and the launch
             cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_parallel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (err != cudaSuccess)
                 return err;
-            jpeg_entropy_parallel_kernel<<<n, threads, smem, stream>>>(descs_dev, min_segment, (uint32_t)smem);
+            jpeg_entropy_parallel_kernel<<<n, threads, smem, stream>>>(descs_dev, min_segment, (uint32_t)rows, (uint32_t)smem);
             err = cudaGetLastError();
             if (err != cudaSuccess)
                 return err;

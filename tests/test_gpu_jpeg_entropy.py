@@ -372,3 +372,86 @@ def test_regions_that_end_inside_a_restart_interval(ctx, interval):
         _, want, _ = host_planes(blob, roi)
         assert status == 0 and all(np.array_equal(p, w[:p.size]) for p, w in zip(planes, want)), roi
         assert left_to_the_serial_decoder(work, d) == 0, roi
+
+
+def recode(blob, dc_lengths, ac_lengths):
+    """The same coefficients coded with other Huffman tables, one for DC and one for AC symbols: code lengths by symbol."""
+    import struct
+    from aeon_b200 import kernels as K
+    info, coefs, _ = K.jpeg_entropy_decode(blob)
+    zz = [0, 8, 1, 2, 9, 16, 24, 17, 10, 3, 4, 11, 18, 25, 32, 40, 33, 26, 19, 12, 5, 6, 13, 20, 27, 34, 41, 48, 56, 49, 42, 35, 28, 21, 14, 7,
+          15, 22, 29, 36, 43, 50, 57, 58, 51, 44, 37, 30, 23, 31, 38, 45, 52, 59, 60, 53, 46, 39, 47, 54, 61, 62, 55, 63]  # column-major
+
+    def canonical(lengths):
+        codes, code, last = {}, 0, 0
+        for sym, ln in sorted(lengths.items(), key=lambda s: (s[1], s[0])):
+            code <<= ln - last
+            codes[sym], code, last = (code, ln), code + 1, ln
+        counts = bytes(sum(v == ln for v in lengths.values()) for ln in range(1, 17))
+        return codes, counts + bytes(s for s, _ in sorted(lengths.items(), key=lambda s: (s[1], s[0])))
+
+    (dc, dc_table), (ac, ac_table) = canonical(dc_lengths), canonical(ac_lengths)
+    bits = []
+
+    def put(code, value, size):
+        bits.append(format(code[0], "0%db" % code[1]))
+        if size:
+            bits.append(format(value if value > 0 else value + (1 << size) - 1, "0%db" % size))
+
+    pred = [0] * info.ncomp
+    for m in range((info.blocks_w[0] // info.hs[0]) * (info.blocks_h[0] // info.vs[0])):
+        mx, my = m % (info.blocks_w[0] // info.hs[0]), m // (info.blocks_w[0] // info.hs[0])
+        for c in range(info.ncomp):
+            for y in range(info.vs[c]):
+                for x in range(info.hs[c]):
+                    at = ((my * info.vs[c] + y) * info.blocks_w[c] + mx * info.hs[c] + x) * 64
+                    block = [int(coefs[c][at + zz[k]]) for k in range(64)]
+                    diff, pred[c] = block[0] - pred[c], block[0]
+                    put(dc[abs(diff).bit_length()], diff, abs(diff).bit_length())
+                    run = 0
+                    for k in range(1, 64):
+                        if block[k] == 0:
+                            run += 1
+                            continue
+                        for _ in range(run // 16):
+                            put(ac[0xf0], 0, 0)
+                        size = abs(block[k]).bit_length()
+                        put(ac[run % 16 << 4 | size], block[k], size)
+                        run = 0
+                    if run:
+                        put(ac[0], 0, 0)
+    text = "".join(bits)
+    text += "1" * (-len(text) % 8)
+    body = bytes(int(text[i:i + 8], 2) for i in range(0, len(text), 8)).replace(b"\xff", b"\xff\x00")
+    out, p = blob[:2], 2
+    while blob[p + 1] != 0xDA:          # the other segments as they are, without the tables
+        end = p + 2 + struct.unpack(">H", blob[p + 2:p + 4])[0]
+        out += blob[p:end] if blob[p + 1] != 0xC4 else b""
+        p = end
+    for kind, table in ((0, dc_table), (0x10, ac_table)):
+        out += b"\xff\xc4" + struct.pack(">H", 3 + len(table)) + bytes([kind]) + table
+    sos = bytearray(blob[p:p + 2 + struct.unpack(">H", blob[p + 2:p + 4])[0]])
+    for c in range(info.ncomp):
+        sos[6 + 2 * c] = 0
+    return out + bytes(sos) + body + b"\xff\xd9"
+
+
+@pytest.mark.parametrize("dc_long, ac_long, ac_short", [(5, 10, 2), (9, 11, 3), (10, 12, 3), (12, 12, 4), (16, 16, 1), (5, 16, 2)])
+def test_tables_with_codes_longer_than_the_lookup_windows(ctx, dc_long, ac_long, ac_short):
+    """Canonical tables with a few short codes and the rest of one length: just inside the windows (9 bits DC, 11 AC), just outside, and
+    so long that they do not start near the end of the code space, where the tables expect codes beyond the windows.  In one stream of
+    a batch only, in both kernels with a work area."""
+    import cv2
+    rng = np.random.default_rng(70)
+    img = gradient_image(rng, 90, 130)
+    plain = jpeg_bytes(img, 88)
+    dc = {s: (2 if s in (2, 3) else dc_long) for s in range(12)}
+    short = [0x01, 0x00, 0x02, 0x11][:ac_short]
+    ac = {r << 4 | s: ac_long for r in range(16) for s in range(1, 11)}
+    ac.update({0x00: ac_long, 0xf0: ac_long})
+    ac.update({s: k + 1 for k, s in enumerate(short)})
+    assert sum(2.0 ** -v for v in ac.values()) < 1 and sum(2.0 ** -v for v in dc.values()) < 1
+    blob = recode(plain, dc, ac)
+    assert np.array_equal(cv2.imdecode(np.frombuffer(blob, np.uint8), 1), cv2.imdecode(np.frombuffer(plain, np.uint8), 1))
+    check(ctx, [plain, blob, jpeg_bytes(img, 88, [cv2.IMWRITE_JPEG_OPTIMIZE, 1])])
+    check(ctx, [blob])
