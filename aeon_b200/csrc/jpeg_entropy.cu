@@ -468,10 +468,11 @@ namespace aeonb
         // a predicated load beside that chain; with a second, dependent lookup for long codes and a branch for codes in no table a
         // pass took half as long again.
         //
-        // Measured on a B200 (kernel times): one stream of about 40 KB 0.183 ms before, 0.146 ms now; 256 streams of up to 55 KB (4:2:0,
-        // quality 90, crop regions stored) 0.263 / 0.207 ms; 512 streams of 6 KB 0.232 / 0.147 ms.  Phases of a 43 KB stream, thousand
-        // cycles: first pass 62 / 44 (16 of them beside the clearing of the planes), rounds 126 / 77 (five of them), storing pass
-        // 110 / 102 (one 2-byte store per coefficient, each to a line of its own), copy and marker scan 21, DC 14, set-up 18.
+        // Measured on a B200 (kernel times): one stream of about 40 KB 0.183 ms before, 0.136 ms now; 256 streams of up to 55 KB (4:2:0,
+        // quality 90, crop regions stored) 0.263 / 0.196 ms; 512 streams of 6 KB 0.232 / 0.135 ms.  Phases of a 43 KB stream, thousand
+        // cycles: first pass 62 / 40 (14 of them beside the clearing of the planes), rounds 126 / 68 (five of them), storing pass
+        // 110 / 101 (one 2-byte store per coefficient, each to a line of its own; 65 without them), copy and marker scan 21 / 17,
+        // DC 14 (stores again), set-up 18 / 14.
         // A wrong guess falls into step with the true decoder after about 10 blocks on average (the block's
         // position inside the MCU has to match too), and not at all inside flat regions, where every block looks
         // the same: there a chain of segments is settled one round per segment, which is what the slowest streams
@@ -517,85 +518,119 @@ namespace aeonb
 
         struct code_table
         {
-            int     limit[17]; // limit[len]: exclusive upper bound of the codes of length <= len, left-justified to 16 bits
+            alignas(16) int limit[16]; // limit[len - 1]: exclusive upper bound of the codes of length <= len, left-justified to 16 bits
             int     valoff[17];
             uint8_t vals[256];
         };
 
-        // One thread fills the canonical-code limits of a table from the DHT form (16 counts); the values are copied by the caller.
-        __device__ void build_code_table(code_table& T, const uint8_t* __restrict__ dht, int* bad)
+        // A warp fills the canonical-code limits of a table from the DHT form (16 counts); the values are copied by the caller.  With n(l)
+        // codes of length l, those of length <= l end at the sum of n(j) << (16 - j) over j <= l, left-justified.
+        __device__ __forceinline__ void build_code_table(code_table& T, const uint8_t* dht, int lane, int* bad)
         {
-            int code = 0, k = 0;
-            T.limit[0] = 0;
-            for (int len = 1; len <= 16; ++len)
+            const int n = lane < 16 ? dht[lane] : 0, codes = lane < 16 ? n << (15 - lane) : 0;
+            int       k = n, limit = codes;
+#pragma unroll
+            for (int o = 1; o < 16; o <<= 1)
             {
-                const int n   = dht[len - 1];
-                T.valoff[len] = k - code;
-                code += n;
-                k += n;
-                if (code > (1 << len) || k > 256)
-                    *bad = 1;
-                T.limit[len] = code << (16 - len);
-                code <<= 1;
+                const int up_k = __shfl_up_sync(0xffffffffu, k, o), up_limit = __shfl_up_sync(0xffffffffu, limit, o);
+                k += lane >= o ? up_k : 0;
+                limit += lane >= o ? up_limit : 0;
             }
+            if (lane >= 16)
+                return;
+            T.valoff[lane + 1] = k - n - ((limit - codes) >> (15 - lane));
+            T.limit[lane]      = limit;
+            if (limit > 1 << 16 || k > 256)
+                *bad = 1;
         }
-        // Length of the code at the head of the 16 bits c16, known to be at least `from`, if it is no longer than `to`.
-        __device__ __forceinline__ int code_length(const code_table& T, int c16, int from, int to)
+        // The limits of a table in registers: the length of a code is then a count of comparisons that do not wait for one another.
+        struct code_limits
         {
-            while (from < to && c16 >= T.limit[from])
-                ++from;
-            return from;
-        }
-        // A code known to be at least `from` bits long, or an invalid one, at the head of the 16 bits c16.
-        __device__ __noinline__ uint32_t long_symbol(const code_table& T, int c16, bool is_ac, int from)
+            int of[16];
+            __device__ __forceinline__ explicit code_limits(const code_table& T)
+            {
+#pragma unroll
+                for (int k = 0; k < 4; ++k)
+                {
+                    const int4 v = reinterpret_cast<const int4*>(T.limit)[k];
+                    of[4 * k] = v.x, of[4 * k + 1] = v.y, of[4 * k + 2] = v.z, of[4 * k + 3] = v.w;
+                }
+            }
+            // Length of the code at the head of the 16 bits c16, or MOST if it is not shorter (or not a code).
+            template <int MOST>
+            __device__ __forceinline__ int length(int c16) const
+            {
+                int len = 1;
+#pragma unroll
+                for (int l = 1; l < MOST; ++l)
+                    len += c16 >= of[l - 1];
+                return len;
+            }
+        };
+        __device__ __forceinline__ uint32_t code_entry(const code_table& T, int c16, int len, bool is_ac)
         {
-            if (c16 >= T.limit[16])
-                return k_invalid;
-            const int len = code_length(T, c16, from, 16);
             return pack_symbol(len, T.vals[((c16 >> (16 - len)) + T.valoff[len]) & 255], is_ac);
         }
-        __device__ __forceinline__ uint32_t window_entry(const code_table& T, int i, int len, int bits, bool is_ac, int* slow)
+        // The symbol at the head of the 16 bits c16, whatever its length, for codes that are in no table.
+        __device__ __noinline__ uint32_t long_symbol(const code_table& T, int c16, bool is_ac)
         {
-            const int c16 = i << (16 - bits);
-            if (c16 < T.limit[len])
-                return pack_symbol(len, T.vals[((i >> (bits - len)) + T.valoff[len]) & 255], is_ac);
-            if (c16 >= LONG_FROM)
-                return 0;
-            if (c16 >= T.limit[16])
-                return k_invalid;
-            *slow = 1;
-            return k_slow;
+            return c16 >= T.limit[15] ? k_invalid : code_entry(T, c16, code_limits(T).length<16>(c16), is_ac);
         }
         // Where a table starts among the ENTRIES: DC slot 0, DC slot 1, AC slot 0, AC slot 1.
         __device__ __forceinline__ int table_at(int t) { return t < 2 ? t * DC_ENTRIES : 2 * DC_ENTRIES + (t - 2) * AC_ENTRIES; }
-        // `nth` threads (index `tid`) fill the storing pass's entries of the four tables once limits and values are in place.  Eight
-        // neighbouring entries go together: unless a code of the last three lengths starts among them they hold one symbol, so the
-        // length is searched twice per eight entries.
+        // Eight neighbouring entries of a window of BITS bits, from i on.  Unless a code of the last three lengths starts among them they
+        // hold one symbol, so most often two lengths are worked out per eight entries.
+        template <int BITS>
+        __device__ __forceinline__ void fill_window(uint16_t* out, const code_table& T, int i, bool is_ac, int* slow)
+        {
+            const code_limits limits(T);
+            const int         first = limits.length<BITS>(i << (16 - BITS)), last = limits.length<BITS>((i + 7) << (16 - BITS));
+            const auto        entry = [&](int k, int len) -> uint32_t {
+                const int c16 = (i + k) << (16 - BITS);
+                if (c16 < T.limit[len - 1])
+                    return code_entry(T, c16, len, is_ac);
+                if (c16 >= LONG_FROM)
+                    return 0;
+                if (c16 >= T.limit[15])
+                    return k_invalid;
+                *slow = 1;
+                return k_slow;
+            };
+            if (first == last && first <= BITS - 3)
+            {
+                const uint32_t e = entry(0, first) * 0x10001u;
+                *reinterpret_cast<uint4*>(out) = make_uint4(e, e, e, e);
+                return;
+            }
+            uint32_t e[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                e[k] = entry(k, limits.length<BITS>((i + k) << (16 - BITS)));
+            *reinterpret_cast<uint4*>(out) = make_uint4(e[0] | e[1] << 16, e[2] | e[3] << 16, e[4] | e[5] << 16, e[6] | e[7] << 16);
+        }
+        // `nth` threads (index `tid`) fill the storing pass's entries of the four tables once limits and values are in place.
         __device__ void build_tables(uint16_t* store, const code_table* codes, int tid, int nth, int* slow)
         {
             constexpr int ac8 = (1 << AC_BITS) / 8, dc8 = (1 << DC_BITS) / 8;
-            for (int j = tid; j < 2 * (ac8 + dc8); j += nth)
+            for (int j = tid; j < 2 * ac8; j += nth)
+                fill_window<AC_BITS>(store + table_at(2 + j / ac8) + LONG + 8 * (j % ac8), codes[2 + j / ac8], 8 * (j % ac8), true, slow);
+            // the last threads first: they have least to do above
+            for (int j = nth - 1 - tid; j < 2 * dc8; j += nth)
+                fill_window<DC_BITS>(store + table_at(j / dc8) + LONG + 8 * (j % dc8), codes[j / dc8], 8 * (j % dc8), false, slow);
+            for (int j = tid; j < 4 * LONG / 2; j += nth)
             {
-                const bool        is_ac = j < 2 * ac8;
-                const int         t = is_ac ? 2 + j / ac8 : (j - 2 * ac8) / dc8, i = (is_ac ? j % ac8 : (j - 2 * ac8) % dc8) * 8;
-                const int         bits = is_ac ? AC_BITS : DC_BITS;
-                const code_table& T    = codes[t];
-                uint16_t* const   out  = store + table_at(t) + LONG + i;
-                const int first = code_length(T, i << (16 - bits), 1, bits), last = code_length(T, (i + 7) << (16 - bits), first, bits);
-                if (first == last && first <= bits - 3)
+                const int         t = j / (LONG / 2), i = 2 * (j % (LONG / 2));
+                const code_table& T = codes[t];
+                const code_limits limits(T);
+                uint32_t          e[2];
+#pragma unroll
+                for (int k = 0; k < 2; ++k)
                 {
-                    const uint32_t e = window_entry(T, i, first, bits, is_ac, slow) * 0x10001u;
-                    *reinterpret_cast<uint4*>(out) = make_uint4(e, e, e, e);
+                    const int c16 = LONG_FROM + i + k;
+                    e[k]          = c16 >= T.limit[15] ? k_invalid : code_entry(T, c16, limits.length<16>(c16), t >= 2);
                 }
-                else
-                {
-#pragma unroll 1
-                    for (int k = 0; k < 8; ++k)
-                        out[k] = (uint16_t)window_entry(T, i + k, code_length(T, (i + k) << (16 - bits), first, last), bits, is_ac, slow);
-                }
+                *reinterpret_cast<uint32_t*>(store + table_at(t) + i) = e[0] | e[1] << 16;
             }
-            for (int j = tid; j < 4 * LONG; j += nth)
-                store[table_at(j / LONG) + j % LONG] = (uint16_t)long_symbol(codes[j / LONG], LONG_FROM + j % LONG, j >= 2 * LONG, 1);
         }
         // The entries of the other passes from those of the storing pass; eight neighbours per thread and pass so that the lookups of
         // the second symbols overlap.
@@ -805,6 +840,10 @@ namespace aeonb
             // The 32 bits under the position lie in w0 and w1; w2 is the word behind them, fetched when the one before it comes into use.
             Words    ahead(words, p >> 5);
             uint32_t w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
+            // The entry of the symbol under the position is fetched as soon as the position is known, and what else a step has to do is
+            // done while that load is under way.
+            uint32_t h = __funnelshift_l(w1, w0, at); // 32 valid bits; a symbol or a pair takes at most 31
+            uint32_t e = lds_u32(look + ((h >> shift) << 2));
             for (;;)
             {
                 for (uint32_t pos = at & k_position; pos < stop;)
@@ -812,27 +851,27 @@ namespace aeonb
                     // Two symbols at a time as long as the first one cannot reach `stop`: a run stops at the first symbol at or past
                     // it, however it came there.
                     const uint32_t take = at < k_pair_limit && pos + k_pair_first < stop ? k_take_pair : k_take_one;
-                    const uint32_t h    = __funnelshift_l(w1, w0, at); // 32 valid bits; a symbol or a pair takes at most 31
-                    uint32_t       e    = lds_u32(look + ((h >> shift) << 2));
                     if (SLOW && e == k_slow)
                     {
                         const bool is_ac = at > k_position;
                         const int  slot1 = look == shared_address(S.scan + table_at(is_ac ? 3 : 1) + LONG);
-                        e = scan_entry(long_symbol(S.codes[(is_ac ? 2 : 0) + slot1], (int)(h >> 16), is_ac, 1));
+                        e = scan_entry(long_symbol(S.codes[(is_ac ? 2 : 0) + slot1], (int)(h >> 16), is_ac));
                     }
                     const uint32_t by    = __byte_perm(e, 0, take);
                     const uint32_t to    = at + by;
                     const bool     cross = (at ^ to) & 32; // the read position has left w0
                     const bool     end = to >= k_block_end, again = by == 0;
-                    w0                   = cross ? w1 : w0;
-                    w1                   = cross ? w2 : w1;
-                    ahead.next_if(w2, cross);
+                    w0    = cross ? w1 : w0;
+                    w1    = cross ? w2 : w1;
                     look  = again ? look - 4 * LONG - 4 * LONG_FROM : end ? link.next_dc : link.ac;
                     shift = again ? 16 : end ? 32 - DC_BITS : 32 - AC_BITS;
                     at    = end ? to & k_position : to;
+                    h     = __funnelshift_l(w1, w0, at);
+                    e     = lds_u32(look + ((h >> shift) << 2));
                     pos   = to & k_position;
-                    blocks += end;
+                    ahead.next_if(w2, cross);
                     follow_if(link, end);
+                    blocks += end;
                 }
                 if (stop == pend)
                     break;
@@ -891,37 +930,40 @@ namespace aeonb
             const uint32_t zz   = shared_address(S.zz);
             Words          ahead(words, p >> 5);
             uint32_t       w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
+            uint32_t       h = __funnelshift_l(w1, w0, at);
+            uint32_t       e = lds_u16(look + ((h >> shift) << 1));
             while (pos < pend && g < gend)
             {
-                const uint32_t h = __funnelshift_l(w1, w0, at);
-                uint32_t       e = lds_u16(look + ((h >> shift) << 1));
                 if (SLOW && e == k_slow)
                 {
                     const bool is_ac = at > k_position;
                     const int  slot1 = look == shared_address(S.store + table_at(is_ac ? 3 : 1) + LONG);
-                    e                = long_symbol(S.codes[(is_ac ? 2 : 0) + slot1], (int)(h >> 16), is_ac, 1);
+                    e                = long_symbol(S.codes[(is_ac ? 2 : 0) + slot1], (int)(h >> 16), is_ac);
                 }
                 const uint32_t total = entry_total(e), size = entry_size(e), advance = entry_advance(e);
-                const uint32_t kk = (at >> 24) + advance - 1; // the coefficient's place
-                const uint32_t x  = h << (total - size);      // the value bits at the top
+                const uint32_t x     = h << (total - size); // the value bits at the top
+                const uint32_t was = at, to = at + (total | advance << 24);
+                const bool     cross = (at ^ to) & 32;
+                const bool     end = to >= k_block_end, again = e == 0;
+                w0    = cross ? w1 : w0;
+                w1    = cross ? w2 : w1;
+                look  = again ? look - 2 * LONG - 2 * LONG_FROM : end ? place.next_dc : place.ac;
+                shift = again ? 16 : end ? 32 - DC_BITS : 32 - AC_BITS;
+                at    = end ? to & k_position : to;
+                h     = __funnelshift_l(w1, w0, at);
+                e     = lds_u16(look + ((h >> shift) << 1));
+                pos   = to & k_position;
+                ahead.next_if(w2, cross);
+
+                const uint32_t kk = (was >> 24) + advance - 1; // the coefficient's place
                 const int      v  = (int)__funnelshift_l(x, 0u, size) + ((int)x >= 0 ? 1 - (1 << size) : 0);
                 const bool     inside = (uint32_t)mx < roi_w && (uint32_t)my < roi_h;
                 // an invalid code, or a run that leaves the block
                 R.bad |= size != 0 && (int)kk > 63;
-                if (at <= k_position)
+                if (was <= k_position)
                     dcdiff[g] = (int16_t)v;
                 else if (size != 0 && kk <= 63 && inside)
                     place.base[(int64_t)(my * place.dy + mx * place.dx) * 64 + S.zz[kk]] = (int16_t)v;
-                const uint32_t to    = at + (total | advance << 24);
-                const bool     cross = (at ^ to) & 32;
-                const bool     end = to >= k_block_end, again = e == 0;
-                w0                   = cross ? w1 : w0;
-                w1                   = cross ? w2 : w1;
-                ahead.next_if(w2, cross);
-                look  = again ? look - 2 * LONG - 2 * LONG_FROM : end ? place.next_dc : place.ac;
-                shift = again ? 16 : end ? 32 - DC_BITS : 32 - AC_BITS;
-                at    = end ? to & k_position : to;
-                pos   = to & k_position;
                 g += end;
                 mx += end ? place.last : 0;
                 my += mx == mx_end;
@@ -962,6 +1004,29 @@ namespace aeonb
             return (warp ? before : 0) + incl - v;
         }
 
+        // The same of three values at once.
+        __device__ __forceinline__ void cta_exclusive_scan3(const int (&v)[3], uint32_t (*sums)[32], int (&before)[3])
+        {
+            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+            int       incl[3] = {v[0], v[1], v[2]};
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1)
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+                {
+                    const int up = __shfl_up_sync(0xffffffffu, incl[c], o);
+                    incl[c] += lane >= o ? up : 0;
+                }
+            __syncthreads(); // `sums` may still be read from an earlier scan
+            if (lane == 31)
+                for (int c = 0; c < 3; ++c)
+                    sums[c][warp] = (uint32_t)incl[c];
+            __syncthreads();
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+                before[c] = __reduce_add_sync(0xffffffffu, lane < warp ? (int)sums[c][lane] : 0) + incl[c] - v[c];
+        }
+
         // The copy of a stream without stuffed bytes holds big-endian 32-bit words (byte i of the copy is byte i ^ 3 of memory).
         // Resident: the raw scan lies in shared memory, from 16-byte vector 0 on, and the copy takes its place -- a tile's bytes are
         // in registers before any of them is written, and never move up.  Otherwise the copy goes to global memory: a thread's
@@ -975,20 +1040,51 @@ namespace aeonb
             uint32_t  size; // bytes appended so far (the same in every thread)
             uint32_t  rest; // the last, incomplete word (thread 0)
 
-            // Appends the bytes of w whose bits are set in `keep`, `at` being their place among the tile's `total` bytes; every
-            // thread has passed a barrier since it read its part of the tile.
+            // Appends the bytes of w (in memory order) whose bits are set in `keep`, `at` being their place among the tile's `total`
+            // bytes; every thread has passed a barrier since it read its part of the tile.
             __device__ __forceinline__ void append(const uint32_t (&w)[4], uint32_t keep, uint32_t at, uint32_t total)
             {
                 uint8_t* const bytes = reinterpret_cast<uint8_t*>(room);
                 const uint32_t carry = RESIDENT ? size : size & 3;
-                uint32_t       o     = carry + at;
                 if (!RESIDENT && threadIdx.x == 0)
                     for (uint32_t c = 0; c < carry; ++c)
                         bytes[c ^ 3] = (uint8_t)(rest >> (24 - 8 * c));
+                // big-endian words without the bytes that go (as a rule none or one of the sixteen)
+                uint32_t       be[4], n = (uint32_t)__popc(keep);
+                const uint32_t o = carry + at, end = o + n;
 #pragma unroll
-                for (int b = 0; b < 16; ++b)
-                    if (keep >> b & 1)
-                        bytes[o++ ^ 3] = (uint8_t)(w[b >> 2] >> (8 * (b & 3)));
+                for (int k = 0; k < 4; ++k)
+                    be[k] = __byte_perm(w[k], 0, 0x0123);
+                for (uint32_t gone = ~keep & 0xFFFF; gone;)
+                {
+                    const uint32_t g = 31 - __clz(gone), in = 8 * (g & 3); // the last one: what lies behind it moves up a byte
+                    gone ^= 1u << g;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4; ++k)
+                    {
+                        const uint32_t up   = __funnelshift_l(k < 3 ? be[k + 1] : 0, be[k], 8);
+                        const uint32_t mask = k < g >> 2 ? 0 : k > g >> 2 ? 0xFFFFFFFFu : 0xFFFFFFFFu >> in;
+                        be[k]               = (be[k] & ~mask) | (up & mask);
+                    }
+                }
+                // They start anywhere in a word: whole words are stored as such, the ends, which belong to two threads, by bytes.
+                const uint32_t shift = 8 * (o & 3), w0 = o >> 2, w1 = end >> 2;
+                uint32_t       head = 0, tail = 0;
+#pragma unroll
+                for (uint32_t k = 0; k < 5; ++k)
+                {
+                    const uint32_t word = __funnelshift_r(k < 4 ? be[k < 4 ? k : 0] : 0, k > 0 ? be[k - 1] : 0, shift);
+                    if ((k > 0 || shift == 0) && w0 + k < w1)
+                        room[w0 + k] = word;
+                    head = k == 0 ? word : head;
+                    tail = w0 + k == w1 ? word : tail;
+                }
+                if (shift != 0)
+                    for (uint32_t b = o; b < min(end, (o | 3) + 1); ++b)
+                        bytes[b ^ 3] = (uint8_t)(head >> (24 - 8 * (b & 3)));
+                if (w1 > w0 || shift == 0)
+                    for (uint32_t b = end & ~3u; b < end; ++b)
+                        bytes[b ^ 3] = (uint8_t)(tail >> (24 - 8 * (b & 3)));
                 if (!RESIDENT)
                 {
                     __syncthreads();
@@ -1029,50 +1125,41 @@ namespace aeonb
         __device__ __forceinline__ void set_up_stream(par_state& S, int tid, int nth)
         {
             const aeonb_entropy_desc& d = S.d;
-            if (tid == 0)
-            {
-                int b = 0;
-                for (int c = 0; c < d.ncomp; ++c)
-                {
-                    const int64_t row_blocks = (int64_t)(d.roi[2] - d.roi[0]) * d.hs[c]; // blocks in a row of the compact plane
-                    for (int y = 0; y < d.vs[c]; ++y)
-                        for (int x = 0; x < d.hs[c]; ++x, ++b)
-                        {
-                            S.comp[b]       = (uint8_t)c;
-                            S.link[b].ac    = shared_address(S.scan + table_at(2 + (d.ac_table[c] & 1)) + LONG);
-                            S.place[b].ac   = shared_address(S.store + table_at(2 + (d.ac_table[c] & 1)) + LONG);
-                            S.link[b].block = (uint32_t)b;
-                            S.place[b].base = d.coef[c] + (y * row_blocks + x) * 64;
-                            S.place[b].dy   = (int32_t)(d.vs[c] * row_blocks);
-                            S.place[b].dx   = d.hs[c];
-                        }
-                }
-                S.bpm = b;
-            }
-            // The tables in DHT form are brought in whole: the head of a table is a chain over its 16 code counts, which one
-            // thread walks from shared memory rather than from L2.
+            // The tables in DHT form are brought in whole by the last threads, while the first ones see to the blocks of an MCU.
+            const int back = nth - 1 - tid;
             if ((reinterpret_cast<uintptr_t>(d.tables) & 15) == 0)
             {
-                for (int i = tid; i < 4 * 272 / 16; i += nth)
+                for (int i = back; i < 4 * 272 / 16; i += nth)
                     reinterpret_cast<uint4*>(S.dht)[i] = __ldg(reinterpret_cast<const uint4*>(d.tables) + i);
             }
             else
-                for (int i = tid; i < 4 * 272; i += nth)
+                for (int i = back; i < 4 * 272; i += nth)
                     S.dht[i] = __ldg(d.tables + i);
-            __syncthreads();
-            if (tid < S.bpm)
+            int bpm = 0;
+            for (int c = 0; c < d.ncomp; ++c)
+                bpm += d.hs[c] * d.vs[c];
+            if (tid < bpm)
             {
-                const int next       = tid + 1 < S.bpm ? tid + 1 : 0;
-                const int dc         = table_at(d.dc_table[S.comp[next]] & 1) + LONG;
-                S.link[tid].next_dc  = shared_address(S.scan + dc);
-                S.link[tid].next     = shared_address(&S.link[next]);
-                S.place[tid].next_dc = shared_address(S.store + dc);
-                S.place[tid].next    = shared_address(&S.place[next]);
-                S.place[tid].last    = next == 0;
+                const auto part_of = [&](int b, int& at) -> int { // component of block b of an MCU, and the number of its first block
+                    at = 0;
+                    for (int c = 0;; at += d.hs[c] * d.vs[c], ++c)
+                        if (c + 1 == d.ncomp || b < at + d.hs[c] * d.vs[c])
+                            return c;
+                };
+                int           at, unused;
+                const int     c = part_of(tid, at), x = (tid - at) % d.hs[c], y = (tid - at) / d.hs[c], next = tid + 1 < bpm ? tid + 1 : 0;
+                const int64_t row_blocks = (int64_t)(d.roi[2] - d.roi[0]) * d.hs[c]; // blocks in a row of the compact plane
+                const int     ac = table_at(2 + (d.ac_table[c] & 1)) + LONG, dc = table_at(d.dc_table[part_of(next, unused)] & 1) + LONG;
+                S.comp[tid]  = (uint8_t)c;
+                S.link[tid]  = block_link{shared_address(S.scan + ac), shared_address(S.scan + dc), shared_address(&S.link[next]), (uint32_t)tid};
+                S.place[tid] = block_place{shared_address(S.store + ac), shared_address(S.store + dc), shared_address(&S.place[next]),
+                                           (uint32_t)(next == 0), d.coef[c] + (y * row_blocks + x) * 64, (int32_t)(d.vs[c] * row_blocks), d.hs[c]};
             }
-            if ((tid & 31) == 0)
-                for (int t = tid >> 5; t < 4; t += nth >> 5)
-                    build_code_table(S.codes[t], S.dht + t * 272, &S.bad);
+            if (tid == 0)
+                S.bpm = bpm;
+            __syncthreads();
+            for (int t = tid >> 5; t < 4; t += nth >> 5)
+                build_code_table(S.codes[t], S.dht + t * 272, tid & 31, &S.bad);
             for (int i = tid; i < 4 * 256; i += nth)
                 S.codes[i >> 8].vals[i & 255] = S.dht[(i >> 8) * 272 + 16 + (i & 255)];
             __syncthreads();
@@ -1176,6 +1263,18 @@ namespace aeonb
             }
         }
 
+        // Of 16 bytes, a bit each: those equal to the bytes of `value`; those from number `n` on, and those below it (n may lie outside).
+        __device__ __forceinline__ uint32_t byte_mask(const uint32_t (&w)[4], uint32_t value)
+        {
+            uint32_t m = 0;
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                m |= ((__vcmpeq4(w[k], value) & 0x08040201u) * 0x01010101u >> 24) << (4 * k);
+            return m;
+        }
+        __device__ __forceinline__ uint32_t bits_below(int n) { return n >= 16 ? 0xFFFFu : n <= 0 ? 0 : (1u << n) - 1; }
+        __device__ __forceinline__ uint32_t bits_from(int n) { return 0xFFFFu & ~bits_below(n); }
+
         // Copies the scan without stuffed bytes, up to the first marker; returns the bytes of the copy.  RESIDENT: in place in `room`,
         // where the scan's vectors have been brought; otherwise from `vec` to `out` through the tile `room`.
         template <bool RESIDENT>
@@ -1199,27 +1298,13 @@ namespace aeonb
                         prev = !RESIDENT  ? (uint32_t)__ldg(reinterpret_cast<const uint8_t*>(vec) + 16 * i - 1)
                                : tid == 0 ? S.tile_end[odd ^ 1] // its place may have been taken
                                           : (uint32_t) reinterpret_cast<const uint8_t*>(room)[16 * i - 1];
-                    // Nearly every vector lies inside the stream and has no 0xFF in front of any of its bytes: all 16 are kept.
-                    const bool inside = 16 * i > lead && 16 * i + 16 - lead <= raw_end;
-                    const bool no_ff  = prev != 0xFF && !__vcmpeq4(w[0], 0xFFFFFFFFu) && !__vcmpeq4(w[1], 0xFFFFFFFFu) &&
-                                       !__vcmpeq4(w[2], 0xFFFFFFFFu) && !(__vcmpeq4(w[3], 0xFFFFFFFFu) & 0x00FFFFFFu);
-                    if (inside && no_ff)
-                        keep = 0xFFFF;
-                    else
-                    {
-#pragma unroll
-                        for (int b = 0; b < 16; ++b)
-                        {
-                            const uint32_t v   = (w[b >> 2] >> (8 * (b & 3))) & 255;
-                            const uint32_t pos = 16 * i + b; // offset from the aligned address
-                            if (pos == lead)
-                                prev = 0;
-                            const bool in = pos >= lead && pos - lead < N;
-                            keep |= (uint32_t)(in && pos - lead < raw_end && !(prev == 0xFF && v == 0)) << b;
-                            marker |= (uint32_t)(in && prev == 0xFF && v != 0) << b;
-                            prev = v;
-                        }
-                    }
+                    // bytes of the vector that belong to the stream, and those in front of the first marker found so far
+                    const uint32_t own  = bits_from((int)lead - (int)(16 * i)) & bits_below((int)(lead + N) - (int)(16 * i));
+                    const uint32_t data = own & bits_below((int)(lead + raw_end) - (int)(16 * i));
+                    const uint32_t ff = byte_mask(w, 0xFFFFFFFFu), zero = byte_mask(w, 0);
+                    const uint32_t follows = ((ff & own) << 1 | (prev == 0xFF && 16 * i > lead)) & 0xFFFF; // bytes that follow 0xFF
+                    keep   = data & ~(follows & zero);
+                    marker = own & follows & ~zero;
                     // The second byte of a marker whose first is the tile's last lies in the next tile, which is too late.
                     if (tid == T - 1 && i + 1 < nv && w[3] >> 24 == 0xFF)
                         marker |= (uint32_t)((RESIDENT ? reinterpret_cast<const uint8_t*>(room)[16 * i + 16]
@@ -1361,7 +1446,7 @@ namespace aeonb
             const bool         resident  = scan_room <= room_bytes;
             if (resident)
                 fetch_raw(room, vec, 0, nv); // arrives while the tables are being built
-            if (tid == 0)
+            if (tid == 64) // not a thread that sets anything else up
                 S.marker_at = N > 0 && __ldg(d.scan + N - 1) == 0xFF ? N - 1 : N;
             set_up_stream(S, tid, (int)T);
             asm volatile("cp.async.wait_all;" ::: "memory");
@@ -1405,12 +1490,7 @@ namespace aeonb
                     sum[2] += c == 2 ? v : 0;
                 }
             int pred[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-            {
-                uint32_t total;
-                pred[c] = (int)cta_exclusive_scan((uint32_t)sum[c], S.warp_sums[c], total);
-            }
+            cta_exclusive_scan3(sum, S.warp_sums, pred);
             store_dc(S, dcdiff, m0, m1, bpm, pred);
             __syncthreads();
             if (tid == 0 && d.status)
@@ -1637,6 +1717,27 @@ namespace aeonb
             return copy.size;
         }
 
+        // Clears the coefficients of the MCUs [m0, m1) inside the region: row by row, runs of blocks that follow one another.
+        __device__ __forceinline__ void clear_mcus(const aeonb_entropy_desc& d, uint32_t m0, uint32_t m1, uint32_t tid, uint32_t nth)
+        {
+            const int mcux = d.mcux;
+            for (int my = max((int)(m0 / (uint32_t)mcux), d.roi[1]); my < d.mcuy; ++my)
+            {
+                const int64_t row = (int64_t)my * mcux;
+                if (row >= (int64_t)m1)
+                    break;
+                const int x0 = (int)max((int64_t)d.roi[0], (int64_t)m0 - row), x1 = (int)min((int64_t)min(d.roi[2], mcux), (int64_t)m1 - row);
+                for (int c = 0; c < d.ncomp && x0 < x1; ++c)
+                    for (int y = 0; y < d.vs[c]; ++y)
+                    {
+                        const int64_t block = ((int64_t)(my - d.roi[1]) * d.vs[c] + y) * ((d.roi[2] - d.roi[0]) * d.hs[c]) + (x0 - d.roi[0]) * d.hs[c];
+                        uint4* const  p     = reinterpret_cast<uint4*>(d.coef[c] + block * 64);
+                        for (uint32_t i = tid; i < (uint32_t)((x1 - x0) * d.hs[c] * 8); i += nth)
+                            p[i] = make_uint4(0, 0, 0, 0);
+                    }
+            }
+        }
+
         // Segments of a part's intervals, their true entry states, and the storing pass.
         template <bool SLOW, typename Words>
         __device__ __forceinline__ void decode_intervals(rst_state& R, const seg_arrays& A, const uint32_t* words, uint32_t first, uint32_t I,
@@ -1670,7 +1771,13 @@ namespace aeonb
                     hi = mid;
             }
             const uint32_t pbeg = (R.clean[iv] + (tid - R.seg[iv]) * seg) * 8, pend = min(R.clean[iv + 1] * 8, pbeg + seg * 8);
-            const uint32_t step       = seg * 8 / (NCHECK + 1);
+            const uint32_t step = seg * 8 / (NCHECK + 1);
+            // ---- clear the coefficients of these intervals' MCUs: warps without a segment, if there are four of them, while the others
+            // decode; the barriers between here and the storing pass order the two
+            const uint32_t busy = (nseg + 31) & ~31u, from = T >= busy + 128 ? busy : 0;
+            if (tid >= from)
+                clear_mcus(S.d, (uint32_t)min((uint64_t)needed_mcus, (uint64_t)first * ri),
+                           (uint32_t)min((uint64_t)needed_mcus, (uint64_t)(first + I) * ri), tid - from, T - from);
             const uint32_t run_blocks = settle_segments<SLOW, Words>(S, A, words, nseg, R.seg[iv] == tid, pbeg, pend, step);
 
             // ---- first block number of every segment, counted from its interval's first block
@@ -1763,20 +1870,9 @@ namespace aeonb
                 fetch_raw(room, vec, i0, i1); // arrives while the tables are being built
             set_up_stream(S, (int)tid, (int)T);
 
-            // ---- clear the coefficients of this part's MCUs (a warp per MCU, a lane per 16 bytes)
             const uint32_t needed_mcus = (uint32_t)min(d.roi[3], d.mcuy) * d.mcux;
             const uint32_t ri          = (uint32_t)d.restart_interval;
-            const uint32_t mcu0 = (uint32_t)min((uint64_t)needed_mcus, (uint64_t)first * ri);
-            const uint32_t mcu1 = (uint32_t)min((uint64_t)needed_mcus, (uint64_t)(first + I) * ri);
             const uint32_t lane = tid & 31, warp = tid >> 5;
-            for (uint32_t m = mcu0 + warp; m < mcu1; m += T / 32)
-            {
-                const int my = (int)(m / (uint32_t)d.mcux), mx = (int)(m - (uint32_t)my * d.mcux);
-                if (my < d.roi[1] || mx < d.roi[0] || mx >= d.roi[2])
-                    continue;
-                for (uint32_t u = lane; u < (uint32_t)bpm * 8; u += 32)
-                    reinterpret_cast<uint4*>(block_home(S, mx, my, (int)(u >> 3)))[u & 7] = make_uint4(0, 0, 0, 0);
-            }
             asm volatile("cp.async.wait_all;" ::: "memory");
             __syncthreads();
             int16_t* const dcdiff = w.dcdiff;
