@@ -547,7 +547,7 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
             }
         launch_timer timer(ctx, AEONB_KERNEL_ENTROPY, bytes);
         uint32_t longest     = 0;
-        uint64_t most_blocks = 0;
+        uint64_t most_blocks = 0, most_places = 0;
         for (int i = 0; i < n; ++i)
             if (descs[i].scratch && descs[i].restart_interval == 0)
             {
@@ -556,9 +556,10 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
                     bpm += (uint64_t)descs[i].hs[c] * descs[i].vs[c];
                 longest     = std::max(longest, descs[i].scan_size);
                 most_blocks = std::max(most_blocks, bpm * descs[i].mcux * descs[i].roi[3]);
+                most_places = std::max(most_places, bpm);
             }
         cudaError_t  e = launch_jpeg_entropy(ddev, n, any_parallel, any_serial, jpeg_entropy_min_segment(), longest, most_blocks,
-                                             parts_dev, (int)parts.size(), ctx->stream);
+                                             (int)std::min<uint64_t>(most_places, 1 << 20), parts_dev, (int)parts.size(), ctx->stream);
         if (e != cudaSuccess)
             throw error(AEONB_ERR_CUDA, cuda_message("jpeg entropy kernel launch", e));
         ctx->launches += (any_parallel ? 1 : 0) + (parts.empty() ? 0 : 2) + (any_serial ? 1 : 0);

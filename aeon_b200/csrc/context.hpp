@@ -124,9 +124,10 @@ namespace aeonb
     // Entropy kernels: the block-parallel one takes the records that have a work area and no restart markers, the interval one
     // those with a work area and restart markers (in the `parts` jpeg_restart_parts cuts them into: record, first interval,
     // intervals, number within the record), the one-warp serial one the rest and what the interval one leaves.  min_segment: smallest segment (bytes) a thread of the parallel kernel decodes;
-    // longest, most_blocks: bytes of the longest stream for the block-parallel kernel, and the most blocks one has.
+    // longest, most_blocks, most_places: bytes of the longest stream for the block-parallel kernel, the most blocks one has, and the
+    // most places in an MCU.
     cudaError_t launch_jpeg_entropy(const aeonb_entropy_desc* descs_dev, int n, bool any_parallel, bool any_serial, int min_segment,
-                                    uint32_t longest, uint64_t most_blocks, const int4* parts_dev, int n_parts,
+                                    uint32_t longest, uint64_t most_blocks, int most_places, const int4* parts_dev, int n_parts,
                                     cudaStream_t stream);
     void        jpeg_restart_parts(const aeonb_entropy_desc* descs, int n, std::vector<int4>& parts);
     int64_t     jpeg_entropy_scratch_bytes(const aeonb_entropy_desc& d);

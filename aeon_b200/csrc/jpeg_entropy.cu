@@ -1,13 +1,15 @@
 // Device-side JPEG entropy decoding for sm_100a: the Huffman stage of cv::imdecode (src/etl_image.cpp:90).
 //
 // Huffman decoding of a baseline scan is a serial chain -- every code starts where the previous one ended --
-// and on the host it was the end-to-end bottleneck of the record path.  Three kernels take it over:
+// and on the host it was the end-to-end bottleneck of the record path.  Four kernels take it over:
 //
 //  * jpeg_entropy_parallel_kernel, one thread block per stream, for scans without restart markers (the
 //    common case).  The stream is cut into one segment per thread; every thread decodes its segment from a
 //    guessed state, and because Huffman streams re-synchronise, most guesses leave their segment in the
 //    true state.  Rounds in which each thread restarts from its left neighbour's exit state settle the rest
 //    (details at the kernel).  Coefficients are stored in a last pass once every entry state is known.
+//  * jpeg_entropy_spread_kernel, a cluster of up to eight thread blocks per stream, for launches of few such
+//    scans: shorter segments, each entered once for every place in the MCU, settle without rounds.
 //  * jpeg_entropy_restart_kernel, several thread blocks per stream, for scans with restart markers: the
 //    intervals between the markers are independent, so a stream is cut into runs of intervals, and each
 //    interval into segments as above (jpeg_restart_index_kernel finds the intervals first).
@@ -469,11 +471,11 @@ namespace aeonb
         // a predicated load beside that chain; with a second, dependent lookup for long codes and a branch for codes in no table a
         // pass took half as long again.
         //
-        // Measured on a B200 (kernel times): one stream of about 40 KB 0.183 ms before, 0.136 ms now; 256 streams of up to 55 KB (4:2:0,
-        // quality 90, crop regions stored) 0.263 / 0.196 ms; 512 streams of 6 KB 0.232 / 0.135 ms.  Phases of a 43 KB stream, thousand
-        // cycles: first pass 62 / 40 (14 of them beside the clearing of the planes), rounds 126 / 68 (five of them), storing pass
-        // 110 / 101 (one 2-byte store per coefficient, each to a line of its own; 65 without them), copy and marker scan 21 / 17,
-        // DC 14 (stores again), set-up 18 / 14.
+        // Measured on a B200 (kernel times): one stream of about 40 KB 0.183 ms before, 0.133 ms now; 256 streams of up to 55 KB (4:2:0,
+        // quality 90, crop regions stored) 0.263 / 0.178 ms; 512 streams of 6 KB 0.232 / 0.123 ms.  Phases of the 256 streams, thousand
+        // cycles on average: first pass 56 / 36, rounds 149 / 89 (five of them; the stream that takes longest spends 160 there), storing
+        // pass 90 / 56, copy and marker scan 23 / 22, DC 8, set-up 24 / 20.  Of one 43 KB stream that has an SM to itself the
+        // storing pass takes 101, 65 without its stores: one of 2 bytes per coefficient, each to a line of its own.
         // A wrong guess falls into step with the true decoder after about 10 blocks on average (the block's
         // position inside the MCU has to match too), and not at all inside flat regions, where every block looks
         // the same: there a chain of segments is settled one round per segment, which is what the slowest streams
@@ -694,7 +696,7 @@ namespace aeonb
             code_table  codes[4]; // DC slot 0, DC slot 1, AC slot 0, AC slot 1
             alignas(16) uint8_t dht[4 * 272]; // the tables as they came
             uint32_t    warp_sums[3][32];
-            uint8_t     zz[64 + 128];            // in front of a run that leaves the block, or of a look further on, anything is read
+            uint8_t     zz[16 + 64 + 128];       // from 16 on; around them lies what is read for a symbol without a place and not used
             block_place place[16];               // per block of an MCU
             block_link  link[16];
             uint8_t     comp[16];
@@ -735,21 +737,46 @@ namespace aeonb
             asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
             return v;
         }
-        // link = the link at its `next` where `yes`
-        __device__ __forceinline__ void follow_if(block_link& link, bool yes)
+        // Predicated loads and stores of the symbol loops.  They work their conditions out from what they are given: a condition handed
+        // over as a number costs two instructions more, in loops whose time is the issue of their instructions.
+        //
+        // Past the end of a block (`to` is the state): link = the link at its `next`, and one more block.
+        __device__ __forceinline__ void follow_past(block_link& link, uint32_t to, uint32_t& blocks)
         {
-            asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %4, 0;\n\t@q ld.shared.v4.u32 {%0, %1, %2, %3}, [%2];\n\t}"
-                         : "+r"(link.ac), "+r"(link.next_dc), "+r"(link.next), "+r"(link.block)
-                         : "r"((uint32_t)yes));
+            asm volatile("{\n\t.reg .pred q;\n\tsetp.ge.u32 q, %5, %6;\n\t@q ld.shared.v4.u32 {%0, %1, %2, %3}, [%2];\n\t@q add.u32 %4, %4, 1;\n\t}"
+                         : "+r"(link.ac), "+r"(link.next_dc), "+r"(link.next), "+r"(link.block), "+r"(blocks)
+                         : "r"(to), "n"(64u << 24));
         }
-        __device__ __forceinline__ void follow_if(block_place& at, bool yes)
+        __device__ __forceinline__ void follow_past(block_place& at, uint32_t to, uint32_t& blocks)
         {
-            uint64_t base = reinterpret_cast<uint64_t>(at.base);
-            asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 a;\n\tsetp.ne.u32 q, %7, 0;\n\tmov.b32 a, %2;\n\t"
-                         "@q ld.shared.v4.u32 {%0, %1, %2, %3}, [a];\n\t@q ld.shared.u64 %4, [a + 16];\n\t@q ld.shared.v2.s32 {%5, %6}, [a + 24];\n\t}"
-                         : "+r"(at.ac), "+r"(at.next_dc), "+r"(at.next), "+r"(at.last), "+l"(base), "+r"(at.dy), "+r"(at.dx)
-                         : "r"((uint32_t)yes));
-            at.base = reinterpret_cast<int16_t*>(base);
+            const uint64_t was = reinterpret_cast<uint64_t>(at.base);
+            uint32_t       lo = (uint32_t)was, hi = (uint32_t)(was >> 32);
+            asm volatile("{\n\t.reg .pred q;\n\t.reg .b32 a;\n\tsetp.ge.u32 q, %9, %10;\n\tmov.b32 a, %2;\n\t"
+                         "@q ld.shared.v4.u32 {%0, %1, %2, %3}, [a];\n\t@q ld.shared.v4.u32 {%4, %5, %6, %7}, [a + 16];\n\t@q add.u32 %8, %8, 1;\n\t}"
+                         : "+r"(at.ac), "+r"(at.next_dc), "+r"(at.next), "+r"(at.last), "+r"(lo), "+r"(hi), "+r"(at.dy), "+r"(at.dx), "+r"(blocks)
+                         : "r"(to), "n"(64u << 24));
+            at.base = reinterpret_cast<int16_t*>((uint64_t)hi << 32 | lo);
+        }
+        __device__ __forceinline__ uint32_t lds_u8(uint32_t addr)
+        {
+            uint16_t v;
+            asm volatile("ld.shared.u8 %0, [%1];" : "=h"(v) : "r"(addr));
+            return v;
+        }
+        // *p = value for a DC symbol (the state in front of it has index 0)
+        __device__ __forceinline__ void store_dc_symbol(int16_t* p, int value, uint32_t was)
+        {
+            asm volatile("{\n\t.reg .pred q;\n\tsetp.le.u32 q, %2, %3;\n\t@q st.s16 [%0], %1;\n\t}" ::"l"(p), "h"((int16_t)value), "r"(was), "n"(0x00ffffff) : "memory");
+        }
+        // *p = value for an AC symbol with value bits whose place kk lies in the block, inside the region (mx < w, my < h)
+        __device__ __forceinline__ void store_ac_symbol(int16_t* p, int value, uint32_t was, uint32_t size, uint32_t kk, uint32_t mx, uint32_t w, uint32_t my,
+                                                        uint32_t h)
+        {
+            asm volatile("{\n\t.reg .pred q;\n\tsetp.gt.u32 q, %2, %9;\n\tsetp.ne.and.u32 q, %3, 0, q;\n\tsetp.lt.and.u32 q, %4, 64, q;\n\t"
+                         "setp.lt.and.u32 q, %5, %6, q;\n\tsetp.lt.and.u32 q, %7, %8, q;\n\t@q st.global.s16 [%0], %1;\n\t}" ::"l"(
+                             __cvta_generic_to_global(p)),
+                         "h"((int16_t)value), "r"(was), "r"(size), "r"(kk), "r"(mx), "r"(w), "r"(my), "r"(h), "n"(0x00ffffff)
+                         : "memory");
         }
 
         // Words of the copy of a stream, from shared or from global memory.  `next_if` replaces `value` by the next word where
@@ -770,8 +797,9 @@ namespace aeonb
             }
             __device__ __forceinline__ void next_if(uint32_t& value, uint32_t yes)
             {
-                asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.shared.u32 %0, [%1];\n\t}" : "+r"(value) : "r"(at), "r"(yes));
-                at += yes ? 4 : 0;
+                asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.shared.u32 %0, [%1];\n\t@q add.u32 %1, %1, 4;\n\t}"
+                             : "+r"(value), "+r"(at)
+                             : "r"(yes));
             }
         };
         struct global_words
@@ -784,8 +812,9 @@ namespace aeonb
             __device__ __forceinline__ uint32_t next() { return *at++; }
             __device__ __forceinline__ void     next_if(uint32_t& value, uint32_t yes)
             {
-                asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.u32 %0, [%1];\n\t}" : "+r"(value) : "l"(at), "r"(yes));
-                at += yes ? 1 : 0;
+                asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q ld.global.u32 %0, [%1];\n\t@q add.u64 %1, %1, 4;\n\t}"
+                             : "+r"(value), "+l"(at)
+                             : "r"(yes));
             }
         };
 
@@ -807,46 +836,39 @@ namespace aeonb
             bool     merged; // the run fell into step with the remembered run: the exit state is that run's (p, b, k unset)
         };
 
-        // Decodes symbols from bit position p in state (b, k) until the first symbol that starts at or past pend.  The copy of the
-        // stream holds big-endian words, so the 32 bits under p are one funnel shift of two words.
-        // The state at the checkpoints (first one at bit check_at, then every check_step bits) goes to chk[0],
-        // chk[check_stride], ... and the blocks completed by then NCHECK rows further on; with `compare`, the run stops at the
-        // first checkpoint that an earlier run over this segment (old_blocks blocks in all) passed in the same state, and the
-        // block counts from there on are renumbered for this run.
+        // Decodes symbols from bit position p in state (b, k) on, without their values.  The copy of the stream holds big-endian words, so
+        // the 32 bits under a position are one funnel shift of two words.
         template <bool SLOW, typename Words>
-        __device__ __forceinline__ seg_result scan_segment(const par_state& S, const uint32_t* words, uint32_t p, int b, int k, uint32_t pend,
-                                                           uint32_t* chk, uint32_t check_stride, uint32_t check_at, uint32_t check_step,
-                                                           bool compare, uint32_t old_blocks)
+        struct scanner
         {
-            seg_result R;
-            R.merged        = false;
-            uint32_t blocks = 0;
-            // The table of the next symbol: the AC one of this block, or after the block's last symbol the DC one of the
-            // next.  Both are at hand before the symbol is known, so that only a select hangs on it.
-            block_link link = S.link[b];
-            uint32_t   look = k == 0 ? S.link[b ? b - 1 : S.bpm - 1].next_dc : link.ac, shift = k == 0 ? 32 - DC_BITS : 32 - AC_BITS;
-            // Bit positions count from the word that the run starts in; `at` is the state: position, and zig-zag index in the top byte.
-            const uint32_t base = p & ~31u;
-            uint32_t       at   = (p - base) | (uint32_t)k << 24;
-            pend                = pend > base ? pend - base : 0;
-            // checkpoints: `slot` walks down this thread's column (state; the blocks so far NCHECK rows further on); `old_key` is
-            // the state an earlier run noted at the next checkpoint (no state has all bits set)
-            const uint32_t rows    = NCHECK * check_stride;
-            uint32_t*      slot    = chk;
-            uint32_t       old_key = compare ? chk[0] : 0xffffffffu;
-            // A checkpoint at or past the segment's end is never taken: a run can step over it with its last symbol or stop short
-            // of it, so what is noted there could be left from an older run than the one whose block count goes with it.
-            check_at -= base;
-            uint32_t stop = check_at >= pend ? pend : check_at;
-            // The 32 bits under the position lie in w0 and w1; w2 is the word behind them, fetched when the one before it comes into use.
-            Words    ahead(words, p >> 5);
-            uint32_t w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
-            // The entry of the symbol under the position is fetched as soon as the position is known, and what else a step has to do is
-            // done while that load is under way.
-            uint32_t h = __funnelshift_l(w1, w0, at); // 32 valid bits; a symbol or a pair takes at most 31
-            uint32_t e = lds_u32(look + ((h >> shift) << 2));
-            for (;;)
+            block_link link;   // of the block in progress
+            uint32_t   base;   // bit positions count from the word that the run starts in
+            uint32_t   at;     // the state: position, and zig-zag index in the top byte
+            uint32_t   look;   // the table of the symbol under the position
+            uint32_t   w0, w1, w2; // the 32 bits under the position lie in w0 and w1; w2 is fetched when w1 comes into use
+            uint32_t   h, e;   // those bits (a symbol or a pair takes at most 31), and the entry of the symbol
+            uint32_t   blocks; // completed
+            Words      ahead;
+
+            __device__ __forceinline__ scanner(const par_state& S, const uint32_t* words, uint32_t p, int b, int k)
+                : link(S.link[b]), base(p & ~31u), at((p & 31) | (uint32_t)k << 24), look(k == 0 ? S.link[b ? b - 1 : S.bpm - 1].next_dc : link.ac),
+                  blocks(0), ahead(words, p >> 5)
             {
+                w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
+                h  = __funnelshift_l(w1, w0, at);
+                e  = lds_u32(look + ((h >> (k == 0 ? 32 - DC_BITS : 32 - AC_BITS)) << 2));
+            }
+            __device__ __forceinline__ uint32_t position() const { return base + (at & k_position); }
+            // The state at the first symbol at or past `stop` (by at most 30 bits), once the run is there.
+            __device__ __forceinline__ uint32_t key(uint32_t stop) const { return (position() - stop) << 10 | link.block << 6 | at >> 24; }
+
+            // Goes on until the first symbol that starts at or past bit `until`.  The entry of the symbol under the position is fetched as
+            // soon as the position is known, and what else a step has to do is done while that load is under way.  The next table -- the AC
+            // one of this block, or after the block's last symbol the DC one of the next -- is at hand before the symbol is known, so
+            // that only a select hangs on it.
+            __device__ __forceinline__ void run_to(const par_state& S, uint32_t until)
+            {
+                const uint32_t stop = until > base ? until - base : 0;
                 for (uint32_t pos = at & k_position; pos < stop;)
                 {
                     // Two symbols at a time as long as the first one cannot reach `stop`: a run stops at the first symbol at or past
@@ -860,45 +882,71 @@ namespace aeonb
                     }
                     const uint32_t by    = __byte_perm(e, 0, take);
                     const uint32_t to    = at + by;
-                    const bool     cross = (at ^ to) & 32; // the read position has left w0
+                    const uint32_t cross = (at ^ to) & 32; // the read position has left w0
                     const bool     end = to >= k_block_end, again = by == 0;
-                    w0    = cross ? w1 : w0;
-                    w1    = cross ? w2 : w1;
-                    look  = again ? look - 4 * LONG - 4 * LONG_FROM : end ? link.next_dc : link.ac;
-                    shift = again ? 16 : end ? 32 - DC_BITS : 32 - AC_BITS;
-                    at    = end ? to & k_position : to;
-                    h     = __funnelshift_l(w1, w0, at);
-                    e     = lds_u32(look + ((h >> shift) << 2));
-                    pos   = to & k_position;
+                    w0                   = cross ? w1 : w0;
+                    w1                   = cross ? w2 : w1;
+                    look                 = again ? look - 4 * LONG - 4 * LONG_FROM : end ? link.next_dc : link.ac;
+                    const uint32_t shift = again ? 16 : end ? 32 - DC_BITS : 32 - AC_BITS;
+                    at                   = end ? to & k_position : to;
+                    h                    = __funnelshift_l(w1, w0, at);
+                    e                    = lds_u32(look + ((h >> shift) << 2));
+                    pos                  = to & k_position;
                     ahead.next_if(w2, cross);
-                    follow_if(link, end);
-                    blocks += end;
+                    follow_past(link, to, blocks);
                 }
+            }
+        };
+
+        // Decodes symbols from bit position p in state (b, k) until the first symbol that starts at or past pend.
+        // The state at the checkpoints (first one at bit check_at, then every check_step bits) goes to chk[0],
+        // chk[check_stride], ... and the blocks completed by then NCHECK rows further on; with `compare`, the run stops at the
+        // first checkpoint that an earlier run over this segment (old_blocks blocks in all) passed in the same state, and the
+        // block counts from there on are renumbered for this run.
+        template <bool SLOW, typename Words>
+        __device__ __forceinline__ seg_result scan_segment(const par_state& S, const uint32_t* words, uint32_t p, int b, int k, uint32_t pend,
+                                                           uint32_t* chk, uint32_t check_stride, uint32_t check_at, uint32_t check_step,
+                                                           bool compare, uint32_t old_blocks)
+        {
+            seg_result R;
+            R.merged = false;
+            scanner<SLOW, Words> run(S, words, p, b, k);
+            // checkpoints: `slot` walks down this thread's column (state; the blocks so far NCHECK rows further on); `old_key` is
+            // the state an earlier run noted at the next checkpoint (no state has all bits set)
+            const uint32_t rows    = NCHECK * check_stride;
+            uint32_t*      slot    = chk;
+            uint32_t       old_key = compare ? chk[0] : 0xffffffffu;
+            // A checkpoint at or past the segment's end is never taken: a run can step over it with its last symbol or stop short
+            // of it, so what is noted there could be left from an older run than the one whose block count goes with it.
+            uint32_t stop = check_at >= pend ? pend : check_at;
+            for (;;)
+            {
+                run.run_to(S, stop);
                 if (stop == pend)
                     break;
                 // a checkpoint
-                const uint32_t key = ((at & k_position) - stop) << 10 | link.block << 6 | at >> 24; // position - stop <= 30
+                const uint32_t key = run.key(stop);
                 if (key == old_key)
                 {
                     // in step with the earlier run: its blocks from here on are this run's too
                     const uint32_t was = slot[rows];
                     for (uint32_t* later = slot; later < chk + rows; later += check_stride)
-                        later[rows] += blocks - was;
-                    blocks += old_blocks - was;
+                        later[rows] += run.blocks - was;
+                    run.blocks += old_blocks - was;
                     R.merged = true;
                     break;
                 }
                 slot[0]    = key;
-                slot[rows] = blocks;
+                slot[rows] = run.blocks;
                 slot += check_stride;
                 const bool more = slot < chk + rows && stop + check_step < pend;
                 old_key         = more && compare ? slot[0] : 0xffffffffu; // fetched now, wanted at the next checkpoint
                 stop            = more ? stop + check_step : pend;
             }
-            R.p      = base + (at & k_position);
-            R.b      = (int)link.block;
-            R.k      = (int)(at >> 24);
-            R.blocks = blocks;
+            R.p      = run.position();
+            R.b      = (int)run.link.block;
+            R.k      = (int)(run.at >> 24);
+            R.blocks = run.blocks;
             return R;
         }
 
@@ -924,15 +972,15 @@ namespace aeonb
             const uint32_t mcu = g / (uint32_t)S.bpm, row = mcu / (uint32_t)S.d.mcux;
             int            my = (int)row - S.d.roi[1], mx = (int)(mcu - row * (uint32_t)S.d.mcux) - S.d.roi[0];
             block_place    place = S.place[b];
-            uint32_t       look = k == 0 ? S.place[b ? b - 1 : S.bpm - 1].next_dc : place.ac, shift = k == 0 ? 32 - DC_BITS : 32 - AC_BITS;
+            uint32_t       look = k == 0 ? S.place[b ? b - 1 : S.bpm - 1].next_dc : place.ac;
             const uint32_t base = p & ~31u;
             uint32_t       at   = (p - base) | (uint32_t)k << 24, pos = p - base;
             pend                = pend > base ? pend - base : 0;
-            const uint32_t zz   = shared_address(S.zz);
+            const uint32_t zz   = shared_address(S.zz) + 16;
             Words          ahead(words, p >> 5);
             uint32_t       w0 = ahead.next(), w1 = ahead.next(), w2 = ahead.next();
             uint32_t       h = __funnelshift_l(w1, w0, at);
-            uint32_t       e = lds_u16(look + ((h >> shift) << 1));
+            uint32_t       e = lds_u16(look + ((h >> (k == 0 ? 32 - DC_BITS : 32 - AC_BITS)) << 1));
             while (pos < pend && g < gend)
             {
                 if (SLOW && e == k_slow)
@@ -944,32 +992,30 @@ namespace aeonb
                 const uint32_t total = entry_total(e), size = entry_size(e), advance = entry_advance(e);
                 const uint32_t x     = h << (total - size); // the value bits at the top
                 const uint32_t was = at, to = at + (total | advance << 24);
-                const bool     cross = (at ^ to) & 32;
+                const uint32_t kk   = (was >> 24) + advance - 1; // the coefficient's place
+                const uint32_t cross = (at ^ to) & 32;
                 const bool     end = to >= k_block_end, again = e == 0;
                 w0    = cross ? w1 : w0;
                 w1    = cross ? w2 : w1;
                 look  = again ? look - 2 * LONG - 2 * LONG_FROM : end ? place.next_dc : place.ac;
-                shift = again ? 16 : end ? 32 - DC_BITS : 32 - AC_BITS;
+                const uint32_t shift = again ? 16 : end ? 32 - DC_BITS : 32 - AC_BITS;
                 at    = end ? to & k_position : to;
                 h     = __funnelshift_l(w1, w0, at);
                 e     = lds_u16(look + ((h >> shift) << 1));
-                pos   = to & k_position;
+                const uint32_t column = lds_u8(zz + kk);
                 ahead.next_if(w2, cross);
+                pos   = to & k_position;
 
-                const uint32_t kk = (was >> 24) + advance - 1; // the coefficient's place
-                const int      v  = (int)__funnelshift_l(x, 0u, size) + ((int)x >= 0 ? 1 - (1 << size) : 0);
-                const bool     inside = (uint32_t)mx < roi_w && (uint32_t)my < roi_h;
+                const int v = (int)__funnelshift_l(x, 0u, size) + ((int)x >= 0 ? 1 - (1 << size) : 0);
                 // an invalid code, or a run that leaves the block
                 R.bad |= size != 0 && (int)kk > 63;
-                if (was <= k_position)
-                    dcdiff[g] = (int16_t)v;
-                else if (size != 0 && kk <= 63 && inside)
-                    place.base[(int64_t)(my * place.dy + mx * place.dx) * 64 + S.zz[kk]] = (int16_t)v;
-                g += end;
+                store_dc_symbol(dcdiff + g, v, was);
+                store_ac_symbol(place.base + (int64_t)(my * place.dy + mx * place.dx) * 64 + column, v, was, size, kk, (uint32_t)mx, roi_w,
+                                (uint32_t)my, roi_h);
                 mx += end ? place.last : 0;
                 my += mx == mx_end;
                 mx = mx == mx_end ? mx_first : mx;
-                follow_if(place, end);
+                follow_past(place, to, g);
             }
             R.p      = base + pos;
             R.blocks = g - first;
@@ -1276,6 +1322,19 @@ namespace aeonb
         __device__ __forceinline__ uint32_t bits_below(int n) { return n >= 16 ? 0xFFFFu : n <= 0 ? 0 : (1u << n) - 1; }
         __device__ __forceinline__ uint32_t bits_from(int n) { return 0xFFFFu & ~bits_below(n); }
 
+        // Bit b of `keep`: byte b of vector i is part of the data, which ends at `raw_end`; of `marker`: it is not zero and follows 0xFF.
+        // `prev` is the byte in front of the vector; the byte in front of the stream (of n bytes, `lead` into the first vector) is not 0xFF.
+        __device__ __forceinline__ void scan_masks(const uint32_t (&w)[4], uint32_t prev, uint32_t i, uint32_t lead, uint32_t n, uint32_t raw_end,
+                                                   uint32_t& keep, uint32_t& marker)
+        {
+            const int      at  = (int)(16 * i) - (int)lead;
+            const uint32_t own = bits_from(-at) & bits_below((int)n - at), data = own & bits_below((int)raw_end - at);
+            const uint32_t ff = byte_mask(w, 0xFFFFFFFFu), zero = byte_mask(w, 0);
+            const uint32_t follows = ((ff & own) << 1 | (prev == 0xFF && at > 0)) & 0xFFFF; // bytes that follow 0xFF
+            keep   = data & ~(follows & zero);
+            marker = own & follows & ~zero;
+        }
+
         // Copies the scan without stuffed bytes, up to the first marker; returns the bytes of the copy.  RESIDENT: in place in `room`,
         // where the scan's vectors have been brought; otherwise from `vec` to `out` through the tile `room`.
         template <bool RESIDENT>
@@ -1286,8 +1345,7 @@ namespace aeonb
             clean_writer<RESIDENT> copy{room, out, 0, 0};
             for (uint32_t tile = 0, odd = 0; tile < nv; tile += T, odd ^= 1)
             {
-                // bit b of `keep` = byte b is part of the data, of `marker` = byte b (16: of the next vector) is non-zero and follows
-                // 0xFF; the byte before the stream is not 0xFF
+                // (bit 16 of `marker`: the first byte of the next vector)
                 const uint32_t i = tile + tid;
                 uint32_t       w[4] = {0, 0, 0, 0}, keep = 0, marker = 0;
                 if (i < nv)
@@ -1299,13 +1357,7 @@ namespace aeonb
                         prev = !RESIDENT  ? (uint32_t)__ldg(reinterpret_cast<const uint8_t*>(vec) + 16 * i - 1)
                                : tid == 0 ? S.tile_end[odd ^ 1] // its place may have been taken
                                           : (uint32_t) reinterpret_cast<const uint8_t*>(room)[16 * i - 1];
-                    // bytes of the vector that belong to the stream, and those in front of the first marker found so far
-                    const uint32_t own  = bits_from((int)lead - (int)(16 * i)) & bits_below((int)(lead + N) - (int)(16 * i));
-                    const uint32_t data = own & bits_below((int)(lead + raw_end) - (int)(16 * i));
-                    const uint32_t ff = byte_mask(w, 0xFFFFFFFFu), zero = byte_mask(w, 0);
-                    const uint32_t follows = ((ff & own) << 1 | (prev == 0xFF && 16 * i > lead)) & 0xFFFF; // bytes that follow 0xFF
-                    keep   = data & ~(follows & zero);
-                    marker = own & follows & ~zero;
+                    scan_masks(w, prev, i, lead, N, raw_end, keep, marker);
                     // The second byte of a marker whose first is the tile's last lies in the next tile, which is too late.
                     if (tid == T - 1 && i + 1 < nv && w[3] >> 24 == 0xFF)
                         marker |= (uint32_t)((RESIDENT ? reinterpret_cast<const uint8_t*>(room)[16 * i + 16]
@@ -1399,6 +1451,18 @@ namespace aeonb
             __syncthreads();
         }
 
+        __device__ __forceinline__ bool parallel_shape_ok(const aeonb_entropy_desc& d, int& bpm, uint64_t& clean_room)
+        {
+            bpm = 0;
+            for (int c = 0; c < 3; ++c)
+                if (c < d.ncomp)
+                    bpm += d.hs[c] * d.vs[c];
+            const uint64_t total_blocks = (uint64_t)d.mcux * d.mcuy * bpm, dc_room = (total_blocks * 2 + 15) & ~15ull;
+            clean_room = ((uint64_t)d.scan_size + 32 + 15) & ~15ull;
+            return d.ncomp >= 1 && d.ncomp <= 3 && d.mcux > 0 && d.mcuy > 0 && d.scan && d.tables && bpm <= 16 && d.scan_size < (1u << 27) &&
+                   total_blocks < (1ull << 30) && d.scratch_bytes >= clean_room + dc_room && (reinterpret_cast<uintptr_t>(d.scratch) & 3) == 0;
+        }
+
         // Shared memory of a block: par_state, SEG_BYTES for each of `rows` segments, and what is left of `smem_bytes` for the scan and
         // behind it the DC differences, where they fit; otherwise they live in the record's work area.
         __global__ void __launch_bounds__(PAR_THREADS) jpeg_entropy_parallel_kernel(const aeonb_entropy_desc* __restrict__ descs, int min_segment,
@@ -1415,24 +1479,16 @@ namespace aeonb
             for (int i = tid; i < (int)(sizeof(aeonb_entropy_desc) / 4); i += T)
                 reinterpret_cast<uint32_t*>(&S.d)[i] = reinterpret_cast<const uint32_t*>(descs + blockIdx.x)[i];
             if (tid < 64)
-                S.zz[tid] = k_zz_colmajor[tid];
+                S.zz[16 + tid] = k_zz_colmajor[tid];
             if (tid == 0)
                 S.bad = S.slow = 0;
             __syncthreads();
             const aeonb_entropy_desc& d = S.d;
             if (!d.scratch || d.restart_interval != 0)
                 return; // the other kernels' stream
-            int bpm = 0;
-            for (int c = 0; c < 3; ++c)
-                if (c < d.ncomp)
-                    bpm += d.hs[c] * d.vs[c];
-            const uint64_t total_blocks64 = (uint64_t)d.mcux * d.mcuy * bpm;
-            const uint64_t clean_room     = ((uint64_t)d.scan_size + 32 + 15) & ~15ull;
-            const uint64_t dc_room        = (total_blocks64 * 2 + 15) & ~15ull;
-            const bool     shape_ok = d.ncomp >= 1 && d.ncomp <= 3 && d.mcux > 0 && d.mcuy > 0 && d.scan && d.tables && bpm <= 16 &&
-                                  d.scan_size < (1u << 27) && total_blocks64 < (1ull << 30) && d.scratch_bytes >= clean_room + dc_room &&
-                                  (reinterpret_cast<uintptr_t>(d.scratch) & 3) == 0;
-            if (!shape_ok)
+            uint64_t clean_room; // of the work area, for the copy; the DC differences lie behind it
+            int      bpm;
+            if (!parallel_shape_ok(d, bpm, clean_room))
             {
                 if (tid == 0 && d.status)
                     *d.status = 1;
@@ -1496,6 +1552,500 @@ namespace aeonb
             __syncthreads();
             if (tid == 0 && d.status)
                 *d.status = S.bad ? 1 : 0;
+        }
+
+        // ------------------------------------------------------------------------------------------------
+        // Few streams without restart markers: a cluster of thread blocks per stream.
+        //
+        // With fewer streams than SMs the kernel above leaves most of the chip idle, and more threads would not help it: its time
+        // is the chain of symbols that a wrong guess takes to fall into step, 820 bits on average and 5000 at the worst place of a
+        // 40 KB stream (4:2:0), and most of that is waiting for the block's place in the MCU to match; codes alone are in step after 80
+        // bits, 1100 at worst.  So here every segment (128 bytes) is entered once for each place in the MCU; one of these runs
+        // is in step after half a segment nearly always.  A run that leaves its segment goes on into the next ones until it is at one
+        // of their checkpoints in the state of one of their runs.  That makes a graph -- from each run to the run
+        // it falls into step with, and the blocks in between -- in which the stream is the path from the first segment's
+        // run 0.  Following the path takes no decoding; it is shortened by following it from the first segment of every group of
+        // segments, and of every block, at the same time.  The storing pass is dealt out in the pieces between the known states.
+        // The tables are built in every block of the cluster, each cleans an equal part of the scan; what crosses blocks are the clean
+        // scan (through the work area), the states at the checkpoints, the graph and sums of DC differences.
+        //
+        // Measured on a B200 (kernel times), one block per stream / this: one stream of 43 KB (eight blocks) 133 us / 56 us, 4 of them
+        // 153 / 54, 32 (four blocks) 170 / 84; the work is about 2.5 times that of the rounds, so it is for SMs that would be idle.
+        // Phases of the one stream, thousand cycles: set-up 13, copy 11, first pass 25, going on 11 on average and 16 at worst,
+        // path 8, storing pass 16, DC 4.  The first pass is bound by the issue of integer instructions; so short
+        // segments do not pay, and more checkpoints (eight) cost it more than the shorter pieces of the storing pass give.
+        constexpr int SPREAD_MOST   = 8;    // blocks in a cluster
+        constexpr int SPREAD_PLACES = 6;    // places in an MCU, at most
+        constexpr int SPREAD_CHECKS = 4;    // checkpoints of a segment, the last one at its end
+        constexpr int SPREAD_SEG    = 128;  // bytes of a segment, at least (64 with two checkpoints: 4 us more for 32 streams)
+        constexpr int SPREAD_GROUP  = 16;   // segments
+        constexpr int SPREAD_EXTRA  = 256;  // states noted between a run's exit and where it falls into step
+        constexpr uint32_t k_none = 0xffffffffu;
+
+        // A place on a path: checkpoint of a run (segment << 6 | place in the MCU << 3 | checkpoint), k_none behind the stream's
+        // end; `blocks`: how many more blocks are complete there than the run itself counts (at the end: how many in all).
+        struct spread_hop
+        {
+            uint32_t to, blocks;
+        };
+        struct spread_extra
+        {
+            uint32_t node, p, bk, blocks, end; // the run; state, blocks since the run's start; where the next known state is
+        };
+        struct spread_state
+        {
+            par_state    S;
+            spread_extra extra[SPREAD_EXTRA];
+            // What the blocks of the cluster tell one another: each writes its own entry in all blocks (a block that fetched the others'
+            // would wait for one after the other).
+            struct
+            {
+                uint32_t   bytes, marker;          // of its part of the scan: bytes without stuffed ones, first marker
+                uint32_t   kept;                   // its bytes in front of the stream's first marker
+                int32_t    dc[3];                  // sums of its DC differences
+                uint32_t   bad;
+                spread_hop through[SPREAD_PLACES]; // from its first segment's runs to the first run outside the block
+            } all[SPREAD_MOST];
+            uint32_t extras, bytes, marker;
+            int32_t  dc[3];
+        };
+        // Of each run, states as scanner::key gives them at the checkpoints (k_none: the stream ended in front of it), blocks by then,
+        // the run it falls into step with, and where the next known state behind its exit is.
+        struct spread_nodes
+        {
+            uint32_t*   key; // SPREAD_CHECKS rows of `cap`
+            uint16_t*   cnt; // as many
+            spread_hop* next;
+            uint32_t*   end;
+            spread_hop* group;  // from the runs of each group's first segment to the first run outside the group
+            spread_hop* inside; // per group: where the path comes in
+            spread_hop* truth;  // per segment: the path's run and checkpoint there
+        };
+        __host__ __device__ inline uint32_t spread_bytes(uint32_t cap)
+        {
+            return cap * (8 + SPREAD_CHECKS * 6 + 4) + (cap / SPREAD_GROUP + 2 * SPREAD_PLACES) * 16 + (cap + 2) * 8;
+        }
+        __device__ __forceinline__ spread_nodes spread_nodes_at(unsigned char* p, uint32_t cap)
+        {
+            spread_nodes N;
+            N.next   = reinterpret_cast<spread_hop*>(p);
+            N.group  = N.next + cap;
+            N.inside = N.group + cap / SPREAD_GROUP + 2 * SPREAD_PLACES;
+            N.truth  = N.inside + cap / SPREAD_GROUP + 2 * SPREAD_PLACES;
+            N.key    = reinterpret_cast<uint32_t*>(N.truth + cap + 2);
+            N.end    = N.key + SPREAD_CHECKS * cap;
+            N.cnt    = reinterpret_cast<uint16_t*>(N.end + cap);
+            return N;
+        }
+
+        template <typename T>
+        __device__ __forceinline__ T* in_block(T* p, uint32_t rank)
+        {
+            return cooperative_groups::this_cluster().map_shared_rank(p, rank);
+        }
+
+        // Copies the scan without stuffed bytes, up to the first marker: each block the vectors [v0, v1), which have been brought to
+        // `room`, to the work area, and from there every block all of it to `room`.  Returns the bytes of the copy.
+        __device__ __forceinline__ uint32_t copy_spread(spread_state& D, uint32_t* room, uint32_t* work, const uint4* vec, uint32_t v0, uint32_t v1,
+                                                        uint32_t lead)
+        {
+            cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+            par_state&     S = D.S;
+            const uint32_t tid = threadIdx.x, T = blockDim.x, C = cluster.num_blocks(), rank = cluster.block_rank();
+            const uint32_t n = S.d.scan_size;
+            auto look = [&](uint32_t i, uint32_t prev, uint32_t raw_end, uint32_t (&w)[4], uint32_t& keep, uint32_t& marker) {
+                const uint4 x = reinterpret_cast<const uint4*>(room)[i - v0];
+                w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
+                scan_masks(w, prev, i, lead, n, raw_end, keep, marker);
+            };
+            const uint32_t first_prev = v0 > 0 && v0 < v1 ? (uint32_t)__ldg(reinterpret_cast<const uint8_t*>(vec) + 16 * v0 - 1) : 0;
+            // once as if no part in front held a marker, for the markers and the counts
+            uint32_t kept = 0;
+            for (uint32_t i = v0 + tid; i < v1; i += T)
+            {
+                uint32_t w[4], keep, marker;
+                look(i, i == v0 ? first_prev : reinterpret_cast<const uint8_t*>(room)[16 * (i - v0) - 1], S.marker_at, w, keep, marker);
+                kept += __popc(keep);
+                if (marker)
+                    atomicMin(&D.marker, 16 * i + (uint32_t)__ffs(marker) - 1 - lead - 1); // the 0xFF before it
+            }
+            uint32_t all;
+            cta_exclusive_scan(kept, S.warp_sums[0], all);
+            if (tid < C)
+            {
+                in_block(D.all, tid)[rank].bytes  = all;
+                in_block(D.all, tid)[rank].marker = D.marker;
+            }
+            cluster.sync();
+            uint32_t before = 0, raw_end = S.marker_at;
+            for (uint32_t r = 0; r < C; ++r)
+            {
+                raw_end = min(raw_end, D.all[r].marker);
+                before += r < rank ? D.all[r].bytes : 0;
+            }
+            // the copy of this part, in place; what lies behind the marker goes
+            clean_writer<true> copy{room, nullptr, 0, 0};
+            for (uint32_t tile = v0, odd = 0; tile < v1; tile += T, odd ^= 1)
+            {
+                const uint32_t i = tile + tid;
+                uint32_t       w[4] = {0, 0, 0, 0}, keep = 0, marker;
+                if (i < v1)
+                    look(i, i == v0 ? first_prev : tid == 0 ? S.tile_end[odd ^ 1] : reinterpret_cast<const uint8_t*>(room)[16 * (i - v0) - 1],
+                         raw_end, w, keep, marker);
+                if (tid == T - 1)
+                    S.tile_end[odd] = w[3] >> 24; // the next tile finds its place taken
+                uint32_t       total;
+                const uint32_t at = cta_exclusive_scan((uint32_t)__popc(keep), S.warp_sums[0], total);
+                copy.append(w, keep, at, total);
+            }
+            __syncthreads();
+            // to its place in the work area: whole words, and bytes where two parts share a word
+            if (tid < C)
+                in_block(D.all, tid)[rank].kept = copy.size;
+            uint8_t* const bytes = reinterpret_cast<uint8_t*>(work);
+            const uint32_t end = before + copy.size, shift = 8 * (before & 3);
+            for (uint32_t i = (before >> 2) + tid; 4 * i < end; i += T)
+            {
+                const uint32_t k    = i - (before >> 2); // the word of the part that begins in it
+                const uint32_t word = __funnelshift_r(room[k], k ? room[k - 1] : 0, shift);
+                if (4 * i >= before && 4 * i + 4 <= end)
+                    work[i] = word;
+                else
+                    for (uint32_t b = max(4 * i, before); b < min(4 * i + 4, end); ++b)
+                        bytes[b ^ 3] = (uint8_t)(word >> (24 - 8 * (b & 3)));
+            }
+            cluster.sync();
+            uint32_t size = 0;
+            for (uint32_t r = 0; r < C; ++r)
+                size += D.all[r].kept;
+            // (the last vector brings what lies behind the copy too; the readers want 32 zero bytes there)
+            fetch_raw(room, reinterpret_cast<const uint4*>(work), 0, (size + 15) >> 4);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            if (tid < 32)
+                reinterpret_cast<uint8_t*>(room)[(size + tid) ^ 3] = 0;
+            __syncthreads();
+            return size;
+        }
+
+        template <bool SLOW>
+        __device__ __forceinline__ void decode_spread(spread_state& D, const spread_nodes& N, const uint32_t* words, uint32_t clean_size, uint32_t cap,
+                                                      uint32_t needed_blocks, int16_t* dcdiff)
+        {
+            using run = scanner<SLOW, shared_words>;
+            cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+            par_state&     S = D.S;
+            const uint32_t tid = threadIdx.x, T = blockDim.x, C = cluster.num_blocks(), rank = cluster.block_rank();
+            const uint32_t H = (uint32_t)S.bpm, total = clean_size * 8;
+            // segments: a multiple of SPREAD_CHECKS bytes; a block's runs fit `cap` nodes
+            const uint32_t most = C * (cap / H - 2);
+            const uint32_t seg  = max((uint32_t)SPREAD_SEG, ((clean_size + most - 1) / most + SPREAD_CHECKS - 1) & ~(SPREAD_CHECKS - 1u));
+            const uint32_t bits = seg * 8, step = bits / SPREAD_CHECKS; // at least 128: a symbol passes one checkpoint at most
+            const uint32_t nseg = (clean_size + seg - 1) / seg, per = max((nseg + C - 1) / C, 1u);
+            const uint32_t s0 = rank * per, mine = s0 < nseg ? min(per, nseg - s0) : 0, nodes = mine * H;
+
+            // ---- clear this block's share of the planes: warps without a run, if there are four of them, while the others decode.  The
+            // cluster's barriers stand between here and the storing pass.
+            const uint32_t busy = (nodes + 31) & ~31u, from = T >= busy + 128 ? busy : 0;
+            if (tid >= from)
+                for (int c = 0; c < S.d.ncomp; ++c)
+                {
+                    const size_t n16 = (size_t)(S.d.roi[2] - S.d.roi[0]) * S.d.hs[c] * (S.d.roi[3] - S.d.roi[1]) * S.d.vs[c] * 8; // 16-byte units
+                    uint4*       p   = reinterpret_cast<uint4*>(S.d.coef[c]);
+                    for (size_t i = n16 * rank / C + tid - from, last = n16 * (rank + 1) / C; i < last; i += T - from)
+                        p[i] = make_uint4(0, 0, 0, 0);
+                }
+
+            // ---- every segment from every place in the MCU.  Neighbouring threads have the same segment.
+            for (uint32_t t = tid; t < nodes; t += T)
+            {
+                const uint32_t ls = t / H, beg = (s0 + ls) * bits;
+                run            r(S, words, beg, (int)(t - ls * H), 0);
+                uint32_t       j = 0;
+                for (uint32_t stop = beg + step; j < SPREAD_CHECKS && stop < total; ++j, stop += step)
+                {
+                    r.run_to(S, stop);
+                    N.key[j * cap + t] = r.key(stop);
+                    N.cnt[j * cap + t] = (uint16_t)r.blocks;
+                }
+                if (j < SPREAD_CHECKS)
+                {
+                    r.run_to(S, total);
+                    for (; j < SPREAD_CHECKS; ++j)
+                    {
+                        N.key[j * cap + t] = k_none;
+                        N.cnt[j * cap + t] = (uint16_t)r.blocks;
+                    }
+                }
+            }
+            cluster.sync();
+
+            // ---- from every exit on until the run falls into step with another one
+            for (uint32_t t = tid; t < nodes; t += T)
+            {
+                const uint32_t key = N.key[(SPREAD_CHECKS - 1) * cap + t], had = N.cnt[(SPREAD_CHECKS - 1) * cap + t];
+                spread_hop     hop{k_none, had};
+                if (key != k_none)
+                {
+                    uint32_t  q = s0 + t / H + 1, j = 0, stop = q * bits;
+                    run       r(S, words, stop + (key >> 10), (int)(key >> 6 & 15), (int)(key & 63));
+                    uint32_t* end = N.end + t; // the end of the piece under way
+                    for (;;)
+                    {
+                        stop += step;
+                        if (stop >= total)
+                        {
+                            r.run_to(S, total);
+                            *end = total;
+                            hop  = spread_hop{k_none, had + r.blocks};
+                            break;
+                        }
+                        r.run_to(S, stop);
+                        const uint32_t        at = r.key(stop), owner = q / per, first = j * cap + (q - owner * per) * H;
+                        const uint32_t* const there = (owner == rank ? N.key : in_block(N.key, owner)) + first;
+                        uint32_t              h     = H;
+#pragma unroll
+                        for (uint32_t k = 0; k < SPREAD_PLACES; ++k) // the loads do not wait for one another
+                            h = k < H && there[k] == at ? k : h;
+                        if (h < H)
+                        {
+                            *end = r.position();
+                            hop  = spread_hop{q << 6 | h << 3 | j, had + r.blocks - (owner == rank ? N.cnt : in_block(N.cnt, owner))[first + h]};
+                            break;
+                        }
+                        const uint32_t x = atomicAdd(&D.extras, 1);
+                        if (x < SPREAD_EXTRA)
+                        {
+                            *end       = r.position();
+                            D.extra[x] = spread_extra{t, r.position(), at & 1023, had + r.blocks, 0};
+                            end        = &D.extra[x].end;
+                        }
+                        j = (j + 1) % SPREAD_CHECKS;
+                        q += j == 0;
+                    }
+                }
+                N.next[t] = hop;
+            }
+            for (uint32_t i = tid; i < mine; i += T)
+                N.truth[i] = spread_hop{k_none, 0};
+            const uint32_t groups = (mine + SPREAD_GROUP - 1) / SPREAD_GROUP;
+            for (uint32_t i = tid; i < groups; i += T)
+                N.inside[i] = spread_hop{k_none, 0};
+            __syncthreads();
+
+            // ---- the path.  From the runs of each group's first segment to the first run outside the group
+            auto segment = [](uint32_t to) { return to >> 6; };
+            auto place   = [](uint32_t to) { return to >> 3 & 7; };
+            auto local   = [&](const spread_hop& a) { return a.to != k_none && segment(a.to) - s0 < mine; };
+            auto through_group = [&](spread_hop a, uint32_t g, auto visit) {
+                for (const uint32_t last = min((g + 1) * SPREAD_GROUP, mine); a.to != k_none && segment(a.to) - s0 < last;)
+                {
+                    const uint32_t   ls = segment(a.to) - s0;
+                    const spread_hop b  = N.next[ls * H + place(a.to)];
+                    visit(ls, a);
+                    a = spread_hop{b.to, a.blocks + b.blocks};
+                }
+                return a;
+            };
+            for (uint32_t i = tid; i < groups * H; i += T)
+            {
+                const uint32_t g = i / H;
+                N.group[i]       = through_group(spread_hop{(s0 + g * SPREAD_GROUP) << 6 | (i - g * H) << 3, 0}, g, [](uint32_t, const spread_hop&) {});
+            }
+            __syncthreads();
+            // one hop from a run of a block whose first segment is `base`: through its group where the run is of the group's first segment
+            auto hop = [&](const spread_hop& a, const spread_hop* next, const spread_hop* group, uint32_t base) {
+                const uint32_t   ls = segment(a.to) - base;
+                const spread_hop b  = ls % SPREAD_GROUP == 0 ? group[ls / SPREAD_GROUP * H + place(a.to)] : next[ls * H + place(a.to)];
+                return spread_hop{b.to, a.blocks + b.blocks};
+            };
+            if (tid < H && nodes)
+            {
+                spread_hop a{s0 << 6 | tid << 3, 0};
+                while (local(a))
+                    a = hop(a, N.next, N.group, s0);
+                for (uint32_t r = rank + 1; r < C; ++r)
+                    in_block(D.all, r)[rank].through[tid] = a;
+            }
+            cluster.sync();
+            if (tid == 0)
+            {
+                spread_hop a{nseg ? 0u : k_none, 0};
+                while (a.to != k_none && segment(a.to) < s0) // in a block in front of this one
+                {
+                    const uint32_t owner = segment(a.to) / per;
+                    if (segment(a.to) == owner * per)
+                    {
+                        const spread_hop b = D.all[owner].through[place(a.to)];
+                        a                  = spread_hop{b.to, a.blocks + b.blocks};
+                    }
+                    else
+                        a = hop(a, in_block(N.next, owner), in_block(N.group, owner), owner * per);
+                }
+                // and through this one, noting where each group is entered
+                const bool comes = local(a) || (nseg == 0 && rank == 0);
+                while (local(a))
+                {
+                    const uint32_t g = (segment(a.to) - s0) / SPREAD_GROUP;
+                    if (N.inside[g].to == k_none)
+                        N.inside[g] = a;
+                    a = hop(a, N.next, N.group, s0);
+                }
+                // the block in which the path ends knows how many blocks the stream holds
+                if (comes && a.to == k_none && a.blocks < needed_blocks)
+                    S.bad = 1;
+            }
+            __syncthreads();
+            for (uint32_t g = tid; g < groups; g += T)
+                through_group(N.inside[g], g, [&](uint32_t ls, const spread_hop& a) { N.truth[ls] = a; });
+            __syncthreads();
+
+            // ---- store.  Pieces: from each checkpoint of the path's runs to the next one, from their exits to the next known state, from
+            // the states noted on the way, and the stream's beginning.
+            const uint32_t extras = min(D.extras, (uint32_t)SPREAD_EXTRA), checks = SPREAD_CHECKS * mine;
+            const uint32_t pieces = checks + extras + (rank == 0 && mine > 0);
+            bool           bad    = false;
+            for (uint32_t i = tid; i < pieces; i += T)
+            {
+                uint32_t p, bk, g, end;
+                if (i < checks)
+                {
+                    const uint32_t   ls = i / SPREAD_CHECKS, j = i % SPREAD_CHECKS, t = ls * H, beg = (s0 + ls) * bits;
+                    const spread_hop a = N.truth[ls];
+                    if (a.to == k_none || j < (a.to & 7))
+                        continue; // the path does not come here, or comes in further on
+                    const uint32_t row = j * cap + t + place(a.to), key = N.key[row];
+                    if (key == k_none)
+                        continue; // the stream ended in front of it
+                    p   = beg + (j + 1) * step + (key >> 10);
+                    bk  = key & 1023;
+                    g   = a.blocks + N.cnt[row];
+                    end = j < SPREAD_CHECKS - 1 ? min(beg + (j + 2) * step, total) : N.end[t + place(a.to)];
+                }
+                else if (i < checks + extras)
+                {
+                    const spread_extra x = D.extra[i - checks];
+                    const spread_hop   a = N.truth[x.node / H];
+                    if (a.to == k_none || place(a.to) != x.node % H)
+                        continue;
+                    p = x.p, bk = x.bk, g = a.blocks + x.blocks, end = x.end;
+                }
+                else
+                    p = bk = g = 0, end = min(step, total);
+                const store_result r = store_segment<SLOW, shared_words>(S, words, p, (int)(bk >> 6), (int)(bk & 63), end, g, needed_blocks, dcdiff);
+                bad |= r.bad;
+            }
+            if (bad)
+                S.bad = 1;
+        }
+
+        __global__ void __launch_bounds__(PAR_THREADS) jpeg_entropy_spread_kernel(const aeonb_entropy_desc* __restrict__ descs, uint32_t cap)
+        {
+            cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+            const uint32_t T = blockDim.x, C = cluster.num_blocks(), rank = cluster.block_rank(), tid = threadIdx.x;
+            extern __shared__ __align__(16) unsigned char smem_raw[];
+            spread_state&      D    = *reinterpret_cast<spread_state*>(smem_raw);
+            par_state&         S    = D.S;
+            const spread_nodes N    = spread_nodes_at(smem_raw + sizeof(spread_state), cap);
+            uint32_t* const    room = reinterpret_cast<uint32_t*>(smem_raw + ((sizeof(spread_state) + spread_bytes(cap) + 15) & ~15u));
+            for (uint32_t i = tid; i < sizeof(aeonb_entropy_desc) / 4; i += T)
+                reinterpret_cast<uint32_t*>(&S.d)[i] = reinterpret_cast<const uint32_t*>(descs + blockIdx.x / C)[i];
+            if (tid < 64)
+                S.zz[16 + tid] = k_zz_colmajor[tid];
+            if (tid == 0)
+                S.bad = S.slow = 0, D.extras = 0, D.marker = k_none;
+            __syncthreads();
+            const aeonb_entropy_desc& d = S.d;
+            if (!d.scratch || d.restart_interval != 0)
+                return; // the other kernels' stream; all blocks of the cluster leave here
+            uint64_t clean_room;
+            int      bpm;
+            if (!parallel_shape_ok(d, bpm, clean_room))
+            {
+                if (tid == 0 && rank == 0 && d.status)
+                    *d.status = 1;
+                return;
+            }
+            const uint32_t     n = d.scan_size;
+            const uint32_t     lead = (uint32_t)(reinterpret_cast<uintptr_t>(d.scan) & 15);
+            const uint4* const vec  = reinterpret_cast<const uint4*>(d.scan - lead);
+            const uint32_t     nv   = (lead + n + 15) >> 4;
+            // this block's share of the scan, which arrives while the tables are being built
+            const uint32_t part = (nv + C - 1) / C, v0 = min(nv, rank * part), v1 = min(nv, v0 + part);
+            fetch_raw(room, vec, v0, v1);
+            if (tid == 64) // not a thread that sets anything else up
+                S.marker_at = n > 0 && __ldg(d.scan + n - 1) == 0xFF ? n - 1 : n;
+            set_up_stream(S, (int)tid, (int)T);
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncthreads();
+            const uint32_t needed_mcus = (uint32_t)min(d.roi[3], d.mcuy) * d.mcux;
+            int16_t* const dcdiff      = reinterpret_cast<int16_t*>(static_cast<uint8_t*>(d.scratch) + clean_room);
+            const uint32_t clean_size  = copy_spread(D, room, reinterpret_cast<uint32_t*>(d.scratch), vec, v0, v1, lead);
+            if (S.slow)
+                decode_spread<true>(D, N, room, clean_size, cap, needed_mcus * bpm, dcdiff);
+            else
+                decode_spread<false>(D, N, room, clean_size, cap, needed_mcus * bpm, dcdiff);
+            cluster.sync(); // the differences are there
+
+            // ---- DC: sum the differences per component in scan order; block r of the cluster owns the r-th run of MCUs, its thread t
+            // MCUs [m0, m1).  The differences of an MCU are fetched together.
+            const uint32_t share = (needed_mcus + C - 1) / C, b0 = min(needed_mcus, rank * share), b1 = min(needed_mcus, b0 + share);
+            const uint32_t mchunk = (share + T - 1) / T, m0 = min(b1, b0 + tid * mchunk), m1 = min(b1, m0 + mchunk);
+            int            sum[3] = {0, 0, 0}, pred[3], diff[SPREAD_PLACES];
+            for (uint32_t m = m0; m < m1; ++m)
+            {
+#pragma unroll
+                for (int b = 0; b < SPREAD_PLACES; ++b)
+                    diff[b] = b < bpm ? dcdiff[(size_t)m * bpm + b] : 0;
+#pragma unroll
+                for (int b = 0; b < SPREAD_PLACES; ++b)
+                {
+                    const int c = b < bpm ? S.comp[b] : 0;
+                    sum[0] += c == 0 ? diff[b] : 0;
+                    sum[1] += c == 1 ? diff[b] : 0;
+                    sum[2] += c == 2 ? diff[b] : 0;
+                }
+            }
+            cta_exclusive_scan3(sum, S.warp_sums, pred);
+            if (tid == T - 1)
+                for (int c = 0; c < 3; ++c)
+                    D.dc[c] = pred[c] + sum[c];
+            __syncthreads();
+            if (tid < C)
+            {
+                auto& mine = in_block(D.all, tid)[rank];
+                mine.dc[0] = D.dc[0], mine.dc[1] = D.dc[1], mine.dc[2] = D.dc[2];
+                mine.bad   = (uint32_t)S.bad;
+            }
+            cluster.sync(); // nothing touches another block's memory afterwards
+            for (uint32_t r = 0; r < rank; ++r)
+                for (int c = 0; c < 3; ++c)
+                    pred[c] += D.all[r].dc[c];
+            if (m1 == m0 + 1)
+            {
+                const int my = (int)(m0 / (uint32_t)d.mcux), mx = (int)(m0 - (uint32_t)my * d.mcux);
+#pragma unroll
+                for (int b = 0; b < SPREAD_PLACES; ++b)
+                    if (b < bpm)
+                    {
+                        const int c   = S.comp[b];
+                        const int now = (c == 0 ? pred[0] : c == 1 ? pred[1] : pred[2]) + diff[b];
+                        pred[0] = c == 0 ? now : pred[0];
+                        pred[1] = c == 1 ? now : pred[1];
+                        pred[2] = c == 2 ? now : pred[2];
+                        if (int16_t* const out = block_home(S, mx, my, b))
+                            out[0] = (int16_t)now;
+                    }
+            }
+            else
+                store_dc(S, dcdiff, m0, m1, bpm, pred);
+            if (tid == 0 && rank == 0 && d.status)
+            {
+                uint32_t bad = 0;
+                for (uint32_t r = 0; r < C; ++r)
+                    bad |= D.all[r].bad;
+                *d.status = bad ? 1 : 0;
+            }
         }
 
         // ------------------------------------------------------------------------------------------------
@@ -1827,7 +2377,7 @@ namespace aeonb
             for (uint32_t i = tid; i < sizeof(aeonb_entropy_desc) / 4; i += T)
                 reinterpret_cast<uint32_t*>(&S.d)[i] = reinterpret_cast<const uint32_t*>(descs + part.x)[i];
             if (tid < 64)
-                S.zz[tid] = k_zz_colmajor[tid];
+                S.zz[16 + tid] = k_zz_colmajor[tid];
             if (tid == 0)
                 S.bad = S.slow = 0;
             __syncthreads();
@@ -2012,13 +2562,60 @@ namespace aeonb
         return std::max(fixed, std::min(want, std::min<size_t>(most, 227 * 1024)));
     }
 
+    // How a launch of few streams is spread: blocks in the cluster of each stream (0: not spread), and runs a block has room for.
+    struct spread_plan
+    {
+        int      blocks = 0, threads = 0;
+        uint32_t cap    = 0;
+        size_t   smem   = 0;
+    };
+    static spread_plan jpeg_entropy_spread(int n, uint32_t longest, int most_places)
+    {
+        spread_plan p;
+        if (n > 66 || most_places < 1 || most_places > SPREAD_PLACES)
+            return p;
+        // As many blocks as all streams' clusters find room for at once, one block to an SM: 15 clusters of eight, 33 of four, 66 of two
+        // (what cudaOccupancyMaxActiveClusters says for a B200).  A block has less than a warp for each of its schedulers to decode with
+        // if it has fewer than 128 runs.
+        const uint32_t segments = longest / SPREAD_SEG + 1;
+        int            blocks   = n <= 15 ? SPREAD_MOST : n <= 33 ? 4 : 2;
+        while (blocks > 1 && segments * (uint32_t)most_places <= (uint32_t)blocks / 2 * 128)
+            blocks /= 2;
+        p.threads = 512;
+        p.cap     = std::min<uint32_t>(1200, ((segments + blocks - 1) / blocks + 3) * most_places);
+        p.smem    = ((sizeof(spread_state) + spread_bytes(p.cap) + 15) & ~(size_t)15) + longest + 16 + 64;
+        p.blocks  = p.smem <= 227 * 1024 ? blocks : 0;
+        return p;
+    }
+
     cudaError_t launch_jpeg_entropy(const aeonb_entropy_desc* descs_dev, int n, bool any_parallel, bool any_serial, int min_segment,
-                                    uint32_t longest, uint64_t most_blocks, const int4* parts_dev, int n_parts,
+                                    uint32_t longest, uint64_t most_blocks, int most_places, const int4* parts_dev, int n_parts,
                                     cudaStream_t stream)
     {
         if (n <= 0)
             return cudaSuccess;
-        if (any_parallel)
+        const spread_plan spread = any_parallel ? jpeg_entropy_spread(n, longest, most_places) : spread_plan();
+        if (spread.blocks > 0)
+        {
+            cudaError_t err = cudaFuncSetAttribute(jpeg_entropy_spread_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+            if (err != cudaSuccess)
+                return err;
+            cudaLaunchConfig_t  cfg  = {};
+            cudaLaunchAttribute attr = {};
+            cfg.gridDim              = dim3(n * spread.blocks);
+            cfg.blockDim             = dim3(spread.threads);
+            cfg.dynamicSmemBytes     = spread.smem;
+            cfg.stream               = stream;
+            attr.id                  = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x    = spread.blocks;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.attrs    = &attr;
+            cfg.numAttrs = 1;
+            err          = cudaLaunchKernelEx(&cfg, jpeg_entropy_spread_kernel, descs_dev, spread.cap);
+            if (err != cudaSuccess)
+                return err;
+        }
+        else if (any_parallel)
         {
             const int    threads = jpeg_entropy_block(n, longest);
             const int    rows = std::min(threads, (int)(longest / (uint32_t)min_segment) + 1);

@@ -455,3 +455,63 @@ def test_tables_with_codes_longer_than_the_lookup_windows(ctx, dc_long, ac_long,
     assert np.array_equal(cv2.imdecode(np.frombuffer(blob, np.uint8), 1), cv2.imdecode(np.frombuffer(plain, np.uint8), 1))
     check(ctx, [plain, blob, jpeg_bytes(img, 88, [cv2.IMWRITE_JPEG_OPTIMIZE, 1])])
     check(ctx, [blob])
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 34, 66, 67])
+def test_streams_spread_over_clusters(ctx, n):
+    """Launches at the edges of the number of blocks a stream is spread over, with streams of every length in one launch (one MCU up to
+    more than the longest one's share per block), of every number of places in an MCU, of regions, of pictures so flat that a
+    run entered at a wrong bit stays out of step to the end of the flat part, and of streams that a marker ends early."""
+    import cv2
+    from aeon_b200 import kernels as K
+    rng = np.random.default_rng(710 + n)
+    modes = [cv2.IMWRITE_JPEG_SAMPLING_FACTOR_420, cv2.IMWRITE_JPEG_SAMPLING_FACTOR_444, cv2.IMWRITE_JPEG_SAMPLING_FACTOR_422,
+             cv2.IMWRITE_JPEG_SAMPLING_FACTOR_411, None]
+    blobs, rois = [], []
+    for i in range(n + 5):
+        h, w = [(430, 470), (8, 8), (300, 200), (64, 500), (17, 33)][i % 5]
+        img = gradient_image(rng, h, w)
+        kind = (i // 5) % 4 if n > 1 else i
+        if kind == 1:
+            img[h // 4:] = 128          # flat from a quarter on
+        elif kind == 2:
+            img = np.full((h, w, 3), int(rng.integers(0, 256)), np.uint8)
+        elif kind == 3:
+            img = rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
+        mode = modes[(i // 3) % 5]
+        blob = (jpeg_bytes(img[..., 0], 90) if mode is None else jpeg_bytes(img, int(rng.choice([60, 90, 97])), [cv2.IMWRITE_JPEG_SAMPLING_FACTOR, mode]))
+        info = K.jpeg_parse(blob)
+        mcux, mcuy = info.blocks_w[0] // info.hs[0], info.blocks_h[0] // info.vs[0]
+        x0, y0 = int(rng.integers(0, mcux)), int(rng.integers(0, mcuy))
+        blobs.append(blob)
+        rois.append((0, 0, mcux, mcuy) if i % 2 else (x0, y0, int(rng.integers(x0 + 1, mcux + 1)), int(rng.integers(y0 + 1, mcuy + 1))))
+    for first in (0, 5):
+        check(ctx, blobs[first:first + n], rois[first:first + n])
+    if n == 1:
+        for blob, roi in zip(blobs, rois):
+            check(ctx, [blob], [roi])
+
+
+def test_spread_streams_cut_short(ctx):
+    """A stream of which a part is missing: the status is 1 unless the region needs none of it, at cuts around the places where the
+    blocks of a cluster share the stream out; bytes behind the end marker are no part of the stream."""
+    from aeon_b200 import kernels as K
+    rng = np.random.default_rng(72)
+    blob = jpeg_bytes(np.clip(gradient_image(rng, 320, 448).astype(np.int16) + rng.integers(-20, 21, (320, 448, 3)), 0, 255).astype(np.uint8), 92)
+    start = blob.index(b"\xff\xda") + 14
+    info = K.jpeg_parse(blob)
+    mcux, mcuy = info.blocks_w[0] // info.hs[0], info.blocks_h[0] // info.vs[0]
+    size = len(blob) - 2 - start
+    tail = bytes(rng.integers(0, 256, 3000, dtype=np.uint8))
+    whole, upper = (0, 0, mcux, mcuy), (0, 0, mcux, 2)
+    for cut in sorted({0, 1, size // 2, size - 1, *(size * r // 8 // 16 * 16 + d for r in range(1, 8) for d in (-1, 0, 1))}):
+        for k in (0, 3000):
+            data = blob[:start + cut] + b"\xff\xd9" + tail[:k]
+            got = K.jpeg_entropy_decode_device(ctx, [data, data], [whole, upper])
+            assert got[0][3] == 1, (cut, k)
+            if cut > size // 4:
+                assert got[1][3] == 0, (cut, k)
+                want = host_planes(blob, upper)[1]
+                for c in range(info.ncomp):
+                    assert np.array_equal(got[1][1][c].cpu().numpy(), want[c][:got[1][1][c].numel()]), (cut, k, c)
+    check(ctx, [blob + tail])
