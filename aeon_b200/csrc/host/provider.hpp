@@ -157,6 +157,37 @@ namespace aeonb
         int    n_device_jobs = 0; // streams Huffman-decoded on the GPU
         bool   anchor_planes_on_device = false; // localization_rcnn: the planes with a value or four per anchor are written by kernels
         std::vector<char*> produced; // where each device-produced output is written
+
+        // Empties the plan of a finished batch for the next one; its vectors keep their memory.
+        void clear()
+        {
+            jobs.clear();
+            copies.clear();
+            rotations.clear();
+            rotation_of_job.clear();
+            for (auto* v : {&desc_job, &pre_job, &desc_rot, &pre_rot, &desc_pre})
+                for (auto& of_stage : *v)
+                    of_stage.clear();
+            for (auto* v : {&desc_dst, &desc_area})
+                for (auto& of_stage : *v)
+                    of_stage.clear();
+            for (auto* v : {&descs, &pre_descs})
+                for (auto& of_stage : *v)
+                    of_stage.clear();
+            for (auto& of_stage : rcnn)
+                of_stage.clear();
+            for (auto& of_stage : sdescs)
+                of_stage.clear();
+            for (auto& of_stage : sdesc_off)
+                of_stage.clear();
+            for (auto& output : out_host)
+                output.clear();
+            slice_end.clear();
+            area_bytes = stage_bytes = pixel_bytes = coef_bytes = oriented_bytes = rotated_bytes = status_room = 0;
+            n_device_jobs           = 0;
+            anchor_planes_on_device = false;
+            produced.clear();
+        }
     };
 }
 
@@ -247,6 +278,12 @@ struct aeonb_provider
     std::mutex                              m_job_mutex;
     std::condition_variable                 m_job_cv, m_done_cv;
     std::deque<std::unique_ptr<batch_job>>  m_jobs;
+    // Finished batches, emptied for the next ones: the jobs of 256 photos are 1 MB, which a new batch would get from the kernel page by
+    // page (with the copies made while the vector grows more than half of the planning time).
+    static constexpr size_t                 k_spare = 4; // as many as can be under way at once: one planned, two queued, one in work
+    std::vector<std::unique_ptr<batch_job>> m_spare;
+    std::unique_ptr<batch_job>              new_job();
+    void                                    recycle(std::unique_ptr<batch_job> job); // with m_job_mutex held
     int64_t                                 m_processed = 0; // last batch the driver has finished enqueuing (or failed on)
     bool                                    m_driver_stop = false;
     std::exception_ptr                      m_failed[k_events]; // what the driver threw for the batch of that slot

@@ -298,7 +298,7 @@ void aeonb_provider::run(const void* const* elems, const size_t* sizes, int n, v
     if (n <= 0 || n > batch_size)
         throw std::invalid_argument("aeonb_provider_run: record count must be in [1, batch_size]");
     const auto t0 = std::chrono::steady_clock::now();
-    auto job = std::make_unique<batch_job>((int)stages.size());
+    auto job = new_job();
     // the big planes of localization_rcnn never exist on the host when they are delivered to device memory as they are
     job->plan.anchor_planes_on_device = on_device && batch_major;
     for (size_t o = 0; o < outputs.size(); ++o)
@@ -321,6 +321,28 @@ void aeonb_provider::run(const void* const* elems, const size_t* sizes, int n, v
     m_job_cv.notify_one();
     if (wait)
         wait_ticket(ticket);
+}
+
+std::unique_ptr<aeonb_provider::batch_job> aeonb_provider::new_job()
+{
+    {
+        std::lock_guard<std::mutex> lk(m_job_mutex);
+        if (!m_spare.empty())
+        {
+            std::unique_ptr<batch_job> job = std::move(m_spare.back());
+            m_spare.pop_back();
+            return job;
+        }
+    }
+    return std::make_unique<batch_job>((int)stages.size());
+}
+
+void aeonb_provider::recycle(std::unique_ptr<batch_job> job)
+{
+    if (m_spare.size() >= k_spare)
+        return;
+    job->plan.clear();
+    m_spare.push_back(std::move(job));
 }
 
 void aeonb_provider::driver_loop()
@@ -350,6 +372,7 @@ void aeonb_provider::driver_loop()
             std::lock_guard<std::mutex> lk(m_job_mutex);
             m_failed[slot] = failed;
             m_processed    = job->ticket;
+            recycle(std::move(job));
         }
         m_done_cv.notify_all();
     }
@@ -447,7 +470,8 @@ void aeonb_provider::plan_records(batch_plan& B, const void* const* elems, const
 
     // Parses the headers of one JPEG stream and registers it as a decode job (sizes only; no layout yet).
     auto plan_jpeg = [&](const void* data, size_t size) -> int {
-        jpeg_job job;
+        B.jobs.emplace_back();
+        jpeg_job& job = B.jobs.back();
         job.data = static_cast<const uint8_t*>(data);
         job.size = size;
         if (is_png(data, size))
@@ -457,14 +481,12 @@ void aeonb_provider::plan_records(batch_plan& B, const void* const* elems, const
             job.pw                     = job.pinfo.width;
             job.ph                     = job.pinfo.height;
             job.frame.info.orientation = 1;
-            B.jobs.push_back(job);
             return (int)B.jobs.size() - 1;
         }
         jpeg_parse(data, size, job.frame);
         const bool swapped = job.frame.info.orientation >= 5;
         job.pw             = swapped ? job.frame.info.height : job.frame.info.width;
         job.ph             = swapped ? job.frame.info.width : job.frame.info.height;
-        B.jobs.push_back(job);
         return (int)B.jobs.size() - 1;
     };
     // Fixes the region of the picture a job has to produce -- the MCUs that the crop box of `d` (given in

@@ -1,6 +1,7 @@
 """End-to-end parity of the provider (header parsing and seeded draws on the host; entropy decoding, JPEG back end and
 image kernel on the GPU) with the record-level oracle, through the C ABI, on the benchmark configurations at reduced
 batch size and on every other stage the provider offers (tests/test_gpu_configs_full.py runs the stated batch sizes)."""
+import json
 import os
 import struct
 
@@ -729,3 +730,66 @@ def test_audio_slices_only_when_no_earlier_batch_is_under_way(ctx):
     assert prov.stats()["launches"] == 8
     for w, o in zip(want, outs):
         assert np.array_equal(o["audio"].cpu().numpy(), w)
+
+
+def test_calls_of_every_shape_after_one_another(ctx):
+    """A provider plans every batch in the memory of an earlier one: batches of changing size, kind of record (JPEG, PNG, turned, progressive,
+    bytes and other buffers) and delivery give what a provider of their own gives."""
+    import cv2
+    import torch
+    cfg = {"batch_size": 8, "random_seed": 5,
+           "etl": [{"type": "image", "height": 1000, "width": 1000},
+                   {"type": "localization_rcnn", "height": 1000, "width": 1000, "max_gt_boxes": 8, "class_names": ["a", "b"],
+                    "debug_deterministic": True}],
+           "augmentation": [{"type": "image", "fixed_aspect_ratio": True, "fixed_scaling_factor": 1.6, "crop_enable": False}]}
+    rng = np.random.default_rng(3)
+
+    def record(kind, boxes):
+        h, w = int(rng.integers(200, 400)), int(rng.integers(300, 500))
+        img = gradient_image(rng, h, w)
+        if kind == "png":
+            data = cv2.imencode(".png", img)[1].tobytes()
+        else:
+            data = jpeg_bytes(img, 90, [cv2.IMWRITE_JPEG_PROGRESSIVE, 1] if kind == "progressive" else ())
+        objs = [{"name": "ab"[i % 2], "difficult": False, "bndbox": {"xmin": 5 * i, "ymin": 9 * i, "xmax": 60 + 9 * i, "ymax": 90 + 5 * i}} for i in range(boxes)]
+        note = json.dumps({"object": objs, "size": {"width": w, "height": h, "depth": 3}}).encode()
+        return (bytearray(data) if kind == "buffer" else data, note)
+
+    calls = [(["jpeg"] * 8, True), (["png", "jpeg"], False), (["progressive"], True), (["buffer"] * 3, True), (["jpeg"] * 8, False),
+             (["jpeg", "png", "progressive", "buffer"] * 2, True), (["jpeg"], False), (["jpeg"] * 5, True)]
+    prov = make_provider(ctx, cfg)
+    for kinds, on_device in calls:
+        recs = [record(k, 1 + i) for i, k in enumerate(kinds)]
+        alone = make_provider(ctx, cfg)
+        for p in (prov, alone):
+            if on_device:
+                out = p.run_device(recs)
+                torch.cuda.synchronize()
+                p.result = {k: v.cpu().numpy()[:len(recs)] for k, v in out.items()}
+            else:
+                p.result = {k: np.array(v[:len(recs)]) for k, v in p.run_host(recs).items()}
+        assert prov.result.keys() == alone.result.keys() and prov.result["image"].any()
+        for name in prov.result:
+            assert np.array_equal(prov.result[name], alone.result[name]), (kinds, on_device, name)
+
+
+def test_pointers_of_packed_records():
+    """The packed pointers of a batch lead to the records' own bytes, with and without the short cut for bytes objects."""
+    import ctypes as C
+    from aeon_b200 import provider as P
+
+    class Shape:
+        input_count = 2
+
+    recs = [(os.urandom(5 + i), b"" if i % 3 == 0 else struct.pack("<i", i)) for i in range(40)]
+    shortcut = P._BYTES_AT
+    try:
+        for P._BYTES_AT in (shortcut, None):
+            for batch in (recs, [(bytearray(a), b) for a, b in recs], recs[:1], []):
+                ptrs, sizes, keep = P.Provider._pack(Shape(), batch)
+                flat = [e for rec in batch for e in rec]
+                assert [C.string_at(ptrs[i], sizes[i]) if sizes[i] else b"" for i in range(len(flat))] == [bytes(e) for e in flat]
+    finally:
+        P._BYTES_AT = shortcut
+    with pytest.raises(ValueError, match="record 1 has 1 elements, the configuration needs 2"):
+        P.Provider._pack(Shape(), [(b"a", b"b"), (b"a",)])
