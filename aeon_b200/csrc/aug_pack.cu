@@ -30,9 +30,11 @@
 
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #include "../../include/aeon_b200.h"
+#include "context.hpp"
 #include "device_common.cuh"
 
 namespace cg = cooperative_groups;
@@ -49,7 +51,6 @@ namespace aeonb
 
         struct aug_launch
         {
-            const aeonb_image_desc* descs; // device copy
             aeonb_image_layout      layout;
             int                     rows_per_band;
             int                     tile_pitch;  // bytes per tile row (multiple of 16)
@@ -479,7 +480,7 @@ namespace aeonb
 
         // RUNS: how the band is stored -- 0: store_band, 1: store_runs, planes, 2: store_runs, channels side by side.
         template <typename T, int PIX, int RUNS>
-        __global__ void __launch_bounds__(AUG_MAX_THREADS, 5) aug_pack_kernel(const aug_launch L)
+        __global__ void __launch_bounds__(AUG_MAX_THREADS, 5) aug_pack_kernel(const aug_launch L, const __grid_constant__ launch_data data)
         {
             // Dynamic shared memory, addressed by 32-bit byte offsets:
             //   tile     [3][rows_per_band][pitch]   the band, planar uint8, output channel order
@@ -525,17 +526,16 @@ namespace aeonb
             {
                 // ---- record descriptor -> shared memory
                 {
-                    const int* g = reinterpret_cast<const int*>(L.descs + rec);
-                    int*       s = reinterpret_cast<int*>(&d);
-                    for (int i = tid; i < (int)(sizeof(aeonb_image_desc) / sizeof(int)); i += nt)
-                        s[i] = g[i];
+                    data.fetch(d, rec, tid, nt);
                     if (tid < 3)
                         part_sum[tid] = cta_sum[tid] = 0;
                     if (tid == 32 % nt) // the two scale factors of the resize, once per CTA (two double divisions each)
                     {
-                        const aeonb_image_desc& gd = L.descs[rec];
-                        tap_scale[0] = 1.0 / ((double)gd.out_w / (double)gd.crop_w);
-                        tap_scale[1] = 1.0 / ((double)gd.out_h / (double)gd.crop_h);
+                        auto field = [&](size_t offset) {
+                            return (double)(int)data.word(((size_t)rec * sizeof(aeonb_image_desc) + offset) / 4);
+                        };
+                        tap_scale[0] = 1.0 / (field(offsetof(aeonb_image_desc, out_w)) / field(offsetof(aeonb_image_desc, crop_w)));
+                        tap_scale[1] = 1.0 / (field(offsetof(aeonb_image_desc, out_h)) / field(offsetof(aeonb_image_desc, crop_h)));
                     }
                 }
                 __syncthreads();
@@ -906,7 +906,7 @@ namespace aeonb
         }
 
         template <typename T>
-        cudaError_t launch_typed(const aug_launch& L, int clusters, int bands, int cluster_size, int threads, size_t smem, int pix, int runs,
+        cudaError_t launch_typed(const aug_launch& L, const launch_data& data, int clusters, int bands, int cluster_size, int threads, size_t smem, int pix, int runs,
                                  cudaStream_t stream)
         {
             // Planes of 4- and 8-byte elements that do not start on 16 bytes stay with store_band (64 of 225 x 225 floats: 71 us, 86 in
@@ -932,13 +932,13 @@ namespace aeonb
             attr[0].val.clusterDim.z = 1;
             cfg.attrs                = attr;
             cfg.numAttrs             = 1;
-            return cudaLaunchKernelEx(&cfg, kern, L);
+            return cudaLaunchKernelEx(&cfg, kern, L, data);
         }
     }
 
     // Host entry used by the C ABI: `descs_dev` is the device copy of the descriptors `descs_host`.
     // Returns a CUDA error; *why is set for configurations the kernel does not cover.
-    cudaError_t launch_aug_pack(const aeonb_image_desc* descs_dev, const aeonb_image_desc* descs_host, int n,
+    cudaError_t launch_aug_pack(const launch_data& data, const aeonb_image_desc* descs_host, int n,
                                 const aeonb_image_layout& layout, int pixel_stride, bool slots_aligned, cudaStream_t stream,
                                 const char** why)
     {
@@ -985,7 +985,6 @@ namespace aeonb
             *why = "a contrast change on an output too large for 8 on-chip bands (rows/8 * width * 3 over 200 KB) is outside the accelerated path";
             return cudaErrorInvalidValue;
         }
-        L.descs         = descs_dev;
         L.layout        = layout;
         L.rows_per_band = (layout.slot_h + bands - 1) / bands;
         const size_t elem = layout.dtype == AEONB_F64 ? 8 : layout.dtype == AEONB_F32 || layout.dtype == AEONB_I32 ? 4
@@ -1011,13 +1010,13 @@ namespace aeonb
         const int clusters = n;
         switch (layout.dtype)
         {
-        case AEONB_U8: return launch_typed<uint8_t>(L, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
-        case AEONB_I8: return launch_typed<int8_t>(L, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
-        case AEONB_I16: return launch_typed<int16_t>(L, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
-        case AEONB_U16: return launch_typed<uint16_t>(L, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
-        case AEONB_I32: return launch_typed<int32_t>(L, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
-        case AEONB_F32: return launch_typed<float>(L, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
-        case AEONB_F64: return launch_typed<double>(L, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
+        case AEONB_U8: return launch_typed<uint8_t>(L, data, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
+        case AEONB_I8: return launch_typed<int8_t>(L, data, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
+        case AEONB_I16: return launch_typed<int16_t>(L, data, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
+        case AEONB_U16: return launch_typed<uint16_t>(L, data, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
+        case AEONB_I32: return launch_typed<int32_t>(L, data, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
+        case AEONB_F32: return launch_typed<float>(L, data, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
+        case AEONB_F64: return launch_typed<double>(L, data, clusters, bands, cluster_size, threads, smem, pixel_stride, runs, stream);
         }
         *why = "unknown output dtype";
         return cudaErrorInvalidValue;
@@ -1038,7 +1037,6 @@ namespace aeonb
 #include <mutex>
 #include <string>
 
-#include "context.hpp"
 
 
 
@@ -1092,8 +1090,10 @@ extern "C" int aeonb_image_batch_noalloc(const aeonb_image_desc* descs, int n, c
         cudaStream_t st      = static_cast<cudaStream_t>(stream);
         // Every descriptor the kernel reads is overwritten here, so nothing of the previous call survives.
         AEONB_CUDA(cudaMemcpyAsync(scratch, descs, sizeof(aeonb_image_desc) * n, cudaMemcpyHostToDevice, st));
+        launch_data data;
+        data.far        = scratch;
         const char* why = nullptr;
-        cudaError_t e   = launch_aug_pack(scratch, descs, n, *layout, pixel_stride, aligned, st, &why);
+        cudaError_t e   = launch_aug_pack(data, descs, n, *layout, pixel_stride, aligned, st, &why);
         if (why)
             throw error(AEONB_ERR_UNSUPPORTED, why);
         if (e != cudaSuccess)

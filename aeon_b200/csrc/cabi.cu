@@ -122,6 +122,15 @@ void* aeonb_ctx::upload(const void* host, size_t bytes)
     return slot.dev;
 }
 
+void aeonb_ctx::carry(launch_data& to, const void* host, size_t bytes)
+{
+    to.far = nullptr;
+    if (bytes <= launch_data::k_near)
+        std::memcpy(to.near, host, bytes);
+    else
+        to.far = upload(host, bytes);
+}
+
 extern "C" {
 
 const char* aeonb_last_error(void)
@@ -360,10 +369,11 @@ int aeonb_image_batch(aeonb_ctx* ctx, const aeonb_image_desc* descs, int n, cons
         ordered.reserve(n);
         for (const auto& o : order)
             ordered.push_back(descs[o.second]);
-        auto* dev = static_cast<const aeonb_image_desc*>(ctx->upload(ordered.data(), sizeof(aeonb_image_desc) * n));
+        launch_data data;
+        ctx->carry(data, ordered.data(), sizeof(aeonb_image_desc) * n);
         const char*  why = nullptr;
         launch_timer timer(ctx, AEONB_KERNEL_IMAGE, ctx->profiling ? aeonb_image_batch_bytes(descs, n, layout) : 0);
-        cudaError_t  e   = launch_aug_pack(dev, ordered.data(), n, *layout, pixel_stride, aligned, ctx->stream, &why);
+        cudaError_t  e   = launch_aug_pack(data, ordered.data(), n, *layout, pixel_stride, aligned, ctx->stream, &why);
         if (why)
             throw error(AEONB_ERR_UNSUPPORTED, why);
         if (e != cudaSuccess)
@@ -453,10 +463,15 @@ int aeonb_jpeg_backend_batch(aeonb_ctx* ctx, const aeonb_jpeg_desc* descs, int n
         if (smem > 200 * 1024)
             throw error(AEONB_ERR_UNSUPPORTED, "image too wide for the on-chip MCU-row strip");
         AEONB_CUDA(cudaSetDevice(ctx->device));
-        auto* ddev = static_cast<const aeonb_jpeg_desc*>(ctx->upload(descs, sizeof(aeonb_jpeg_desc) * n));
-        auto* wdev = static_cast<const int2*>(ctx->upload(work.data(), sizeof(int2) * work.size()));
+        static_assert(sizeof(aeonb_jpeg_desc) % alignof(int2) == 0, "the work list lies behind the descriptors");
+        std::vector<unsigned char> both(sizeof(aeonb_jpeg_desc) * n + sizeof(int2) * work.size());
+        std::memcpy(both.data(), descs, sizeof(aeonb_jpeg_desc) * n);
+        if (!work.empty())
+            std::memcpy(both.data() + sizeof(aeonb_jpeg_desc) * n, work.data(), sizeof(int2) * work.size());
+        launch_data data;
+        ctx->carry(data, both.data(), both.size());
         launch_timer timer(ctx, AEONB_KERNEL_JPEG_BACKEND, ctx->profiling ? aeonb_jpeg_backend_bytes(descs, n) : 0);
-        cudaError_t  e = launch_jpeg_backend(ddev, wdev, (int)work.size(), smem, ctx->stream);
+        cudaError_t  e = launch_jpeg_backend(data, n, (int)work.size(), smem, ctx->stream);
         if (e != cudaSuccess)
             throw error(AEONB_ERR_CUDA, cuda_message("jpeg back-end kernel launch", e));
         ctx->launches++;
@@ -532,7 +547,8 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
                 ordered[b] = descs[by_size[next++]];
             descs = ordered.data();
         }
-        auto* ddev = static_cast<const aeonb_entropy_desc*>(ctx->upload(descs, sizeof(aeonb_entropy_desc) * n));
+        launch_data data;
+        ctx->carry(data, descs, sizeof(aeonb_entropy_desc) * n);
         std::vector<int4> parts; // of the streams with restart markers
         jpeg_restart_parts(descs, n, parts);
         const int4* parts_dev = parts.empty() ? nullptr : static_cast<const int4*>(ctx->upload(parts.data(), sizeof(int4) * parts.size()));
@@ -558,7 +574,7 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
                 most_blocks = std::max(most_blocks, bpm * descs[i].mcux * descs[i].roi[3]);
                 most_places = std::max(most_places, bpm);
             }
-        cudaError_t  e = launch_jpeg_entropy(ddev, n, any_parallel, any_serial, jpeg_entropy_min_segment(), longest, most_blocks,
+        cudaError_t  e = launch_jpeg_entropy(data, n, any_parallel, any_serial, jpeg_entropy_min_segment(), longest, most_blocks,
                                              (int)std::min<uint64_t>(most_places, 1 << 20), parts_dev, (int)parts.size(), ctx->stream);
         if (e != cudaSuccess)
             throw error(AEONB_ERR_CUDA, cuda_message("jpeg entropy kernel launch", e));

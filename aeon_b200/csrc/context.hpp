@@ -53,6 +53,33 @@ namespace aeonb
         }
     }
 
+    // The descriptors of a launch.  Where they fit they travel with the launch as a kernel parameter; otherwise `far` is their device
+    // copy, which takes a launch of its own in front of the kernel: 9.3 us for the two (device time) against 3.6 for one launch
+    // with 8 KB of parameters, which takes no longer than one with a pointer (16 KB: 0.7 us longer, 31 KB: 3.5).  A provider call
+    // of one photo, which had four such launches: 154 -> 137 us.  (Not for kernels of many short blocks: each reads its descriptor
+    // from the parameters a little later than from L2, and the area resize of 32 pictures took 127 instead of 104 us.)
+    struct launch_data
+    {
+        static constexpr size_t k_near = 8064;
+        const void*             far = nullptr;
+        alignas(16) unsigned char near[k_near];
+#ifdef __CUDACC__
+        // 32-bit word i.  (Not through one pointer to either place: parameters read by a generic address are slower.)
+        __device__ __forceinline__ uint32_t word(size_t i) const
+        {
+            return far ? static_cast<const uint32_t*>(far)[i] : reinterpret_cast<const uint32_t*>(near)[i];
+        }
+        // Descriptor `index` to shared memory, by nth threads.
+        template <typename T>
+        __device__ __forceinline__ void fetch(T& to, int index, int tid, int nth) const
+        {
+            static_assert(sizeof(T) % 4 == 0, "copied word by word");
+            for (int i = tid; i < (int)(sizeof(T) / 4); i += nth)
+                reinterpret_cast<uint32_t*>(&to)[i] = word((size_t)index * (sizeof(T) / 4) + i);
+        }
+#endif
+    };
+
     // A pinned host buffer paired with a device buffer of the same size; used to ship small
     // descriptor arrays (and, in the provider, coefficient planes) with one async copy.
     struct staging_slot
@@ -94,6 +121,8 @@ struct aeonb_ctx
     // Copies `bytes` of host data to the device on the stream; the returned device pointer is
     // valid for kernels enqueued after this call.
     void* upload(const void* host, size_t bytes);
+    // Puts `bytes` of host data into `to`, or brings them to the device where they do not fit.
+    void carry(aeonb::launch_data& to, const void* host, size_t bytes);
 };
 
 namespace aeonb
@@ -114,11 +143,11 @@ namespace aeonb
     void check_image_batch(const aeonb_image_desc* d, int n, const aeonb_image_layout& L, int& pixel_stride, bool& aligned);
 
     // Kernel launchers (defined next to the kernels).
-    cudaError_t launch_aug_pack(const aeonb_image_desc* descs_dev, const aeonb_image_desc* descs_host, int n,
+    cudaError_t launch_aug_pack(const launch_data& descs, const aeonb_image_desc* descs_host, int n,
                                 const aeonb_image_layout& layout, int pixel_stride, bool slots_aligned, cudaStream_t stream,
                                 const char** why);
-    cudaError_t launch_jpeg_backend(const aeonb_jpeg_desc* descs_dev, const int2* work_dev, int n_work, size_t smem,
-                                    cudaStream_t stream);
+    // `data`: n descriptors, and behind them (record, first MCU row) of every block
+    cudaError_t launch_jpeg_backend(const launch_data& data, int n, int n_work, size_t smem, cudaStream_t stream);
     size_t      jpeg_backend_smem(const aeonb_jpeg_desc& d);
     int         jpeg_backend_strip(); // MCU rows one CTA of the back-end kernel handles
     // Entropy kernels: the block-parallel one takes the records that have a work area and no restart markers, the interval one
@@ -126,7 +155,7 @@ namespace aeonb
     // intervals, number within the record), the one-warp serial one the rest and what the interval one leaves.  min_segment: smallest segment (bytes) a thread of the parallel kernel decodes;
     // longest, most_blocks, most_places: bytes of the longest stream for the block-parallel kernel, the most blocks one has, and the
     // most places in an MCU.
-    cudaError_t launch_jpeg_entropy(const aeonb_entropy_desc* descs_dev, int n, bool any_parallel, bool any_serial, int min_segment,
+    cudaError_t launch_jpeg_entropy(const launch_data& descs, int n, bool any_parallel, bool any_serial, int min_segment,
                                     uint32_t longest, uint64_t most_blocks, int most_places, const int4* parts_dev, int n_parts,
                                     cudaStream_t stream);
     void        jpeg_restart_parts(const aeonb_entropy_desc* descs, int n, std::vector<int4>& parts);

@@ -20,6 +20,7 @@
 #include <stdint.h>
 
 #include "../../include/aeon_b200.h"
+#include "context.hpp"
 
 namespace aeonb
 {
@@ -27,12 +28,6 @@ namespace aeonb
     {
         constexpr int JPG_THREADS = 256;
         constexpr int JPG_STRIP   = 2; // MCU rows per CTA: the chroma context rows are transformed once per strip
-
-        struct jpeg_launch
-        {
-            const aeonb_jpeg_desc* descs; // device
-            const int2*            work;  // device: (record, mcu row) per CTA
-        };
 
         __device__ __forceinline__ int clamp255(int v) { return min(max(v, 0), 255); }
 
@@ -174,7 +169,7 @@ namespace aeonb
             }
         }
 
-        __global__ void __launch_bounds__(JPG_THREADS, 3) jpeg_backend_kernel(const jpeg_launch L)
+        __global__ void __launch_bounds__(JPG_THREADS, 3) jpeg_backend_kernel(const __grid_constant__ launch_data data, int n)
         {
             extern __shared__ __align__(16) unsigned char smem[];
             __shared__ aeonb_jpeg_desc d;
@@ -184,14 +179,10 @@ namespace aeonb
             __shared__ int             job_first[JPG_STRIP * 4 + 5]; // first work item of each job, and the total
 
             const int  tid  = threadIdx.x;
-            const int2 wk   = L.work[blockIdx.x];
+            const size_t at = (size_t)n * (sizeof(aeonb_jpeg_desc) / 4) + 2 * (size_t)blockIdx.x;
+            const int2 wk   = make_int2((int)data.word(at), (int)data.word(at + 1));
             const int  mrow = wk.y; // first MCU row of this CTA's strip
-            {
-                const int* g = reinterpret_cast<const int*>(L.descs + wk.x);
-                int*       s = reinterpret_cast<int*>(&d);
-                for (int i = tid; i < (int)(sizeof(aeonb_jpeg_desc) / sizeof(int)); i += JPG_THREADS)
-                    s[i] = g[i];
-            }
+            data.fetch(d, wk.x, tid, JPG_THREADS);
             __syncthreads();
             for (int i = tid; i < d.ncomp * 64; i += JPG_THREADS)
                 quant[i >> 6][i & 63] = __ldg(d.quant[i >> 6] + (i & 63));
@@ -582,8 +573,7 @@ namespace aeonb
         }
     }
 
-    cudaError_t launch_jpeg_backend(const aeonb_jpeg_desc* descs_dev, const int2* work_dev, int n_work, size_t smem,
-                                    cudaStream_t stream)
+    cudaError_t launch_jpeg_backend(const launch_data& data, int n, int n_work, size_t smem, cudaStream_t stream)
     {
         if (n_work <= 0)
             return cudaSuccess;
@@ -591,8 +581,7 @@ namespace aeonb
         cudaError_t err = cudaFuncSetAttribute(jpeg_backend_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
         if (err != cudaSuccess)
             return err;
-        jpeg_launch L{descs_dev, work_dev};
-        jpeg_backend_kernel<<<n_work, JPG_THREADS, smem, stream>>>(L);
+        jpeg_backend_kernel<<<n_work, JPG_THREADS, smem, stream>>>(data, n);
         return cudaGetLastError();
     }
 

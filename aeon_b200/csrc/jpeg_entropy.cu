@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "../../include/aeon_b200.h"
+#include "context.hpp"
 
 namespace aeonb
 {
@@ -252,7 +253,7 @@ namespace aeonb
             }
         };
 
-        __global__ void __launch_bounds__(32) jpeg_entropy_kernel(const aeonb_entropy_desc* __restrict__ descs)
+        __global__ void __launch_bounds__(32) jpeg_entropy_kernel(const __grid_constant__ launch_data data)
         {
             extern __shared__ __align__(16) unsigned char smem_raw[];
             warp_state&              S    = *reinterpret_cast<warp_state*>(smem_raw);
@@ -262,8 +263,7 @@ namespace aeonb
             __shared__ int           bad;
             __shared__ uint32_t      fetched; // bytes of the scan loaded into the window so far
             static_assert(sizeof(aeonb_entropy_desc) % 4 == 0, "descriptor is copied word by word");
-            for (int i = lane; i < (int)(sizeof(aeonb_entropy_desc) / 4); i += 32)
-                reinterpret_cast<uint32_t*>(&d)[i] = reinterpret_cast<const uint32_t*>(descs + blockIdx.x)[i];
+            data.fetch(d, (int)(blockIdx.x), (int)lane, (int)32);
             if (lane == 0)
             {
                 bad     = 0;
@@ -1465,7 +1465,7 @@ namespace aeonb
 
         // Shared memory of a block: par_state, SEG_BYTES for each of `rows` segments, and what is left of `smem_bytes` for the scan and
         // behind it the DC differences, where they fit; otherwise they live in the record's work area.
-        __global__ void __launch_bounds__(PAR_THREADS) jpeg_entropy_parallel_kernel(const aeonb_entropy_desc* __restrict__ descs, int min_segment,
+        __global__ void __launch_bounds__(PAR_THREADS) jpeg_entropy_parallel_kernel(const __grid_constant__ launch_data data, int min_segment,
                                                                                     uint32_t rows, uint32_t smem_bytes)
         {
             const uint32_t T = blockDim.x;
@@ -1476,8 +1476,7 @@ namespace aeonb
             uint32_t* const  room       = reinterpret_cast<uint32_t*>(smem_raw + room_at);
             const uint32_t   room_bytes = smem_bytes - room_at;
             const int        tid        = threadIdx.x;
-            for (int i = tid; i < (int)(sizeof(aeonb_entropy_desc) / 4); i += T)
-                reinterpret_cast<uint32_t*>(&S.d)[i] = reinterpret_cast<const uint32_t*>(descs + blockIdx.x)[i];
+            data.fetch(S.d, (int)(blockIdx.x), (int)tid, (int)T);
             if (tid < 64)
                 S.zz[16 + tid] = k_zz_colmajor[tid];
             if (tid == 0)
@@ -1939,7 +1938,7 @@ namespace aeonb
                 S.bad = 1;
         }
 
-        __global__ void __launch_bounds__(PAR_THREADS) jpeg_entropy_spread_kernel(const aeonb_entropy_desc* __restrict__ descs, uint32_t cap)
+        __global__ void __launch_bounds__(PAR_THREADS) jpeg_entropy_spread_kernel(const __grid_constant__ launch_data data, uint32_t cap)
         {
             cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
             const uint32_t T = blockDim.x, C = cluster.num_blocks(), rank = cluster.block_rank(), tid = threadIdx.x;
@@ -1948,8 +1947,7 @@ namespace aeonb
             par_state&         S    = D.S;
             const spread_nodes N    = spread_nodes_at(smem_raw + sizeof(spread_state), cap);
             uint32_t* const    room = reinterpret_cast<uint32_t*>(smem_raw + ((sizeof(spread_state) + spread_bytes(cap) + 15) & ~15u));
-            for (uint32_t i = tid; i < sizeof(aeonb_entropy_desc) / 4; i += T)
-                reinterpret_cast<uint32_t*>(&S.d)[i] = reinterpret_cast<const uint32_t*>(descs + blockIdx.x / C)[i];
+            data.fetch(S.d, (int)(blockIdx.x / C), (int)tid, (int)T);
             if (tid < 64)
                 S.zz[16 + tid] = k_zz_colmajor[tid];
             if (tid == 0)
@@ -2090,15 +2088,14 @@ namespace aeonb
         // it goes through twice, counting markers and then numbering them from the counts of the warps in front.  What bounds
         // it is the latency of those passes: 32 streams of 0.3 MB took 85 us with one block each, about 20 with eight.
         __global__ void __cluster_dims__(RST_INDEX_BLOCKS, 1, 1) __launch_bounds__(RST_INDEX_THREADS)
-            jpeg_restart_index_kernel(const aeonb_entropy_desc* __restrict__ descs)
+            jpeg_restart_index_kernel(const __grid_constant__ launch_data data)
         {
             namespace cg = cooperative_groups;
             constexpr uint32_t            warps = RST_INDEX_THREADS / 32;
             __shared__ aeonb_entropy_desc d;
             __shared__ uint32_t           counts[warps], other, total;
             const uint32_t                tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x % RST_INDEX_BLOCKS;
-            for (uint32_t i = tid; i < sizeof(aeonb_entropy_desc) / 4; i += RST_INDEX_THREADS)
-                reinterpret_cast<uint32_t*>(&d)[i] = reinterpret_cast<const uint32_t*>(descs + blockIdx.x / RST_INDEX_BLOCKS)[i];
+            data.fetch(d, (int)(blockIdx.x / RST_INDEX_BLOCKS), (int)tid, (int)RST_INDEX_THREADS);
             __syncthreads();
             if (!d.scratch || d.restart_interval == 0)
                 return; // as all blocks of the cluster
@@ -2361,7 +2358,7 @@ namespace aeonb
 
         // Part blockIdx.x = {record, first interval, intervals, number of the part within its stream}.  Shared memory: rst_state,
         // SEG_BYTES per thread, and what is left of `smem_bytes` for the part's bytes, where they fit.
-        __global__ void __launch_bounds__(RST_THREADS, 2) jpeg_entropy_restart_kernel(const aeonb_entropy_desc* __restrict__ descs,
+        __global__ void __launch_bounds__(RST_THREADS, 2) jpeg_entropy_restart_kernel(const __grid_constant__ launch_data data,
                                                                                    const int4* __restrict__ parts, int min_segment,
                                                                                    uint32_t smem_bytes)
         {
@@ -2374,8 +2371,7 @@ namespace aeonb
             uint32_t* const  room    = reinterpret_cast<uint32_t*>(smem_raw + room_at);
             const uint32_t   tid     = threadIdx.x;
             const int4       part    = __ldg(parts + blockIdx.x);
-            for (uint32_t i = tid; i < sizeof(aeonb_entropy_desc) / 4; i += T)
-                reinterpret_cast<uint32_t*>(&S.d)[i] = reinterpret_cast<const uint32_t*>(descs + part.x)[i];
+            data.fetch(S.d, (int)(part.x), (int)tid, (int)T);
             if (tid < 64)
                 S.zz[16 + tid] = k_zz_colmajor[tid];
             if (tid == 0)
@@ -2588,7 +2584,7 @@ namespace aeonb
         return p;
     }
 
-    cudaError_t launch_jpeg_entropy(const aeonb_entropy_desc* descs_dev, int n, bool any_parallel, bool any_serial, int min_segment,
+    cudaError_t launch_jpeg_entropy(const launch_data& descs, int n, bool any_parallel, bool any_serial, int min_segment,
                                     uint32_t longest, uint64_t most_blocks, int most_places, const int4* parts_dev, int n_parts,
                                     cudaStream_t stream)
     {
@@ -2611,7 +2607,7 @@ namespace aeonb
             attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
             cfg.attrs    = &attr;
             cfg.numAttrs = 1;
-            err          = cudaLaunchKernelEx(&cfg, jpeg_entropy_spread_kernel, descs_dev, spread.cap);
+            err          = cudaLaunchKernelEx(&cfg, jpeg_entropy_spread_kernel, descs, spread.cap);
             if (err != cudaSuccess)
                 return err;
         }
@@ -2625,7 +2621,7 @@ namespace aeonb
             cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_parallel_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
             if (err != cudaSuccess)
                 return err;
-            jpeg_entropy_parallel_kernel<<<n, threads, smem, stream>>>(descs_dev, min_segment, (uint32_t)rows, (uint32_t)smem);
+            jpeg_entropy_parallel_kernel<<<n, threads, smem, stream>>>(descs, min_segment, (uint32_t)rows, (uint32_t)smem);
             err = cudaGetLastError();
             if (err != cudaSuccess)
                 return err;
@@ -2636,11 +2632,11 @@ namespace aeonb
             cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_restart_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (err != cudaSuccess)
                 return err;
-            jpeg_restart_index_kernel<<<n * RST_INDEX_BLOCKS, RST_INDEX_THREADS, 0, stream>>>(descs_dev);
+            jpeg_restart_index_kernel<<<n * RST_INDEX_BLOCKS, RST_INDEX_THREADS, 0, stream>>>(descs);
             err = cudaGetLastError();
             if (err != cudaSuccess)
                 return err;
-            jpeg_entropy_restart_kernel<<<n_parts, RST_THREADS, smem, stream>>>(descs_dev, parts_dev, min_segment, (uint32_t)smem);
+            jpeg_entropy_restart_kernel<<<n_parts, RST_THREADS, smem, stream>>>(descs, parts_dev, min_segment, (uint32_t)smem);
             err = cudaGetLastError();
             if (err != cudaSuccess)
                 return err;
@@ -2651,7 +2647,7 @@ namespace aeonb
             cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (err != cudaSuccess)
                 return err;
-            jpeg_entropy_kernel<<<n, 32, smem, stream>>>(descs_dev);
+            jpeg_entropy_kernel<<<n, 32, smem, stream>>>(descs);
             return cudaGetLastError();
         }
         return cudaSuccess;
