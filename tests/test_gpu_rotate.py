@@ -84,3 +84,35 @@ def test_bad_arguments(ctx):
     d = (L.RotateDesc * 1)()
     assert ctx.lib.aeonb_rotate_batch(ctx.handle, d, 1) == L.ERR_INVALID
     assert ctx.lib.aeonb_rotate_batch(ctx.handle, d, 0) == 0
+
+
+@pytest.mark.parametrize("nearest", [False, True])
+def test_rotation_at_the_edges_of_tiles_and_words(ctx, nearest):
+    """Widths and heights around a tile (512 x 8) and four pixels, sources and destinations at every alignment: rows, and nothing beside them,
+    are written as the oracle has them."""
+    from aeon_b200 import _lib as L
+    rng = np.random.default_rng(93)
+    dev = torch.device("cuda", ctx.device)
+    cases = [(h, w) for w in (1, 2, 3, 4, 5, 511, 512, 513, 1030) for h in (1, 8, 9)] + [(17, 515)]
+    descs = (L.RotateDesc * len(cases))()
+    keep = []
+    for i, (h, w) in enumerate(cases):
+        img = rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
+        angle, lead, pitch, at = int(rng.integers(-30, 31)), i % 4, 3 * w + i % 3, (i // 4) % 4
+        src = torch.zeros(8 + h * 3 * w, dtype=torch.uint8, device=dev)
+        src[lead:lead + img.size] = torch.from_numpy(img.reshape(-1)).to(dev)
+        dst = torch.full((8 + h * pitch,), 123, dtype=torch.uint8, device=dev)
+        d = descs[i]
+        d.src, d.src_pitch, d.src_pixel_stride = src.data_ptr() + lead, 3 * w, 3
+        d.width, d.height, d.angle, d.nearest = w, h, angle, int(nearest)
+        d.dst, d.dst_pitch, d.dst_pixel_stride = dst.data_ptr() + at, pitch, 3
+        want = np.full(8 + h * pitch, 123, np.uint8)
+        turned = ops.rotate(img, angle, False) if nearest else ops.rotate(img, angle)
+        for y in range(h):
+            want[at + y * pitch:at + y * pitch + 3 * w] = turned[y].reshape(-1)
+        keep.append((src, dst, want))
+    torch.cuda.synchronize(dev)
+    L.check(ctx.lib.aeonb_rotate_batch(ctx.handle, descs, len(cases)))
+    ctx.synchronize()
+    for (h, w), (_, dst, want) in zip(cases, keep):
+        assert np.array_equal(dst.cpu().numpy(), want), (h, w)
