@@ -149,11 +149,55 @@ namespace aeonb
             return t;
         }
 
+        // AREA_TAPS pixels of STRIDE bytes from p on, of which `count` are wanted, as whole words with the first pixel's first byte at the
+        // bottom.  A word is loaded only if a byte of a wanted pixel lies in it, and none waits for another.
+        constexpr int AREA_TAPS = 5;
+        template <int STRIDE>
+        __device__ __forceinline__ void area_words(const uint8_t* p, int count, uint32_t (&v)[(AREA_TAPS * STRIDE + 3) / 4])
+        {
+            constexpr int   V     = (AREA_TAPS * STRIDE + 3) / 4;
+            const uint32_t  lead  = (uint32_t)((uintptr_t)p & 3);
+            const uint32_t* word  = reinterpret_cast<const uint32_t*>(p - lead);
+            const int       bytes = (int)lead + min(count, AREA_TAPS) * STRIDE;
+            uint32_t        w[V + 1];
+#pragma unroll
+            for (int j = 0; j <= V; ++j)
+                w[j] = 4 * j < bytes ? __ldg(word + j) : 0;
+#pragma unroll
+            for (int j = 0; j < V; ++j)
+                v[j] = __funnelshift_r(w[j], w[j + 1], 8 * lead);
+        }
+        // The sums of one source row of a cell, tap after tap as OpenCV adds them.  Taps behind the last one have weight zero, which
+        // leaves a sum of non-negative terms as it is.  A byte becomes a float as the low bits of 2^23, from which 2^23 is taken.
+        template <int STRIDE>
+        __device__ __forceinline__ void area_row(const uint8_t* p, int count, const float (&first)[AREA_TAPS], const cell_taps& cell, float (&buf)[3])
+        {
+            for (int k0 = 0; k0 < count; k0 += AREA_TAPS)
+            {
+                uint32_t v[(AREA_TAPS * STRIDE + 3) / 4];
+                area_words<STRIDE>(p + k0 * STRIDE, count - k0, v);
+#pragma unroll
+                for (int k = 0; k < AREA_TAPS; ++k)
+                {
+                    const float alpha = k0 == 0 ? first[k] : k0 + k < count ? tap_weight(cell, k0 + k) : 0.f;
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+                    {
+                        const int      at   = k * STRIDE + c;
+                        const uint32_t bits = __byte_perm(v[at / 4], 0x4B000000u, 0x7440u + (uint32_t)(at % 4));
+                        buf[c] = __fadd_rn(buf[c], __fmul_rn(__fsub_rn(__uint_as_float(bits), 8388608.f), alpha));
+                    }
+                }
+            }
+        }
+
         // Mode 1, the shrinking regime.  A block takes `rows` destination rows; the cells of its columns and rows, whose float64
         // divisions cost more than the taps of a pixel, are worked out once per block.  A cell that lies inside the picture reads its
-        // source rows as aligned words, the other ones pixel by pixel.  Bound by the issue of the float32 chain that OpenCV's order
-        // prescribes (six operations per tap) and the byte conversions.  32 crops of about 850 x 850 to
-        // 224 x 224: 142 us with the cells worked out for every pixel and a load for every byte, 105 us so.
+        // source rows as aligned words, five pixels at a time, the other ones pixel by pixel.  Bound by the issue of the float32 chain that
+        // OpenCV's order prescribes (six operations per tap) and the byte conversions.  32 crops of about 850 x 850 to
+        // 224 x 224: 142 us with the cells worked out for every pixel and a load for every byte, 105 us with words loaded one after
+        // the other and converted by I2F (a quarter of the rate of the rest), 88 us so.  (Three blocks fit an SM by their registers; held
+        // to the registers of four or five they take 104 us.)
         constexpr int AREA_COLS = 512, AREA_ROWS = 8;
         __device__ void area_cells(const area_job& J, int rows)
         {
@@ -177,35 +221,21 @@ namespace aeonb
                         const cell_taps cx = tx[x], cy = ty[r];
                         const int       sx = J.crop_x + cx.first - J.canvas_x, sy = J.crop_y + cy.first - J.canvas_y;
                         const bool      inside = sx >= 0 && sy >= 0 && sx + cx.count <= J.src_w && sy + cy.count <= J.src_h;
-                        float           acc[3] = {0.f, 0.f, 0.f};
+                        float           acc[3] = {0.f, 0.f, 0.f}, alpha_first[AREA_TAPS];
+#pragma unroll
+                        for (int k = 0; k < AREA_TAPS; ++k)
+                            alpha_first[k] = k < cx.count ? tap_weight(cx, k) : 0.f;
                         for (int ky = 0; ky < cy.count; ++ky)
                         {
                             const float beta   = tap_weight(cy, ky);
                             float       buf[3] = {0.f, 0.f, 0.f};
                             if (inside)
                             {
-                                const uint8_t*  p    = J.src + (size_t)(sy + ky) * J.src_pitch + (size_t)sx * J.src_stride;
-                                const uint32_t  lead = (uint32_t)((uintptr_t)p & 3);
-                                const uint32_t* word = reinterpret_cast<const uint32_t*>(p - lead);
-                                // `have` bytes from the next pixel on lie at the bottom of `bytes`; a word is loaded only if a byte
-                                // of the pixel lies in it
-                                uint64_t bytes = (uint64_t)__ldg(word++) >> (8 * lead);
-                                int      have  = 4 - (int)lead;
-                                for (int kx = 0; kx < cx.count; ++kx)
-                                {
-                                    if (have < J.src_stride)
-                                    {
-                                        bytes |= (uint64_t)__ldg(word++) << (8 * have);
-                                        have += 4;
-                                    }
-                                    const float    alpha = tap_weight(cx, kx);
-                                    const uint32_t v     = (uint32_t)bytes;
-                                    buf[0] = __fadd_rn(buf[0], __fmul_rn((float)(v & 255), alpha));
-                                    buf[1] = __fadd_rn(buf[1], __fmul_rn((float)(v >> 8 & 255), alpha));
-                                    buf[2] = __fadd_rn(buf[2], __fmul_rn((float)(v >> 16 & 255), alpha));
-                                    bytes >>= 8 * J.src_stride;
-                                    have -= J.src_stride;
-                                }
+                                const uint8_t* p = J.src + (size_t)(sy + ky) * J.src_pitch + (size_t)sx * J.src_stride;
+                                if (J.src_stride == 3)
+                                    area_row<3>(p, cx.count, alpha_first, cx, buf);
+                                else
+                                    area_row<4>(p, cx.count, alpha_first, cx, buf);
                             }
                             else
                                 for (int kx = 0; kx < cx.count; ++kx)
@@ -456,8 +486,9 @@ extern "C" int aeonb_resize_batch(aeonb_ctx* ctx, const aeonb_resize_desc* descs
         const int  per  = (int)std::min<int64_t>((most + 255) / 256, 148 * 8);
         const dim3 grid((unsigned)std::max(per, 1), (unsigned)n);
         launch_timer timer(ctx, AEONB_KERNEL_OTHER, 0);
-        // rows of a block in the shrinking regime: as many share its column cells as leave about six blocks for every SM
-        const int rows = (int)std::max<int64_t>(1, std::min<int64_t>(area_rows / (148 * 6), AREA_ROWS));
+        // rows of a block in the shrinking regime: as many share its column cells as leave about 24 blocks for every SM, eight rounds (six
+        // blocks, two rounds: 92 us instead of 88 for 32 crops)
+        const int rows = (int)std::max<int64_t>(1, std::min<int64_t>(area_rows / (148 * 24), AREA_ROWS));
         resize_area_kernel<<<grid, 256, 0, ctx->stream>>>(jdev, rows);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess)

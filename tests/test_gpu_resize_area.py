@@ -119,3 +119,19 @@ def test_shrinking_cells_over_blocks_of_rows_and_columns(ctx, records):
     for stride in (3, 4):
         for (img, cxy, crop, (ow, oh)), g in zip(jobs, resize_gpu(ctx, jobs, stride)):
             assert np.array_equal(g, ops.resize_area_u8(window(img, cxy, crop), ow, oh)), (img.shape, ow, oh, stride)
+
+
+@pytest.mark.parametrize("src_stride", [3, 4])
+@pytest.mark.parametrize("taps", [2, 3.9, 4.1, 4.9, 5.1, 9.9, 10.2])
+def test_cells_around_the_pixels_taken_together(ctx, src_stride, taps):
+    """Cells of about one, two and three groups of five source pixels, rows that start at every place of a word."""
+    rng = np.random.default_rng(81)
+    jobs = []
+    for out in (1, 7, 24):
+        for crop_x in range(4):
+            w, h = int(out * taps + 1), int(5 * taps + 1)
+            img = rng.integers(0, 256, (h + 2, w + 5, 3), dtype=np.uint8)
+            jobs.append((img, (0, 0), (crop_x, 1, w, h), (out, 5)))
+    got = resize_gpu(ctx, jobs, src_stride)
+    for (img, at, crop, (dw, dh)), g in zip(jobs, got):
+        assert np.array_equal(g, ops.resize_area_u8(np.ascontiguousarray(window(img, at, crop)), dw, dh)), (crop, dw)
