@@ -1644,7 +1644,8 @@ namespace aeonb
         }
 
         // Copies the scan without stuffed bytes, up to the first marker: each block the vectors [v0, v1), which have been brought to
-        // `room`, to the work area, and from there every block all of it to `room`.  Returns the bytes of the copy.
+        // `room`, to the work area, and from there every block all of it to `room`.  Returns the bytes of the copy.  Takes the wait that
+        // belongs to the arrival at the cluster's barrier at the kernel's beginning.
         __device__ __forceinline__ uint32_t copy_spread(spread_state& D, uint32_t* room, uint32_t* work, const uint4* vec, uint32_t v0, uint32_t v1,
                                                         uint32_t lead)
         {
@@ -1670,6 +1671,7 @@ namespace aeonb
             }
             uint32_t all;
             cta_exclusive_scan(kept, S.warp_sums[0], all);
+            cluster.barrier_wait(); // every block of the cluster has started (it arrived on entry): its memory may be written from now on
             if (tid < C)
             {
                 in_block(D.all, tid)[rank].bytes  = all;
@@ -1964,6 +1966,9 @@ namespace aeonb
                     *d.status = 1;
                 return;
             }
+            // Nothing else promises that the other blocks have started by the time this one first writes to their memory; copy_spread
+            // waits for all of them there, behind the tables, so that the wait costs nothing.
+            cluster.barrier_arrive();
             const uint32_t     n = d.scan_size;
             const uint32_t     lead = (uint32_t)(reinterpret_cast<uintptr_t>(d.scan) & 15);
             const uint4* const vec  = reinterpret_cast<const uint4*>(d.scan - lead);
