@@ -2,7 +2,7 @@
 //
 // orient_kernel: the EXIF orientation turn cv::imdecode applies after decoding (a pure permutation of pixels).
 //
-// rotate_kernel: aeon's image::rotate (src/image.cpp:53-75), i.e.
+// rotate_pixels_kernel, rotate_tiles_kernel: aeon's image::rotate (src/image.cpp:53-75), i.e.
 // cv::warpAffine(src, dst, getRotationMatrix2D(centre, angle, 1), src.size(), INTER_LINEAR, BORDER_CONSTANT, 0)
 // on 8-bit interleaved pictures, bit for bit; and its INTER_NEAREST form (interpolate == false), which the
 // pixelmask and depthmap transformers use (src/etl_pixel_mask.cpp:71-73): the same fixed-point source coordinates
@@ -11,7 +11,7 @@
 // OpenCV maps every destination pixel back through the inverted matrix in 10-bit fixed point -- the products are
 // formed in float64 and rounded half to even per column (M0*x*1024, M3*x*1024) and per row ((M1*y+M2)*1024,
 // (M4*y+M5)*1024) -- keeps 5 fractional bits, and blends the four neighbours with integer weights
-// (32-fx)(32-fy)*32 ... that sum to 2^15; neighbours outside the picture count as zero.  The kernel does exactly
+// (32-fx)(32-fy)*32 ... that sum to 2^15; neighbours outside the picture count as zero.  The kernels do exactly
 // that per destination pixel: the float64 products with explicit round-to-nearest multiplies (no contraction),
 // __double2int_rn for the rounding, then integer arithmetic.  HBM traffic is one read of the source (neighbouring
 // threads share their taps through L1/L2) and one write of the destination.
@@ -37,14 +37,8 @@ namespace aeonb
             double         m[6]; // inverse map: source = m * (x, y, 1)
         };
 
-        // A block takes tiles of ROT_COLS x ROT_ROWS destination pixels.  What depends on the column or the row alone -- the float64
-        // products -- is worked out once per tile; a thread makes four neighbouring pixels, which leave as three words.  The six bytes of
-        // two neighbouring source pixels are cut out of aligned words, and each channel takes two 16 x 8 bit dot products.  Bound by
-        // the issue of integer instructions: 16 pictures and 16 masks of about 437 x 437 took 58 us with a thread per pixel, a
-        // division and four float64 products for each and loads and stores of bytes, 38 us so (tiles of 16 rows 41, of four 39).
-        constexpr int ROT_COLS = 512, ROT_ROWS = 8;
-
-        // The bytes of pixel `x` of a row and, with `two`, of the one behind it, from the bottom of v[0] on.
+        // The bytes of pixel `x` of a row and, with `two`, of the one behind it, from the bottom of v[0] on: cut out of aligned words
+        // that hold a byte of them (loads of single bytes: 16 pictures of 437 x 437 35 us, 31 so, a thread per pixel in both).
         __device__ __forceinline__ void source_bytes(const rotate_job& J, const uint8_t* row, int x, bool two, uint32_t (&v)[2])
         {
             const uint8_t*  p     = row + (size_t)x * J.src_stride;
@@ -106,13 +100,42 @@ namespace aeonb
             return pixel;
         }
 
-        __global__ void __launch_bounds__(256) rotate_kernel(const rotate_job* __restrict__ jobs)
+        // The parts of a fixed-point source coordinate that depend on the column and on the row (the rounding included).
+        __device__ __forceinline__ int2 column_part(const rotate_job& J, int x)
+        {
+            return make_int2(__double2int_rn(__dmul_rn(__dmul_rn(J.m[0], (double)x), 1024.0)), __double2int_rn(__dmul_rn(__dmul_rn(J.m[3], (double)x), 1024.0)));
+        }
+        __device__ __forceinline__ int2 row_part(const rotate_job& J, int y)
+        {
+            const int round = J.nearest ? 512 : 16; // half of the last kept bit: 10 bits dropped, or 5
+            return make_int2(__double2int_rn(__dmul_rn(__dadd_rn(__dmul_rn(J.m[1], (double)y), J.m[2]), 1024.0)) + round,
+                             __double2int_rn(__dmul_rn(__dadd_rn(__dmul_rn(J.m[4], (double)y), J.m[5]), 1024.0)) + round);
+        }
+        __device__ __forceinline__ void store_pixel(uint8_t* p, uint32_t v) { p[0] = (uint8_t)v, p[1] = (uint8_t)(v >> 8), p[2] = (uint8_t)(v >> 16); }
+
+        // Few pixels, narrow pictures, destinations with four bytes per pixel: a thread per pixel, as many blocks as the pixels fill.
+        __global__ void __launch_bounds__(256) rotate_pixels_kernel(const rotate_job* __restrict__ jobs)
+        {
+            const rotate_job J      = jobs[blockIdx.y];
+            const int        pixels = J.width * J.height;
+            for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pixels; i += gridDim.x * blockDim.x)
+            {
+                const int  y = i / J.width, x = i - y * J.width;
+                const int2 column = column_part(J, x), line = row_part(J, y);
+                store_pixel(J.dst + (size_t)y * J.dst_pitch + (size_t)x * J.dst_stride, rotated_pixel(J, line.x + column.x, line.y + column.y));
+            }
+        }
+
+        // Many pixels: a block takes tiles of ROT_COLS x ROT_ROWS destination pixels.  What depends on the column or the row alone -- the
+        // float64 products -- is worked out once per tile; a thread makes four neighbouring pixels, which leave as three words (the
+        // destination's rows start on words, three bytes per pixel).  Bound by the issue of integer instructions: 16 pictures and 16 masks
+        // of about 437 x 437 take 38 us (tiles of 16 rows 41, of four 39).
+        constexpr int ROT_COLS = 512, ROT_ROWS = 8;
+        __global__ void __launch_bounds__(256) rotate_tiles_kernel(const rotate_job* __restrict__ jobs)
         {
             __shared__ int2  column[ROT_COLS], line[ROT_ROWS];
             const rotate_job J       = jobs[blockIdx.y];
-            const int        round   = J.nearest ? 512 : 16; // half of the last kept bit: 10 bits dropped, or 5
             const int        tiles_x = (J.width + ROT_COLS - 1) / ROT_COLS, tiles = tiles_x * ((J.height + ROT_ROWS - 1) / ROT_ROWS);
-            const bool       words   = J.dst_stride == 3 && (((uintptr_t)J.dst | (uintptr_t)J.dst_pitch) & 3) == 0;
             for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x)
             {
                 const int x_first = tile % tiles_x * ROT_COLS, y_first = tile / tiles_x * ROT_ROWS;
@@ -120,13 +143,10 @@ namespace aeonb
                 __syncthreads(); // the tile before has been used
                 for (int i = threadIdx.x; i < cols + rows; i += blockDim.x)
                 {
-                    const double at = (double)(i < cols ? x_first + i : y_first + i - cols);
                     if (i < cols)
-                        column[i] = make_int2(__double2int_rn(__dmul_rn(__dmul_rn(J.m[0], at), 1024.0)),
-                                              __double2int_rn(__dmul_rn(__dmul_rn(J.m[3], at), 1024.0)));
+                        column[i] = column_part(J, x_first + i);
                     else
-                        line[i - cols] = make_int2(__double2int_rn(__dmul_rn(__dadd_rn(__dmul_rn(J.m[1], at), J.m[2]), 1024.0)) + round,
-                                                   __double2int_rn(__dmul_rn(__dadd_rn(__dmul_rn(J.m[4], at), J.m[5]), 1024.0)) + round);
+                        line[i - cols] = row_part(J, y_first + i - cols);
                 }
                 __syncthreads();
                 const int quads = (cols + 3) / 4;
@@ -138,8 +158,8 @@ namespace aeonb
 #pragma unroll
                     for (int k = 0; k < 4; ++k)
                         px[k] = k < n ? rotated_pixel(J, from.x + column[x + (k < n ? k : 0)].x, from.y + column[x + (k < n ? k : 0)].y) : 0;
-                    uint8_t* const d = J.dst + (size_t)(y_first + r) * J.dst_pitch + (size_t)(x_first + x) * J.dst_stride;
-                    if (words && n == 4)
+                    uint8_t* const d = J.dst + (size_t)(y_first + r) * J.dst_pitch + (size_t)(x_first + x) * 3;
+                    if (n == 4)
                     {
                         uint32_t* const w = reinterpret_cast<uint32_t*>(d);
                         w[0] = px[0] | px[1] << 24;
@@ -150,10 +170,7 @@ namespace aeonb
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             if (k < n)
-                            {
-                                uint8_t* const p = d + k * J.dst_stride;
-                                p[0] = (uint8_t)px[k], p[1] = (uint8_t)(px[k] >> 8), p[2] = (uint8_t)(px[k] >> 16);
-                            }
+                                store_pixel(d + 3 * k, px[k]);
                 }
             }
         }
@@ -234,7 +251,8 @@ extern "C" int aeonb_rotate_batch(aeonb_ctx* ctx, const aeonb_rotate_desc* descs
         if (n <= 0)
             return AEONB_OK;
         std::vector<rotate_job> jobs(n);
-        int64_t                 most = 0;
+        int64_t                 most = 0, most_tiles = 0, pixels = 0; // (pixels without interpolation four times)
+        bool                    wide = true, words = true;
         for (int i = 0; i < n; ++i)
         {
             const aeonb_rotate_desc& r = descs[i];
@@ -259,14 +277,27 @@ extern "C" int aeonb_rotate_batch(aeonb_ctx* ctx, const aeonb_rotate_desc* descs
             j.height      = r.height;
             j.nearest     = r.nearest != 0;
             rotation_inverse_map(r.width, r.height, r.angle, j.m);
-            most = std::max<int64_t>(most, (int64_t)((r.width + ROT_COLS - 1) / ROT_COLS) * ((r.height + ROT_ROWS - 1) / ROT_ROWS));
+            most       = std::max<int64_t>(most, (int64_t)r.width * r.height);
+            most_tiles = std::max<int64_t>(most_tiles, (int64_t)((r.width + ROT_COLS - 1) / ROT_COLS) * ((r.height + ROT_ROWS - 1) / ROT_ROWS));
+            pixels += (int64_t)r.width * r.height * (r.nearest ? 4 : 1);
+            wide &= r.width >= 128;
+            words &= r.dst_pixel_stride == 3 && (((uintptr_t)r.dst | (uintptr_t)r.dst_pitch) & 3) == 0;
         }
         AEONB_CUDA(cudaSetDevice(ctx->device));
         auto*      jdev = static_cast<const rotate_job*>(ctx->upload(jobs.data(), sizeof(rotate_job) * n));
-        const int  per  = (int)std::min<int64_t>(most, 148 * 8); // blocks per record
+        // A tile is a longer chain of work than a pixel, and tiles narrower than 128 pixels leave threads idle: below about four million
+        // pixels, of masks one million, there are too few of them to fill the SMs.  Pixels / tiles: one picture of 437 x 437 8.5 / 14.4 us,
+        // 16 of them 30.7 / 32.8, 16 of 512 x 512 39.2 / 36.9, 64 of 437 x 437 102 / 87; four masks of 437 x 437 10.6 / 11.9, eight 14.6 / 12.3;
+        // 64 pictures of 30 x 3000 41 / 69.  With destinations of four bytes per pixel, which a tile would store by bytes, 16 pictures
+        // of 437 x 437 30.7 / 40.5.
+        const bool tiles = words && wide && pixels >= 1 << 22;
+        const int  per   = (int)std::min<int64_t>(tiles ? most_tiles : (most + 255) / 256, 148 * 8); // blocks per record
         const dim3 grid((unsigned)std::max(per, 1), (unsigned)n);
         launch_timer timer(ctx, AEONB_KERNEL_OTHER, 0);
-        rotate_kernel<<<grid, 256, 0, ctx->stream>>>(jdev);
+        if (tiles)
+            rotate_tiles_kernel<<<grid, 256, 0, ctx->stream>>>(jdev);
+        else
+            rotate_pixels_kernel<<<grid, 256, 0, ctx->stream>>>(jdev);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess)
             throw error(AEONB_ERR_CUDA, cuda_message("rotate kernel launch", e));

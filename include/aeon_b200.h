@@ -180,7 +180,9 @@ int aeonb_image_batch_noalloc(const aeonb_image_desc* descs, int n, const aeonb_
  * then the source of aeonb_image_batch. */
 typedef struct aeonb_rotate_desc
 {
-    const uint8_t* src;      /* device: interleaved B,G,R[,x] picture */
+    const uint8_t* src;      /* device: interleaved B,G,R[,x] picture.  Read in aligned 4-byte words: up to three bytes on
+                                either side of it that share a word with one of its own must be readable memory, which
+                                holds for any placement inside a cudaMalloc'd buffer */
     int32_t src_pitch, src_pixel_stride;
     int32_t width, height;
     int32_t angle;           /* degrees, counter-clockwise */
@@ -213,7 +215,8 @@ int aeonb_orient_batch(aeonb_ctx* ctx, const aeonb_orient_desc* descs, int n);
  * aeonb_image_batch then takes as a source of the same size (no further resampling). */
 typedef struct aeonb_resize_desc
 {
-    const uint8_t* src;      /* device: interleaved B,G,R[,x]; NULL = all-zero canvas */
+    const uint8_t* src;      /* device: interleaved B,G,R[,x]; NULL = all-zero canvas.  INTER_AREA reads it in aligned 4-byte
+                                words, as aeonb_rotate_desc describes */
     int32_t src_pitch, src_pixel_stride;
     int32_t src_w, src_h;
     int32_t canvas_x, canvas_y;

@@ -87,18 +87,26 @@ def test_bad_arguments(ctx):
 
 
 @pytest.mark.parametrize("nearest", [False, True])
-def test_rotation_at_the_edges_of_tiles_and_words(ctx, nearest):
-    """Widths and heights around a tile (512 x 8) and four pixels, sources and destinations at every alignment: rows, and nothing beside them,
-    are written as the oracle has them."""
+@pytest.mark.parametrize("tiles", [False, True])
+def test_rotation_at_the_edges_of_tiles_and_words(ctx, nearest, tiles):
+    """Widths and heights around a tile (512 x 8) and four pixels, sources at every alignment: rows, and nothing beside them, are written as
+    the oracle has them.  Launches of at least 2**22 pixels (masks: a quarter) of pictures at least 128 wide, with destinations of three bytes per pixel on
+    words, go through tiles, others through a thread per pixel, with destinations at every alignment."""
     from aeon_b200 import _lib as L
     rng = np.random.default_rng(93)
     dev = torch.device("cuda", ctx.device)
-    cases = [(h, w) for w in (1, 2, 3, 4, 5, 511, 512, 513, 1030) for h in (1, 8, 9)] + [(17, 515)]
+    cases = [(h, w) for w in (1, 2, 3, 4, 5, 128, 129, 511, 512, 513, 1030) for h in (1, 8, 9)] + [(17, 515)]
+    if tiles:
+        cases = [c for c in cases if c[1] >= 128] + [(2051, 2047)]      # the last one brings the pixels
+    pixels = sum(h * w for h, w in cases) * (4 if nearest else 1)
+    assert (pixels >= 1 << 22) == tiles
     descs = (L.RotateDesc * len(cases))()
     keep = []
     for i, (h, w) in enumerate(cases):
         img = rng.integers(0, 256, (h, w, 3), dtype=np.uint8)
         angle, lead, pitch, at = int(rng.integers(-30, 31)), i % 4, 3 * w + i % 3, (i // 4) % 4
+        if tiles:
+            pitch, at = (3 * w + 3) // 4 * 4, 4 * (i % 2)
         src = torch.zeros(8 + h * 3 * w, dtype=torch.uint8, device=dev)
         src[lead:lead + img.size] = torch.from_numpy(img.reshape(-1)).to(dev)
         dst = torch.full((8 + h * pitch,), 123, dtype=torch.uint8, device=dev)
@@ -116,3 +124,31 @@ def test_rotation_at_the_edges_of_tiles_and_words(ctx, nearest):
     ctx.synchronize()
     for (h, w), (_, dst, want) in zip(cases, keep):
         assert np.array_equal(dst.cpu().numpy(), want), (h, w)
+
+
+def test_rotation_on_either_side_of_the_rule_for_tiles(ctx):
+    """The same pictures in launches that go through tiles and in ones that one property each keeps from it: too few pixels, a narrow picture,
+    a destination off a word, four bytes per pixel."""
+    from aeon_b200 import _lib as L
+    rng = np.random.default_rng(94)
+    dev = torch.device("cuda", ctx.device)
+    shapes = [(1025, 2048), (1024, 2048)]
+    images = [rng.integers(0, 256, (h, w, 3), dtype=np.uint8) for h, w in shapes]
+    small = rng.integers(0, 256, (40, 127, 3), dtype=np.uint8)
+    want = [ops.rotate(img, 13) for img in images] + [ops.rotate(small, 13)]
+    for name, pictures, at, stride in [("tiles", images, 0, 3), ("few pixels", images[1:], 0, 3), ("narrow", images + [small], 0, 3), ("off a word", images, 2, 3),
+                                       ("four bytes", images, 0, 4)]:
+        descs, keep = (L.RotateDesc * len(pictures))(), []
+        for d, img in zip(descs, pictures):
+            h, w = img.shape[:2]
+            src, dst = torch.from_numpy(img).to(dev), torch.zeros(at + h * w * stride, dtype=torch.uint8, device=dev)
+            d.src, d.src_pitch, d.src_pixel_stride = src.data_ptr(), 3 * w, 3
+            d.width, d.height, d.angle = w, h, 13
+            d.dst, d.dst_pitch, d.dst_pixel_stride = dst.data_ptr() + at, w * stride, stride
+            keep.append((src, dst))
+        torch.cuda.synchronize(dev)
+        L.check(ctx.lib.aeonb_rotate_batch(ctx.handle, descs, len(pictures)))
+        ctx.synchronize()
+        for img, (_, dst), ref in zip(pictures, keep, want[1:] if len(pictures) == 1 else want):
+            got = dst[at:].cpu().numpy().reshape(img.shape[0], img.shape[1], stride)[..., :3]
+            assert np.array_equal(got, ref), (name, img.shape)
