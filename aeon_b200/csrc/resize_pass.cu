@@ -47,6 +47,7 @@ namespace aeonb
             int32_t        src_pitch, src_stride, src_w, src_h, canvas_x, canvas_y;
             int32_t        crop_x, crop_y, crop_w, crop_h;
             int32_t        dst_pitch, dst_stride, out_w, out_h;
+            int32_t        taps; // mode 1: pixels taken at a time
             int32_t        mode; // 0: whole-factor boxes, 1: weighted cells, 2: bilinear with area taps, 3: bicubic, 4: Lanczos
             const int32_t* lanczos; // mode 4: out_w x (start, 8 weights), then out_h x (start, 8 weights), 9 ints each
             int32_t        ix, iy;
@@ -149,16 +150,15 @@ namespace aeonb
             return t;
         }
 
-        // AREA_TAPS pixels of STRIDE bytes from p on, of which `count` are wanted, as whole words with the first pixel's first byte at the
+        // TAPS pixels of STRIDE bytes from p on, of which `count` are wanted, as whole words with the first pixel's first byte at the
         // bottom.  A word is loaded only if a byte of a wanted pixel lies in it, and none waits for another.
-        constexpr int AREA_TAPS = 5;
-        template <int STRIDE>
-        __device__ __forceinline__ void area_words(const uint8_t* p, int count, uint32_t (&v)[(AREA_TAPS * STRIDE + 3) / 4])
+        template <int TAPS, int STRIDE>
+        __device__ __forceinline__ void area_words(const uint8_t* p, int count, uint32_t (&v)[(TAPS * STRIDE + 3) / 4])
         {
-            constexpr int   V     = (AREA_TAPS * STRIDE + 3) / 4;
+            constexpr int   V     = (TAPS * STRIDE + 3) / 4;
             const uint32_t  lead  = (uint32_t)((uintptr_t)p & 3);
             const uint32_t* word  = reinterpret_cast<const uint32_t*>(p - lead);
-            const int       bytes = (int)lead + min(count, AREA_TAPS) * STRIDE;
+            const int       bytes = (int)lead + min(count, TAPS) * STRIDE;
             uint32_t        w[V + 1];
 #pragma unroll
             for (int j = 0; j <= V; ++j)
@@ -169,15 +169,15 @@ namespace aeonb
         }
         // The sums of one source row of a cell, tap after tap as OpenCV adds them.  Taps behind the last one have weight zero, which
         // leaves a sum of non-negative terms as it is.  A byte becomes a float as the low bits of 2^23, from which 2^23 is taken.
-        template <int STRIDE>
-        __device__ __forceinline__ void area_row(const uint8_t* p, int count, const float (&first)[AREA_TAPS], const cell_taps& cell, float (&buf)[3])
+        template <int TAPS, int STRIDE>
+        __device__ __forceinline__ void area_row(const uint8_t* p, int count, const float (&first)[TAPS], const cell_taps& cell, float (&buf)[3])
         {
-            for (int k0 = 0; k0 < count; k0 += AREA_TAPS)
+            for (int k0 = 0; k0 < count; k0 += TAPS)
             {
-                uint32_t v[(AREA_TAPS * STRIDE + 3) / 4];
-                area_words<STRIDE>(p + k0 * STRIDE, count - k0, v);
+                uint32_t v[(TAPS * STRIDE + 3) / 4];
+                area_words<TAPS, STRIDE>(p + k0 * STRIDE, count - k0, v);
 #pragma unroll
-                for (int k = 0; k < AREA_TAPS; ++k)
+                for (int k = 0; k < TAPS; ++k)
                 {
                     const float alpha = k0 == 0 ? first[k] : k0 + k < count ? tap_weight(cell, k0 + k) : 0.f;
 #pragma unroll
@@ -193,15 +193,21 @@ namespace aeonb
 
         // Mode 1, the shrinking regime.  A block takes `rows` destination rows; the cells of its columns and rows, whose float64
         // divisions cost more than the taps of a pixel, are worked out once per block.  A cell that lies inside the picture reads its
-        // source rows as aligned words, five pixels at a time, the other ones pixel by pixel.  Bound by the issue of the float32 chain that
-        // OpenCV's order prescribes (six operations per tap) and the byte conversions.  32 crops of about 850 x 850 to
-        // 224 x 224: 142 us with the cells worked out for every pixel and a load for every byte, 105 us with words loaded one after
-        // the other and converted by I2F (a quarter of the rate of the rest), 88 us so.  (Three blocks fit an SM by their registers; held
-        // to the registers of four or five they take 104 us.)
+        // source rows as aligned words, TAPS pixels at a time, the other ones pixel by pixel.  Bound by the issue of the float32 chain that
+        // OpenCV's order prescribes (six operations per tap) and the byte conversions.  32 pictures of 850 x 850 to 224 x 224: 85 us
+        // with words loaded one after the other and converted by I2F (a quarter of the rate of the rest), 64 us so.  (Three blocks fit
+        // an SM by their registers; held to the registers of four or five they took a fifth longer.)
         constexpr int AREA_COLS = 512, AREA_ROWS = 8;
-        __device__ void area_cells(const area_job& J, int rows)
+        // Pixels taken at a time, 3, 4 or 5, for rows of up to `most` taps: those behind the last tap cost as much as the others, and beginning
+        // a group costs about one more.  128 pictures of 1400 x 1000 to 224 x 224 (up to 6 x 8 taps): 446 us by fives, 355 by fours.
+        inline int area_taps(int most)
         {
-            __shared__ cell_taps tx[AREA_COLS], ty[AREA_ROWS];
+            const auto cost = [&](int t) { return (most + t - 1) / t * (t + 1); };
+            return cost(5) <= cost(4) && cost(5) <= cost(3) ? 5 : cost(4) <= cost(3) ? 4 : 3;
+        }
+        template <int TAPS>
+        __device__ __forceinline__ void area_cells(const area_job& J, int rows, cell_taps* tx, cell_taps* ty)
+        {
             for (int y0 = blockIdx.x * rows; y0 < J.out_h; y0 += gridDim.x * rows)
                 for (int x0 = 0; x0 < J.out_w; x0 += AREA_COLS)
                 {
@@ -221,9 +227,9 @@ namespace aeonb
                         const cell_taps cx = tx[x], cy = ty[r];
                         const int       sx = J.crop_x + cx.first - J.canvas_x, sy = J.crop_y + cy.first - J.canvas_y;
                         const bool      inside = sx >= 0 && sy >= 0 && sx + cx.count <= J.src_w && sy + cy.count <= J.src_h;
-                        float           acc[3] = {0.f, 0.f, 0.f}, alpha_first[AREA_TAPS];
+                        float           acc[3] = {0.f, 0.f, 0.f}, alpha_first[TAPS];
 #pragma unroll
-                        for (int k = 0; k < AREA_TAPS; ++k)
+                        for (int k = 0; k < TAPS; ++k)
                             alpha_first[k] = k < cx.count ? tap_weight(cx, k) : 0.f;
                         for (int ky = 0; ky < cy.count; ++ky)
                         {
@@ -233,9 +239,9 @@ namespace aeonb
                             {
                                 const uint8_t* p = J.src + (size_t)(sy + ky) * J.src_pitch + (size_t)sx * J.src_stride;
                                 if (J.src_stride == 3)
-                                    area_row<3>(p, cx.count, alpha_first, cx, buf);
+                                    area_row<TAPS, 3>(p, cx.count, alpha_first, cx, buf);
                                 else
-                                    area_row<4>(p, cx.count, alpha_first, cx, buf);
+                                    area_row<TAPS, 4>(p, cx.count, alpha_first, cx, buf);
                             }
                             else
                                 for (int kx = 0; kx < cx.count; ++kx)
@@ -263,7 +269,13 @@ namespace aeonb
             const int      pixels = J.out_w * J.out_h;
             if (J.mode == 1)
             {
-                area_cells(J, area_rows);
+                __shared__ cell_taps tx[AREA_COLS], ty[AREA_ROWS];
+                if (J.taps == 3)
+                    area_cells<3>(J, area_rows, tx, ty);
+                else if (J.taps == 4)
+                    area_cells<4>(J, area_rows, tx, ty);
+                else
+                    area_cells<5>(J, area_rows, tx, ty);
                 return;
             }
             for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < pixels; i += gridDim.x * blockDim.x)
@@ -417,6 +429,7 @@ extern "C" int aeonb_resize_batch(aeonb_ctx* ctx, const aeonb_resize_desc* descs
         std::vector<int32_t>  tables;      // Lanczos taps of every record that wants them
         std::vector<size_t>   table_first(n, 0);
         int64_t               most = 0, area_rows = 0;
+        int                   narrowest = AREA_COLS;
         for (int i = 0; i < n; ++i)
         {
             const aeonb_resize_desc& r = descs[i];
@@ -472,7 +485,12 @@ extern "C" int aeonb_resize_batch(aeonb_ctx* ctx, const aeonb_resize_desc* descs
             else
                 j.mode = 2;
             most = std::max<int64_t>(most, (int64_t)r.out_w * r.out_h);
-            area_rows += j.mode == 1 ? r.out_h : 0;
+            j.taps = area_taps((int)std::min(std::ceil(j.scale_x), 1e6) + 1);
+            if (j.mode == 1)
+            {
+                area_rows += r.out_h;
+                narrowest = std::min(narrowest, r.out_w);
+            }
         }
         AEONB_CUDA(cudaSetDevice(ctx->device));
         if (!tables.empty())
@@ -486,9 +504,12 @@ extern "C" int aeonb_resize_batch(aeonb_ctx* ctx, const aeonb_resize_desc* descs
         const int  per  = (int)std::min<int64_t>((most + 255) / 256, 148 * 8);
         const dim3 grid((unsigned)std::max(per, 1), (unsigned)n);
         launch_timer timer(ctx, AEONB_KERNEL_OTHER, 0);
-        // rows of a block in the shrinking regime: as many share its column cells as leave about 24 blocks for every SM, eight rounds (six
-        // blocks, two rounds: 92 us instead of 88 for 32 crops)
-        const int rows = (int)std::max<int64_t>(1, std::min<int64_t>(area_rows / (148 * 24), AREA_ROWS));
+        // Rows of a block in the shrinking regime, 1, 2, 4 or 8: as many share its column cells as leave about ten blocks for every SM, and at
+        // least as many as give each of its threads a pixel.  One row / that many, five pixels at a time: 128 crops of 850 x 850 to 16 x 16 2389 / 333 us, 32 of
+        // 300 x 400 to 112 x 112 34 / 23, four of 850 x 850 to 800 x 800 68 / 58, 32 of 850 x 850 to 224 x 224 76 / 66.
+        int rows = 1;
+        while (rows < AREA_ROWS && (rows * narrowest < 256 || area_rows >= (int64_t)148 * 10 * 2 * rows))
+            rows *= 2;
         resize_area_kernel<<<grid, 256, 0, ctx->stream>>>(jdev, rows);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess)

@@ -107,7 +107,7 @@ def test_lanczos4_matches_the_oracle(ctx):
 @pytest.mark.parametrize("records", [1, 40])
 def test_shrinking_cells_over_blocks_of_rows_and_columns(ctx, records):
     """More columns than a block holds cells for (512), rows that do not fill a block's group (one row a block for one record, eight for
-    many), cells of one to nine pixels, cells that hang over the picture's edge on an expanded canvas, 4-byte source pixels."""
+    many, the narrowest of which is 31 pixels wide), cells of one to nine pixels, cells that hang over the picture's edge on an expanded canvas, 4-byte source pixels."""
     rng = np.random.default_rng(85)
     jobs = []
     for i in range(records):
@@ -135,3 +135,17 @@ def test_cells_around_the_pixels_taken_together(ctx, src_stride, taps):
     got = resize_gpu(ctx, jobs, src_stride)
     for (img, at, crop, (dw, dh)), g in zip(jobs, got):
         assert np.array_equal(g, ops.resize_area_u8(np.ascontiguousarray(window(img, at, crop)), dw, dh)), (crop, dw)
+
+
+@pytest.mark.parametrize("width, rows", [(512, 1), (255, 2), (127, 4), (63, 8), (1, 8)])
+@pytest.mark.parametrize("taps", [1.3, 2.6, 3.7, 5.2, 6.6, 8.8, 11.5])
+def test_rows_of_a_block_and_pixels_taken_together(ctx, width, rows, taps):
+    """Every number of rows that a block takes of a narrow picture, with one row left over and one missing, at every number of pixels that
+    are taken together (three to five, by the pixels of a cell)."""
+    rng = np.random.default_rng(86)
+    jobs = []
+    for oh in (1, rows + 1, 3 * rows - 1):
+        w, h = int(width * taps) + 1, int(oh * 2.3) + 1
+        jobs.append((rng.integers(0, 256, (h, w, 3), dtype=np.uint8), (0, 0), (0, 0, w, h), (width, oh)))
+    for (img, _, _, (ow, oh)), g in zip(jobs, resize_gpu(ctx, jobs)):
+        assert np.array_equal(g, ops.resize_area_u8(img, ow, oh)), (img.shape, ow, oh)
