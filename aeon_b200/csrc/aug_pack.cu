@@ -418,7 +418,7 @@ namespace aeonb
         // lies together in the output -- a channel's band, the whole band, or one line of it where lines are apart -- is written in
         // whole 16-byte pieces, the elements at its two ends one by one.  Written element by element, as they were, with a warp's
         // threads 16 elements apart, these stores were most of the kernel: four pictures of 1000 x 1000 bytes 67 us, now 43; 32 of
-        // 224 x 224 x 3 bytes 53 us, now 28; 128 of 300 x 300 bytes 189 us, now 122.
+        // 224 x 224 x 3 bytes 53 us, now 27; 128 of 300 x 300 bytes 189 us, now 119.
         template <typename T, bool WHOLE, bool IDENT, bool INTERLEAVED>
         __device__ __forceinline__ void store_runs(const store_args<T>& A, int tid, int nt)
         {
@@ -909,13 +909,11 @@ namespace aeonb
         cudaError_t launch_typed(const aug_launch& L, const launch_data& data, int clusters, int bands, int cluster_size, int threads, size_t smem, int pix, int runs,
                                  cudaStream_t stream)
         {
-            // Planes of 4- and 8-byte elements that do not start on 16 bytes stay with store_band (64 of 225 x 225 floats: 71 us, 86 in
-            // runs): four stores of a warp fill what one would.
             auto kern = pix == 4 ? aug_pack_kernel<T, 4, 0> : aug_pack_kernel<T, 3, 0>;
             if (runs == 2)
                 kern = pix == 4 ? aug_pack_kernel<T, 4, 2> : aug_pack_kernel<T, 3, 2>;
-            else if (runs == 1 && sizeof(T) <= 2)
-                kern = pix == 4 ? aug_pack_kernel<T, 4, sizeof(T) <= 2 ? 1 : 0> : aug_pack_kernel<T, 3, sizeof(T) <= 2 ? 1 : 0>;
+            else if (runs == 1)
+                kern = pix == 4 ? aug_pack_kernel<T, 4, sizeof(T) == 1 ? 1 : 0> : aug_pack_kernel<T, 3, sizeof(T) == 1 ? 1 : 0>;
             // the most launch_aug_pack lets through, so that threads with smaller tiles do not lower it between this call and the launch
             cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, AUG_MAX_SMEM);
             if (err != cudaSuccess)
@@ -995,8 +993,12 @@ namespace aeonb
         bool at_elements = true; // every slot starts on a multiple of the element's size
         for (int i = 0; i < n; ++i)
             at_elements &= ((uintptr_t)descs_host[i].dst & (elem - 1)) == 0;
-        const int runs = L.vector_ok || !at_elements ? 0 : layout.stride_x == 1 ? 1
-                       : layout.stride_c == 1 && layout.stride_x == layout.channels ? 2 : 0;
+        // How a band is stored (see RUNS).  Wider elements than bytes fill what a store takes sooner: planes of 2, 4 and 8 bytes per element stay
+        // with store_band (element by element / in runs: 256 of 64 x 64 x int16 35.5 / 40.4 us, 256 of 448 x 448 704 / 796, 64 of 225 x 225
+        // floats 71 / 86), and so do narrow or few pictures of 8-byte elements side by side, for which the runs' arithmetic costs more than
+        // they save (256 of 64 x 64 doubles 45 / 52, one of 1000 x 1000 33 / 42; 64 of 300 x 300 155 / 111).
+        const int runs = L.vector_ok || !at_elements ? 0 : layout.stride_x == 1 ? (elem == 1 ? 1 : 0)
+                       : layout.stride_c == 1 && layout.stride_x == layout.channels && (elem < 8 || (layout.slot_w >= 256 && n >= 8)) ? 2 : 0;
         const size_t smem = smem_for(bands);
         if (smem > AUG_MAX_SMEM)
         {

@@ -297,3 +297,22 @@ def test_outputs_that_do_not_start_on_16_bytes(ctx, otype, layout):
                 K.image_batch(ctx, srcs, params, got, K.make_layout(w, h, dt, strides=(sc, sy, sx)), record_stride=slot + 4)
                 ctx.synchronize()
                 assert torch.equal(room, expect), (w, h, lead)
+
+
+@pytest.mark.parametrize("n, w", [(7, 256), (8, 255), (8, 256), (9, 301)])
+def test_doubles_side_by_side(ctx, n, w):
+    """8-byte elements with the channels side by side go out in runs from eight pictures of 256 columns on, element by element below."""
+    from aeon_b200 import kernels as K
+    rng = np.random.default_rng(22)
+    h, dt, dev = 37, K.DTYPE_BY_NAME["double"], torch.device("cuda", ctx.device)
+    srcs = [torch.from_numpy(gradient_image(rng, 50, 80)).to(dev) for _ in range(n)]
+    params = [random_params(rng, 80, 50, w, h, False) for _ in srcs]
+    with torch.cuda.stream(ctx.torch_stream):
+        want = torch.full((n, 3, h, w), 99, dtype=K._TORCH_DTYPE[dt], device=dev)
+        K.image_batch(ctx, srcs, params, want, K.make_layout(w, h, dt))
+        for lead in (0, 1):
+            room = torch.full((lead + n * h * w * 3 + 8,), 77, dtype=K._TORCH_DTYPE[dt], device=dev)
+            got = room[lead:lead + n * h * w * 3].view(n, h, w, 3)
+            K.image_batch(ctx, srcs, params, got, K.make_layout(w, h, dt, channel_major=False))
+            ctx.synchronize()
+            assert torch.equal(got, want.permute(0, 2, 3, 1)) and torch.all(room[:lead] == 77) and torch.all(room[lead + n * h * w * 3:] == 77)
