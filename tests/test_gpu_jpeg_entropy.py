@@ -235,6 +235,21 @@ def test_block_sizes_on_either_side_of_a_stream_per_sm(ctx, golden_dir, copies):
         check(ctx, [blob] if blob else [blobs[i % len(blobs)] for i in range(copies)])
 
 
+def test_streams_that_fit_with_fewer_segments(ctx):
+    """Streams around the longest that two blocks on an SM can hold: the launch's longest one decides how many segments there is room for
+    beside it (382 of them at 57 KB, 128 at 69 KB; behind that the copy goes to global memory)."""
+    rng = np.random.default_rng(79)
+    img = np.clip(gradient_image(rng, 400, 900).astype(np.int16) + rng.integers(-24, 25, (400, 900, 3)), 0, 255).astype(np.uint8)
+    blobs, w = [], 240
+    for size in (54_000, 58_000, 62_000, 66_000, 68_500, 71_000):
+        while len(jpeg_bytes(img[:, :w], 90)) < size:
+            w += 4
+        blobs.append(jpeg_bytes(img[:, :w], 90))
+        assert len(blobs[-1]) < size + 1500
+    for longest in range(1, len(blobs) + 1):
+        check(ctx, [blobs[longest - 1 - i % min(longest, 2)] for i in range(149)])
+
+
 def decode_descs(ctx, blobs, rois=None, lead=0, scratch=True, scan_bytes=None):
     """Entropy decode with the descriptors in hand: (status, [planes], work area, descriptor) of every record.  `lead`: offset of a scan from a
     16-byte boundary; `scan_bytes`: cuts the scans off; work areas are zeroed before."""
