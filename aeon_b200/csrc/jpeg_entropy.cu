@@ -2055,7 +2055,7 @@ namespace aeonb
         // Streams with restart markers.
         //
         // Behind every restart marker a decoder starts afresh -- byte aligned, first block of an MCU, DC predictors zero -- so the
-        // intervals between them are independent and their first block numbers known.  An index kernel (one block per stream)
+        // intervals between them are independent and their first block numbers known.  An index kernel (a cluster of blocks per stream)
         // notes where the intervals start; the stream is then cut into parts of up to RST_MAX_INTERVALS whole intervals, one thread
         // block each, and inside a part the intervals into segments as in the kernel above, except that the first segment of
         // every interval starts in the true state and block numbers are counted from there: a wrong guess travels to the end of
@@ -2068,7 +2068,7 @@ namespace aeonb
         // each): 88 ms with the serial kernel (one warp per stream), 0.22 ms with these two.  Two blocks of 512 threads fit an SM by
         // their tables; five of 128 threads with parts of at most 10 KB took 0.09 ms more, most of it spent on building tables.
         constexpr int RST_THREADS       = 512;
-        constexpr int RST_INDEX_THREADS = 1024, RST_INDEX_BLOCKS = 8;
+        constexpr int RST_INDEX_THREADS = 1024;
         constexpr int RST_ROOM          = 46 * 1024; // shared memory for a part's bytes (see jpeg_restart_parts): 2 blocks fit an SM
 
         struct rst_state
@@ -2089,18 +2089,18 @@ namespace aeonb
                    (uint64_t)d.mcux * d.mcuy * bpm < (1ull << 30) && d.scratch_bytes >= w.bytes && (reinterpret_cast<uintptr_t>(d.scratch) & 15) == 0;
         }
 
-        // Finds the intervals of a stream: RST_INDEX_BLOCKS blocks of a cluster per stream, every warp a run of 16-byte vectors, which
+        // Finds the intervals of a stream: the blocks of a cluster per stream, every warp a run of 16-byte vectors, which
         // it goes through twice, counting markers and then numbering them from the counts of the warps in front.  What bounds
-        // it is the latency of those passes: 32 streams of 0.3 MB took 85 us with one block each, about 20 with eight.
-        __global__ void __cluster_dims__(RST_INDEX_BLOCKS, 1, 1) __launch_bounds__(RST_INDEX_THREADS)
-            jpeg_restart_index_kernel(const __grid_constant__ launch_data data)
+        // it is the latency of those passes: 16 streams of 0.6 MB took 82 us with one block each, about 20 with four.
+        __global__ void __launch_bounds__(RST_INDEX_THREADS) jpeg_restart_index_kernel(const __grid_constant__ launch_data data)
         {
             namespace cg = cooperative_groups;
             constexpr uint32_t            warps = RST_INDEX_THREADS / 32;
             __shared__ aeonb_entropy_desc d;
             __shared__ uint32_t           counts[warps], other, total;
-            const uint32_t                tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, rank = blockIdx.x % RST_INDEX_BLOCKS;
-            data.fetch(d, (int)(blockIdx.x / RST_INDEX_BLOCKS), (int)tid, (int)RST_INDEX_THREADS);
+            cg::cluster_group             cluster = cg::this_cluster();
+            const uint32_t                tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, C = cluster.num_blocks(), rank = cluster.block_rank();
+            data.fetch(d, (int)(blockIdx.x / C), (int)tid, (int)RST_INDEX_THREADS);
             __syncthreads();
             if (!d.scratch || d.restart_interval == 0)
                 return; // as all blocks of the cluster
@@ -2132,7 +2132,7 @@ namespace aeonb
                 return follows & restart;
             };
             // a warp owns a run of vectors, so that markers are numbered by warp, then by pass, then by lane
-            const uint32_t per = (nv + warps * RST_INDEX_BLOCKS - 1) / (warps * RST_INDEX_BLOCKS);
+            const uint32_t per = (nv + warps * C - 1) / (warps * C);
             const uint32_t v0 = (rank * warps + warp) * per, v1 = min(nv, v0 + per);
             uint32_t       count = 0;
             for (uint32_t base = v0; base < v1; base += 32)
@@ -2155,10 +2155,9 @@ namespace aeonb
             uint32_t       before = __reduce_add_sync(0xffffffffu, lane < warp ? here : 0);
             if (tid == 0)
                 total = mine;
-            cg::cluster_group cluster = cg::this_cluster();
             cluster.sync();
             uint32_t all = 0, end = other;
-            for (uint32_t r = 0; r < RST_INDEX_BLOCKS; ++r)
+            for (uint32_t r = 0; r < C; ++r)
             {
                 const uint32_t theirs = *cluster.map_shared_rank(&total, r);
                 before += r < rank ? theirs : 0;
@@ -2567,6 +2566,10 @@ namespace aeonb
         return (size_t)std::max(least, std::min(want, most));
     }
 
+    // Blocks of the cluster of each of n streams: as many as all clusters find room for at once, one block to an SM: 15 clusters of eight, 33
+    // of four, 66 of two (what cudaOccupancyMaxActiveClusters says for a B200 and blocks that have an SM to themselves).
+    static int jpeg_entropy_cluster(int n) { return n <= 15 ? 8 : n <= 33 ? 4 : n <= 66 ? 2 : 1; }
+
     // How a launch of few streams is spread: blocks in the cluster of each stream (0: not spread), and runs a block has room for.
     struct spread_plan
     {
@@ -2577,13 +2580,11 @@ namespace aeonb
     static spread_plan jpeg_entropy_spread(int n, uint32_t longest, int most_places)
     {
         spread_plan p;
-        if (n > 66 || most_places < 1 || most_places > SPREAD_PLACES)
+        if (jpeg_entropy_cluster(n) == 1 || most_places < 1 || most_places > SPREAD_PLACES)
             return p;
-        // As many blocks as all streams' clusters find room for at once, one block to an SM: 15 clusters of eight, 33 of four, 66 of two
-        // (what cudaOccupancyMaxActiveClusters says for a B200).  A block has less than a warp for each of its schedulers to decode with
-        // if it has fewer than 128 runs.
+        // A block has less than a warp for each of its schedulers to decode with if it has fewer than 128 runs.
         const uint32_t segments = longest / SPREAD_SEG + 1;
-        int            blocks   = n <= 15 ? SPREAD_MOST : n <= 33 ? 4 : 2;
+        int            blocks   = jpeg_entropy_cluster(n);
         while (blocks > 1 && segments * (uint32_t)most_places <= (uint32_t)blocks / 2 * 128)
             blocks /= 2;
         p.threads = 512;
@@ -2641,8 +2642,20 @@ namespace aeonb
             cudaError_t  err  = cudaFuncSetAttribute(jpeg_entropy_restart_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (err != cudaSuccess)
                 return err;
-            jpeg_restart_index_kernel<<<n * RST_INDEX_BLOCKS, RST_INDEX_THREADS, 0, stream>>>(descs);
-            err = cudaGetLastError();
+            // Both kernels, us, with one / two / four / eight blocks per stream: 256 streams of 1.6 KB 60 / 69 / 92 / 153, 64 of 42 KB
+            // 145 / 143 / 147 / 167, 16 of 0.6 MB 336 / 297 / 273 / 277, one of 0.6 MB 163 / 124 / 102 / 92.
+            const int           blocks = jpeg_entropy_cluster(n);
+            cudaLaunchConfig_t  cfg    = {};
+            cudaLaunchAttribute attr   = {};
+            cfg.gridDim                = dim3(n * blocks);
+            cfg.blockDim               = dim3(RST_INDEX_THREADS);
+            cfg.stream                 = stream;
+            attr.id                    = cudaLaunchAttributeClusterDimension;
+            attr.val.clusterDim.x      = blocks;
+            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+            cfg.attrs    = &attr;
+            cfg.numAttrs = 1;
+            err          = cudaLaunchKernelEx(&cfg, jpeg_restart_index_kernel, descs);
             if (err != cudaSuccess)
                 return err;
             jpeg_entropy_restart_kernel<<<n_parts, RST_THREADS, smem, stream>>>(descs, parts_dev, min_segment, (uint32_t)smem);

@@ -189,6 +189,20 @@ def test_restart_intervals(ctx, interval):
     check(ctx, blobs[:1], rois[:1])
 
 
+@pytest.mark.parametrize("n", [1, 15, 16, 33, 34, 66, 67])
+def test_restart_index_over_clusters(ctx, n):
+    """Launches at the edges of the number of blocks that look for a stream's markers: streams of a few vectors, whose blocks are mostly
+    empty, beside one of 100 KB, markers at every place of a vector and on both sides of a block's share."""
+    import cv2
+    rng = np.random.default_rng(690 + n)
+    long = jpeg_bytes(rng.integers(0, 256, (230, 400, 3), dtype=np.uint8), 95, [cv2.IMWRITE_JPEG_RST_INTERVAL, 1])
+    assert len(long) > 100_000
+    small = [jpeg_bytes(gradient_image(rng, int(rng.integers(8, 60)), int(rng.integers(8, 60))), 85, [cv2.IMWRITE_JPEG_RST_INTERVAL, int(rng.integers(1, 5))])
+             for _ in range(8)]
+    check(ctx, [long if i == n // 2 else small[i % 8] for i in range(n)])
+    check(ctx, [small[i % 8] for i in range(n)])
+
+
 def test_damaged_restart_streams_are_left_to_the_serial_decoder(ctx):
     """Streams whose intervals are not all there, or do not end where they should: with and without a work area the same status,
     and the same planes where the status is good."""
