@@ -1,12 +1,12 @@
-"""The bookkeeping of the block-parallel entropy kernel, as a model on the CPU (tests/entropy_model.py): what the kernel
-counts must be what the stream holds, every piece of the storing pass must start at the right block in a known state."""
+"""The bookkeeping of the block-parallel entropy kernels, as a model on the CPU (tests/entropy_model.py): what the kernels
+count must be what the stream holds, every piece of the storing pass must start at the right block in a known state."""
 import os
 
 import cv2
 import numpy as np
 import pytest
 
-from tests.entropy_model import simulate
+from tests.entropy_model import SPREAD_EXTRA, simulate, simulate_spread
 from tests.synth import gradient_image
 
 
@@ -50,3 +50,41 @@ def test_a_thread_for_every_piece_of_the_storing_pass(golden_dir, quality):
         assert r["counted"] == r["total_blocks"] and not r["problems"], r
         pieces = 4 * r["segments"]
         assert pieces <= 1024 or r["segment"] == 160 or pieces % 1024 == 0 or pieces % 1024 > 256, r
+
+
+def spread_streams(rng):
+    """Streams of one to a thousand segments, of two to six places in an MCU, with much, little and nothing to fall into step on."""
+    modes = [cv2.IMWRITE_JPEG_SAMPLING_FACTOR_420, cv2.IMWRITE_JPEG_SAMPLING_FACTOR_444, cv2.IMWRITE_JPEG_SAMPLING_FACTOR_422,
+             cv2.IMWRITE_JPEG_SAMPLING_FACTOR_411, None]
+    for k, (h, w) in enumerate([(300, 400), (8, 8), (33, 47), (430, 470), (120, 160)] * 4):
+        img = gradient_image(rng, h, w, int(rng.integers(2, 40)))
+        if k // 5 == 1:
+            img[h // 3:] = 128
+        elif k // 5 == 2:
+            img[:] = (np.arange(w) // 8 % 2 * 255)[None, :, None]
+        elif k // 5 == 3:
+            img = rng.integers(0, 256, img.shape, dtype=np.uint8)
+        mode = modes[(k + k // 5) % 5]
+        blob = cv2.imencode(".jpg", img if mode else img[..., 0], [cv2.IMWRITE_JPEG_QUALITY, int(rng.choice([60, 90, 97]))] +
+                            ([cv2.IMWRITE_JPEG_SAMPLING_FACTOR, mode] if mode else []))[1].tobytes()
+        yield k, blob
+
+
+@pytest.mark.parametrize("streams", [1, 16, 66])
+def test_streams_spread_over_clusters(streams):
+    for k, blob in spread_streams(np.random.default_rng(200 + streams)):
+        if len(blob) < 110_000:
+            r = simulate_spread(blob, streams)
+            assert not r["problems"], (k, r)
+
+
+@pytest.mark.parametrize("room", [0, 1, 30])
+def test_more_states_than_there_is_room_for(room):
+    """A run that notes no state makes the piece in front of it longer, and nothing else."""
+    rng = np.random.default_rng(205)
+    for img in (gradient_image(rng, 300, 400), rng.integers(0, 256, (100, 150, 3), dtype=np.uint8)):
+        r = simulate_spread(cv2.imencode(".jpg", img, [cv2.IMWRITE_JPEG_QUALITY, 90])[1].tobytes(), extra_room=room)
+        assert max(r["noted"]) > room and not r["problems"], r
+    noise = cv2.imencode(".jpg", rng.integers(0, 256, (160, 200, 3), dtype=np.uint8), [cv2.IMWRITE_JPEG_QUALITY, 100])[1].tobytes()
+    r = simulate_spread(noise)
+    assert max(r["noted"]) > SPREAD_EXTRA and not r["problems"], r
