@@ -209,14 +209,18 @@ def test_pictures_as_wide_as_two_mcu_rows_in_shared_memory_allow(ctx, mode, wide
         decode_gpu(ctx, blobs[2:])
 
 
-@pytest.mark.parametrize("n", [1, 26, 27, 28, 47, 48, 49, 60])
+@pytest.mark.parametrize("n", [1, 53, 54, 59, 60])
 def test_batches_around_the_size_that_travels_with_a_launch(ctx, n):
-    """Descriptors go with the launch up to about 8 KB (48 streams, 27 images, fewer pictures with their work lists) and through device memory
-    beyond: the same pictures either way."""
+    """Descriptors go with the launch up to 8064 bytes and through device memory beyond: 53 streams or images, 59 pictures of one strip of MCU
+    rows with their work lists.  The same pictures on either side."""
+    import ctypes as C
+    from aeon_b200 import _lib as L
+    near = 8064
+    assert near // C.sizeof(L.EntropyDesc) == near // C.sizeof(L.ImageDesc) == 53 and near // (C.sizeof(L.JpegDesc) + 8) == 59
     from aeon_b200.provider import Provider
     from tests.pipeline_oracle import PipelineOracle
     rng = np.random.default_rng(80 + n)
-    recs = [(jpeg_bytes(gradient_image(rng, int(rng.integers(20, 90)), int(rng.integers(20, 90))), 90),) for _ in range(n)]
+    recs = [(jpeg_bytes(gradient_image(rng, int(rng.integers(20, 33)), int(rng.integers(20, 90))), 90),) for _ in range(n)]
     cfg = {"batch_size": n, "random_seed": 3, "etl": [{"type": "image", "height": 64, "width": 48}],
            "augmentation": [{"type": "image", "crop_enable": True, "center": False, "scale": [0.5, 1.0], "flip_enable": True}]}
     prov = Provider(ctx, cfg)

@@ -1,5 +1,9 @@
-"""Device entropy decoders (a thread block per JPEG stream decoding segments speculatively; a block per run of intervals for streams
-with restart markers; one warp per stream) against the host decoder and against the oracle: identical coefficient planes."""
+"""Device entropy decoders (a cluster of thread blocks per JPEG stream, or a block, decoding segments speculatively; a block per run of
+intervals for streams with restart markers; one warp per stream) against the host decoder and against the oracle: identical coefficient
+planes.
+
+Launches of up to 66 streams, none longer than about 120 KB and none with more than six blocks in an MCU, go through the kernel that spreads
+a stream over a cluster; padded to 67 (1024 threads at most) or 149 (512) they go through the one with a block per stream."""
 import ctypes as C
 import os
 
@@ -77,7 +81,8 @@ def test_natural_batch_and_reference_fixtures(ctx, golden_dir, parallel):
     check(ctx, blobs, parallel=parallel)
 
 
-def test_regions(ctx, parallel):
+@pytest.mark.parametrize("parallel, n", [(True, 12), (True, 67), (True, 149), (False, 12)])
+def test_regions(ctx, parallel, n):
     from aeon_b200 import kernels as K
     rng = np.random.default_rng(64)
     blobs, rois = [], []
@@ -90,10 +95,11 @@ def test_regions(ctx, parallel):
         x1, y1 = int(rng.integers(x0 + 1, mcux + 1)), int(rng.integers(y0 + 1, mcuy + 1))
         blobs.append(blob)
         rois.append((x0, y0, x1, y1))
-    check(ctx, blobs, rois, parallel)
+    check(ctx, [blobs[i % 12] for i in range(n)], [rois[i % 12] for i in range(n)], parallel)
 
 
-def test_malformed_stream_sets_status_and_returns(ctx, parallel):
+@pytest.mark.parametrize("parallel, n", [(True, 3), (True, 67), (True, 149), (False, 3)])
+def test_malformed_stream_sets_status_and_returns(ctx, parallel, n):
     """A scan of 0xFF filler and one of random bytes: the kernel flags them (or decodes garbage) and terminates."""
     from aeon_b200 import kernels as K
     rng = np.random.default_rng(65)
@@ -102,11 +108,11 @@ def test_malformed_stream_sets_status_and_returns(ctx, parallel):
     head = good[:sos + 14]
     truncated = good[:sos + 14 + 200] + b"\xff\xd9"
     noise = head + bytes(rng.integers(0, 255, 3000, dtype=np.uint8)) + b"\xff\xd9"
-    got = K.jpeg_entropy_decode_device(ctx, [good, truncated, noise], None, parallel)
-    assert got[0][3] == 0
+    got = K.jpeg_entropy_decode_device(ctx, [good, truncated, noise] + [good] * (n - 3), None, parallel)
+    assert [g[3] for g in got[:1] + got[3:]] == [0] * (n - 2)
     assert got[1][3] in (0, 1) and got[2][3] in (0, 1)
     # and the context is still usable
-    check(ctx, [good], parallel=parallel)
+    check(ctx, [good] * (n - 2), parallel=parallel)
 
 
 def test_large_picture_and_many_streams(ctx, parallel):
@@ -148,7 +154,9 @@ def test_streams_with_more_segments_than_the_smallest_segment_allows(ctx, golden
     check(ctx, [blob])
     info = host_planes(blob)[0]
     mcux, mcuy = info.blocks_w[0] // info.hs[0], info.blocks_h[0] // info.vs[0]
-    check(ctx, [blob] * 4, rois=[(0, 0, mcux, mcuy), (3, 5, mcux - 2, mcuy), (0, mcuy - 1, mcux, mcuy), (0, 0, mcux, mcuy - 1)])
+    rois = [(0, 0, mcux, mcuy), (3, 5, mcux - 2, mcuy), (0, mcuy - 1, mcux, mcuy), (0, 0, mcux, mcuy - 1)]
+    for n in (4, 68, 149):
+        check(ctx, [blob] * n, [rois[i % 4] for i in range(n)])
     rng = np.random.default_rng(77)
     big = []
     for k in range(24):   # 84-140 KB: segments of 164 to 280 bytes, last segments of every length
@@ -157,6 +165,7 @@ def test_streams_with_more_segments_than_the_smallest_segment_allows(ctx, golden
         big.append(jpeg_bytes(img, 92))
     assert min(len(b) for b in big) > 84000
     check(ctx, big)
+    check(ctx, [big[i % 24] for i in range(67)])
 
 
 def restart_offsets(blob):
@@ -367,25 +376,27 @@ def coded_grey(rng, size, whole):
             mark(0xDA, bytes([1, 1, 0, 0, 63, 0])) + bytes(out) + b"\xff\xd9" + bytes(20))
 
 
-@pytest.mark.parametrize("tile", [2048, 4096, 13 * 16384])
-def test_streams_that_end_at_the_edge_of_a_tile(ctx, tile):
-    """The end marker at every place around a multiple of the bytes a block copies at a time (128 threads for a short stream; 1024 and the
-    copy in the work area for the long one): a whole stream decodes, one cut short in front of its last code is reported, also where the
-    marker's first byte is the last of a tile."""
+@pytest.mark.parametrize("n, tile", [(1, 8192), (67, 4096), (149, 4096), (67, 8192), (1, 13 * 16384)])
+def test_streams_that_end_at_the_edge_of_a_tile(ctx, n, tile):
+    """The end marker at every place around a multiple of the bytes a block copies at a time -- 16 for each of its threads: 512 of a cluster's
+    only block, 256 of the blocks that short streams get in launches of more than 66, 1024 and the copy in the work area for
+    the long one: a whole stream decodes, one cut short in front of its last code is reported, also where the marker's first byte is
+    the last of a tile."""
     rng = np.random.default_rng(tile)
-    for size, lead in [(tile - 2, 0), (tile - 1, 0), (tile, 0), (tile - 1 - 6, 6), (tile - 1 - 15, 15)][:5 if tile < 10000 else 3]:
+    for size, lead in [(tile - 2, 0), (tile - 1, 0), (tile, 0), (tile + 1, 0), (tile - 1 - 6, 6), (tile - 1 - 15, 15)][:6 if tile < 10000 else 3]:
         blob = coded_grey(rng, size, True)
-        (status, planes, _, _), = decode_descs(ctx, [blob], lead=lead)
-        assert status == 0 and np.array_equal(planes[0], host_planes(blob)[1][0][:planes[0].size]), (size, lead)
-        (status, _, _, _), = decode_descs(ctx, [coded_grey(rng, size, False)], lead=lead)
-        assert status == 1, (size, lead)
+        want = host_planes(blob)[1][0]
+        for status, planes, _, _ in decode_descs(ctx, [blob] * n, lead=lead):
+            assert status == 0 and np.array_equal(planes[0], want[:planes[0].size]), (size, lead)
+        cut = decode_descs(ctx, [coded_grey(rng, size, False)] * n, lead=lead)
+        assert all(status == 1 for status, _, _, _ in cut), (size, lead)
 
 
 def left_to_the_serial_decoder(work, d):
     """The first word of the work area's header: not 0 where the interval decoder has given a stream up."""
     mcus, bpm = d.mcux * d.mcuy, sum(d.hs[c] * d.vs[c] for c in range(d.ncomp))
     intervals = -(-mcus // d.restart_interval)
-    parts = intervals if intervals < 96 else intervals // 64 + 96
+    parts = intervals if intervals < 96 else intervals // 256 + 96
     at = (d.scan_size + 64 * (parts + 2) + 15) // 16 * 16 + (mcus * bpm * 2 + 15) // 16 * 16
     return int(work[at:at + 4].view(np.uint32)[0])
 
@@ -403,8 +414,28 @@ def test_regions_that_end_inside_a_restart_interval(ctx, interval):
         assert left_to_the_serial_decoder(work, d) == 0, roi
 
 
-def recode(blob, dc_lengths, ac_lengths):
-    """The same coefficients coded with other Huffman tables, one for DC and one for AC symbols: code lengths by symbol."""
+@pytest.mark.parametrize("h, w, interval, parts_of", [(16 * 20 - 3, 16 * 26 - 5, 1, 6), (16 * 16, 16 * 16, 1, 3), (16 * 40, 16 * 40, 2, 9), (24, 16 * 400, 1, 9)])
+def test_many_restart_intervals(ctx, h, w, interval, parts_of):
+    """More than 256 intervals, the most that a block takes, and as many as that (the work area's layout changes at 96 and with every 256):
+    identical planes, and the stream stays with the interval decoder, for the whole picture and for regions.  `parts_of`: one stream in a
+    launch, or beside enough others that its parts hold more intervals."""
+    import cv2
+    rng = np.random.default_rng(73)
+    blob = jpeg_bytes(gradient_image(rng, h, w), 85, [cv2.IMWRITE_JPEG_RST_INTERVAL, interval])
+    mcux, mcuy = -(-w // 16), -(-h // 16)
+    assert -(-mcux * mcuy // interval) >= 256
+    whole, part = (0, 0, mcux, mcuy), (1, mcuy // 3, mcux - 2, max(mcuy - 1, mcuy // 3 + 1))
+    for n in (1, parts_of, 40):
+        rois = [whole if i % 2 == 0 else part for i in range(n)]
+        for roi, (status, planes, work, d) in zip(rois, decode_descs(ctx, [blob] * n, rois)):
+            _, want, _ = host_planes(blob, roi)
+            assert status == 0 and all(np.array_equal(p, x[:p.size]) for p, x in zip(planes, want)), roi
+            assert left_to_the_serial_decoder(work, d) == 0, roi
+
+
+def recode(blob, dc_lengths, ac_lengths, interval=0):
+    """The same coefficients coded with other Huffman tables, one for DC and one for AC symbols: code lengths by symbol.  With `interval`, a
+    restart marker after every so many MCUs."""
     import struct
     from aeon_b200 import kernels as K
     info, coefs, _ = K.jpeg_entropy_decode(blob)
@@ -420,16 +451,25 @@ def recode(blob, dc_lengths, ac_lengths):
         return codes, counts + bytes(s for s, _ in sorted(lengths.items(), key=lambda s: (s[1], s[0])))
 
     (dc, dc_table), (ac, ac_table) = canonical(dc_lengths), canonical(ac_lengths)
-    bits = []
+    bits, body = [], b""
 
     def put(code, value, size):
         bits.append(format(code[0], "0%db" % code[1]))
         if size:
             bits.append(format(value if value > 0 else value + (1 << size) - 1, "0%db" % size))
 
+    def whole_bytes():
+        text = "".join(bits)
+        text += "1" * (-len(text) % 8)
+        bits.clear()
+        return bytes(int(text[i:i + 8], 2) for i in range(0, len(text), 8)).replace(b"\xff", b"\xff\x00")
+
     pred = [0] * info.ncomp
     for m in range((info.blocks_w[0] // info.hs[0]) * (info.blocks_h[0] // info.vs[0])):
         mx, my = m % (info.blocks_w[0] // info.hs[0]), m // (info.blocks_w[0] // info.hs[0])
+        if interval and m and m % interval == 0:
+            body += whole_bytes() + bytes([0xFF, 0xD0 + (m // interval - 1) % 8])
+            pred = [0] * info.ncomp
         for c in range(info.ncomp):
             for y in range(info.vs[c]):
                 for x in range(info.hs[c]):
@@ -449,14 +489,13 @@ def recode(blob, dc_lengths, ac_lengths):
                         run = 0
                     if run:
                         put(ac[0], 0, 0)
-    text = "".join(bits)
-    text += "1" * (-len(text) % 8)
-    body = bytes(int(text[i:i + 8], 2) for i in range(0, len(text), 8)).replace(b"\xff", b"\xff\x00")
+    body += whole_bytes()
     out, p = blob[:2], 2
     while blob[p + 1] != 0xDA:          # the other segments as they are, without the tables
         end = p + 2 + struct.unpack(">H", blob[p + 2:p + 4])[0]
         out += blob[p:end] if blob[p + 1] != 0xC4 else b""
         p = end
+    out += b"\xff\xdd" + struct.pack(">HH", 4, interval) if interval else b""
     for kind, table in ((0, dc_table), (0x10, ac_table)):
         out += b"\xff\xc4" + struct.pack(">H", 3 + len(table)) + bytes([kind]) + table
     sos = bytearray(blob[p:p + 2 + struct.unpack(">H", blob[p + 2:p + 4])[0]])
@@ -469,7 +508,8 @@ def recode(blob, dc_lengths, ac_lengths):
 def test_tables_with_codes_longer_than_the_lookup_windows(ctx, dc_long, ac_long, ac_short):
     """Canonical tables with a few short codes and the rest of one length: just inside the windows (9 bits DC, 11 AC), just outside, and
     so long that they do not start near the end of the code space, where the tables expect codes beyond the windows.  In one stream of
-    a batch only, in both kernels with a work area."""
+    a launch only, in the kernel for few streams, in the one with a block per stream, in shared memory and too long for it, and in the one
+    for restart markers."""
     import cv2
     rng = np.random.default_rng(70)
     img = gradient_image(rng, 90, 130)
@@ -484,6 +524,16 @@ def test_tables_with_codes_longer_than_the_lookup_windows(ctx, dc_long, ac_long,
     assert np.array_equal(cv2.imdecode(np.frombuffer(blob, np.uint8), 1), cv2.imdecode(np.frombuffer(plain, np.uint8), 1))
     check(ctx, [plain, blob, jpeg_bytes(img, 88, [cv2.IMWRITE_JPEG_OPTIMIZE, 1])])
     check(ctx, [blob])
+    for n in (67, 149):
+        check(ctx, [plain] * (n - 1) + [blob])
+    restart = [recode(plain, dc, ac, interval) for interval in (1, 9, 1000)]
+    assert np.array_equal(cv2.imdecode(np.frombuffer(restart[0], np.uint8), 1), cv2.imdecode(np.frombuffer(plain, np.uint8), 1))
+    for status, planes, work, d in decode_descs(ctx, restart):
+        assert status == 0 and all(np.array_equal(p, x[:p.size]) for p, x in zip(planes, host_planes(plain)[1]))
+        assert left_to_the_serial_decoder(work, d) == 0
+    tall = recode(jpeg_bytes(np.concatenate([img[:80]] * 26), 98), dc, ac)
+    assert len(tall) > 227 * 1024
+    check(ctx, [tall])
 
 
 @pytest.mark.parametrize("n", [1, 15, 16, 34, 66, 67])
@@ -521,7 +571,18 @@ def test_streams_spread_over_clusters(ctx, n):
             check(ctx, [blob], [roi])
 
 
-def test_spread_streams_cut_short(ctx):
+def test_more_noted_states_than_there_is_room_for(ctx):
+    """Noise of which hardly any run falls into step with another: more states on the way than a block has room for."""
+    from tests.entropy_model import SPREAD_EXTRA, simulate_spread
+    rng = np.random.default_rng(74)
+    blobs = [jpeg_bytes(rng.integers(0, 256, (160, 120 + 40 * k, 3), dtype=np.uint8), 100) for k in range(3)]
+    for blob in blobs:
+        assert max(simulate_spread(blob, len(blobs))["noted"]) > SPREAD_EXTRA
+    check(ctx, blobs)
+
+
+@pytest.mark.parametrize("n", [2, 67, 149])
+def test_streams_cut_short(ctx, n):
     """A stream of which a part is missing: the status is 1 unless the region needs none of it, at cuts around the places where the
     blocks of a cluster share the stream out; bytes behind the end marker are no part of the stream."""
     from aeon_b200 import kernels as K
@@ -533,10 +594,11 @@ def test_spread_streams_cut_short(ctx):
     size = len(blob) - 2 - start
     tail = bytes(rng.integers(0, 256, 3000, dtype=np.uint8))
     whole, upper = (0, 0, mcux, mcuy), (0, 0, mcux, 2)
+    small = jpeg_bytes(gradient_image(rng, 8, 8), 90)
     for cut in sorted({0, 1, size // 2, size - 1, *(size * r // 8 // 16 * 16 + d for r in range(1, 8) for d in (-1, 0, 1))}):
         for k in (0, 3000):
             data = blob[:start + cut] + b"\xff\xd9" + tail[:k]
-            got = K.jpeg_entropy_decode_device(ctx, [data, data], [whole, upper])
+            got = K.jpeg_entropy_decode_device(ctx, [data, data] + [small] * (n - 2), [whole, upper] + [None] * (n - 2))
             assert got[0][3] == 1, (cut, k)
             if cut > size // 4:
                 assert got[1][3] == 0, (cut, k)
