@@ -520,8 +520,8 @@ int aeonb_jpeg_entropy_batch(aeonb_ctx* ctx, const aeonb_entropy_desc* descs, in
         // are resident at once up to four to an SM (fewer, of larger streams); the first `sms` blocks of a grid land on SMs of
         // their own.  So the longest streams go to the blocks that keep their SM to themselves (the last ones of the first wave
         // when the second wave is not full), the next longest to the rest of the first wave, the shortest to the second wave.
-        // Measured on B200, streams of 20-80 KB: 256 of them 277 us against 320 us in arrival order, 200 275 against 315, 400
-        // 387 against 440, up to 149 the same.  AEONB_ENTROPY_ORDER=0 keeps the arrival order.
+        // Measured on B200, streams of 22-82 KB: 256 of them 385 us against 486 us in arrival order, 200 339 against 479, 400
+        // 544 against 617, up to 149 the same.  AEONB_ENTROPY_ORDER=0 keeps the arrival order.
         std::vector<aeonb_entropy_desc> ordered;
         static const bool reorder = [] {
             const char* e = std::getenv("AEONB_ENTROPY_ORDER");

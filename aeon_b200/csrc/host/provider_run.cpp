@@ -1021,8 +1021,8 @@ void aeonb_provider::stage_inputs(batch_plan& B, int par, bool alone)
     if (nwork > 0)
     {
         const int                     groups = std::max(1, std::min(k_slices, nwork));
-        // A batch of nothing but clips: the spectrogram kernel of a slice runs while the next slices are on their way.  Under
-        // 2 MB the copy takes about as long as the launches that this adds.  Behind a batch that is still under way it gains
+        // A batch of nothing but clips: once all of them are staged, the spectrogram kernel is launched slice by slice, and that of a
+        // slice runs while the next slices are still crossing the link.  Under 2 MB the copy takes about as long as the launches that this adds.  Behind a batch that is still under way it gains
         // nothing, since that one's kernel runs beside the upload already, and the launches cost: with four batches in flight 32 clips
         // (400-sample frames, 13 cepstra) take 266 us in slices and 190 us in one launch, 64 clips (320, 64 filters) 490 and 420 us.
         int clip_stages = 0;

@@ -2065,7 +2065,7 @@ namespace aeonb
         // marked doubtful and the serial kernel, launched behind, decodes it anew.
         //
         // Measured on a B200, 32 pictures of 900-1400 pixels a side (4:2:2, quality 92, a marker after every MCU row, 0.3 MB
-        // each): 88 ms with the serial kernel (one warp per stream), 0.22 ms with these two.  Two blocks of 512 threads fit an SM by
+        // each): 88 ms with the serial kernel (one warp per stream), 0.21 ms with these two.  Two blocks of 512 threads fit an SM by
         // their tables; five of 128 threads with parts of at most 10 KB took 0.09 ms more, most of it spent on building tables.
         constexpr int RST_THREADS       = 512;
         constexpr int RST_INDEX_THREADS = 1024;

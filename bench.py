@@ -785,11 +785,11 @@ def main():
 
 
 # DRAM bytes per launch (ncu dram__bytes_read.sum + dram__bytes_write.sum) of the kernels of the headline step, from the
-# captures summarised under profiles/ (same workload, same batch size; in the three-kernel chain part of the coefficient
+# captures kept beside the benchmark (same workload, same batch size; in the three-kernel chain part of the coefficient
 # planes and pictures stays in the 126 MB L2 between kernels, so a kernel's DRAM traffic can be below its algorithmic bytes).
 # Reported beside, never inside, the achieved figure, which comes from the algorithmic bytes and the time of this run.
 TRAFFIC = {"bytes": {"jpeg_entropy": 48.9e6, "jpeg_backend": 74.9e6, "aug_pack": 147.8e6},
-           "source": "profiles/*_config2.md (one launch each under ncu, config2 batch 256, device entropy decoding)"}
+           "source": "one launch each under ncu, config2 batch 256, device entropy decoding"}
 
 
 if __name__ == "__main__":

@@ -257,9 +257,8 @@ int64_t aeonb_jpeg_backend_bytes(const aeonb_jpeg_desc* descs, int n);
 
 /* ------------------------------------------------------------------------------------------------
  * 1b'. JPEG entropy decoding on the device: the Huffman stage of cv::imdecode
- *      (src/etl_image.cpp:90).  A stream without restart markers that is given a work area is decoded by a whole
- *      thread block (segments decoded speculatively, then synchronised on each other); other streams by one
- *      warp that walks the stream serially.  Fills the coefficient planes that
+ *      (src/etl_image.cpp:90).  A stream that is given a work area is decoded by one or several thread blocks; other
+ *      streams, and damaged ones with restart markers, by one warp that walks the stream serially.  Fills the coefficient planes that
  *      aeonb_jpeg_desc describes, so aeonb_jpeg_entropy_batch followed by aeonb_jpeg_backend_batch
  *      decodes a batch of JPEG files without per-record host work beyond header parsing.
  * ---------------------------------------------------------------------------------------------- */
@@ -284,9 +283,10 @@ typedef struct aeonb_entropy_desc
     int32_t* status;         /* device: set to 0 on success, 1 when the stream is malformed (may be NULL) */
     void*    scratch;        /* device: work area of aeonb_jpeg_entropy_scratch_bytes() bytes, 16-byte aligned.  With it, a
                                 stream without restart markers is decoded by a whole thread block (speculative decoding
-                                of segments that synchronise on each other), one with restart markers by several, each a
-                                run of the intervals between the markers; without it (NULL) a single warp walks the
-                                stream serially */
+                                of segments that synchronise on each other) or, in calls of up to 66 streams of up to
+                                about 120 KB, by a cluster of them; one with restart markers by several, each a run of
+                                the intervals between the markers; without it (NULL) a single warp walks the stream
+                                serially */
     uint64_t scratch_bytes;
 } aeonb_entropy_desc;
 
