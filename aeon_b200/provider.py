@@ -72,10 +72,11 @@ class Provider:
             r = next(r for r, rec in enumerate(records) if len(rec) != k)
             raise ValueError("record %d has %d elements, the configuration needs %d" % (r, len(records[r]), k))
         flat = list(chain.from_iterable(records))
-        sizes = (C.c_size_t * (n * k)).from_buffer(array("Q", map(len, flat)) or array("Q", (0,)))
+        few = n * k < 8  # ctypes converts a few elements sooner than the arrays are made (two: 3.7 / 5.5 us; 16: 10.6 / 7.4)
+        sizes = (C.c_size_t * (n * k))(*map(len, flat)) if few else (C.c_size_t * (n * k)).from_buffer(array("Q", map(len, flat)))
         if not set(map(type, flat)) - {bytes}:
             # each element points at the bytes object's own buffer, which `flat` keeps alive
-            if _BYTES_AT is not None:
+            if _BYTES_AT is not None and not few:
                 at = np.fromiter(map(id, flat), np.uint64, n * k) + _BYTES_AT
                 return C.cast(at.ctypes.data, C.POINTER(C.c_void_p)), sizes, (at, flat)
             ptrs = (C.c_char_p * (n * k))(*flat)
