@@ -129,6 +129,7 @@ aeonb_provider::aeonb_provider(aeonb_ctx* c, const json& cfg) : ctx(c)
 {
     if (!ctx)
         throw std::invalid_argument("provider needs a context");
+    m_spare.reserve(k_spare); // the driver thread, which fills it, has nobody to throw to
     const json* etl = cfg.find("etl");
     if (!etl || !etl->is_array())
         throw std::invalid_argument("Required Argument: 'etl' not set");
