@@ -941,12 +941,13 @@ namespace aeonb
                                 const char** why)
     {
         *why = nullptr;
-        bool any_contrast = false;
+        bool any_contrast = false, as_they_are = layout.dtype == AEONB_U8; // bytes go out without a look into the value table
         int  max_cols     = 1; // widest stretch of source columns any record reads
         for (int i = 0; i < n; ++i)
         {
             const aeonb_image_desc& r = descs_host[i];
             any_contrast |= r.contrast != 1.0f;
+            as_they_are &= r.contrast == 1.0f && !r.lighting_enable;
             if (r.src)
                 max_cols = std::max(max_cols, std::min(r.crop_w, r.src_w));
         }
@@ -993,13 +994,25 @@ namespace aeonb
         bool at_elements = true; // every slot starts on a multiple of the element's size
         for (int i = 0; i < n; ++i)
             at_elements &= ((uintptr_t)descs_host[i].dst & (elem - 1)) == 0;
-        // How a band is stored (see RUNS).  Wider elements than bytes fill what a store takes sooner: planes of 2, 4 and 8 bytes per element stay
-        // with store_band (element by element / in runs: 256 of 64 x 64 x int16 35.5 / 40.4 us, 256 of 448 x 448 704 / 796, 64 of 225 x 225
-        // floats 71 / 86), and so do narrow or few pictures of 8-byte elements side by side, for which the runs' arithmetic costs more than
-        // they save (256 of 64 x 64 doubles 45 / 52, one of 1000 x 1000 33 / 42; 64 of 300 x 300 155 / 111).
-        const int runs = L.vector_ok || !at_elements ? 0 : layout.stride_x == 1 ? (elem == 1 ? 1 : 0)
-                       : layout.stride_c == 1 && layout.stride_x == layout.channels && (elem < 8 || (layout.slot_w >= 256 && n >= 8)) ? 2 : 0;
         const size_t smem = smem_for(bands);
+        // How a band is stored (see RUNS).  Runs take fewer and wider stores and more arithmetic: they pay where the stores of several blocks
+        // of an SM wait for one another, and a block that has its SM to itself is slower with them.  Element by element / in runs, us:
+        // 225 x 225 floats side by side, 4 pictures 20 / 24, 16 32 / 28, 128 162 / 145; with all photometric steps and so at most eight blocks
+        // a picture, one picture 57 / 71, 16 69 / 75, 64 102 / 89; byte planes of 225 x 225 with lighting, 4 pictures 21 / 24, 16 30 / 28;
+        // 20 of 1001 x 1001, whose blocks do not share an SM, 395 / 489.  Bytes side by side that go out as they are gain always (8 of
+        // 300 x 300 32 / 20, one 19 / 17).  Planes of wider elements do not gain (256 of 64 x 64 x int16 35.5 / 40.4, 256 of 448 x 448
+        // 704 / 796, 64 of 225 x 225 floats 71 / 86), 8-byte elements side by side only in wide pictures with three blocks on an SM (64 of
+        // 300 x 300 159 / 112; 16 with a contrast change 85 / 107; 40 of 449 x 449, two blocks on an SM, 276 / 323).
+        const int64_t blocks   = (int64_t)n * bands;
+        const size_t  resident = (size_t)228 * 1024 / (smem + 9 * 1024); // blocks that an SM has room for: 8 KB static, 1 KB of the system
+        int           runs     = 0;
+        if (!L.vector_ok && at_elements)
+        {
+            if (layout.stride_x == 1)
+                runs = elem == 1 && blocks >= 256 && resident >= 2 ? 1 : 0;
+            else if (layout.stride_c == 1 && layout.stride_x == layout.channels)
+                runs = (elem == 8 ? blocks >= 384 && resident >= 3 && layout.slot_w >= 256 : blocks >= 256 || as_they_are) ? 2 : 0;
+        }
         if (smem > AUG_MAX_SMEM)
         {
             *why = "output image too large for the on-chip band tile (one row of width * 3 bytes must stay under 200 KB)";

@@ -271,37 +271,42 @@ def test_launches_of_several_sizes_at_once(ctx):
 
 @pytest.mark.parametrize("otype", ["uint8_t", "int8_t", "uint16_t", "float", "double"])
 @pytest.mark.parametrize("layout", ["planes", "planes apart", "lines apart", "side by side", "side by side, lines apart", "strides"])
-def test_outputs_that_do_not_start_on_16_bytes(ctx, otype, layout):
-    """Every way a band is stored, at widths around a piece of 16 bytes, slots larger than the picture, one row to many bands, first
-    elements at every place of a piece: what lies in the slots equals an output of aligned lines, what lies between them is left alone."""
+@pytest.mark.parametrize("records", [3, 260])
+def test_outputs_that_do_not_start_on_16_bytes(ctx, records, otype, layout):
+    """Every way a band is stored (260 records have enough blocks for the stores in runs, three only where bytes go out as they are), at widths
+    around a piece of 16 bytes, slots larger than the picture, one row to many bands, first elements at every place of a piece: what lies in the
+    slots equals an output of aligned lines, what lies between them is left alone."""
     from aeon_b200 import kernels as K
     rng = np.random.default_rng(21)
     dt, dev = K.DTYPE_BY_NAME[otype], torch.device("cuda", ctx.device)
     for w, h, margin in [(1, 1, 0), (3, 7, 2), (15, 16, 0), (16, 9, 1), (17, 33, 0), (31, 5, 3), (225, 40, 0), (229, 301, 5), (500, 64, 0), (1000, 61, 0)]:
+        if records > 3:
+            h = min(h, 33)
         srcs = [torch.from_numpy(gradient_image(rng, 40 + 9 * k, 70 + 5 * k)).to(dev) for k in range(3)]
+        srcs = [srcs[k % 3] for k in range(records)]
         params = [random_params(rng, s.shape[1], s.shape[0], max(w - margin, 1), max(h - margin, 1), False) for s in srcs]
         pitch = (w + 31) // 16 * 16
         with torch.cuda.stream(ctx.torch_stream):
-            want = torch.full((3, 3, h, pitch), 99, dtype=K._TORCH_DTYPE[dt], device=dev)
+            want = torch.full((records, 3, h, pitch), 99, dtype=K._TORCH_DTYPE[dt], device=dev)
             K.image_batch(ctx, srcs, params, want, K.make_layout(w, h, dt, strides=(h * pitch, pitch, 1)))
             sc, sy, sx = {"planes": (h * w, w, 1), "planes apart": (h * w + 5, w, 1), "lines apart": (h * (w + 3), w + 3, 1),
                           "side by side": (1, 3 * w, 3), "side by side, lines apart": (1, 3 * w + 7, 3), "strides": (2, 7 * w, 7)}[layout]
             if w % 16 == 0 and layout in ("planes", "lines apart"):
                 sc, sy = h * (w + 1), w + 1
             slot = 2 * sc + (h - 1) * sy + (w - 1) * sx + 1
-            for lead in range(0, 16, 1 if w == 17 else 5):
-                room = torch.full((lead + 3 * (slot + 4) + 16,), 77, dtype=K._TORCH_DTYPE[dt], device=dev)
-                got = torch.as_strided(room, (3, 3, h, w), (slot + 4, sc, sy, sx), lead)
+            for lead in range(0, 16, 1 if w == 17 and records == 3 else 5):
+                room = torch.full((lead + records * (slot + 4) + 16,), 77, dtype=K._TORCH_DTYPE[dt], device=dev)
+                got = torch.as_strided(room, (records, 3, h, w), (slot + 4, sc, sy, sx), lead)
                 expect = room.clone()
-                torch.as_strided(expect, (3, 3, h, w), (slot + 4, sc, sy, sx), lead).copy_(want[..., :w])
+                torch.as_strided(expect, (records, 3, h, w), (slot + 4, sc, sy, sx), lead).copy_(want[..., :w])
                 K.image_batch(ctx, srcs, params, got, K.make_layout(w, h, dt, strides=(sc, sy, sx)), record_stride=slot + 4)
                 ctx.synchronize()
                 assert torch.equal(room, expect), (w, h, lead)
 
 
-@pytest.mark.parametrize("n, w", [(7, 256), (8, 255), (8, 256), (9, 301)])
+@pytest.mark.parametrize("n, w", [(47, 256), (48, 255), (48, 256), (60, 301)])
 def test_doubles_side_by_side(ctx, n, w):
-    """8-byte elements with the channels side by side go out in runs from eight pictures of 256 columns on, element by element below."""
+    """8-byte elements with the channels side by side go out in runs from 384 blocks (eight a picture here) and 256 columns on."""
     from aeon_b200 import kernels as K
     rng = np.random.default_rng(22)
     h, dt, dev = 37, K.DTYPE_BY_NAME["double"], torch.device("cuda", ctx.device)
