@@ -55,9 +55,9 @@ namespace aeonb
 
     // The descriptors of a launch.  Where they fit they travel with the launch as a kernel parameter; otherwise `far` is their device
     // copy, which takes a launch of its own in front of the kernel: 9.3 us for the two (device time) against 3.6 for one launch
-    // with 8 KB of parameters, which takes no longer than one with a pointer (16 KB: 0.7 us longer, 31 KB: 3.5).  A provider call
-    // of one photo, which had four such launches: 154 -> 137 us.  (Not for kernels of many short blocks: each reads its descriptor
-    // from the parameters a little later than from L2, and the area resize of 32 pictures took 127 instead of 104 us.)
+    // with 8 KB of parameters, up to 1 us more than with a pointer alone, also where `far` is used (16 KB: 0.7 us more, 31 KB: 3.5).
+    // A provider call of one photo, which had four such launches: 154 -> 137 us.  (Not for kernels of many short blocks: each reads
+    // its descriptor from the parameters a little later than from L2, and the area resize of 32 pictures took 127 instead of 104 us.)
     struct launch_data
     {
         static constexpr size_t k_near = 8064;
